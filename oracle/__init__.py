@@ -43,9 +43,10 @@ def build(force: bool = False) -> str:
 
 
 def reference_dir() -> str:
-    """The reference checkout the recipes read: $GQF_REFERENCE_DIR, else the
-    folder this build was set up with."""
-    return os.environ.get("GQF_REFERENCE_DIR", "/root/reference")
+    """The reference checkout the recipes read: $GQF_REFERENCE_DIR, else its
+    usual folder; "" when that folder is empty (no checkout to read)."""
+    d = os.environ.get("GQF_REFERENCE_DIR", "/root/reference")
+    return "" if os.path.isdir(d) and not os.listdir(d) else d
 
 
 def build_ref(ref: str | None = None) -> bool:
