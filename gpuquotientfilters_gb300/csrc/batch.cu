@@ -93,8 +93,8 @@ __global__ void __launch_bounds__(1024) k_mf_scan(const uint32_t *__restrict__ c
     }
 }
 
-template <int THREADS, int QPT, int BPE>
-__global__ void __launch_bounds__(THREADS, (THREADS >= 1024 ? 1 : 2)) k_mf_layout(MfParams p)
+template <int THREADS, int QPT, int BPE, bool SET>
+__global__ void __launch_bounds__(THREADS, (SET ? 1024 / THREADS : 2)) k_mf_layout(MfParams p)
 {
     __shared__ uint32_t s_gb, s_f;
     if (threadIdx.x == 0) {
@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(THREADS, (THREADS >= 1024 ? 1 : 2)) k_mf_layou
     a.cap_items = p.cap_items;
     a.op = OP_BUILD;
     a.nodup = p.nodup;
-    a.bitmap_ok = p.bitmap_ok;
+    a.set_ok = p.bitmap_ok;
     a.a_dups = nullptr;
     a.status = p.status + f.bucket0;
     a.ticket = p.ticket;
@@ -125,7 +125,8 @@ __global__ void __launch_bounds__(THREADS, (THREADS >= 1024 ? 1 : 2)) k_mf_layou
     a.fix_cap = f.fix_cap;
     a.fix_soft = 1;
     a.err = p.err;
-    bucket_layout_body<THREADS, QPT, BPE>(a, s_gb - f.bucket0);
+    if (SET) bucket_layout_set<THREADS, QPT, ListSource>(a, s_gb - f.bucket0);
+    else bucket_layout_body<THREADS, QPT, BPE>(a, s_gb - f.bucket0);
 }
 
 template <int BPE>
@@ -207,15 +208,22 @@ static cudaError_t mf_with_scatter(uint32_t chunk, Fn fn)
     }
 }
 
-template <int BPE, typename Fn>
-static cudaError_t mf_with_layout(uint32_t tb, Fn fn)
+template <int BPE, bool SET, typename Fn>
+static cudaError_t mf_with_layout_of(uint32_t tb, Fn fn)
 {
     switch (tb) {
-    case 13: return fn(k_mf_layout<256, 32, BPE>, 256);
-    case 12: return fn(k_mf_layout<128, 32, BPE>, 128);
-    case 11: return fn(k_mf_layout<64, 32, BPE>, 64);
-    default: return fn(k_mf_layout<32, 32, BPE>, 32);
+    case 13: return fn(k_mf_layout<256, 32, BPE, SET>, 256);
+    case 12: return fn(k_mf_layout<128, 32, BPE, SET>, 128);
+    case 11: return fn(k_mf_layout<64, 32, BPE, SET>, 64);
+    default: return fn(k_mf_layout<32, 32, BPE, SET>, 32);
     }
+}
+
+template <int BPE, typename Fn>
+static cudaError_t mf_with_layout(uint32_t tb, bool set, Fn fn)
+{
+    if (BPE == 1 && set) return mf_with_layout_of<1, true>(tb, fn);
+    return mf_with_layout_of<BPE, false>(tb, fn);
 }
 
 template <int BPE>
@@ -232,7 +240,7 @@ static int mf_record(Batch &b, cudaStream_t s)
             kscat<<<b.total_chunks, threads, (size_t)chunk * 4 + (size_t)b.nbmax * 8, s>>>(b.p);
             return cudaGetLastError();
         }));
-        GQF_CK(mf_with_layout<BPE>(b.p.tb, [&](auto klay, int threads) {
+        GQF_CK(mf_with_layout<BPE>(b.p.tb, b.p.bitmap_ok != 0, [&](auto klay, int threads) {
             klay<<<b.total_buckets, threads, b.layout_smem, s>>>(b.p);
             return cudaGetLastError();
         }));
@@ -343,9 +351,10 @@ static int mf_create(Batch *b, const gqf_sqf_job *jobs, int count, int no_duplic
     size_t maxsm = (size_t)(di.smem_optin > 0 ? di.smem_optin : 99 * 1024) - 4096;
     uint32_t cap = (uint32_t)std::min<double>(max_avg * 1.25 + 10.0 * std::sqrt(max_avg) + 512.0, 65520.0);
     cap = (cap + 15) & ~15u;
-    size_t sm = layout_smem_bytes(tb, cap, (int)b->bpe, bitmap);
+    // bitmap mode: thread counts of the graph (32 quotients a thread) and the persistent form
+    size_t sm = bitmap ? set_plan(tb, std::max(S / 32, (uint32_t)b->tune.cta_threads)).total
+                       : layout_smem_bytes(tb, cap, (int)b->bpe);
     if (sm > maxsm) return GQF_ERR_ARG;
-    (void)S;
     b->layout_smem = sm;
     // one allocation: descriptors | zeroed control | bases | items | fix-ups
     Sizer z;
@@ -391,9 +400,9 @@ static int mf_create(Batch *b, const gqf_sqf_job *jobs, int count, int no_duplic
         return e != cudaSuccess ? e : mf_smem(kscat, (size_t)chunk * 4 + (size_t)b->nbmax * 8);
     }));
     if (b->bpe == 1)
-        GQF_CK(mf_with_layout<1>(tb, [&](auto klay, int) { return mf_smem(klay, b->layout_smem); }));
+        GQF_CK(mf_with_layout<1>(tb, bitmap, [&](auto klay, int) { return mf_smem(klay, b->layout_smem); }));
     else
-        GQF_CK(mf_with_layout<2>(tb, [&](auto klay, int) { return mf_smem(klay, b->layout_smem); }));
+        GQF_CK(mf_with_layout<2>(tb, bitmap, [&](auto klay, int) { return mf_smem(klay, b->layout_smem); }));
     // the persistent shape: quotients per layout thread = 2^tb / threads
     b->px.total_chunks = pchunks;
     b->px.total_buckets = buckets;

@@ -4,6 +4,7 @@
 // grid, phases separated by a bounded grid barrier.  Per filter the results
 // are exactly those of the kernel-per-phase pipeline (same per-unit code).
 #include "batch.cuh"
+#include "grid_sync.cuh"
 
 namespace gqf {
 
@@ -13,41 +14,6 @@ namespace gqf {
 // units from the same lists as the kernels above, and the phases are
 // separated by a grid barrier.  The layout's buckets are taken by ticket, so
 // a bucket's predecessors were taken by CTAs that are running.
-// Grid-wide barrier for a co-resident grid: thread 0 of each CTA arrives,
-// the last one opens the next generation.  The wait is bounded; a CTA that
-// gives up records DEV_ERR_TIMEOUT and the abort word, and every CTA leaves
-// at the next barrier.  Returns false when the pipeline must stop.
-__device__ __forceinline__ bool mf_grid_sync(uint32_t *bar, uint32_t *err)
-{
-    __shared__ uint32_t s_go;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t go = 1;
-        volatile uint32_t *vbar = bar;
-        const uint32_t gen = vbar[1];
-        __threadfence();  // this CTA's phase writes before its arrival
-        if (atomicAdd(bar, 1u) == gridDim.x - 1) {
-            vbar[0] = 0u;
-            __threadfence();
-            atomicAdd(bar + 1, 1u);
-        } else {
-            uint32_t i = 0;
-            while (vbar[1] == gen) {
-                if (++i > SPIN_LIMIT) {
-                    atomicOr(err, DEV_ERR_TIMEOUT);
-                    atomicExch(bar + 2, 1u);
-                    break;
-                }
-            }
-        }
-        __threadfence();
-        if (vbar[2]) go = 0;
-        s_go = go;
-    }
-    __syncthreads();
-    return s_go != 0;
-}
-
 template <int THREADS, int IPT, int QPT, int BPE>
 __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_mf_persistent(MfParams p, MfPersist x)
 {
@@ -68,7 +34,7 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_mf_persistent(MfPara
             const MfFilter &f = p.f[s_f];
             bucket_hist_chunk<THREADS, IPT>(u - f.pchunk0, f.keys, f.n_keys, mf_geom(f, p.tb), p.bcnt + f.bucket0);
         }
-        if (!mf_grid_sync(x.bar, p.err)) return;
+        if (!grid_sync(x.bar, p.err)) return;
         // exclusive scan of all bucket counts (one CTA)
         if (blockIdx.x == 0) {
             __shared__ uint32_t sw[THREADS / 32];
@@ -92,7 +58,7 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_mf_persistent(MfPara
                 run += p.bcnt[b];
             }
         }
-        if (!mf_grid_sync(x.bar, p.err)) return;
+        if (!grid_sync(x.bar, p.err)) return;
         for (uint32_t u = blockIdx.x; u < x.total_chunks; u += gridDim.x) {
             __syncthreads();
             if (tid == 0) s_f = mf_owner<&MfFilter::pchunk0>(p.f, p.nf, u);
@@ -102,7 +68,7 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_mf_persistent(MfPara
                                                    p.bbase + f.bucket0, 0xFFFFFFFFu, p.bfill + f.bucket0, p.items,
                                                    nullptr, p.err);
         }
-        if (!mf_grid_sync(x.bar, p.err)) return;
+        if (!grid_sync(x.bar, p.err)) return;
         for (;;) {
             __syncthreads();
             if (tid == 0) {
@@ -126,7 +92,7 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_mf_persistent(MfPara
             a.cap_items = p.cap_items;
             a.op = OP_BUILD;
             a.nodup = p.nodup;
-            a.bitmap_ok = p.bitmap_ok;
+            a.set_ok = p.bitmap_ok;
             a.a_dups = nullptr;
             a.status = p.status + f.bucket0;
             a.ticket = p.ticket;
@@ -135,14 +101,15 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_mf_persistent(MfPara
             a.fix_cap = f.fix_cap;
             a.fix_soft = 1;
             a.err = p.err;
-            bucket_layout_body<THREADS, QPT, BPE>(a, gb - f.bucket0);
+            if (BPE == 1 && p.bitmap_ok) bucket_layout_set<THREADS, QPT, ListSource>(a, gb - f.bucket0);
+            else bucket_layout_body<THREADS, QPT, BPE>(a, gb - f.bucket0);
         }
-        if (!mf_grid_sync(x.bar, p.err)) return;
+        if (!grid_sync(x.bar, p.err)) return;
         for (uint32_t fi = blockIdx.x; fi < p.nf; fi += gridDim.x) {
             const MfFilter &f = p.f[fi];
             if (f.n_keys) mf_occupied_bits<BPE>(p, f, fi, tid, THREADS);
         }
-        if (!mf_grid_sync(x.bar, p.err)) return;
+        if (!grid_sync(x.bar, p.err)) return;
     }
     if (x.any_lookup) {
         for (uint32_t u = blockIdx.x; u < x.total_qchunks; u += gridDim.x) {

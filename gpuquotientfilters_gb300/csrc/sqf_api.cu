@@ -9,8 +9,10 @@
 #include "host_common.cuh"
 #include "sqf_build.cuh"
 #include "sqf_extract.cuh"
+#include "sqf_fallback.cuh"
 #include "sqf_lookup.cuh"
 #include "sqf_mirror.cuh"
+#include "sqf_update.cuh"
 
 namespace gqf {
 
@@ -50,18 +52,23 @@ struct LayoutPlan {
     uint32_t stride;     // speculative bucket stride (items)
     uint32_t cap_items;  // per-CTA item capacity of k_bucket_layout
     size_t smem;
-    int threads;
 };
 
 // Bucket geometry for `n_expect` items over 2^q quotients: about 12k items
 // per bucket (one CTA sorts a bucket in shared memory), at most 4096 buckets
-// (the scatter keeps two u32 per bucket in shared memory).
-static LayoutPlan plan_layout(uint32_t q, uint32_t r, uint64_t n_expect, uint64_t n_b_expect, bool bitmap)
+// (the scatter keeps two u32 per bucket in shared memory).  `spread`: also at
+// least 512 buckets (of 256 quotients or more), so a small filter's layout
+// uses every SM; its buckets cost little beyond their items.  (A bucketed
+// lookup stages spill slots with each bucket, so it keeps the large ones.)
+// `general`: k_bucket_layout may run.
+static LayoutPlan plan_layout(uint32_t q, uint32_t r, uint64_t n_expect, uint64_t n_b_expect, bool general,
+                              bool spread)
 {
     const DeviceInfo &di = device_info(current_device());
     LayoutPlan p;
     uint32_t tb_lo = std::max<uint32_t>(7, q > 12 ? q - 12 : 0);
     uint32_t tb_hi = std::min<uint32_t>(q, 15);
+    if (spread) tb_hi = std::min(tb_hi, std::max<uint32_t>(q > 9 ? q - 9 : 0, std::min<uint32_t>(q, 8)));
     uint64_t denom = n_expect ? n_expect : 1;
     uint32_t tb = ceil_log2((12000ull << q) / denom);
     tb = std::min(std::max(tb, tb_lo), tb_hi);
@@ -73,25 +80,30 @@ static LayoutPlan plan_layout(uint32_t q, uint32_t r, uint64_t n_expect, uint64_
     p.g.fp_mask = (q + r >= 32) ? 0xFFFFFFFFu : ((1u << (q + r)) - 1u);
     double avg_b = (double)n_b_expect / p.g.nb;
     p.stride = (uint32_t)align_up((size_t)(avg_b + 10.0 * std::sqrt(avg_b) + 64.0), 32);
+    p.cap_items = 0;
+    p.smem = 0;
+    if (!general) return p;
     int bpe = (r + 3) / 8;
     double avg = (double)n_expect / p.g.nb;
     uint32_t need = (uint32_t)(avg * 1.05 + 10.0 * std::sqrt(avg) + 256.0);
-    p.threads = tb >= 10 ? (1 << (tb - 5)) : 32;
     size_t S = (size_t)1 << tb;
     size_t tile = tile_bytes(tb, bpe) + S / 8;
     size_t counters = 4 * (S / 2 + S / 32 + 8);
-    size_t bitmaps = 4 * (S + S / 8);
     size_t budget = 100 * 1024;
     size_t maxsm = (size_t)(di.smem_optin > 0 ? di.smem_optin : 99 * 1024) - 4096;
-    size_t need_bytes = std::max(counters + (size_t)need * bpe, bitmap ? bitmaps : 0) + tile + 16;
-    if (need_bytes > budget) budget = maxsm;
+    if (counters + (size_t)need * bpe + tile + 16 > budget) budget = maxsm;
     size_t r0 = budget > tile + 16 ? budget - tile - 16 : 0;
     size_t cap = r0 > counters ? (r0 - counters) / bpe : 0;
     cap = std::min<size_t>(cap & ~(size_t)15, 65520);
     p.cap_items = (uint32_t)cap;
-    p.smem = layout_smem_bytes(tb, p.cap_items, bpe, bitmap);
+    p.smem = layout_smem_bytes(tb, p.cap_items, bpe);
     return p;
 }
+
+// Layout buckets of an in-place update: 8192 quotients (three CTAs per SM
+// hold their sets, index and tile), fewer where the filter would otherwise
+// give less than 512 buckets, down to 1024.
+static uint32_t update_tb(uint32_t q) { return std::min<uint32_t>(q, std::min<uint32_t>(13, std::max<uint32_t>(10, q > 9 ? q - 9 : 0))); }
 
 static size_t scatter_smem(uint32_t nb, bool pairs)
 {
@@ -156,6 +168,8 @@ struct ScratchReq {
     bool extract2;  // second table (merge)
     uint32_t nslots;
     size_t snap_bytes = 0;  // in-place update: snapshot of the table
+    uint32_t upd_nb = 0;    // and its layout buckets
+    bool every_fix = false; // room for a fix-up of every quotient
 };
 
 static Scratch carve(void *base, const ScratchReq &r, bool sizing_only, size_t *bytes_out)
@@ -164,14 +178,14 @@ static Scratch carve(void *base, const ScratchReq &r, bool sizing_only, size_t *
     auto lay = [&](auto &c) {
         size_t nb = r.nb;
         s.bcnt = c.template take<uint32_t>(nb, 8);
-        s.status = c.template take<unsigned long long>(nb, 8);
+        s.status = c.template take<unsigned long long>(std::max<size_t>(nb, r.upd_nb), 8);
         s.ticket = c.template take<uint32_t>(1, 4);
         s.fix_cnt = c.template take<uint32_t>(1, 4);
         s.a_dups = c.template take<uint32_t>(1, 4);
         s.fused_fail = c.template take<uint32_t>(1, 4);
         s.ctrl_bytes = c.off;
         s.bbase = c.template take<uint32_t>(nb + 1);
-        s.fix_cap = std::max<uint32_t>(65536u, r.nslots / 8);
+        s.fix_cap = std::max<uint32_t>(65536u, r.every_fix ? r.nslots : r.nslots / 8);
         s.fix_list = c.template take<uint32_t>(s.fix_cap);
         s.bitems = c.template take<uint32_t>(std::max<size_t>(r.batch_items, 1));
         s.bidx = r.pairs ? c.template take<uint32_t>(std::max<size_t>(r.batch_items, 1)) : nullptr;
@@ -282,9 +296,8 @@ static int bucket_batch(const uint32_t *keys, uint32_t n, const LayoutPlan &p, S
 
 template <int BPE>
 static int launch_layout(const LayoutPlan &p, const SqfGeom &tg, uint8_t *table, const BucketSrc &A,
-                         const BucketSrc &B, int op, int nodup, bool bitmap_ok, const uint32_t *a_dups, Scratch &sc,
-                         uint32_t *err, cudaStream_t s, const uint8_t *src_table = nullptr,
-                         const uint32_t *gate = nullptr)
+                         const BucketSrc &B, int op, int nodup, bool set_ok, const uint32_t *a_dups, Scratch &sc,
+                         uint32_t *err, cudaStream_t s, const uint32_t *gate = nullptr)
 {
     // slots past the last bucket's quotients only receive spill: clear them
     // (a gated launch leaves that to k_fallback_prepare)
@@ -302,7 +315,7 @@ static int launch_layout(const LayoutPlan &p, const SqfGeom &tg, uint8_t *table,
     a.cap_items = p.cap_items;
     a.op = op;
     a.nodup = nodup;
-    a.bitmap_ok = bitmap_ok ? 1 : 0;
+    a.set_ok = set_ok ? 1 : 0;
     a.a_dups = a_dups;
     a.status = sc.status;
     a.ticket = sc.ticket;
@@ -310,61 +323,103 @@ static int launch_layout(const LayoutPlan &p, const SqfGeom &tg, uint8_t *table,
     a.fix_cnt = sc.fix_cnt;
     a.fix_cap = sc.fix_cap;
     a.err = err;
-    a.src_table = src_table;
-    a.fused_fail = src_table ? sc.fused_fail : nullptr;
     a.gate = gate;
-    const size_t smem = p.smem + (src_table ? layout_fused_bytes(p.g.tb) + 16 : 0);
-    // one thread per 32 consecutive quotients (fewer per thread below 1024
-    // quotients per bucket)
+    const int threads = (int)layout_threads(p.g.tb);
     cudaError_t e = cudaSuccess;
-    auto go = [&](auto kernel, int threads) {
+    auto go = [&](auto kernel, size_t smem) {
         e = set_smem(kernel, smem);
         if (e == cudaSuccess) kernel<<<p.g.nb, threads, smem, s>>>(a);
     };
-    if (src_table && BPE == 1 && op == OP_INSERT) {
-        // in-place insert: merge into the staged old slices
-        const size_t msm = merge_plan(p.g.tb).total;
-        auto gm = [&](auto kernel, int threads) {
-            e = set_smem(kernel, msm);
-            if (e == cudaSuccess) kernel<<<p.g.nb, threads, msm, s>>>(a);
-        };
+    if (BPE == 1 && set_ok) {
+        const size_t smem = set_plan(p.g.tb, threads).total;
         switch (p.g.tb) {
-        case 15: gm(k_bucket_insert_merge<1024>, 1024); break;
-        case 14: gm(k_bucket_insert_merge<512>, 512); break;
-        case 13: gm(k_bucket_insert_merge<256>, 256); break;
-        case 12: gm(k_bucket_insert_merge<128>, 128); break;
-        case 11: gm(k_bucket_insert_merge<64>, 64); break;
-        default: gm(k_bucket_insert_merge<32>, 32); break;
+        case 15: go(k_set_layout<1024, 32>, smem); break;
+        case 14: go(k_set_layout<512, 32>, smem); break;
+        case 13: go(k_set_layout<256, 32>, smem); break;
+        case 12: go(k_set_layout<256, 16>, smem); break;
+        case 11: go(k_set_layout<128, 16>, smem); break;
+        case 10: go(k_set_layout<128, 8>, smem); break;
+        case 9: go(k_set_layout<64, 8>, smem); break;
+        case 8: go(k_set_layout<32, 8>, smem); break;
+        default: go(k_set_layout<32, 4>, smem); break;
         }
-    } else if (src_table && BPE == 1) {
+        GQF_CK(e);
+        count_launches(1);
+    }
+    if (!set_ok || a_dups) {
         switch (p.g.tb) {
-        case 15: go(k_bucket_layout<1024, 32, BPE, true>, 1024); break;
-        case 14: go(k_bucket_layout<512, 32, BPE, true>, 512); break;
-        case 13: go(k_bucket_layout<256, 32, BPE, true>, 256); break;
-        case 12: go(k_bucket_layout<128, 32, BPE, true>, 128); break;
-        case 11: go(k_bucket_layout<64, 32, BPE, true>, 64); break;
-        case 10: go(k_bucket_layout<32, 32, BPE, true>, 32); break;
-        case 9: go(k_bucket_layout<32, 16, BPE, true>, 32); break;
-        case 8: go(k_bucket_layout<32, 8, BPE, true>, 32); break;
-        default: go(k_bucket_layout<32, 4, BPE, true>, 32); break;
+        case 15: go(k_bucket_layout<1024, 32, BPE>, p.smem); break;
+        case 14: go(k_bucket_layout<512, 32, BPE>, p.smem); break;
+        case 13: go(k_bucket_layout<256, 32, BPE>, p.smem); break;
+        case 12: go(k_bucket_layout<256, 16, BPE>, p.smem); break;
+        case 11: go(k_bucket_layout<128, 16, BPE>, p.smem); break;
+        case 10: go(k_bucket_layout<128, 8, BPE>, p.smem); break;
+        case 9: go(k_bucket_layout<64, 8, BPE>, p.smem); break;
+        case 8: go(k_bucket_layout<32, 8, BPE>, p.smem); break;
+        default: go(k_bucket_layout<32, 4, BPE>, p.smem); break;
         }
-    } else {
-        switch (p.g.tb) {
-        case 15: go(k_bucket_layout<1024, 32, BPE>, 1024); break;
-        case 14: go(k_bucket_layout<512, 32, BPE>, 512); break;
-        case 13: go(k_bucket_layout<256, 32, BPE>, 256); break;
-        case 12: go(k_bucket_layout<128, 32, BPE>, 128); break;
-        case 11: go(k_bucket_layout<64, 32, BPE>, 64); break;
-        case 10: go(k_bucket_layout<32, 32, BPE>, 32); break;
-        case 9: go(k_bucket_layout<32, 16, BPE>, 32); break;
-        case 8: go(k_bucket_layout<32, 8, BPE>, 32); break;
-        default: go(k_bucket_layout<32, 4, BPE>, 32); break;
-        }
+        GQF_CK(e);
+        count_launches(1);
+    }
+    const DeviceInfo &di = device_info(current_device());
+    count_launches(1);
+    k_fixup_occ<BPE><<<di.sms * 2, 256, 0, s>>>(table, sc.fix_list, sc.fix_cnt, sc.fix_cap, gate);
+    GQF_CK(cudaGetLastError());
+    return GQF_OK;
+}
+
+// In-place update of one-byte slots: old contents from the snapshot (and
+// `src2`), batch buckets of geometry p.
+static int launch_update(const LayoutPlan &p, const SqfGeom &tg, uint8_t *table, const uint8_t *src2,
+                         const BucketSrc &B, int op, Scratch &sc, uint32_t *err, cudaStream_t s)
+{
+    const size_t tail = (size_t)1 << tg.q;
+    if (tg.T > tail) GQF_CK(cudaMemsetAsync(table + tail, 0, tg.T - tail, s));
+    LayoutArgs a;
+    a.A = BucketSrc{nullptr, nullptr, 0, nullptr};
+    a.B = B;
+    a.table = table;
+    a.q = tg.q;
+    a.r = tg.r;
+    a.tb = update_tb(tg.q);
+    a.nb = 1u << (tg.q - a.tb);
+    a.nslots = tg.nslots;
+    a.cap_items = 0;
+    a.op = op;
+    a.nodup = 1;
+    a.set_ok = 1;
+    a.a_dups = nullptr;
+    a.status = sc.status;
+    a.ticket = sc.ticket;
+    a.fix_list = sc.fix_list;
+    a.fix_cnt = sc.fix_cnt;
+    a.fix_cap = sc.fix_cap;
+    a.err = err;
+    a.src_table = sc.snap;
+    a.src2 = src2;
+    a.sub = p.g.tb - a.tb;
+    a.fused_fail = sc.fused_fail;
+    const int threads = (int)layout_threads(a.tb);
+    const size_t smem = set_update_smem(a.tb, threads, src2 != nullptr);
+    cudaError_t e = cudaSuccess;
+    auto go = [&](auto one, auto two) {
+        auto kernel = src2 ? two : one;
+        e = set_smem(kernel, smem);
+        if (e == cudaSuccess) kernel<<<a.nb, threads, smem, s>>>(a);
+    };
+    switch (a.tb) {
+    case 13: go(k_set_update<256, 32, false>, k_set_update<256, 32, true>); break;
+    case 12: go(k_set_update<256, 16, false>, k_set_update<256, 16, true>); break;
+    case 11: go(k_set_update<128, 16, false>, k_set_update<128, 16, true>); break;
+    case 10: go(k_set_update<128, 8, false>, k_set_update<128, 8, true>); break;
+    case 9: go(k_set_update<64, 8, false>, k_set_update<64, 8, true>); break;
+    case 8: go(k_set_update<32, 8, false>, k_set_update<32, 8, true>); break;
+    default: go(k_set_update<32, 4, false>, k_set_update<32, 4, true>); break;
     }
     GQF_CK(e);
     const DeviceInfo &di = device_info(current_device());
+    k_fixup_occ<1><<<di.sms * 2, 256, 0, s>>>(table, sc.fix_list, sc.fix_cnt, sc.fix_cap, nullptr);
     count_launches(2);
-    k_fixup_occ<BPE><<<di.sms * 2, 256, 0, s>>>(table, sc.fix_list, sc.fix_cnt, sc.fix_cap, gate);
     GQF_CK(cudaGetLastError());
     return GQF_OK;
 }
@@ -390,7 +445,7 @@ __global__ void k_fallback_prepare(const uint32_t *__restrict__ gate, unsigned l
     }
 }
 
-enum class Src { NONE, TABLE, KEYS, TABLE2 };
+constexpr size_t SNAP_BESIDE = 16u << 20;  // table bytes from which a snapshot is copied on the side stream
 
 // Scratch bytes of rebuild() for an insert or delete of n keys (the same
 // sizing as below).
@@ -398,7 +453,7 @@ static size_t update_scratch_bytes(uint32_t q, uint32_t r, uint32_t n)
 {
     const uint32_t nslots = gqf_sqf_num_slots(q);
     const uint64_t expect = std::min<uint64_t>((uint64_t)(nslots * 0.9) + n, (uint64_t)nslots * 2);
-    LayoutPlan p = plan_layout(q, r, expect, n, r == 5);
+    LayoutPlan p = plan_layout(q, r, expect, n, true, false);
     ScratchReq req{p.g.nb, (size_t)p.g.nb * p.stride, false, true, false, nslots};
     size_t bytes = 0, bytes_exact = 0;
     carve(nullptr, req, true, &bytes);
@@ -416,18 +471,29 @@ static int rebuild(const gqf_sqf *qf, const gqf_sqf *qf2, const uint32_t *keys, 
     const SqfGeom tg = geom_of(qf);
     const bool needA = op != OP_BUILD;
     const bool bFromTable = qf2 != nullptr;
-    uint64_t nA = needA ? tg.nslots : 0;  // worst case for sizing
-    uint64_t nB = bFromTable ? tg.nslots : n;
     // expected items: the table holds at most nslots
     uint64_t expect = std::min<uint64_t>((needA ? (uint64_t)(tg.nslots * 0.9) : 0) + (bFromTable ? (uint64_t)(tg.nslots * 0.9) : n),
                                          (uint64_t)tg.nslots * 2);
-    // r = 5 and set semantics: remainder bitmaps (see LayoutArgs::bitmap_ok)
-    const bool bitmap_ok = tg.r == 5 && (((op == OP_BUILD || op == OP_MERGE) && nodup) || op == OP_INSERT ||
-                                         op == OP_DELETE);
-    LayoutPlan p = plan_layout(tg.q, tg.r, expect, bFromTable ? 0 : n, bitmap_ok);
+    // r = 5 and set semantics: remainder sets (see LayoutArgs::set_ok)
+    const bool set_ok = tg.r == 5 && (((op == OP_BUILD || op == OP_MERGE) && nodup) || op == OP_INSERT);
+    // duplicates in the table veto the set mode of an insert
+    const bool update = op == OP_INSERT;
+    // In-place update: on one-byte slots with set semantics the old contents
+    // are decoded bucket by bucket from a snapshot of the table (no
+    // extraction pass, see LayoutArgs).  If a bucket cannot be decoded (a
+    // table holding duplicate fingerprints, a run past its slice), the op
+    // reruns the general way from the snapshot: a synchronous call decides on
+    // the host; an asynchronous one queues the general path behind the
+    // in-place kernels with every launch gated on the device-side failure
+    // flag, so it costs only empty launches when the in-place path held.
+    const bool fused = BPE == 1 && set_ok && needA;
+    // an update's batch keeps the large buckets (a layout bucket reads its
+    // part of one); a build's are the layout's
+    LayoutPlan p = plan_layout(tg.q, tg.r, expect, bFromTable ? 0 : n, !set_ok || update, !fused);
     ScratchReq req{p.g.nb, bFromTable ? 0 : (size_t)p.g.nb * p.stride, false, needA, bFromTable, tg.nslots};
-    (void)nA;
-    (void)nB;
+    // small filters are laid out in small buckets, which a nearly full table's
+    // spill can pass whole
+    req.every_fix = tg.q <= 22;
     int dev = current_device();
     Arena &ar = arena(dev, s);
     std::lock_guard<std::mutex> lk(ar.mu);
@@ -438,21 +504,9 @@ static int rebuild(const gqf_sqf *qf, const gqf_sqf *qf2, const uint32_t *keys, 
     ScratchReq req_exact = req;
     req_exact.batch_items = std::max<size_t>(n, 1);
     carve(nullptr, req_exact, true, &bytes_exact);
-    // In-place update: an insert or delete on one-byte slots with set
-    // semantics decodes every bucket's old contents straight from a snapshot
-    // of the table (no extraction pass, see LayoutArgs).  If a bucket cannot
-    // be placed that way (a table holding duplicate fingerprints), the op
-    // reruns the general way from the snapshot: a synchronous call decides
-    // on the host; an asynchronous one queues the general path behind the
-    // in-place kernels with every launch gated on the device-side failure
-    // flag, so it costs only empty launches when the in-place path held.
-    // An insert whose batch averages more than half of MERGE_ITEMS new
-    // fingerprints per bucket would send buckets over the in-place merge's
-    // capacity and end up on the general path anyway: it goes there directly.
-    const bool merge_fits = op != OP_INSERT || (uint64_t)n * 2 <= (uint64_t)p.g.nb * MERGE_ITEMS;
-    const bool fused = BPE == 1 && bitmap_ok && (op == OP_INSERT || op == OP_DELETE) && !bFromTable && merge_fits;
     ScratchReq req_fused = req_exact;
     req_fused.snap_bytes = tg.T;
+    req_fused.upd_nb = 1u << (tg.q - update_tb(tg.q));
     size_t bytes_fused = 0;
     if (fused) carve(nullptr, req_fused, true, &bytes_fused);
     void *base = arena_reserve(ar, std::max(std::max(bytes, bytes_exact), bytes_fused));
@@ -462,13 +516,19 @@ static int rebuild(const gqf_sqf *qf, const gqf_sqf *qf2, const uint32_t *keys, 
         Scratch sc = carve(base, req_fused, false, &bytes);
         int st = call_begin(ar, s, ms != nullptr);
         if (st) return st;
-        // the snapshot is copied on the side stream while the batch is bucketed
-        cudaStream_t side = arena_side(ar);
-        if (!side) return GQF_ERR_CUDA;
-        GQF_CK(cudaEventRecord(ar.fork, s));
-        GQF_CK(cudaStreamWaitEvent(side, ar.fork, 0));
-        GQF_CK(cudaMemcpyAsync(sc.snap, qf->table, tg.T, cudaMemcpyDeviceToDevice, side));
-        GQF_CK(cudaEventRecord(ar.join, side));
+        // a large snapshot is copied on the side stream while the batch is
+        // bucketed; a small one costs less than the two event waits
+        const bool beside = n != 0 && tg.T > SNAP_BESIDE;
+        if (beside) {
+            cudaStream_t side = arena_side(ar);
+            if (!side) return GQF_ERR_CUDA;
+            GQF_CK(cudaEventRecord(ar.fork, s));
+            GQF_CK(cudaStreamWaitEvent(side, ar.fork, 0));
+            GQF_CK(cudaMemcpyAsync(sc.snap, qf->table, tg.T, cudaMemcpyDeviceToDevice, side));
+            GQF_CK(cudaEventRecord(ar.join, side));
+        } else {
+            GQF_CK(cudaMemcpyAsync(sc.snap, qf->table, tg.T, cudaMemcpyDeviceToDevice, s));
+        }
         GQF_CK(cudaMemsetAsync(sc.bcnt, 0, sc.ctrl_bytes, s));
         BucketSrc A{nullptr, nullptr, 0, nullptr}, B{nullptr, nullptr, 0, nullptr};
         if (n) {
@@ -476,8 +536,10 @@ static int rebuild(const gqf_sqf *qf, const gqf_sqf *qf2, const uint32_t *keys, 
             if (st) return st;
             B = BucketSrc{sc.bitems, sc.bbase, 0, sc.bcnt};
         }
-        GQF_CK(cudaStreamWaitEvent(s, ar.join, 0));
-        st = launch_layout<BPE>(p, tg, qf->table, A, B, op, nodup, true, nullptr, sc, ar.err, s, sc.snap);
+        if (beside) GQF_CK(cudaStreamWaitEvent(s, ar.join, 0));
+        // a filter merged with itself is read from the snapshot twice
+        const uint8_t *src2 = !qf2 ? nullptr : qf2->table == qf->table ? sc.snap : qf2->table;
+        st = launch_update(p, tg, qf->table, src2, B, op, sc, ar.err, s);
         if (st) return st;
         if (!ms) {
             // the general path, gated on the failure flag: contents from the
@@ -490,11 +552,17 @@ static int rebuild(const gqf_sqf *qf, const gqf_sqf *qf2, const uint32_t *keys, 
                                                            tg.T > tail ? tg.T - tail : 0);
             GQF_CK(cudaGetLastError());
             st = extract_into<BPE>(sc.snap, tg.nslots, tg.T, tg.r, p.g, sc.tiles, sc.Q, sc.E, sc.abase, sc.acnt,
-                                   sc.a_dups, s, sc.fused_fail);
+                                   update ? sc.a_dups : nullptr, s, sc.fused_fail);
             if (st) return st;
             A = BucketSrc{sc.E, sc.abase, 0, sc.acnt};
-            st = launch_layout<BPE>(p, tg, qf->table, A, B, op, nodup, bitmap_ok, sc.a_dups, sc, ar.err, s, nullptr,
-                                    sc.fused_fail);
+            if (src2) {
+                st = extract_into<BPE>(src2, tg.nslots, tg.T, tg.r, p.g, sc.tiles, sc.Q, sc.E2, sc.a2base, sc.a2cnt,
+                                       nullptr, s, sc.fused_fail);
+                if (st) return st;
+                B = BucketSrc{sc.E2, sc.a2base, 0, sc.a2cnt};
+            }
+            st = launch_layout<BPE>(p, tg, qf->table, A, B, op, nodup, set_ok, update ? sc.a_dups : nullptr, sc,
+                                    ar.err, s, sc.fused_fail);
             if (st) return st;
             return call_end(ar, s, nullptr);
         }
@@ -536,8 +604,7 @@ static int rebuild(const gqf_sqf *qf, const gqf_sqf *qf2, const uint32_t *keys, 
             if (st) return st;
             B = exact ? BucketSrc{sc.bitems, sc.bbase, 0, sc.bcnt} : BucketSrc{sc.bitems, nullptr, p.stride, sc.bcnt};
         }
-        st = launch_layout<BPE>(p, tg, qf->table, A, B, op, nodup, bitmap_ok,
-                                (op == OP_INSERT || op == OP_DELETE) ? sc.a_dups : nullptr, sc, ar.err, s);
+        st = launch_layout<BPE>(p, tg, qf->table, A, B, op, nodup, set_ok, update ? sc.a_dups : nullptr, sc, ar.err, s);
         if (st) return st;
         if (!ms) return call_end(ar, s, nullptr);
         // synchronous: look at the error word before deciding
@@ -554,6 +621,139 @@ static int rebuild(const gqf_sqf *qf, const gqf_sqf *qf2, const uint32_t *keys, 
         return dev_err_to_status(e);
     }
     return GQF_ERR_FULL;
+}
+
+// ------------------------------------------------------ cluster-local updates
+// An insert of at most one key per 16 quotients, and every delete
+// (sqf_update.cuh), with the general path behind it on the device.  Larger
+// inserts connect ever longer runs of clusters and are rebuilt instead.
+static bool insert_is_local(uint32_t q, uint32_t n) { return (uint64_t)n * 16 <= (1ull << q); }
+
+template <int BPE>
+static int local_update(const gqf_sqf *qf, const uint32_t *keys, uint32_t n, int op, cudaStream_t s, float *ms)
+{
+    const SqfGeom tg = geom_of(qf);
+    const DeviceInfo &di = device_info(current_device());
+    const bool ins = op == OP_INSERT;
+    // insert buckets of about 128 keys, one CTA each
+    InsBatch ib{};
+    uint32_t lg = 0;
+    while ((128ull << lg) < n && lg < std::min<uint32_t>(tg.q, 18)) lg++;
+    ib.nb = 1u << lg;
+    ib.shift = tg.q + tg.r - lg;
+    const double avg = (double)n / ib.nb;
+    ib.stride = (uint32_t)align_up((size_t)(avg + 10.0 * std::sqrt(avg) + 32.0), 32);
+    uint32_t hsize = 1024;
+    while (hsize < 2ull * n) hsize <<= 1;
+    ib.hmask = hsize - 1;
+    const size_t nkey = (size_t)ib.nb * ib.stride + n;
+    // a table shorter than any walk's limit needs no fallback
+    const bool fb = tg.nslots > FAR_SLOTS;
+    static_assert((uint64_t)((1u << (FB_TB - 1)) * 1.1) <= FAR_SLOTS, "a fallback table spans whole buckets");
+    const uint32_t fnb = fb ? 1u << (tg.q - FB_TB) : 1u;
+    const uint32_t ntiles = (tg.nslots + EXTRACT_TILE - 1) / EXTRACT_TILE;
+    FallbackArgs f{};
+    uint32_t *far = nullptr, *claim = nullptr, *lead = nullptr;
+    size_t zero_bytes = 0;
+    // control words | delete claims (both zeroed) | then either the update's
+    // arrays or, when the fallback runs, its own over them
+    auto lay = [&](auto &c) {
+        far = c.template take<uint32_t>(1);
+        f.bar = c.template take<uint32_t>(4, 16);
+        f.lay.ticket = c.template take<uint32_t>(1, 4);
+        f.lay.fix_cnt = c.template take<uint32_t>(1, 4);
+        ib.n_over = c.template take<uint32_t>(1, 4);
+        ib.pool = c.template take<uint32_t>(1, 4);
+        f.bcnt = c.template take<uint32_t>(fnb, 4);
+        f.bfill = c.template take<uint32_t>(fnb, 4);
+        f.lay.status = c.template take<unsigned long long>(fnb, 8);
+        if (ins) ib.cnt = c.template take<uint32_t>(ib.nb, 4);
+        else claim = c.template take<uint32_t>((tg.nslots + 15) / 16, 16);
+        zero_bytes = c.off;
+        const size_t at = c.off;
+        if (ins) {
+            ib.seen = c.template take<uint32_t>(hsize);
+            ib.base = c.template take<uint32_t>(ib.nb);
+            ib.fp = c.template take<uint32_t>(nkey);
+            ib.ip = c.template take<uint32_t>(nkey);
+            ib.gap = c.template take<uint32_t>(nkey);
+            ib.over = c.template take<uint32_t>(n);
+        } else {
+            lead = c.template take<uint32_t>(n);
+        }
+        const size_t end = c.off;
+        if (fb) {
+            c.off = at;
+            f.tiles = c.template take<Counts3>(ntiles + 1);
+            f.Q = c.template take<uint32_t>(tg.nslots);
+            f.E = c.template take<uint32_t>(tg.nslots);
+            f.abase = c.template take<uint32_t>(fnb + 1);
+            f.acnt = c.template take<uint32_t>(fnb);
+            f.bbase = c.template take<uint32_t>(fnb + 1);
+            f.bitems = c.template take<uint32_t>(n);
+            f.lay.fix_cap = std::max<uint32_t>(65536u, tg.nslots / 8);
+            f.lay.fix_list = c.template take<uint32_t>(f.lay.fix_cap);
+            c.off = std::max(c.off, end);
+        }
+    };
+    Sizer z;
+    lay(z);
+    Arena &ar = arena(current_device(), s);
+    std::lock_guard<std::mutex> lk(ar.mu);
+    void *base = arena_reserve(ar, z.off);
+    if (!base) return GQF_ERR_NOMEM;
+    Carver c(base);
+    lay(c);
+    int st = call_begin(ar, s, ms != nullptr);
+    if (st) return st;
+    if (n == 0) return call_end(ar, s, ms);
+    GQF_CK(cudaMemsetAsync(base, 0, zero_bytes, s));
+    const SlotTable<BPE> v{qf->table, tg.nslots};
+    const uint32_t grid = (n + UPD_THREADS - 1) / UPD_THREADS;
+    if (ins) {
+        GQF_CK(cudaMemsetAsync(ib.seen, 0xFF, (size_t)hsize * 4, s));
+        k_ins_stage<BPE><<<grid, UPD_THREADS, 0, s>>>(keys, n, v, tg.q, tg.r, ib, far);
+        k_ins_sort<BPE><<<ib.nb, INS_THREADS, 0, s>>>(v, tg.r, ib, far);
+        k_ins_groups<BPE><<<ib.nb, INS_THREADS, 0, s>>>(v, ib, far);
+        k_ins_apply<BPE><<<ib.nb, INS_THREADS, 0, s>>>(v, tg.r, ib, ar.err, far);
+        count_launches(4);
+    } else {
+        k_del_locate<BPE><<<grid, UPD_THREADS, 0, s>>>(keys, n, v, tg.q, tg.r, claim, lead, far);
+        k_del_apply<BPE><<<grid, UPD_THREADS, 0, s>>>(n, v, claim, lead, far);
+        count_launches(2);
+    }
+    GQF_CK(cudaGetLastError());
+    if (fb) {
+        f.far = far;
+        f.keys = keys;
+        f.n = n;
+        f.nbytes = (uint32_t)tg.T;
+        LayoutArgs &a = f.lay;
+        a.A = BucketSrc{f.E, f.abase, 0, f.acnt};
+        a.B = BucketSrc{f.bitems, f.bbase, 0, f.bcnt};
+        a.table = qf->table;
+        a.q = tg.q;
+        a.r = tg.r;
+        a.tb = FB_TB;
+        a.nb = fnb;
+        a.nslots = tg.nslots;
+        a.op = op;
+        a.nodup = ins ? 1 : 0;
+        a.set_ok = 0;
+        a.a_dups = nullptr;
+        a.err = ar.err;
+        // the most items a bucket's u16 counters allow (eight times its average)
+        a.cap_items = 65520;
+        const size_t smem = layout_smem_bytes(FB_TB, a.cap_items, BPE);
+        GQF_CK(set_smem(k_update_fallback<BPE>, smem));
+        // a quarter of the SMs: the launch must find room for all of its CTAs
+        // at once beside other streams' kernels, and it rarely runs
+        void *args[] = {&f};
+        GQF_CK(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_update_fallback<BPE>),
+                                           dim3(std::max(1, di.sms / 4)), dim3(FB_THREADS), args, smem, s));
+        count_launches(1);
+    }
+    return call_end(ar, s, ms);
 }
 
 template <int BPE>
@@ -606,7 +806,7 @@ static int lookup_sorted_t(const gqf_sqf *qf, int n, const uint32_t *keys, uint3
     // a batch of at least one query per 16 slots is answered faster through
     // the bit-plane mirror than by bucketing the queries first.
     if (BPE == 1 && (uint64_t)n * 16 >= tg.nslots) return lookup_unsorted_t<BPE>(qf, n, keys, out, s, ms);
-    LayoutPlan p = plan_layout(tg.q, tg.r, (uint64_t)tg.nslots * 8 / 10, (uint64_t)n, false);
+    LayoutPlan p = plan_layout(tg.q, tg.r, (uint64_t)tg.nslots * 8 / 10, (uint64_t)n, false, false);
     // query buckets: aim for ~4k queries per bucket, table-aligned
     ScratchReq req{p.g.nb, (size_t)std::max(n, 1), true, false, false, tg.nslots};
     Arena &ar = arena(current_device(), s);
@@ -670,8 +870,8 @@ static int bulk_build_noalloc_t(const gqf_sqf *qf, uint32_t n, const uint32_t *k
     }
     char *base = static_cast<char *>(nd->base);
     const SqfGeom tg = geom_of(qf);
-    const bool bitmap_ok = tg.r == 5 && nodup;
-    LayoutPlan p = plan_layout(tg.q, tg.r, n, n, bitmap_ok);
+    const bool set_ok = tg.r == 5 && nodup;
+    LayoutPlan p = plan_layout(tg.q, tg.r, n, n, !set_ok, false);  // few buckets: the fix-up list is small
     ScratchReq req{p.g.nb, std::max<size_t>(n, 1), false, false, false, tg.nslots};
     size_t need = 0;
     carve(nullptr, req, true, &need);
@@ -689,7 +889,7 @@ static int bulk_build_noalloc_t(const gqf_sqf *qf, uint32_t n, const uint32_t *k
         if (st) return st;
         B = BucketSrc{sc.bitems, sc.bbase, 0, sc.bcnt};
     }
-    int st = launch_layout<BPE>(p, tg, qf->table, A, B, OP_BUILD, nodup, bitmap_ok, nullptr, sc, err, s);
+    int st = launch_layout<BPE>(p, tg, qf->table, A, B, OP_BUILD, nodup, set_ok, nullptr, sc, err, s);
     if (st) return st;
     uint32_t e = 0;
     GQF_CK(cudaMemcpyAsync(&e, err, sizeof(e), cudaMemcpyDeviceToHost, s));
@@ -779,6 +979,8 @@ int gqf_sqf_bulk_build_noalloc(const gqf_sqf *qf, int n, const uint32_t *d_keys,
 int gqf_sqf_insert(const gqf_sqf *qf, int n, const uint32_t *d_keys, void *stream, float *ms)
 {
     if (!sqf_ok(qf) || n < 0 || (n > 0 && !d_keys)) return GQF_ERR_ARG;
+    if (insert_is_local(qf->qbits, (uint32_t)n))
+        return BPE_DISPATCH(qf, local_update, qf, d_keys, (uint32_t)n, OP_INSERT, static_cast<cudaStream_t>(stream), ms);
     return BPE_DISPATCH(qf, rebuild, qf, nullptr, d_keys, (uint32_t)n, OP_INSERT, 1, static_cast<cudaStream_t>(stream),
                         ms);
 }
@@ -786,8 +988,7 @@ int gqf_sqf_insert(const gqf_sqf *qf, int n, const uint32_t *d_keys, void *strea
 int gqf_sqf_delete(const gqf_sqf *qf, int n, const uint32_t *d_keys, void *stream, float *ms)
 {
     if (!sqf_ok(qf) || n < 0 || (n > 0 && !d_keys)) return GQF_ERR_ARG;
-    return BPE_DISPATCH(qf, rebuild, qf, nullptr, d_keys, (uint32_t)n, OP_DELETE, 0, static_cast<cudaStream_t>(stream),
-                        ms);
+    return BPE_DISPATCH(qf, local_update, qf, d_keys, (uint32_t)n, OP_DELETE, static_cast<cudaStream_t>(stream), ms);
 }
 
 int gqf_sqf_insert_via_merge(const gqf_sqf *qf, const uint32_t *d_old, int n_old, const uint32_t *d_new, int n_new,

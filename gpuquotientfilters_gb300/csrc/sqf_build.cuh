@@ -342,15 +342,6 @@ __device__ inline uint32_t lookback_cin_warp(unsigned long long *status, uint32_
 // through their runs hit distinct banks.
 __device__ __forceinline__ uint32_t skew16(uint32_t w) { return w + (w >> 4); }
 
-// Bitmap layout: one u32 remainder set per local quotient, one pad uint4
-// after every 8 uint4s, so threads owning 32 consecutive quotients sit 9
-// uint4s apart and a quarter-warp of uint4 loads covers all 32 banks.
-__device__ __forceinline__ uint32_t mask_word(uint32_t x)
-{
-    uint32_t u = x >> 2;
-    return 4 * (u + (u >> 3)) + (x & 3u);
-}
-
 // u16 counters packed two per (skewed) u32 word
 __device__ __forceinline__ uint32_t cnt16_get(const uint32_t *a, uint32_t i)
 {
@@ -443,11 +434,11 @@ struct LayoutArgs {
     uint32_t q, r, tb, nb, nslots;
     uint32_t cap_items;  // tagged remainders one CTA can hold (general mode)
     int op, nodup;
-    // Remainder-bitmap mode: r = 5 and the op has set semantics (NoDup
+    // Set mode (k_set_layout): r = 5 and the op has set semantics (NoDup
     // build/merge, insert/delete into a table without duplicate
     // fingerprints); `a_dups` (device flag, may be null) vetoes it at run
-    // time when the table holds duplicates.
-    int bitmap_ok;
+    // time when the table holds duplicates, and k_bucket_layout runs.
+    int set_ok;
     const uint32_t *a_dups;
     unsigned long long *status;
     uint32_t *ticket;
@@ -459,12 +450,15 @@ struct LayoutArgs {
     // above fix_cap (batched builds).
     int fix_soft = 0;
     uint32_t *err;
-    // In-place update (insert / delete, one-byte slots, bitmap mode): A is
-    // decoded bucket by bucket from this snapshot of the table taken before
-    // the op, instead of from an extracted list.  A bucket it cannot decode
-    // here (duplicate or out-of-order remainders, runs past its staged
-    // slice) sets *fused_fail and the host reruns the op the general way.
-    const uint8_t *src_table = nullptr;
+    // In-place update (k_set_update): the table's old contents are decoded
+    // bucket by bucket from src_table, a snapshot of the table taken before
+    // the op (and from src2, a second table, in a merge of two) instead of
+    // from an extracted list.  B's buckets are 2^sub layout buckets each.  A
+    // bucket that cannot be decoded (duplicate or out-of-order remainders in
+    // an insert or delete, runs past its slice) sets *fused_fail and the op
+    // is done the general way.
+    const uint8_t *src_table = nullptr, *src2 = nullptr;
+    uint32_t sub = 0;
     uint32_t *fused_fail = nullptr;
     // When set, the launch does nothing unless *gate is nonzero (the general
     // path queued behind an asynchronous in-place update, run only if that
@@ -472,15 +466,12 @@ struct LayoutArgs {
     const uint32_t *gate = nullptr;
 };
 
-// Shared-memory plan of k_bucket_layout: region 0 holds either the
-// remainder bitmaps (one u32 per quotient) or the packed u16 group counters
-// plus the tagged remainders; the tile buffer follows.
-__host__ __device__ inline size_t layout_region0_bytes(uint32_t tb, uint32_t cap_items, int bpe, bool bitmap)
+// Shared-memory plan of k_bucket_layout: region 0 holds the packed u16 group
+// counters plus the tagged remainders; the tile buffer follows.
+__host__ __device__ inline size_t layout_region0_bytes(uint32_t tb, uint32_t cap_items, int bpe)
 {
     size_t S = (size_t)1 << tb;
-    size_t gen = 4 * (S / 2 + S / 32 + 8) + (((size_t)cap_items * bpe + 15) & ~(size_t)15);
-    size_t bit = 4 * (S + S / 8);
-    return bitmap && bit > gen ? bit : gen;
+    return 4 * (S / 2 + S / 32 + 8) + (((size_t)cap_items * bpe + 15) & ~(size_t)15);
 }
 // The tile buffer's byte offsets are skewed by 16 bytes per 128: threads
 // emitting slots about 32 apart then write distinct shared-memory banks, and
@@ -490,23 +481,14 @@ __host__ __device__ inline size_t tile_bytes(uint32_t tb, int bpe)
 {
     return (tile_skew((((size_t)1 << tb) + SPILL_SLOTS) * bpe + 32) + 16 + 15) & ~(size_t)15;
 }
-__host__ __device__ inline size_t layout_smem_bytes(uint32_t tb, uint32_t cap_items, int bpe, bool bitmap)
+__host__ __device__ inline size_t layout_smem_bytes(uint32_t tb, uint32_t cap_items, int bpe)
 {
     size_t S = (size_t)1 << tb;
-    size_t r0 = (layout_region0_bytes(tb, cap_items, bpe, bitmap) + 15) & ~(size_t)15;
+    size_t r0 = (layout_region0_bytes(tb, cap_items, bpe) + 15) & ~(size_t)15;
     return r0 + tile_bytes(tb, bpe) + S / 8;  // + occupied bit per quotient
 }
-// Extra shared memory of the in-place update decode: per 32-slot word of
-// the staged slice its run-start mask and the run starts before it, per
-// 32-quotient word of the bucket its occupied mask and the count before it.
-__host__ __device__ inline size_t layout_fused_bytes(uint32_t tb)
-{
-    const size_t S = (size_t)1 << tb, LW = (S + SPILL_SLOTS) / 32, QW = S / 32;
-    return ((LW * 4 + 15) & ~(size_t)15) + ((LW * 2 + 15) & ~(size_t)15) + ((QW * 4 + 15) & ~(size_t)15) +
-           ((QW * 2 + 15) & ~(size_t)15);
-}
 
-// Group walk (general mode): quotients [qb, qb+QPT) in slot order, calling
+// Group walk: quotients [qb, qb+QPT) in slot order, calling
 // emit(xa, rem, k) for every item the rebuilt table holds (k = index of the
 // item within its quotient's run).  Groups hold (rem << 1 | source) sorted.
 template <typename Rem, typename Emit>
@@ -532,21 +514,24 @@ __device__ __forceinline__ void walk_groups(const uint32_t *s_cnt, const Rem *s_
 // ---------------------------------------------------------------------
 // K2: one CTA per bucket (taken in ticket order for the look-back).
 // ---------------------------------------------------------------------
+// Threads of a layout CTA for 2^tb quotients: 32 quotients a thread in the
+// large buckets, fewer in the small ones, whose few CTAs per SM would
+// otherwise be a single warp each.
+__host__ __device__ inline uint32_t layout_threads(uint32_t tb)
+{
+    return tb >= 13 ? 1u << (tb - 5) : tb == 12 ? 256u : tb >= 10 ? 128u : tb == 9 ? 64u : 32u;
+}
+
 // THREADS threads own QPT consecutive quotients each (S = THREADS * QPT).
-// FUSED instantiations carry the in-place update decode (LayoutArgs::
-// src_table); the others compile without it.
-template <int THREADS, int QPT_, int BPE, bool FUSED = false>
+template <int THREADS, int QPT_, int BPE>
 __device__ __forceinline__ void bucket_layout_body(const LayoutArgs &a, const uint32_t b)
 {
     using Rem = typename std::conditional<BPE == 1, uint8_t, uint16_t>::type;
     extern __shared__ __align__(16) uint8_t smem_layout[];
     const uint32_t S = 1u << a.tb;
-    const bool bitmap = BPE == 1 && a.bitmap_ok && (a.src_table || !(a.a_dups && *a.a_dups));
-    uint32_t *s_cnt = reinterpret_cast<uint32_t *>(smem_layout);   // general: u16 counters
-    uint32_t *s_mask = reinterpret_cast<uint32_t *>(smem_layout);  // bitmap: u32 per local quotient
+    uint32_t *s_cnt = reinterpret_cast<uint32_t *>(smem_layout);  // u16 counters
     Rem *s_rem = reinterpret_cast<Rem *>(smem_layout + 4 * ((size_t)S / 2 + S / 32 + 8));
-    uint8_t *s_tile = smem_layout + ((layout_region0_bytes(a.tb, a.cap_items, BPE, a.bitmap_ok != 0) + 15) &
-                                     ~(size_t)15);
+    uint8_t *s_tile = smem_layout + ((layout_region0_bytes(a.tb, a.cap_items, BPE) + 15) & ~(size_t)15);
     const uint32_t BUF = S + SPILL_SLOTS;  // slots the tile buffer holds
 
     __shared__ uint32_t s_warp[33];
@@ -566,7 +551,7 @@ __device__ __forceinline__ void bucket_layout_body(const LayoutArgs &a, const ui
     constexpr uint32_t QPT = QPT_;  // S == THREADS * QPT
     const uint32_t qb = tid * QPT;
 
-    if (!bitmap && n > a.cap_items) {
+    if (n > a.cap_items) {
         // cannot sort here: flag it (the host falls back) and keep the chain alive
         if (tid == 0) {
             atomicOr(a.err, DEV_ERR_BUCKET_CAP);
@@ -580,321 +565,74 @@ __device__ __forceinline__ void bucket_layout_body(const LayoutArgs &a, const ui
     // items are read in batches of LB per thread so LB loads are in flight
     constexpr int LB = 8;
 
-    if (FUSED && BPE == 1 && bitmap && a.src_table) {
-        // In-place update: decode this bucket's old contents from the
-        // snapshot.  Runs are stored in quotient order, one per occupied
-        // quotient; the runs starting at or past x0 are first the D0 still
-        // pending from quotients below x0, then those of the bucket's
-        // occupied quotients in order.
-        const uint32_t L = BUF;
-        uint8_t *s_sl = s_tile;  // the slice, in the tile buffer until the emit
-        uint8_t *fx = smem_layout + ((layout_smem_bytes(a.tb, a.cap_items, BPE, true) + 15) & ~(size_t)15);
-        const size_t o1 = ((size_t)(L / 32) * 4 + 15) & ~(size_t)15, o2 = ((size_t)(L / 32) * 2 + 15) & ~(size_t)15,
-                     o3 = ((size_t)(S / 32) * 4 + 15) & ~(size_t)15;
-        uint32_t *s_rs32 = reinterpret_cast<uint32_t *>(fx);
-        uint16_t *s_rsp = reinterpret_cast<uint16_t *>(fx + o1);
-        uint32_t *s_oc32 = reinterpret_cast<uint32_t *>(fx + o1 + o2);
-        uint16_t *s_ocp = reinterpret_cast<uint16_t *>(fx + o1 + o2 + o3);
-        __shared__ int s_D0;
-        __shared__ uint32_t s_nrs;
-        for (uint32_t i = tid; i < (S + S / 8) / 4; i += THREADS)
-            reinterpret_cast<uint4 *>(s_mask)[i] = make_uint4(0, 0, 0, 0);
-        const uint8_t *src = a.src_table;
-        for (uint32_t i = tid * 16; i < L; i += THREADS * 16) {
-            uint4 w4;
-            if ((size_t)x0 + i + 16 <= a.nslots) {
-                w4 = __ldg(reinterpret_cast<const uint4 *>(src + x0 + i));
-            } else {
-                uint8_t tmp[16];
+    // A: counting sort of tagged remainders by local quotient
+    for (uint32_t i = tid; i < S / 2 + S / 32 + 8; i += THREADS) s_cnt[i] = 0;
+    __syncthreads();
+    for (uint32_t i0 = 0; i0 < n; i0 += THREADS * LB) {
+        uint32_t v[LB];
 #pragma unroll
-                for (int k = 0; k < 16; k++) tmp[k] = (size_t)x0 + i + k < a.nslots ? src[x0 + i + k] : 0;
-                w4 = *reinterpret_cast<uint4 *>(tmp);
-            }
-            *reinterpret_cast<uint4 *>(s_sl + i) = w4;
+        for (int k = 0; k < LB; k++) {
+            uint32_t i = i0 + k * THREADS + tid;
+            v[k] = i < n ? item(i) : 0u;
         }
+#pragma unroll
+        for (int k = 0; k < LB; k++)
+            if (i0 + k * THREADS + tid < n) cnt16_fetch_inc(s_cnt, (v[k] >> a.r) & (S - 1));
+    }
+    __syncthreads();
+    // exclusive scan of the u16 counters: thread owns QPT consecutive quotients
+    {
+        uint32_t sum = 0;
+        for (uint32_t j = 0; j < QPT; j++) sum += cnt16_get(s_cnt, qb + j);
+        uint32_t incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        if (lane == 31) s_warp[wid] = incl;
+        __syncthreads();
         if (wid == 0) {
-            // runs of quotients below x0 still pending at x0
-            const int D = pending_runs_warp(src, x0);
-            if (lane == 0) s_D0 = D;
-        }
-        __syncthreads();
-        // 32-slot masks: run starts over the slice, occupied over the bucket
-        for (uint32_t w = tid; w < L / 32; w += THREADS) {
-            uint32_t rsm = 0, ocm = 0;
-#pragma unroll
-            for (int h = 0; h < 4; h++) {
-                const Flags8 f = flags8(*reinterpret_cast<const uint64_t *>(s_sl + 32 * w + 8 * h));
-                rsm |= ((f.nonempty & ~f.cont) & 0xFFu) << (8 * h);
-                ocm |= (f.occ & 0xFFu) << (8 * h);
-            }
-            s_rs32[w] = rsm;
-            if (w < S / 32) s_oc32[w] = ocm;
-        }
-        __syncthreads();
-        // exclusive prefix counts: thread-contiguous word ranges + block scan
-        {
-            const uint32_t per = (L / 32 + THREADS - 1) / THREADS;
-            const uint32_t w0 = min(L / 32, tid * per), w1 = min(L / 32, w0 + per);
-            uint32_t cr = 0, co = 0;
-            for (uint32_t w = w0; w < w1; w++) {
-                cr += __popc(s_rs32[w]);
-                if (w < S / 32) co += __popc(s_oc32[w]);
-            }
-            uint32_t ir = cr, io = co;
+            uint32_t v = lane < THREADS / 32 ? s_warp[lane] : 0;
+            uint32_t iv = v;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t x = __shfl_up_sync(0xffffffffu, ir, o), y = __shfl_up_sync(0xffffffffu, io, o);
-                if (lane >= o) {
-                    ir += x;
-                    io += y;
-                }
+                uint32_t t = __shfl_up_sync(0xffffffffu, iv, o);
+                if (lane >= o) iv += t;
             }
-            if (lane == 31) {
-                s_wfn[wid].n = ir;
-                s_wfn[wid].F = io;
-            }
-            __syncthreads();
-            uint32_t pr = ir - cr, po = io - co;
-            for (int w = 0; w < wid; w++) {
-                pr += s_wfn[w].n;
-                po += s_wfn[w].F;
-            }
-            if (tid == THREADS - 1) s_nrs = pr + cr;  // run starts in the slice
-            for (uint32_t w = w0; w < w1; w++) {
-                s_rsp[w] = (uint16_t)pr;
-                pr += __popc(s_rs32[w]);
-                if (w < S / 32) {
-                    s_ocp[w] = (uint16_t)po;
-                    po += __popc(s_oc32[w]);
-                }
-            }
-        }
-        // the batch: its remainders, per quotient, into the bitmaps
-        for (uint32_t i0 = 0; i0 < nbn; i0 += THREADS * LB) {
-            uint32_t v[LB];
-#pragma unroll
-            for (int k = 0; k < LB; k++) {
-                const uint32_t i = i0 + k * THREADS + tid;
-                v[k] = i < nbn ? a.B.items[bbase + i] : 0u;
-            }
-#pragma unroll
-            for (int k = 0; k < LB; k++)
-                if (i0 + k * THREADS + tid < nbn)
-                    atomicOr(s_mask + mask_word((v[k] >> a.r) & (S - 1)), 1u << (v[k] & rmask));
+            if (lane < THREADS / 32) s_warp[lane] = iv - v;
         }
         __syncthreads();
-        {
-            // each thread decodes the runs of its own QPT quotients: the run
-            // of its first occupied quotient is run start number D0 + (the
-            // bucket's occupied quotients before qb); later ones follow in
-            // slot order.  Then per quotient: old set | batch (insert) or
-            // old set & ~batch (delete).
-            const int D0 = s_D0;
-            const int nrs = (int)s_nrs;
-            const uint32_t qw = qb >> 5, qs = qb & 31;
-            const uint32_t ocm = (s_oc32[qw] >> qs) & (QPT >= 32 ? 0xFFFFFFFFu : ((1u << (QPT & 31)) - 1u));
-            const int j0 = (int)s_ocp[qw] + __popc(s_oc32[qw] & ((1u << qs) - 1u));
-            const bool del = a.op == OP_DELETE;
-            bool bad = false;
-            uint32_t pos = 0;  // current run start (slot of the slice)
-            if (ocm) {
-                const int k = D0 + j0;
-                if (k < 0 || k >= nrs) {
-                    bad = true;
-                } else {
-                    uint32_t lo = 0, hi = L / 32;  // last word with s_rsp[w] <= k
-                    while (hi - lo > 1) {
-                        const uint32_t mid = (lo + hi) >> 1;
-                        if ((int)s_rsp[mid] <= k) lo = mid;
-                        else hi = mid;
-                    }
-                    pos = (lo << 5) + (uint32_t)select_bit(s_rs32[lo], k - (int)s_rsp[lo]);
-                }
-            }
-            bool first = true;
-#pragma unroll 4
-            for (uint32_t jq = 0; jq < QPT; jq++) {
-                uint32_t am = 0;
-                if (((ocm >> jq) & 1u) && !bad) {
-                    if (!first) {  // the next run start, at or past the previous run's end
-                        uint32_t w = pos >> 5;
-                        uint32_t mm = pos < L ? (s_rs32[w] & ~((1u << (pos & 31)) - 1u)) : 0u;
-                        while (!mm && ++w < L / 32) mm = s_rs32[w];
-                        if (!mm) bad = true;
-                        else pos = (w << 5) + (uint32_t)(__ffs(mm) - 1);
-                    }
-                    first = false;
-                    if (!bad) {
-                        int prev = -1;
-                        for (;;) {
-                            const uint32_t rem = (uint32_t)s_sl[pos] >> 3;
-                            if ((int)rem <= prev) bad = true;  // duplicate or unsorted run
-                            prev = (int)rem;
-                            am |= 1u << rem;
-                            if (++pos >= L) {
-                                bad = true;  // the run may continue past the slice
-                                break;
-                            }
-                            const uint32_t e2 = s_sl[pos];
-                            if (!((e2 & 7u) && (e2 & 2u))) break;
-                        }
-                    }
-                }
-                uint32_t *mw = s_mask + mask_word(qb + jq);
-                *mw = del ? (am & ~*mw) : (am | *mw);
-            }
-            if (bad) atomicOr(a.fused_fail, 1u);
-        }
-        __syncthreads();
-    } else if (bitmap && na == 0 && a.op != OP_DELETE && ((bbase & 3) == 0)) {
-        // build from one 16-byte aligned source (the speculative bucket
-        // stride keeps bucket starts aligned): the first four items per
-        // thread as one 16-byte load issued before the masks are cleared,
-        // the rest four at a time
-        const uint4 *src4 = reinterpret_cast<const uint4 *>(a.B.items + bbase);
-        const uint32_t n4 = nbn >> 2;
-        auto put = [&](uint32_t v) {
-            atomicOr(s_mask + mask_word((v >> a.r) & (S - 1)), 1u << (v & rmask));
-        };
-        constexpr int LV = 4;  // 16-byte loads in flight per thread
-        uint4 w[LV];
-#pragma unroll
-        for (int k = 0; k < LV; k++) {
-            const uint32_t j = k * THREADS + tid;
-            w[k] = j < n4 ? __ldg(src4 + j) : make_uint4(0, 0, 0, 0);
-        }
-        for (uint32_t i = tid; i < (S + S / 8) / 4; i += THREADS)
-            reinterpret_cast<uint4 *>(s_mask)[i] = make_uint4(0, 0, 0, 0);
-        __syncthreads();
-        for (uint32_t j0 = 0;; j0 += LV * THREADS) {
-#pragma unroll
-            for (int k = 0; k < LV; k++) {
-                if (j0 + k * THREADS + tid < n4) {
-                    put(w[k].x);
-                    put(w[k].y);
-                    put(w[k].z);
-                    put(w[k].w);
-                }
-            }
-            if (j0 + LV * THREADS >= n4) break;
-#pragma unroll
-            for (int k = 0; k < LV; k++) {
-                const uint32_t j = j0 + LV * THREADS + k * THREADS + tid;
-                w[k] = j < n4 ? __ldg(src4 + j) : make_uint4(0, 0, 0, 0);
-            }
-        }
-        for (uint32_t i = (n4 << 2) + tid; i < nbn; i += THREADS) put(a.B.items[bbase + i]);  // tail
-        __syncthreads();
-    } else if (bitmap) {
-        // A: remainder sets by quotient (A first, then B); mask of local
-        // quotient x lives at word mask_word(x) (one pad uint4 per 8)
-        for (uint32_t i = tid; i < (S + S / 8) / 4; i += THREADS)
-            reinterpret_cast<uint4 *>(s_mask)[i] = make_uint4(0, 0, 0, 0);
-        __syncthreads();
-        for (int src = 0; src < 2; src++) {
-            const uint32_t lo_i = src ? na : 0u, hi_i = src ? n : na;
-            const bool clear = src == 1 && a.op == OP_DELETE;
-            for (uint32_t i0 = lo_i; i0 < hi_i; i0 += THREADS * LB) {
-                uint32_t v[LB];
-#pragma unroll
-                for (int k = 0; k < LB; k++) {
-                    uint32_t i = i0 + k * THREADS + tid;
-                    v[k] = i < hi_i ? item(i) : 0u;
-                }
-#pragma unroll
-                for (int k = 0; k < LB; k++) {
-                    if (i0 + k * THREADS + tid < hi_i) {
-                        uint32_t w = mask_word((v[k] >> a.r) & (S - 1)), bit = 1u << (v[k] & rmask);
-                        if (clear) atomicAnd(s_mask + w, ~bit);
-                        else atomicOr(s_mask + w, bit);
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    } else {
-        // A: counting sort of tagged remainders by local quotient
-        for (uint32_t i = tid; i < S / 2 + S / 32 + 8; i += THREADS) s_cnt[i] = 0;
-        __syncthreads();
-        for (uint32_t i0 = 0; i0 < n; i0 += THREADS * LB) {
-            uint32_t v[LB];
-#pragma unroll
-            for (int k = 0; k < LB; k++) {
-                uint32_t i = i0 + k * THREADS + tid;
-                v[k] = i < n ? item(i) : 0u;
-            }
-#pragma unroll
-            for (int k = 0; k < LB; k++)
-                if (i0 + k * THREADS + tid < n) cnt16_fetch_inc(s_cnt, (v[k] >> a.r) & (S - 1));
-        }
-        __syncthreads();
-        // exclusive scan of the u16 counters: thread owns QPT consecutive quotients
-        {
-            uint32_t sum = 0;
-            for (uint32_t j = 0; j < QPT; j++) sum += cnt16_get(s_cnt, qb + j);
-            uint32_t incl = sum;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += v;
-            }
-            if (lane == 31) s_warp[wid] = incl;
-            __syncthreads();
-            if (wid == 0) {
-                uint32_t v = lane < THREADS / 32 ? s_warp[lane] : 0;
-                uint32_t iv = v;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    uint32_t t = __shfl_up_sync(0xffffffffu, iv, o);
-                    if (lane >= o) iv += t;
-                }
-                if (lane < THREADS / 32) s_warp[lane] = iv - v;
-            }
-            __syncthreads();
-            uint32_t run = s_warp[wid] + incl - sum;
-            for (uint32_t j = 0; j < QPT; j += 2) {  // QPT even: whole words
-                uint32_t c0 = cnt16_get(s_cnt, qb + j), c1 = cnt16_get(s_cnt, qb + j + 1);
-                s_cnt[skew16((qb + j) >> 1)] = run | ((run + c0) << 16);
-                run += c0 + c1;
-            }
-        }
-        __syncthreads();
-        for (uint32_t i0 = 0; i0 < n; i0 += THREADS * LB) {
-            uint32_t v[LB];
-#pragma unroll
-            for (int k = 0; k < LB; k++) {
-                uint32_t i = i0 + k * THREADS + tid;
-                v[k] = i < n ? item(i) : 0u;
-            }
-#pragma unroll
-            for (int k = 0; k < LB; k++) {
-                uint32_t i = i0 + k * THREADS + tid;
-                if (i < n) {
-                    uint32_t p = cnt16_fetch_inc(s_cnt, (v[k] >> a.r) & (S - 1));
-                    s_rem[p] = (Rem)(((v[k] & rmask) << 1) | (i >= na ? 1u : 0u));
-                }
-            }
-        }
-        __syncthreads();
-        // s_cnt[x] now holds the END of group x; group x = [end(x-1), end(x))
-        for (uint32_t j = 0; j < QPT; j++) {
-            uint32_t x = qb + j;
-            uint32_t g0 = x ? cnt16_get(s_cnt, x - 1) : 0u, g1 = cnt16_get(s_cnt, x);
-            if (g1 - g0 > 1) small_sort(s_rem + g0, g1 - g0);
+        uint32_t run = s_warp[wid] + incl - sum;
+        for (uint32_t j = 0; j < QPT; j += 2) {  // QPT even: whole words
+            uint32_t c0 = cnt16_get(s_cnt, qb + j), c1 = cnt16_get(s_cnt, qb + j + 1);
+            s_cnt[skew16((qb + j) >> 1)] = run | ((run + c0) << 16);
+            run += c0 + c1;
         }
     }
-    // Bitmap mode: this thread's QPT remainder sets, held in registers
-    // (QPT/4 conflict-free uint4 loads: thread strides are 9 uint4 apart).
-    uint32_t mreg[QPT];
-    if (bitmap) {
+    __syncthreads();
+    for (uint32_t i0 = 0; i0 < n; i0 += THREADS * LB) {
+        uint32_t v[LB];
 #pragma unroll
-        for (uint32_t j = 0; j < QPT / 4; j++) {
-            uint4 m4 = reinterpret_cast<const uint4 *>(s_mask)[mask_word(qb + 4 * j) >> 2];
-            mreg[4 * j] = m4.x;
-            mreg[4 * j + 1] = m4.y;
-            mreg[4 * j + 2] = m4.z;
-            mreg[4 * j + 3] = m4.w;
+        for (int k = 0; k < LB; k++) {
+            uint32_t i = i0 + k * THREADS + tid;
+            v[k] = i < n ? item(i) : 0u;
         }
+#pragma unroll
+        for (int k = 0; k < LB; k++) {
+            uint32_t i = i0 + k * THREADS + tid;
+            if (i < n) {
+                uint32_t p = cnt16_fetch_inc(s_cnt, (v[k] >> a.r) & (S - 1));
+                s_rem[p] = (Rem)(((v[k] & rmask) << 1) | (i >= na ? 1u : 0u));
+            }
+        }
+    }
+    __syncthreads();
+    // s_cnt[x] now holds the END of group x; group x = [end(x-1), end(x))
+    for (uint32_t j = 0; j < QPT; j++) {
+        uint32_t x = qb + j;
+        uint32_t g0 = x ? cnt16_get(s_cnt, x - 1) : 0u, g1 = cnt16_get(s_cnt, x);
+        if (g1 - g0 > 1) small_sort(s_rem + g0, g1 - g0);
     }
     auto warp_incl = [&](LayoutFn f) -> LayoutFn {
 #pragma unroll
@@ -907,25 +645,11 @@ __device__ __forceinline__ void bucket_layout_body(const LayoutArgs &a, const ui
         return f;
     };
     // every item the rebuilt bucket keeps, in slot order, for this thread
-    // (general mode)
     auto walk = [&](auto &&emit) { walk_groups(s_cnt, s_rem, qb, QPT, x0, a.op, a.nodup, emit); };
 
     // B/C: this thread's layout map, then a warp scan of the maps
     LayoutFn fn{0u, 0u};
-    if (bitmap) {
-        uint32_t c = 0, cnt_items = 0;
-#pragma unroll
-        for (uint32_t j = 0; j < QPT; j++) {
-            uint32_t k = __popc(mreg[j]);
-            if (k) {
-                uint32_t xa = x0 + qb + j;
-                c = (xa > c ? xa : c) + k;
-                cnt_items += k;
-            }
-        }
-        fn.n = cnt_items;
-        fn.F = cnt_items ? c : 0u;
-    } else {
+    {
         uint32_t c = 0, cnt_items = 0;
         walk([&](uint32_t xa, uint32_t, uint32_t) {
             uint32_t pos = xa > c ? xa : c;
@@ -1005,41 +729,7 @@ __device__ __forceinline__ void bucket_layout_body(const LayoutArgs &a, const ui
     };
     // E: emit elements; record occupied quotients (bit array) and the ones
     // whose slot an earlier bucket writes (fix-ups)
-    if (bitmap) {
-        const LayoutFn texcl = compose(s_wexcl[wid], wexcl);
-        uint32_t c = texcl.apply(cin);
-        // occupied quotients of this thread; those below lo (their slot was
-        // written by an earlier bucket) become fix-ups
-        uint32_t nz = 0;
-#pragma unroll
-        for (uint32_t j = 0; j < QPT; j++) nz |= (mreg[j] != 0u ? 1u : 0u) << j;
-        const uint32_t xb = x0 + qb;
-        const uint32_t nbelow = lo > xb ? min(lo - xb, 32u) : 0u;
-        const uint32_t bmask = nbelow >= 32u ? 0xFFFFFFFFu : ((1u << nbelow) - 1u);
-        for (uint32_t fx = nz & bmask; fx; fx &= fx - 1u) add_fix(xb + (uint32_t)__ffs(fx) - 1u);
-        const uint32_t occ = nz & ~bmask;
-        if (QPT >= 32) s_occ[qb >> 5] = occ;  // this thread owns the whole word
-        else if (occ) atomicOr(s_occ + (qb >> 5), occ << (qb & 31));
-        // the thread's items in slot order, one per iteration (a loop per
-        // quotient would make the warp wait for its fullest quotient at
-        // every step); the next quotient's set comes from shared memory
-        uint32_t m = 0, pos = 0, e0 = 0, nzr = nz;
-        for (uint32_t it = 0; it < fn.n; it++) {
-            if (!m) {
-                const uint32_t j = (uint32_t)__ffs(nzr) - 1u;
-                nzr &= nzr - 1u;
-                m = s_mask[mask_word(qb + j)];
-                const uint32_t xa = xb + j;
-                pos = xa > c ? xa : c;
-                e0 = pos != xa ? 1u : 0u;  // shifted
-            }
-            const uint32_t v = (uint32_t)__ffs(m) - 1u;
-            m &= m - 1u;
-            if (pos < hi) put_elem(pos, (v << 3) | e0);
-            e0 = 3u;  // later items of the run: continuation + shifted
-            c = ++pos;
-        }
-    } else {
+    {
         const LayoutFn texcl = compose(s_wexcl[wid], wexcl);
         uint32_t c = texcl.apply(cin);
         walk([&](uint32_t xa, uint32_t rem, uint32_t kk) {
@@ -1111,14 +801,15 @@ __device__ __forceinline__ void bucket_layout_body(const LayoutArgs &a, const ui
 
 // One CTA per bucket, taken in ticket order so every bucket's predecessors
 // are running or done when it looks back.
-template <int THREADS, int QPT_, int BPE, bool FUSED = false>
+template <int THREADS, int QPT_, int BPE>
 __global__ void __launch_bounds__(THREADS, (THREADS >= 1024 ? 1 : 2)) k_bucket_layout(LayoutArgs a)
 {
     if (a.gate && !*a.gate) return;
+    if (a.set_ok && !*a.a_dups) return;  // done by k_set_layout
     __shared__ uint32_t s_ticket;
     if (threadIdx.x == 0) s_ticket = atomicAdd(a.ticket, 1u);
     __syncthreads();
-    bucket_layout_body<THREADS, QPT_, BPE, FUSED>(a, s_ticket);
+    bucket_layout_body<THREADS, QPT_, BPE>(a, s_ticket);
 }
 
 template <int BPE>
@@ -1133,4 +824,4 @@ __global__ void k_fixup_occ(uint8_t *table, const uint32_t *fix_list, const uint
 
 }  // namespace gqf
 
-#include "sqf_merge.cuh"
+#include "sqf_set.cuh"

@@ -78,9 +78,9 @@ struct ThreadSlots {
     uint32_t e[EXTRACT_WPT][8];
     uint32_t ne[EXTRACT_WPT], rs[EXTRACT_WPT], occ[EXTRACT_WPT];
     uint32_t s0;
-    __device__ __forceinline__ void load(const uint8_t *t, uint32_t nslots, uint32_t nbytes)
+    __device__ __forceinline__ void load(const uint8_t *t, uint32_t nslots, uint32_t nbytes, uint32_t tile)
     {
-        s0 = blockIdx.x * EXTRACT_TILE + threadIdx.x * (EXTRACT_WPT * 8);
+        s0 = tile * EXTRACT_TILE + threadIdx.x * (EXTRACT_WPT * 8);
 #pragma unroll
         for (int w = 0; w < EXTRACT_WPT; w++) load8_elems<BPE>(t, nslots, nbytes, s0 + 8 * w, e[w]);
 #pragma unroll
@@ -103,14 +103,11 @@ struct ThreadSlots {
 // When `dups` is non-null it is set to 1 if the table stores a fingerprint
 // twice: a continuation element whose remainder equals its predecessor's.
 template <int BPE>
-__global__ void __launch_bounds__(EXTRACT_THREADS) k_tile_counts(const uint8_t *__restrict__ t, uint32_t nslots,
-                                                                uint32_t nbytes, Counts3 *__restrict__ tiles,
-                                                                uint32_t *__restrict__ dups,
-                                                                const uint32_t *__restrict__ gate = nullptr)
+__device__ __forceinline__ void tile_counts(uint32_t tile, const uint8_t *t, uint32_t nslots, uint32_t nbytes,
+                                            Counts3 *tiles, uint32_t *dups)
 {
-    if (gate && !*gate) return;
     ThreadSlots<BPE> ts;
-    ts.load(t, nslots, nbytes);
+    ts.load(t, nslots, nbytes, tile);
     if (dups) {
         uint32_t prev = 0;
         if (ts.s0 > 0 && ts.s0 - 1 < nslots) {
@@ -150,8 +147,17 @@ __global__ void __launch_bounds__(EXTRACT_THREADS) k_tile_counts(const uint8_t *
             r.rs += sw[1][w];
             r.occ += sw[2][w];
         }
-        tiles[blockIdx.x] = r;
+        tiles[tile] = r;
     }
+}
+template <int BPE>
+__global__ void __launch_bounds__(EXTRACT_THREADS) k_tile_counts(const uint8_t *__restrict__ t, uint32_t nslots,
+                                                                uint32_t nbytes, Counts3 *__restrict__ tiles,
+                                                                uint32_t *__restrict__ dups,
+                                                                const uint32_t *__restrict__ gate = nullptr)
+{
+    if (gate && !*gate) return;
+    tile_counts<BPE>(blockIdx.x, t, nslots, nbytes, tiles, dups);
 }
 
 // Exclusive scan of the tile counts by one CTA; total written at
@@ -260,15 +266,11 @@ __device__ __forceinline__ void flush_tile(const uint32_t *s_out, uint32_t cnt, 
 // the j-th run).  A tile's entries are staged in shared memory and stored
 // coalesced.
 template <int BPE>
-__global__ void __launch_bounds__(EXTRACT_THREADS) k_occ_list(const uint8_t *__restrict__ t, uint32_t nslots,
-                                                             uint32_t nbytes, const Counts3 *__restrict__ tiles,
-                                                             uint32_t *__restrict__ Q,
-                                                             const uint32_t *__restrict__ gate = nullptr)
+__device__ __forceinline__ void occ_list(uint32_t tile, const uint8_t *t, uint32_t nslots, uint32_t nbytes,
+                                         const Counts3 *tiles, uint32_t *Q, uint32_t *s_out)
 {
-    if (gate && !*gate) return;
-    __shared__ uint32_t s_out[EXTRACT_TILE];
     ThreadSlots<BPE> ts;
-    ts.load(t, nslots, nbytes);
+    ts.load(t, nslots, nbytes, tile);
     const Counts3 ex = block_excl3(ts.totals());
     uint32_t o = ex.occ;
 #pragma unroll
@@ -280,26 +282,31 @@ __global__ void __launch_bounds__(EXTRACT_THREADS) k_occ_list(const uint8_t *__r
             s_out[o++] = ts.s0 + 8 * w + k;
         }
     }
-    const uint32_t base = tiles[blockIdx.x].occ;
-    flush_tile(s_out, tiles[blockIdx.x + 1].occ - base, Q, base);
+    const uint32_t base = tiles[tile].occ;
+    flush_tile(s_out, tiles[tile + 1].occ - base, Q, base);
+}
+template <int BPE>
+__global__ void __launch_bounds__(EXTRACT_THREADS) k_occ_list(const uint8_t *__restrict__ t, uint32_t nslots,
+                                                             uint32_t nbytes, const Counts3 *__restrict__ tiles,
+                                                             uint32_t *__restrict__ Q,
+                                                             const uint32_t *__restrict__ gate = nullptr)
+{
+    if (gate && !*gate) return;
+    __shared__ uint32_t s_out[EXTRACT_TILE];
+    occ_list<BPE>(blockIdx.x, t, nslots, nbytes, tiles, Q, s_out);
 }
 
 // Pass 3: E[i] = fingerprint of the i-th stored element (staged per tile,
 // stored coalesced).
 template <int BPE>
-__global__ void __launch_bounds__(EXTRACT_THREADS) k_extract(const uint8_t *__restrict__ t, uint32_t nslots,
-                                                            uint32_t nbytes, uint32_t r,
-                                                            const Counts3 *__restrict__ tiles,
-                                                            const uint32_t *__restrict__ Q, uint32_t *__restrict__ E,
-                                                            const uint32_t *__restrict__ gate = nullptr)
+__device__ __forceinline__ void extract(uint32_t tile, const uint8_t *t, uint32_t nslots, uint32_t nbytes, uint32_t r,
+                                        const Counts3 *tiles, const uint32_t *Q, uint32_t *E, uint32_t *s_out)
 {
-    if (gate && !*gate) return;
-    __shared__ uint32_t s_out[EXTRACT_TILE];
     ThreadSlots<BPE> ts;
-    ts.load(t, nslots, nbytes);
+    ts.load(t, nslots, nbytes, tile);
     const Counts3 ex = block_excl3(ts.totals());
     uint32_t o = ex.ne;
-    uint32_t runs_before = tiles[blockIdx.x].rs + ex.rs;  // run starts strictly before this thread's slots
+    uint32_t runs_before = tiles[tile].rs + ex.rs;  // run starts strictly before this thread's slots
 #pragma unroll
     for (int w = 0; w < EXTRACT_WPT; w++) {
 #pragma unroll
@@ -312,8 +319,19 @@ __global__ void __launch_bounds__(EXTRACT_THREADS) k_extract(const uint8_t *__re
         }
         runs_before += __popc(ts.rs[w]);
     }
-    const uint32_t base = tiles[blockIdx.x].ne;
-    flush_tile(s_out, tiles[blockIdx.x + 1].ne - base, E, base);
+    const uint32_t base = tiles[tile].ne;
+    flush_tile(s_out, tiles[tile + 1].ne - base, E, base);
+}
+template <int BPE>
+__global__ void __launch_bounds__(EXTRACT_THREADS) k_extract(const uint8_t *__restrict__ t, uint32_t nslots,
+                                                            uint32_t nbytes, uint32_t r,
+                                                            const Counts3 *__restrict__ tiles,
+                                                            const uint32_t *__restrict__ Q, uint32_t *__restrict__ E,
+                                                            const uint32_t *__restrict__ gate = nullptr)
+{
+    if (gate && !*gate) return;
+    __shared__ uint32_t s_out[EXTRACT_TILE];
+    extract<BPE>(blockIdx.x, t, nslots, nbytes, r, tiles, Q, E, s_out);
 }
 
 // Bucket bounds of a sorted fingerprint list: base[b] = lower_bound(b << shift).
