@@ -653,7 +653,9 @@ static int local_update(const gqf_sqf *qf, const uint32_t *keys, uint32_t n, int
     const uint32_t fnb = fb ? 1u << (tg.q - FB_TB) : 1u;
     const uint32_t ntiles = (tg.nslots + EXTRACT_TILE - 1) / EXTRACT_TILE;
     FallbackArgs f{};
-    uint32_t *far = nullptr, *claim = nullptr, *lead = nullptr;
+    uint32_t *far = nullptr, *claim = nullptr, *n_units = nullptr;
+    uint2 *units = nullptr;
+    uint4 *lead = nullptr;
     size_t zero_bytes = 0;
     // control words | delete claims (both zeroed) | then either the update's
     // arrays or, when the fallback runs, its own over them
@@ -664,22 +666,22 @@ static int local_update(const gqf_sqf *qf, const uint32_t *keys, uint32_t n, int
         f.lay.fix_cnt = c.template take<uint32_t>(1, 4);
         ib.n_over = c.template take<uint32_t>(1, 4);
         ib.pool = c.template take<uint32_t>(1, 4);
+        n_units = ib.n_group = c.template take<uint32_t>(1, 4);
         f.bcnt = c.template take<uint32_t>(fnb, 4);
         f.bfill = c.template take<uint32_t>(fnb, 4);
         f.lay.status = c.template take<unsigned long long>(fnb, 8);
         if (ins) ib.cnt = c.template take<uint32_t>(ib.nb, 4);
-        else claim = c.template take<uint32_t>((tg.nslots + 15) / 16, 16);
+        else claim = c.template take<uint32_t>(2 * ((tg.nslots + 31) / 32), 16);
         zero_bytes = c.off;
         const size_t at = c.off;
         if (ins) {
             ib.seen = c.template take<uint32_t>(hsize);
             ib.base = c.template take<uint32_t>(ib.nb);
-            ib.fp = c.template take<uint32_t>(nkey);
-            ib.ip = c.template take<uint32_t>(nkey);
-            ib.gap = c.template take<uint32_t>(nkey);
-            ib.over = c.template take<uint32_t>(n);
+            ib.key = c.template take<uint4>(nkey);
+            ib.over = c.template take<uint4>(n);
         } else {
-            lead = c.template take<uint32_t>(n);
+            lead = c.template take<uint4>(n);
+            units = c.template take<uint2>(n);
         }
         const size_t end = c.off;
         if (fb) {
@@ -710,17 +712,21 @@ static int local_update(const gqf_sqf *qf, const uint32_t *keys, uint32_t n, int
     GQF_CK(cudaMemsetAsync(base, 0, zero_bytes, s));
     const SlotTable<BPE> v{qf->table, tg.nslots};
     const uint32_t grid = (n + UPD_THREADS - 1) / UPD_THREADS;
+    // a warp per listed unit or group, at most every key's
+    const uint32_t lgrid = std::min<uint32_t>((n + LIST_THREADS / 32 - 1) / (LIST_THREADS / 32), (uint32_t)di.sms * 32);
     if (ins) {
         GQF_CK(cudaMemsetAsync(ib.seen, 0xFF, (size_t)hsize * 4, s));
         k_ins_stage<BPE><<<grid, UPD_THREADS, 0, s>>>(keys, n, v, tg.q, tg.r, ib, far);
-        k_ins_sort<BPE><<<ib.nb, INS_THREADS, 0, s>>>(v, tg.r, ib, far);
+        k_ins_sort<<<ib.nb, INS_THREADS, 0, s>>>(ib, far);
         k_ins_groups<BPE><<<ib.nb, INS_THREADS, 0, s>>>(v, ib, far);
         k_ins_apply<BPE><<<ib.nb, INS_THREADS, 0, s>>>(v, tg.r, ib, ar.err, far);
-        count_launches(4);
+        k_ins_lists<BPE><<<lgrid, LIST_THREADS, 0, s>>>(v, tg.r, ib);
+        count_launches(5);
     } else {
         k_del_locate<BPE><<<grid, UPD_THREADS, 0, s>>>(keys, n, v, tg.q, tg.r, claim, lead, far);
-        k_del_apply<BPE><<<grid, UPD_THREADS, 0, s>>>(n, v, claim, lead, far);
-        count_launches(2);
+        k_del_apply<BPE><<<grid, UPD_THREADS, 0, s>>>(n, v, claim, lead, units, n_units, far);
+        k_del_units<BPE><<<lgrid, LIST_THREADS, 0, s>>>(v, claim, units, n_units);
+        count_launches(3);
     }
     GQF_CK(cudaGetLastError());
     if (fb) {

@@ -60,7 +60,18 @@ QF_HD uint32_t fshr32(uint32_t lo, uint32_t hi, uint32_t s)  // (hi:lo >> s), s 
 QF_HD uint32_t nth_bit(uint32_t m, int j)
 {
 #ifdef __CUDA_ARCH__
-    return __fns(m, 0, j + 1);
+    // halving by popcounts: no loop, whatever j is in the warp's other lanes
+    uint32_t at = 0;
+#pragma unroll
+    for (int w = 16; w; w >>= 1) {
+        const int c = __popc(m & ((1u << w) - 1u));
+        if (j >= c) {
+            j -= c;
+            m >>= w;
+            at += w;
+        }
+    }
+    return at;
 #else
     return (uint32_t)select_bit(m, j);
 #endif
