@@ -89,6 +89,27 @@ QF_HD int select_bit(uint32_t m, int j)
     return lowest_bit(m);
 }
 
+// position of the (j+1)-th set bit of m (m has more than j set bits)
+QF_HD uint32_t nth_bit(uint32_t m, int j)
+{
+#ifdef __CUDA_ARCH__
+    // halving by popcounts: no loop, whatever j is in the warp's other lanes
+    uint32_t at = 0;
+#pragma unroll
+    for (int w = 16; w; w >>= 1) {
+        const int c = __popc(m & ((1u << w) - 1u));
+        if (j >= c) {
+            j -= c;
+            m >>= w;
+            at += w;
+        }
+    }
+    return at;
+#else
+    return (uint32_t)select_bit(m, j);
+#endif
+}
+
 // ---- byte-lane SWAR: one flag bit per byte of a u64 (slot k = byte k) ---
 constexpr uint64_t BL_LO = 0x0101010101010101ull;  // bit 0 of every byte
 constexpr uint64_t BL_HI = 0x8080808080808080ull;  // bit 7 of every byte

@@ -792,9 +792,9 @@ static int lookup_unsorted_t(const gqf_sqf *qf, int n, const uint32_t *keys, uin
         count_launches(2);
     } else if (n > 0) {
         const DeviceInfo &di = device_info(current_device());
-        // one-byte slots: two queries per thread (more threads in flight
-        // beat more loads per thread for the dependent word walks)
-        constexpr int QPT = BPE == 1 ? 2 : LOOKUP_QPT;
+        // one or two queries per thread: more threads in flight beat more
+        // loads per thread for the dependent walks
+        constexpr int QPT = BPE == 1 ? 2 : 1;
         const uint32_t per_block = LOOKUP_THREADS * QPT;
         const uint32_t grid = std::min<uint32_t>((n + per_block - 1) / per_block, (uint32_t)di.sms * 32);
         k_lookup_unsorted<BPE, QPT><<<grid, LOOKUP_THREADS, 0, s>>>(keys, (uint32_t)n, v, out);

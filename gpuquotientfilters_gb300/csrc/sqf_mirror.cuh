@@ -56,27 +56,6 @@ QF_HD uint32_t fshr32(uint32_t lo, uint32_t hi, uint32_t s)  // (hi:lo >> s), s 
 #endif
 }
 
-// position of the (j+1)-th set bit of m (m has more than j set bits)
-QF_HD uint32_t nth_bit(uint32_t m, int j)
-{
-#ifdef __CUDA_ARCH__
-    // halving by popcounts: no loop, whatever j is in the warp's other lanes
-    uint32_t at = 0;
-#pragma unroll
-    for (int w = 16; w; w >>= 1) {
-        const int c = __popc(m & ((1u << w) - 1u));
-        if (j >= c) {
-            j -= c;
-            m >>= w;
-            at += w;
-        }
-    }
-    return at;
-#else
-    return (uint32_t)select_bit(m, j);
-#endif
-}
-
 // Record of group G from the slot bytes (bytes past nbytes read as empty);
 // the build kernel's transposition must give exactly this.
 QF_HD void mirror_record(const uint8_t *t, uint32_t nbytes, uint32_t G, int P, uint32_t (&v)[8])
