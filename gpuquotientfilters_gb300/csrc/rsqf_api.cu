@@ -9,6 +9,7 @@
 #include "host_common.cuh"
 #include "rsqf.cuh"
 #include "rsqf_build.cuh"
+#include "rsqf_mirror.cuh"
 #include "sqf_build.cuh"
 
 #ifndef GQF_RSQF_API
@@ -372,11 +373,27 @@ int GQF_RSQF_API(lookup_unsorted)(const gqf_rsqf *cqf, int n, const uint32_t *d_
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     Arena &ar = arena(current_device(), s);
     std::lock_guard<std::mutex> lk(ar.mu);
+    const uint32_t nbl = cqf->numBlocks;
+    // one query per 16 slots pays for the mirror (the staging loads want a
+    // 16-byte aligned table, which initCQFGPU's is)
+    const bool mirror = (uint64_t)n * 16 >= (uint64_t)nbl * RSQF_SPB &&
+                        (reinterpret_cast<uintptr_t>(cqf->blocks) & 15u) == 0;
+    uint64_t *rec = nullptr;
+    if (mirror) {
+        rec = static_cast<uint64_t *>(arena_reserve(ar, rmir_bytes(nbl)));
+        if (!rec) return GQF_ERR_NOMEM;
+    }
     int st = call_begin(ar, s, ms != nullptr);
     if (st) return st;
-    if (n > 0) {
-        RsqfView v{static_cast<const uint8_t *>(cqf->blocks), cqf->numBlocks};
-        const DeviceInfo &di = device_info(current_device());
+    const DeviceInfo &di = device_info(current_device());
+    if (n > 0 && mirror) {
+        k_rsqf_mirror<<<(nbl + RMIR_THREADS) / RMIR_THREADS, RMIR_THREADS, 0, s>>>(
+            static_cast<const uint8_t *>(cqf->blocks), nbl, rec);
+        const uint32_t grid = std::min<uint32_t>((n + RMIR_LOOKUP_THREADS - 1) / RMIR_LOOKUP_THREADS, di.sms * 32);
+        k_rsqf_lookup_mirror<<<grid, RMIR_LOOKUP_THREADS, 0, s>>>(d_keys, (uint32_t)n, rec, nbl, cqf->qbits, d_out);
+        count_launches(2);
+    } else if (n > 0) {
+        RsqfView v{static_cast<const uint8_t *>(cqf->blocks), nbl};
         uint32_t grid = std::min<uint32_t>((n + RSQF_LOOKUP_THREADS - 1) / RSQF_LOOKUP_THREADS, di.sms * 32);
         k_rsqf_lookup_unsorted<<<grid, RSQF_LOOKUP_THREADS, 0, s>>>(d_keys, (uint32_t)n, v, cqf->qbits, d_out);
         count_launches(1);
