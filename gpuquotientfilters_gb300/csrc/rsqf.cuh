@@ -457,6 +457,7 @@ struct RsqfWarpTable {
     bool crossed;
     uint32_t lane;
     bool t0_zero;       // t0 is all zero (a batch into an empty filter)
+    bool left = false;  // crossed below glo
 
     __device__ __forceinline__ uint32_t zero_run_end(uint32_t b) const
     {
@@ -510,6 +511,7 @@ struct RsqfWarpTable {
     {
         if (!in(b)) {
             crossed = true;
+            left = left || b < glo;
             return false;
         }
         return true;

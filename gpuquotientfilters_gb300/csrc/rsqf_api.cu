@@ -164,7 +164,8 @@ constexpr uint32_t RSQF_SMALL_GROUP = 16;      // 1 KB of staging per warp
 constexpr uint32_t RSQF_WARP_GROUP_MAX = 224;  // 14 KB of staging per warp
 __global__ void k_rsqf_groups(uint32_t nblocks, const uint8_t *__restrict__ start, uint8_t *__restrict__ active,
                               const uint32_t *__restrict__ fhome, uint32_t *__restrict__ list0,
-                              uint32_t *__restrict__ list1, uint32_t *__restrict__ list2, uint32_t *__restrict__ counts)
+                              uint32_t *__restrict__ list1, uint32_t *__restrict__ list2, uint32_t *__restrict__ counts,
+                              int build)
 {
     const uint32_t total = nblocks + 1;  // logical blocks + guard block
     for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < total; b += gridDim.x * blockDim.x) {
@@ -173,7 +174,7 @@ __global__ void k_rsqf_groups(uint32_t nblocks, const uint8_t *__restrict__ star
         uint32_t e = b + 1;
         while (e < total && !start[e]) e++;
         if (fhome[min(b, nblocks)] == fhome[min(e, nblocks)]) continue;  // no items: table unchanged
-        const int which = e - b <= RSQF_SMALL_GROUP ? 0 : (e - b <= RSQF_WARP_GROUP_MAX ? 1 : 2);
+        const int which = build ? 1 : e - b <= RSQF_SMALL_GROUP ? 0 : (e - b <= RSQF_WARP_GROUP_MAX ? 1 : 2);
         uint32_t *list = which == 0 ? list0 : (which == 1 ? list1 : list2);
         const uint32_t k = atomicAdd(counts + which, 1u);
         list[2 * k] = b;
@@ -208,7 +209,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_rsqf_round_warp(
     uint8_t *__restrict__ t, const uint8_t *__restrict__ t0, uint32_t nblocks, uint32_t q,
     const uint32_t *__restrict__ fps, const uint32_t *__restrict__ fhome, const uint32_t *__restrict__ list,
     const uint32_t *__restrict__ count, uint8_t *__restrict__ crossed, uint32_t *n_crossed,
-    int32_t *__restrict__ ret, int t0_zero, const uint8_t *__restrict__ sus, const uint32_t *__restrict__ fpos)
+    int32_t *__restrict__ ret, int t0_zero)
 {
     __shared__ __align__(16) uint8_t sm_all[WARPS][MAXB * RSQF_SB];
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -229,31 +230,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_rsqf_round_warp(
         __syncwarp();
         RsqfWarpTable f{sm, t0, nblocks, b, e, false, lane, t0_zero != 0};
         const uint32_t i0 = fhome[min(b, nblocks)], i1 = fhome[min(e, nblocks)];
-        uint32_t istart = i0;
-        if (sus) {
-            // a build: the canonical state of the items before the first
-            // block of offset > 62, then the exact replay from there
-            istart = rsqf_replay_start(sus, fpos, b, min(e, nblocks), i0, i1);
-            for (uint32_t i = i0 + lane; i < istart; i += 32) {
-                const uint32_t fp = fps[i], s = (uint32_t)ret[i];
-                const uint32_t blk = s / RSQF_SPB, sl = s % RSQF_SPB, hb = (fp >> RSQF_R) / RSQF_SPB;
-                unsigned long long *bs = reinterpret_cast<unsigned long long *>(sm + (size_t)(blk - b) * RSQF_SB);
-                unsigned long long *bh = reinterpret_cast<unsigned long long *>(sm + (size_t)(hb - b) * RSQF_SB);
-                atomicOr(bh + 1, 1ull << ((fp >> RSQF_R) % RSQF_SPB));  // occupieds of the home block
-                if (i + 1 == istart || (fps[i + 1] >> RSQF_R) != (fp >> RSQF_R)) atomicOr(bs + 2, 1ull << sl);
-                const uint32_t bit = sl * RSQF_R, wi = bit >> 6, sh = bit & 63;
-                const unsigned long long r = fp & RSQF_RMASK;
-                atomicOr(bs + 3 + wi, r << sh);
-                if (sh + RSQF_R > 64) atomicOr(bs + 4 + wi, r >> (64 - sh));
-            }
-            // offsets: items homed below the block and stored in it
-            for (uint32_t blk = b + lane; blk < e && blk < nblocks; blk += 32) {
-                const uint32_t hi = min(fhome[blk], istart), lo = max(fpos[blk], i0);
-                sm[(size_t)(blk - b) * RSQF_SB] = (uint8_t)(hi > lo ? hi - lo : 0u);
-            }
-            __syncwarp();
-        }
-        for (uint32_t i = istart; i < i1; i++) {
+        for (uint32_t i = i0; i < i1; i++) {
             const int32_t slot = rsqf_insert(f, q, fps[i]);
             if (f.crossed) break;
             if (lane == 0) ret[i] = slot;
@@ -267,6 +244,147 @@ __global__ void __launch_bounds__(32 * WARPS) k_rsqf_round_warp(
         } else {
             for (uint32_t k = lane; k < (e - b) * RSQF_BB; k += 32) {
                 const size_t a = (size_t)b * RSQF_BB + k;
+                t[a] = *f.staged_byte(a);
+            }
+            if (lane == 0) crossed[b] = 0;
+        }
+        __syncwarp();
+    }
+}
+
+// A build's replay of one group, a warp each.  Only a window of the group is
+// staged: from the home block W of the first item that can depart from its
+// canonical position (item fpos[S1] of the group's first block S1 of offset
+// above 62, see rsqf_replay_start) for at most MAXB blocks; blocks below W
+// keep what k_rsqf_assemble wrote.  Ascending items read and write only blocks
+// from their home on, so whenever the blocks from h on are, before the first
+// item homed in h, exactly what the canonical positions put there, every
+// later item is canonical again up to the next block of offset above 62:
+// those are skipped (or the group ends).  A departure of a few slots is
+// absorbed by the next free slots, so a few hundred items are replayed where
+// a group holds thousands.
+// A write past the group's end marks it crossed (merged with its successor
+// and done again); one past the window, or below it, hands the group to
+// k_rsqf_round_big through list 2.
+template <uint32_t MAXB>
+__global__ void __launch_bounds__(32) k_rsqf_replay_build(
+    uint8_t *__restrict__ t, const uint8_t *__restrict__ t0, uint32_t nblocks, uint32_t q,
+    const uint32_t *__restrict__ fps, const uint32_t *__restrict__ fhome, const uint32_t *__restrict__ list,
+    uint32_t *__restrict__ counts, uint8_t *__restrict__ crossed, uint32_t *n_crossed, int32_t *__restrict__ ret,
+    const uint8_t *__restrict__ sus, const uint32_t *__restrict__ fpos, uint32_t *__restrict__ list2)
+{
+    constexpr uint32_t EXPB = 4;  // blocks that spilled items are compared in
+    __shared__ __align__(16) uint8_t sm[MAXB * RSQF_SB];
+    __shared__ __align__(16) unsigned long long s_exp[EXPB * RSQF_SW];
+    const uint32_t lane = threadIdx.x;
+    const uint32_t ng = counts[1];
+    for (uint32_t gi = blockIdx.x; gi < ng; gi += gridDim.x) {
+        const uint32_t b = list[2 * gi], e = list[2 * gi + 1];
+        const uint32_t i0 = fhome[min(b, nblocks)], i1 = fhome[min(e, nblocks)];
+        // first block at or past x (below e) of offset above 62, or e
+        auto next_sus = [&](uint32_t x) -> uint32_t {
+            for (; x < e; x += 32) {
+                const unsigned m = __ballot_sync(~0u, x + lane < min(e, nblocks) && sus[x + lane]);
+                if (m) return x + (uint32_t)__ffs(m) - 1u;
+            }
+            return e;
+        };
+        const uint32_t s1 = next_sus(b);
+        uint32_t i = s1 < e ? min(max(fpos[s1], i0), i1) : i0;
+        if (i >= i1) continue;
+        const uint32_t W = max(b, (fps[i] >> RSQF_R) / RSQF_SPB), we = min(e, W + MAXB);
+        for (uint32_t k = lane; k < (we - W) * RSQF_SW; k += 32) reinterpret_cast<uint64_t *>(sm)[k] = 0;
+        __syncwarp();
+        // adds items [from, to) at their canonical slots to blocks from W on,
+        // and sets the offsets those give from block ob on
+        auto canon = [&](unsigned long long *words, uint32_t wblocks, uint32_t from, uint32_t to, bool by_ret,
+                         uint32_t base, uint32_t slot0) {
+            for (uint32_t x = from + lane; x < to; x += 32) {
+                const uint32_t fp = fps[x], sl = by_ret ? (uint32_t)ret[x] : slot0 + (x - from);
+                const uint32_t blk = sl / RSQF_SPB - base, hb = (fp >> RSQF_R) / RSQF_SPB;
+                if (blk >= wblocks) continue;
+                unsigned long long *bs = words + (size_t)blk * RSQF_SW;
+                if (hb >= base && hb - base < wblocks)
+                    atomicOr(words + (size_t)(hb - base) * RSQF_SW + 1, 1ull << ((fp >> RSQF_R) % RSQF_SPB));
+                if (x + 1 == to || (fps[x + 1] >> RSQF_R) != (fp >> RSQF_R)) atomicOr(bs + 2, 1ull << (sl % RSQF_SPB));
+                const uint32_t bit = (sl % RSQF_SPB) * RSQF_R, wi = bit >> 6, sh = bit & 63;
+                const unsigned long long rem = fp & RSQF_RMASK;
+                atomicOr(bs + 3 + wi, rem << sh);
+                if (sh + RSQF_R > 64) atomicOr(bs + 4 + wi, rem >> (64 - sh));
+            }
+        };
+        auto canon_off = [&](uint32_t blk, uint32_t upto) -> uint32_t {  // items below `upto` homed below blk, stored past it
+            const uint32_t hi = min(fhome[min(blk, nblocks)], upto), lo = fpos[min(blk, nblocks)];
+            return hi > lo ? hi - lo : 0u;
+        };
+        unsigned long long *smw = reinterpret_cast<unsigned long long *>(sm);
+        canon(smw, we - W, max(fpos[W], i0), i, true, W, 0u);
+        for (uint32_t blk = W + lane; blk < we && blk < nblocks; blk += 32)
+            smw[(size_t)(blk - W) * RSQF_SW] = canon_off(blk, i) & 0xFFu;
+        __syncwarp();
+        RsqfWarpTable f{sm, t0, nblocks, W, we, false, lane, true};
+        uint32_t hcur = (fps[i] >> RSQF_R) / RSQF_SPB, wb = we;  // blocks [W, wb) are written back
+        while (i < i1) {
+            const uint32_t h = (fps[i] >> RSQF_R) / RSQF_SPB;
+            if (h > hcur && h < we && i == fhome[h]) {
+                hcur = h;
+                // canonical again from block h on?
+                const uint32_t p0 = fpos[h], nsp = i > p0 ? i - p0 : 0u;
+                bool same = nsp <= (EXPB - 1) * RSQF_SPB && (we == e || h + EXPB <= we);
+                for (uint32_t k = lane; k < EXPB * RSQF_SW; k += 32) s_exp[k] = 0;
+                __syncwarp();
+                if (same) {
+                    canon(s_exp, EXPB, i - nsp, i, false, h, h * RSQF_SPB);
+                    if (lane < EXPB && h + lane < nblocks) s_exp[(size_t)lane * RSQF_SW] = canon_off(h + lane, i) & 0xFFu;
+                }
+                __syncwarp();
+                for (uint32_t k = lane; same && k < (we - h) * RSQF_SW; k += 32)
+                    same = smw[(size_t)(h - W) * RSQF_SW + k] == (k < EXPB * RSQF_SW ? s_exp[k] : 0ull);
+                if (__all_sync(~0u, same)) {
+                    const uint32_t s2 = next_sus(h), i2 = s2 < e ? min(max(fpos[s2], i), i1) : i1;
+                    if (i2 == i1) {  // the rest of the group stays as assembled
+                        wb = h;
+                        break;
+                    }
+                    if (i2 > i) {
+                        if ((fps[i2] >> RSQF_R) / RSQF_SPB >= we || s2 >= we) {  // past the window
+                            f.crossed = true;
+                            break;
+                        }
+                        canon(smw, we - W, i, i2, true, W, 0u);
+                        for (uint32_t blk = h + lane; blk < we && blk < nblocks; blk += 32)
+                            smw[(size_t)(blk - W) * RSQF_SW] = canon_off(blk, i2) & 0xFFu;
+                        __syncwarp();
+                        i = i2;
+                        hcur = (fps[i] >> RSQF_R) / RSQF_SPB;
+                        continue;
+                    }
+                }
+            }
+            if (h >= we) {  // past the window
+                f.crossed = true;
+                break;
+            }
+            const int32_t slot = rsqf_insert(f, q, fps[i]);
+            if (f.crossed) break;
+            if (lane == 0) ret[i] = slot;
+            i++;
+        }
+        __syncwarp();
+        if (f.crossed) {
+            if (lane == 0) {
+                if (f.left || we < e) {
+                    const uint32_t k = atomicAdd(counts + 2, 1u);
+                    list2[2 * k] = b;
+                    list2[2 * k + 1] = e;
+                } else {
+                    crossed[b] = 1;
+                    atomicAdd(n_crossed, 1u);
+                }
+            }
+        } else {
+            for (uint32_t k = lane; k < (wb - W) * RSQF_BB; k += 32) {
+                const size_t a = (size_t)W * RSQF_BB + k;
                 t[a] = *f.staged_byte(a);
             }
             if (lane == 0) crossed[b] = 0;
@@ -488,12 +606,18 @@ static int rsqf_replay_rounds(uint8_t *t, const uint8_t *t0, uint32_t nbl, uint3
     for (int round = 0;; round++) {
         GQF_CK(cudaMemsetAsync(ctr, 0, 4 * sizeof(uint32_t), s));  // three list sizes, crossed
         k_rsqf_groups<<<grid, 256, 0, s>>>(nbl, start, active, fhome, wlist, wlist + 2 * (size_t)(nbl + 1), blist,
-                                           ctr);
-        k_rsqf_round_warp<RSQF_SMALL_GROUP, 8><<<di.sms * 8, 256, 0, s>>>(t, t0, nbl, q, items, fhome, wlist, ctr,
-                                                                        crossed, ctr + 3, d_ret, t0_zero ? 1 : 0, sus, fpos);
-        k_rsqf_round_warp<RSQF_WARP_GROUP_MAX, 1><<<di.sms * 16, 32, 0, s>>>(
-            t, t0, nbl, q, items, fhome, wlist + 2 * (size_t)(nbl + 1), ctr + 1, crossed, ctr + 3, d_ret,
-            t0_zero ? 1 : 0, sus, fpos);
+                                           ctr, sus ? 1 : 0);
+        if (sus) {
+            k_rsqf_replay_build<RSQF_WARP_GROUP_MAX><<<di.sms * 4, 32, 0, s>>>(
+                t, t0, nbl, q, items, fhome, wlist + 2 * (size_t)(nbl + 1), ctr, crossed, ctr + 3, d_ret, sus, fpos,
+                blist);
+        } else {
+            k_rsqf_round_warp<RSQF_SMALL_GROUP, 8><<<di.sms * 8, 256, 0, s>>>(t, t0, nbl, q, items, fhome, wlist, ctr,
+                                                                            crossed, ctr + 3, d_ret, t0_zero ? 1 : 0);
+            k_rsqf_round_warp<RSQF_WARP_GROUP_MAX, 1><<<di.sms * 16, 32, 0, s>>>(
+                t, t0, nbl, q, items, fhome, wlist + 2 * (size_t)(nbl + 1), ctr + 1, crossed, ctr + 3, d_ret,
+                t0_zero ? 1 : 0);
+        }
         k_rsqf_round_big<<<std::max(1, di.sms), 64, 0, s>>>(t, t0, nbl, q, items, fhome, blist, ctr, crossed,
                                                              ctr + 3, d_ret, t0_zero ? 1 : 0, sus, fpos);
         count_launches(4);
