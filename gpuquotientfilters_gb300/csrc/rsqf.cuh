@@ -75,29 +75,9 @@ __device__ __forceinline__ uint64_t lowmask64(uint32_t n) { return n >= 64 ? ~0u
 __device__ __forceinline__ uint32_t select64(uint64_t x, uint32_t k)
 {
     if (k == 0) return 0;
-    if (k > (uint32_t)__popcll(x)) return RSQF_NONE;
-    uint32_t base = 0;
-    uint32_t c = __popc((uint32_t)x);
-    if (k > c) {
-        k -= c;
-        x >>= 32;
-        base = 32;
-    }
-    uint32_t v = (uint32_t)x;
-    c = __popc(v & 0xFFFFu);
-    if (k > c) {
-        k -= c;
-        v >>= 16;
-        base += 16;
-    }
-    c = __popc(v & 0xFFu);
-    if (k > c) {
-        k -= c;
-        v >>= 8;
-        base += 8;
-    }
-    for (uint32_t i = 1; i < k; i++) v &= v - 1;
-    return base + (uint32_t)(__ffs(v) - 1);
+    const uint32_t lo = (uint32_t)x, hi = (uint32_t)(x >> 32), c = (uint32_t)__popc(lo);
+    if (k > c + (uint32_t)__popc(hi)) return RSQF_NONE;
+    return k > c ? 32 + nth_bit(hi, (int)(k - c) - 1) : nth_bit(lo, (int)k - 1);
 }
 __device__ __forceinline__ uint32_t rank64(uint64_t x, uint32_t i)  // ones in [0, i]
 {
@@ -338,6 +318,9 @@ __device__ inline uint32_t rsqf_first_unused(Tab &f, int &bn, uint32_t start)
     return cur;
 }
 
+struct RsqfWarpTable;
+__device__ inline uint32_t rsqf_first_unused(RsqfWarpTable &f, int &bn, uint32_t start);
+
 // insert (RSQF.cpp:367-520 = RSQF.cu:645-875 per item): slot or -1.  On a
 // crossing f.crossed is set and the return value is meaningless.  Tab is
 // the table accessor (per-thread global memory, or a warp's staged blocks).
@@ -458,12 +441,33 @@ struct RsqfWarpTable {
     uint32_t lane;
     bool t0_zero;       // t0 is all zero (a batch into an empty filter)
     bool left = false;  // crossed below glo
+    uint32_t top = 0xFFFFFFFFu;  // t0_zero: no block above it was written
+    uint32_t dlo = 0xFFFFFFFFu, dhi = 0;  // blocks [dlo, dhi] hold every write
 
     __device__ __forceinline__ uint32_t zero_run_end(uint32_t b) const
     {
-        return (t0_zero && b >= ghi) ? nblocks + 1 : b;
+        return (t0_zero && (b >= ghi || b > top)) ? nblocks + 1 : b;
     }
 
+    __device__ __forceinline__ void touched(uint32_t b)
+    {
+        if (t0_zero) top = max(top, b);
+        dlo = min(dlo, b);
+        dhi = max(dhi, b);
+    }
+    // the staged blocks [b0, b1) into the packed table
+    __device__ __forceinline__ void store(uint8_t *t, uint32_t b0, uint32_t b1) const
+    {
+        for (uint32_t b = b0; b < b1; b++) {
+            const uint8_t *src = sb(b);
+            uint8_t *dst = t + (size_t)b * RSQF_BB;
+#pragma unroll
+            for (uint32_t j0 = 0; j0 < RSQF_BB; j0 += 32) {
+                const uint32_t j = j0 + lane;
+                if (j < RSQF_BB) dst[j] = src[j == 0 ? 0u : j + 7];
+            }
+        }
+    }
     __device__ __forceinline__ bool in(uint32_t b) const { return b >= glo && b < ghi; }
     __device__ __forceinline__ uint8_t *sb(uint32_t b) const { return sm + (size_t)(b - glo) * RSQF_SB; }
     __device__ __forceinline__ uint64_t &w64(uint32_t b, uint32_t byte) const
@@ -514,6 +518,7 @@ struct RsqfWarpTable {
             left = left || b < glo;
             return false;
         }
+        touched(b);
         return true;
     }
     __device__ __forceinline__ void set_off(uint32_t b, uint32_t v)
@@ -603,6 +608,8 @@ struct RsqfWarpTable {
         // group-relative slots [sa, sb_) move to [sa + 1, sb_ + 1)
         const uint64_t ga = sa - (uint64_t)glo * RSQF_SPB, gb = sb_ - (uint64_t)glo * RSQF_SPB;
         uint8_t *base = sm;
+        touched((uint32_t)bn);
+        touched((uint32_t)re_block);
         move_bits_up(ga, gb, 1, [base](uint64_t u) {  // runEnds: one word per block
             return reinterpret_cast<uint64_t *>(base + u * RSQF_SB + 16);
         });
@@ -614,5 +621,44 @@ struct RsqfWarpTable {
         return true;
     }
 };
+
+// findFirstUnusedSlot by a warp.  From slot cur of a block the reference steps
+// to sel + 1, sel = select(runEnds past the offset, rank(occupieds, cur)),
+// until cur > sel.  sel does not decrease with cur, so the slots stepped over
+// all have cur <= sel and the result is the first slot from cur on with cur >
+// sel: the lanes test two slots each instead of taking the steps.  (The first
+// block's rank == 0 case and an offset past the block are the reference's.)
+__device__ inline uint32_t rsqf_first_unused(RsqfWarpTable &f, int &bn, uint32_t start)
+{
+    uint32_t cur = start;
+    uint64_t occ = f.occ((uint32_t)bn);
+    uint32_t off = f.off((uint32_t)bn);
+    bool here = true;  // cur may be in this block
+    if (rank64(occ, start) == 0) {
+        if (start > off) return start;
+        if (off == RSQF_SPB - 1) here = false;
+        else cur = off + 1;
+    }
+    for (;;) {
+        if (here) {
+            const uint64_t m = f.re((uint32_t)bn) & ~lowmask64(off);
+            if (cur < RSQF_SPB) {
+                const uint32_t c0 = f.lane, c1 = f.lane + 32;
+                const unsigned b0 = __ballot_sync(~0u, c0 >= cur && c0 > select64(m, rank64(occ, c0)));
+                const unsigned b1 = __ballot_sync(~0u, c1 >= cur && c1 > select64(m, rank64(occ, c1)));
+                if (b0) return (uint32_t)__ffs(b0) - 1u;
+                if (b1) return 31u + (uint32_t)__ffs(b1);
+            } else if (cur > select64(m, rank64(occ, cur))) {
+                return cur;
+            }
+        }
+        bn++;
+        if ((uint32_t)bn > f.nblocks) return RSQF_NONE;
+        occ = f.occ((uint32_t)bn);
+        off = f.off((uint32_t)bn);
+        cur = off;
+        here = true;
+    }
+}
 
 }  // namespace GQF_RSQF_NS

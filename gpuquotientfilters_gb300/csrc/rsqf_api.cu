@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_rsqf_round_warp(
     uint8_t *__restrict__ t, const uint8_t *__restrict__ t0, uint32_t nblocks, uint32_t q,
     const uint32_t *__restrict__ fps, const uint32_t *__restrict__ fhome, const uint32_t *__restrict__ list,
     const uint32_t *__restrict__ count, uint8_t *__restrict__ crossed, uint32_t *n_crossed,
-    int32_t *__restrict__ ret, int t0_zero)
+    int32_t *__restrict__ ret, int t0_zero, int first)
 {
     __shared__ __align__(16) uint8_t sm_all[WARPS][MAXB * RSQF_SB];
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -242,10 +242,10 @@ __global__ void __launch_bounds__(32 * WARPS) k_rsqf_round_warp(
                 atomicAdd(n_crossed, 1u);
             }
         } else {
-            for (uint32_t k = lane; k < (e - b) * RSQF_BB; k += 32) {
-                const size_t a = (size_t)b * RSQF_BB + k;
-                t[a] = *f.staged_byte(a);
-            }
+            // a group's first replay finds the live blocks as in t0: only
+            // those it wrote change (16 blocks a group, two or three written)
+            if (!first) f.store(t, b, e);
+            else if (f.dlo <= f.dhi) f.store(t, f.dlo, f.dhi + 1);
             if (lane == 0) crossed[b] = 0;
         }
         __syncwarp();
@@ -323,6 +323,13 @@ __global__ void __launch_bounds__(32) k_rsqf_replay_build(
             smw[(size_t)(blk - W) * RSQF_SW] = canon_off(blk, i) & 0xFFu;
         __syncwarp();
         RsqfWarpTable f{sm, t0, nblocks, W, we, false, lane, true};
+        // items that fail walk the blocks behind them to the table's end: the
+        // ones above the last written block are all zero and are jumped
+        auto top_of = [&](uint32_t x) -> uint32_t {  // last block the canonical items below x fill, or x's home
+            const uint32_t h = (fps[min(x, i1 - 1)] >> RSQF_R) / RSQF_SPB;
+            return x > i0 ? max(h, (uint32_t)ret[x - 1] / RSQF_SPB) : h;
+        };
+        f.top = top_of(i);
         uint32_t hcur = (fps[i] >> RSQF_R) / RSQF_SPB, wb = we;  // blocks [W, wb) are written back
         while (i < i1) {
             const uint32_t h = (fps[i] >> RSQF_R) / RSQF_SPB;
@@ -356,6 +363,7 @@ __global__ void __launch_bounds__(32) k_rsqf_replay_build(
                             smw[(size_t)(blk - W) * RSQF_SW] = canon_off(blk, i2) & 0xFFu;
                         __syncwarp();
                         i = i2;
+                        f.top = max(f.top, top_of(i));
                         hcur = (fps[i] >> RSQF_R) / RSQF_SPB;
                         continue;
                     }
@@ -383,10 +391,7 @@ __global__ void __launch_bounds__(32) k_rsqf_replay_build(
                 }
             }
         } else {
-            for (uint32_t k = lane; k < (wb - W) * RSQF_BB; k += 32) {
-                const size_t a = (size_t)W * RSQF_BB + k;
-                t[a] = *f.staged_byte(a);
-            }
+            f.store(t, W, wb);
             if (lane == 0) crossed[b] = 0;
         }
         __syncwarp();
@@ -433,6 +438,16 @@ __global__ void k_rsqf_round_big(uint8_t *t, const uint8_t *t0, uint32_t nblocks
         crossed[b] = cross ? 1 : 0;
         if (cross) atomicAdd(n_crossed, 1u);
     }
+}
+
+// What the host decides on after the positions: the error word, and whether
+// the filter held items (1), the batch passed the last slot (2), some cluster
+// departs from its canonical positions (4); into mapped host memory.
+static __global__ void k_rsqf_report(const uint32_t *err, const uint32_t *ctl, uint32_t *host)
+{
+    host[0] = *err;
+    host[1] = (ctl[RCTL_NONEMPTY] ? 1u : 0u) | (ctl[RCTL_OVER] ? 2u : 0u) | (ctl[RCTL_NSUS] ? 4u : 0u);
+    __threadfence_system();
 }
 
 // Merge every crossed group with its successor (chains collapse in one
@@ -524,10 +539,18 @@ static int rsqf_bucket(const uint32_t *keys, uint32_t n, const BucketGeom &g, ui
                        uint32_t *cnt, uint32_t *base, uint32_t *err, cudaStream_t s)
 {
     GQF_CK(cudaMemsetAsync(cnt, 0, g.nb * 4, s));
-    const uint32_t hchunk = SCATTER_THREADS * SCATTER_IPT;
-    GQF_CK(set_smem(k_bucket_hist<SCATTER_THREADS, SCATTER_IPT>, g.nb * 4));
-    k_bucket_hist<SCATTER_THREADS, SCATTER_IPT><<<(n + hchunk - 1) / hchunk, SCATTER_THREADS, g.nb * 4, s>>>(
-        keys, n, g, cnt);
+    // batches of up to 4M keys in 4096-key chunks, so that more than a few
+    // CTAs share them
+    const bool small = n <= (1u << 22);
+    const uint32_t hchunk = small ? 256u * 16u : (uint32_t)(SCATTER_THREADS * SCATTER_IPT);
+    const uint32_t hgrid = (n + hchunk - 1) / hchunk;
+    if (small) {
+        GQF_CK(set_smem(k_bucket_hist<256, 16>, g.nb * 4));
+        k_bucket_hist<256, 16><<<hgrid, 256, g.nb * 4, s>>>(keys, n, g, cnt);
+    } else {
+        GQF_CK(set_smem(k_bucket_hist<SCATTER_THREADS, SCATTER_IPT>, g.nb * 4));
+        k_bucket_hist<SCATTER_THREADS, SCATTER_IPT><<<hgrid, SCATTER_THREADS, g.nb * 4, s>>>(keys, n, g, cnt);
+    }
     k_rsqf_scan_bases<<<1, 1024, 0, s>>>(cnt, g.nb, base);
     GQF_CK(cudaMemsetAsync(cnt, 0, g.nb * 4, s));
     if (idx) {
@@ -536,12 +559,16 @@ static int rsqf_bucket(const uint32_t *keys, uint32_t n, const BucketGeom &g, ui
         GQF_CK(set_smem(kfn, sm));
         const uint32_t chunk = PAIR_THREADS * PAIR_IPT;
         kfn<<<(n + chunk - 1) / chunk, PAIR_THREADS, sm, s>>>(keys, n, g, base, 0xFFFFFFFFu, cnt, items, idx, err);
+    } else if (small) {
+        auto kfn = k_hash_bucket<256, 16, false>;
+        const size_t sm = (size_t)hchunk * 4 + (size_t)g.nb * 8;
+        GQF_CK(set_smem(kfn, sm));
+        kfn<<<hgrid, 256, sm, s>>>(keys, n, g, base, 0xFFFFFFFFu, cnt, items, nullptr, err);
     } else {
         auto kfn = k_hash_bucket<SCATTER_THREADS, SCATTER_IPT, false>;
-        size_t sm = (size_t)SCATTER_THREADS * SCATTER_IPT * 4 + (size_t)g.nb * 8;
+        const size_t sm = (size_t)hchunk * 4 + (size_t)g.nb * 8;
         GQF_CK(set_smem(kfn, sm));
-        kfn<<<(n + hchunk - 1) / hchunk, SCATTER_THREADS, sm, s>>>(keys, n, g, base, 0xFFFFFFFFu, cnt, items,
-                                                                   nullptr, err);
+        kfn<<<hgrid, SCATTER_THREADS, sm, s>>>(keys, n, g, base, 0xFFFFFFFFu, cnt, items, nullptr, err);
     }
     count_launches(3);
     GQF_CK(cudaGetLastError());
@@ -599,7 +626,8 @@ int GQF_RSQF_API(lookup_sorted)(const gqf_rsqf *cqf, int n, const uint32_t *d_ke
 static int rsqf_replay_rounds(uint8_t *t, const uint8_t *t0, uint32_t nbl, uint32_t q, const uint32_t *items,
                               const uint32_t *fhome, uint8_t *start, uint8_t *active, uint8_t *crossed,
                               uint32_t *wlist, uint32_t *blist, uint32_t *ctr, int32_t *d_ret, bool t0_zero,
-                              cudaStream_t s, const uint8_t *sus = nullptr, const uint32_t *fpos = nullptr)
+                              Arena &ar, cudaStream_t s, const uint8_t *sus = nullptr,
+                              const uint32_t *fpos = nullptr)
 {
     const DeviceInfo &di = device_info(current_device());
     const uint32_t grid = std::min<uint32_t>((nbl + 1 + 255) / 256, di.sms * 8);
@@ -612,19 +640,28 @@ static int rsqf_replay_rounds(uint8_t *t, const uint8_t *t0, uint32_t nbl, uint3
                 t, t0, nbl, q, items, fhome, wlist + 2 * (size_t)(nbl + 1), ctr, crossed, ctr + 3, d_ret, sus, fpos,
                 blist);
         } else {
-            k_rsqf_round_warp<RSQF_SMALL_GROUP, 8><<<di.sms * 8, 256, 0, s>>>(t, t0, nbl, q, items, fhome, wlist, ctr,
-                                                                            crossed, ctr + 3, d_ret, t0_zero ? 1 : 0);
-            k_rsqf_round_warp<RSQF_WARP_GROUP_MAX, 1><<<di.sms * 16, 32, 0, s>>>(
+            // the long groups' serial replays run beside the many short ones
+            // (other blocks, other items), on the side stream
+            cudaStream_t side = arena_side(ar);
+            if (!side) return GQF_ERR_CUDA;
+            GQF_CK(cudaEventRecord(ar.fork, s));
+            GQF_CK(cudaStreamWaitEvent(side, ar.fork, 0));
+            k_rsqf_round_warp<RSQF_WARP_GROUP_MAX, 1><<<di.sms * 16, 32, 0, side>>>(
                 t, t0, nbl, q, items, fhome, wlist + 2 * (size_t)(nbl + 1), ctr + 1, crossed, ctr + 3, d_ret,
-                t0_zero ? 1 : 0);
+                t0_zero ? 1 : 0, round == 0 ? 1 : 0);
+            GQF_CK(cudaEventRecord(ar.join, side));
+            k_rsqf_round_warp<RSQF_SMALL_GROUP, 8><<<di.sms * 8, 256, 0, s>>>(t, t0, nbl, q, items, fhome, wlist, ctr,
+                                                                            crossed, ctr + 3, d_ret, t0_zero ? 1 : 0,
+                                                                            round == 0 ? 1 : 0);
+            GQF_CK(cudaStreamWaitEvent(s, ar.join, 0));
         }
         k_rsqf_round_big<<<std::max(1, di.sms), 64, 0, s>>>(t, t0, nbl, q, items, fhome, blist, ctr, crossed,
                                                              ctr + 3, d_ret, t0_zero ? 1 : 0, sus, fpos);
         count_launches(4);
-        uint32_t h_n = 0;
-        GQF_CK(cudaMemcpyAsync(&h_n, ctr + 3, 4, cudaMemcpyDeviceToHost, s));
-        GQF_CK(cudaStreamSynchronize(s));
-        if (h_n == 0) return GQF_OK;
+        uint32_t rep[2];
+        const int st = call_report(ar, s, ctr + 3, rep);
+        if (st) return st;
+        if (rep[1] == 0) return GQF_OK;  // no group crossed
         if (round > 100000) return GQF_ERR_TIMEOUT;
         k_rsqf_merge<<<grid, 256, 0, s>>>(nbl, start, active, crossed);
         count_launches(1);
@@ -694,14 +731,15 @@ int GQF_RSQF_API(insert)(const gqf_rsqf *cqf, int n, const uint32_t *d_keys, int
         k_rsqf_assemble<<<agrid, 256, 0, s>>>(table, items, d_ret, (uint32_t)n, nbl, fpos, fhome, start, sus, ctl, ar.err);
         count_launches(4);
         GQF_CK(cudaGetLastError());
-        uint32_t h_ctl[RCTL_WORDS], h_err = 0;
-        GQF_CK(cudaMemcpyAsync(h_ctl, ctl, sizeof h_ctl, cudaMemcpyDeviceToHost, s));
-        GQF_CK(cudaMemcpyAsync(&h_err, ar.err, sizeof h_err, cudaMemcpyDeviceToHost, s));
-        GQF_CK(cudaStreamSynchronize(s));
+        k_rsqf_report<<<1, 1, 0, s>>>(ar.err, ctl, ar.report_dev);
+        count_launches(1);
+        GQF_CK(cudaEventRecord(ar.ev1, s));
+        GQF_CK(cudaEventSynchronize(ar.ev1));
+        const uint32_t h_err = ar.report[0], h_ctl = ar.report[1];
         if (h_err) return dev_err_to_status(h_err);
         const uint32_t grid = std::min<uint32_t>((nbl + 1 + 255) / 256, di.sms * 16);
-        if (!h_ctl[RCTL_NONEMPTY] && !h_ctl[RCTL_OVER]) {
-            if (h_ctl[RCTL_NSUS]) {
+        if (!(h_ctl & 3u)) {
+            if (h_ctl & 4u) {
                 // replay the clusters the canonical positions do not describe,
                 // each from its empty blocks
                 GQF_CK(cudaMemsetAsync(t0, 0, tbytes, s));
@@ -710,18 +748,18 @@ int GQF_RSQF_API(insert)(const gqf_rsqf *cqf, int n, const uint32_t *d_keys, int
                 k_rsqf_mark_sus<<<grid, 256, 0, s>>>(nbl, start, sus, active);
                 count_launches(1);
                 st = rsqf_replay_rounds(table, t0, nbl, q, items, fhome, start, active, crossed, wlist, blist, ctr,
-                                        d_ret, true, s, sus, fpos);
+                                        d_ret, true, ar, s, sus, fpos);
                 if (st) return st;
             }
         } else {
             GQF_CK(cudaMemcpyAsync(t0, table, tbytes, cudaMemcpyDeviceToDevice, s));
             RsqfView v0{t0, nbl};
             k_pend_reduce<<<ntiles, PEND_THREADS, 0, s>>>(v0, nbl, items, fhome, fn, tile_fn);
-            k_pend_scan_tiles<<<1, 32, 0, s>>>(tile_fn, ntiles);
+            k_pend_scan_tiles<<<1, PEND_SCAN_THREADS, 0, s>>>(tile_fn, ntiles);
             k_pend_apply<<<ntiles, PEND_THREADS, 0, s>>>(nbl, fn, tile_fn, start, active, crossed);
             count_launches(3);
             st = rsqf_replay_rounds(table, t0, nbl, q, items, fhome, start, active, crossed, wlist, blist, ctr, d_ret,
-                                    false, s);
+                                    false, ar, s);
             if (st) return st;
         }
     }

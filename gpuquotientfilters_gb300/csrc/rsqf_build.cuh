@@ -372,7 +372,7 @@ __device__ __forceinline__ PendFn rsqf_block_pend(const RsqfView &v, uint32_t B,
 }
 
 constexpr int PEND_THREADS = 256;
-constexpr int PEND_BPT = 8;
+constexpr int PEND_BPT = 2;  // a block takes hundreds of dependent cycles: few per thread
 constexpr uint32_t PEND_TILE = PEND_THREADS * PEND_BPT;
 
 // Ordered (non-commutative) exclusive block scan of PendFn; `total` gets the
@@ -433,15 +433,21 @@ __global__ void __launch_bounds__(PEND_THREADS) k_pend_reduce(RsqfView v, uint32
     if (threadIdx.x == 0) tile_fn[blockIdx.x] = tot;
 }
 
-// Exclusive composition over the tiles (a few hundred; one thread).
-__global__ void k_pend_scan_tiles(PendFn *tile_fn, uint32_t ntiles)
+// Exclusive composition over the tiles (a few thousand), one CTA: every
+// thread composes a run of tiles, then an ordered block scan.
+constexpr int PEND_SCAN_THREADS = 512;
+__global__ void __launch_bounds__(PEND_SCAN_THREADS) k_pend_scan_tiles(PendFn *tile_fn, uint32_t ntiles)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    PendFn acc{0, 0};
-    for (uint32_t t = 0; t < ntiles; t++) {
+    __shared__ PendFn s_w[PEND_SCAN_THREADS / 32 + 1];
+    const uint32_t per = (ntiles + PEND_SCAN_THREADS - 1) / PEND_SCAN_THREADS;
+    const uint32_t t0 = min(ntiles, threadIdx.x * per), t1 = min(ntiles, t0 + per);
+    PendFn acc{0, 0}, tot;
+    for (uint32_t t = t0; t < t1; t++) acc = pend_compose(acc, tile_fn[t]);
+    PendFn run = block_excl_pend<PEND_SCAN_THREADS>(acc, s_w, tot);
+    for (uint32_t t = t0; t < t1; t++) {
         const PendFn f = tile_fn[t];
-        tile_fn[t] = acc;
-        acc = pend_compose(acc, f);
+        tile_fn[t] = run;
+        run = pend_compose(run, f);
     }
 }
 
