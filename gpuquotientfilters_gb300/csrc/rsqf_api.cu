@@ -63,39 +63,56 @@ __global__ void __launch_bounds__(1024) k_rsqf_scan_bases(const uint32_t *cnt, u
     if (threadIdx.x == 0) base[nb] = tot;
 }
 
-// Sorts each bucket of fingerprints in place (exact bucket bases, so the
-// whole array ends up sorted): counting sort by local quotient in shared
-// memory, then the (small) groups of equal quotient by value.
+// Sorts each bucket's fingerprints into dst[base[b]..] (the whole dst ends up
+// sorted): counting sort by local quotient in shared memory, then every item
+// ranks itself in its (small) group of equal quotients and is stored at its
+// place.  src holds bucket b from src_base[b], or from b * stride.
+// Buckets of lo < n <= cap items; a second launch with more shared memory
+// takes the few larger ones, so that two CTAs share an SM in the first.
+// 60.4M fingerprints, q = 26: one thread per quotient sorting its group, one
+// CTA per SM, took 852 us; this takes 335 us.
+// With bmax non-null it also stores, per bucket, max(quotient_j - j) over
+// the bucket's items (j = index in the whole sorted array), the input of the
+// canonical-position scan.
 constexpr int SORT_THREADS = 512;
 __host__ __device__ inline size_t sort_smem_bytes(uint32_t tb, uint32_t cap)
 {
     size_t S = (size_t)1 << tb;
     return 4 * (S / 2 + S / 32 + 8) + 4 * (size_t)cap;
 }
-// With bmax non-null it also stores, per bucket, max(quotient_j - j) over
-// the bucket's items (j = index in the whole sorted array), the input of the
-// canonical-position scan.
-__global__ void __launch_bounds__(SORT_THREADS) k_bucket_sort(uint32_t *items, const uint32_t *base,
-                                                             const uint32_t *cnt, uint32_t tb, uint32_t cap,
-                                                             uint32_t *err, int32_t *bmax)
+__global__ void __launch_bounds__(SORT_THREADS, 2) k_bucket_sort(const uint32_t *__restrict__ src,
+                                                                const uint32_t *__restrict__ src_base, uint32_t stride,
+                                                                const uint32_t *__restrict__ base,
+                                                                const uint32_t *__restrict__ cnt, uint32_t tb,
+                                                                uint32_t lo, uint32_t cap, int last,
+                                                                uint32_t *__restrict__ dst, uint32_t *err,
+                                                                int32_t *bmax)
 {
     extern __shared__ __align__(16) uint32_t smem_sort[];
     const uint32_t S = 1u << tb;
     uint32_t *s_cnt = smem_sort;
     uint32_t *s_it = smem_sort + (S / 2 + S / 32 + 8);
     __shared__ uint32_t s_warp[33];
-    const uint32_t b = blockIdx.x, n = cnt[b];
-    const size_t b0 = base[b];
-    if (n <= 1 || n > cap) {
+    const uint32_t b = blockIdx.x, n = src_base ? cnt[b] : min(cnt[b], stride);
+    if (n > cap || (lo && n <= lo)) {  // the other launch's
+        if (n > cap && last && threadIdx.x == 0) {
+            atomicOr(err, DEV_ERR_BUCKET_CAP);
+            bmax[b] = INT_MIN;
+        }
+        return;
+    }
+    const size_t s0 = src_base ? (size_t)src_base[b] : (size_t)b * stride, b0 = base[b];
+    if (n <= 1) {
         if (threadIdx.x == 0) {
-            if (n > cap) atomicOr(err, DEV_ERR_BUCKET_CAP);
-            if (bmax) bmax[b] = n == 1 ? (int32_t)(items[b0] >> RSQF_R) - (int32_t)b0 : INT_MIN;
+            if (n) dst[b0] = src[s0];
+            bmax[b] = n ? (int32_t)(src[s0] >> RSQF_R) - (int32_t)b0 : INT_MIN;
         }
         return;
     }
     for (uint32_t i = threadIdx.x; i < S / 2 + S / 32 + 8; i += SORT_THREADS) s_cnt[i] = 0;
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < n; i += SORT_THREADS) cnt16_fetch_inc(s_cnt, (items[b0 + i] >> RSQF_R) & (S - 1));
+    for_each_item<SORT_THREADS>(src, s0, n, threadIdx.x,
+                                [&](uint32_t v) { cnt16_fetch_inc(s_cnt, (v >> RSQF_R) & (S - 1)); });
     __syncthreads();
     // exclusive scan of the packed u16 counters, S/2 words in skewed order
     {
@@ -104,7 +121,10 @@ __global__ void __launch_bounds__(SORT_THREADS) k_bucket_sort(uint32_t *items, c
         const uint32_t per = max(2u, ((S + SORT_THREADS - 1) / SORT_THREADS + 1) & ~1u);
         const uint32_t q0 = min(S, threadIdx.x * per), q1 = min(S, q0 + per);
         uint32_t sum = 0;
-        for (uint32_t x = q0; x < q1; x++) sum += cnt16_get(s_cnt, x);
+        for (uint32_t x = q0; x < q1; x += 2) {
+            const uint32_t c = s_cnt[skew16(x >> 1)];
+            sum += (c & 0xFFFFu) + (c >> 16);
+        }
         const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
         uint32_t incl = sum;
         for (int o = 1; o < 32; o <<= 1) {
@@ -123,36 +143,32 @@ __global__ void __launch_bounds__(SORT_THREADS) k_bucket_sort(uint32_t *items, c
         }
         __syncthreads();
         uint32_t run = s_warp[wid] + incl - sum;
-        __syncthreads();
-        for (uint32_t x = q0; x < q1; x++) {
-            uint32_t c = cnt16_get(s_cnt, x);
-            uint32_t w = skew16(x >> 1), sh = (x & 1) * 16;
-            s_cnt[w] = (s_cnt[w] & ~(0xFFFFu << sh)) | (run << sh);
-            run += c;
+        for (uint32_t x = q0; x < q1; x += 2) {
+            const uint32_t w = skew16(x >> 1), c = s_cnt[w], c0 = c & 0xFFFFu;
+            s_cnt[w] = run | ((run + c0) << 16);
+            run += c0 + (c >> 16);
         }
     }
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < n; i += SORT_THREADS) {
-        uint32_t v = items[b0 + i];
-        s_it[cnt16_fetch_inc(s_cnt, (v >> RSQF_R) & (S - 1))] = v;
-    }
+    for_each_item<SORT_THREADS>(src, s0, n, threadIdx.x,
+                                [&](uint32_t v) { s_it[cnt16_fetch_inc(s_cnt, (v >> RSQF_R) & (S - 1))] = v; });
     __syncthreads();
-    for (uint32_t x = threadIdx.x; x < S; x += SORT_THREADS) {
-        uint32_t g0 = x ? cnt16_get(s_cnt, x - 1) : 0u, g1 = cnt16_get(s_cnt, x);
-        if (g1 - g0 > 1) small_sort(s_it + g0, g1 - g0);
-    }
-    __syncthreads();
+    // group x is now [end of x - 1, end of x)
     int32_t m = INT_MIN;
     for (uint32_t i = threadIdx.x; i < n; i += SORT_THREADS) {
-        const uint32_t v = s_it[i];
-        items[b0 + i] = v;
-        m = max(m, (int32_t)(v >> RSQF_R) - (int32_t)(b0 + i));
+        const uint32_t v = s_it[i], x = (v >> RSQF_R) & (S - 1);
+        const uint32_t g0 = x ? cnt16_get(s_cnt, x - 1) : 0u, g1 = cnt16_get(s_cnt, x);
+        uint32_t p = g0;
+        for (uint32_t j = g0; j < g1; j++) {
+            const uint32_t y = s_it[j];
+            p += (y < v || (y == v && j < i)) ? 1u : 0u;
+        }
+        dst[b0 + p] = v;
+        m = max(m, (int32_t)(v >> RSQF_R) - (int32_t)(b0 + p));
     }
-    if (bmax) {
-        int32_t tot;
-        block_excl_max<SORT_THREADS>(m, reinterpret_cast<int32_t *>(s_warp), tot);
-        if (threadIdx.x == 0) bmax[b] = tot;
-    }
+    int32_t tot;
+    block_excl_max<SORT_THREADS>(m, reinterpret_cast<int32_t *>(s_warp), tot);
+    if (threadIdx.x == 0) bmax[b] = tot;
 }
 
 // Lists this round's groups: every active group start with batch items.
@@ -534,9 +550,12 @@ int GQF_RSQF_API(lookup_unsorted)(const gqf_rsqf *cqf, int n, const uint32_t *d_
     return call_end(ar, s, ms);
 }
 
-// Hash + exact bucketing of a batch into (items, optional idx, base, cnt).
-static int rsqf_bucket(const uint32_t *keys, uint32_t n, const BucketGeom &g, uint32_t *items, uint32_t *idx,
-                       uint32_t *cnt, uint32_t *base, uint32_t *err, cudaStream_t s)
+// Hash + bucketing of a batch: (items, optional idx) by bucket, counts, and
+// the counts' exclusive scan.  stride 0: histogram first, bucket b at base[b];
+// else one pass, bucket b at b * stride (a bucket past it sets
+// DEV_ERR_BUCKET_OVER).
+static int rsqf_bucket(const uint32_t *keys, uint32_t n, const BucketGeom &g, uint32_t stride, uint32_t *items,
+                       uint32_t *idx, uint32_t *cnt, uint32_t *base, uint32_t *err, cudaStream_t s)
 {
     GQF_CK(cudaMemsetAsync(cnt, 0, g.nb * 4, s));
     // batches of up to 4M keys in 4096-key chunks, so that more than a few
@@ -544,33 +563,42 @@ static int rsqf_bucket(const uint32_t *keys, uint32_t n, const BucketGeom &g, ui
     const bool small = n <= (1u << 22);
     const uint32_t hchunk = small ? 256u * 16u : (uint32_t)(SCATTER_THREADS * SCATTER_IPT);
     const uint32_t hgrid = (n + hchunk - 1) / hchunk;
-    if (small) {
-        GQF_CK(set_smem(k_bucket_hist<256, 16>, g.nb * 4));
-        k_bucket_hist<256, 16><<<hgrid, 256, g.nb * 4, s>>>(keys, n, g, cnt);
-    } else {
-        GQF_CK(set_smem(k_bucket_hist<SCATTER_THREADS, SCATTER_IPT>, g.nb * 4));
-        k_bucket_hist<SCATTER_THREADS, SCATTER_IPT><<<hgrid, SCATTER_THREADS, g.nb * 4, s>>>(keys, n, g, cnt);
+    if (!stride) {
+        if (small) {
+            GQF_CK(set_smem(k_bucket_hist<256, 16>, g.nb * 4));
+            k_bucket_hist<256, 16><<<hgrid, 256, g.nb * 4, s>>>(keys, n, g, cnt);
+        } else {
+            GQF_CK(set_smem(k_bucket_hist<SCATTER_THREADS, SCATTER_IPT>, g.nb * 4));
+            k_bucket_hist<SCATTER_THREADS, SCATTER_IPT><<<hgrid, SCATTER_THREADS, g.nb * 4, s>>>(keys, n, g, cnt);
+        }
+        k_rsqf_scan_bases<<<1, 1024, 0, s>>>(cnt, g.nb, base);
+        GQF_CK(cudaMemsetAsync(cnt, 0, g.nb * 4, s));
+        count_launches(2);
     }
-    k_rsqf_scan_bases<<<1, 1024, 0, s>>>(cnt, g.nb, base);
-    GQF_CK(cudaMemsetAsync(cnt, 0, g.nb * 4, s));
+    const uint32_t *at = stride ? nullptr : base;
+    const uint32_t cap = stride ? stride : 0xFFFFFFFFu;
     if (idx) {
         auto kfn = k_hash_bucket<PAIR_THREADS, PAIR_IPT, true>;
         size_t sm = (size_t)2 * PAIR_THREADS * PAIR_IPT * 4 + (size_t)g.nb * 8;
         GQF_CK(set_smem(kfn, sm));
         const uint32_t chunk = PAIR_THREADS * PAIR_IPT;
-        kfn<<<(n + chunk - 1) / chunk, PAIR_THREADS, sm, s>>>(keys, n, g, base, 0xFFFFFFFFu, cnt, items, idx, err);
+        kfn<<<(n + chunk - 1) / chunk, PAIR_THREADS, sm, s>>>(keys, n, g, at, cap, cnt, items, idx, err);
     } else if (small) {
         auto kfn = k_hash_bucket<256, 16, false>;
         const size_t sm = (size_t)hchunk * 4 + (size_t)g.nb * 8;
         GQF_CK(set_smem(kfn, sm));
-        kfn<<<hgrid, 256, sm, s>>>(keys, n, g, base, 0xFFFFFFFFu, cnt, items, nullptr, err);
+        kfn<<<hgrid, 256, sm, s>>>(keys, n, g, at, cap, cnt, items, nullptr, err);
     } else {
         auto kfn = k_hash_bucket<SCATTER_THREADS, SCATTER_IPT, false>;
         const size_t sm = (size_t)hchunk * 4 + (size_t)g.nb * 8;
         GQF_CK(set_smem(kfn, sm));
-        kfn<<<hgrid, SCATTER_THREADS, sm, s>>>(keys, n, g, base, 0xFFFFFFFFu, cnt, items, nullptr, err);
+        kfn<<<hgrid, SCATTER_THREADS, sm, s>>>(keys, n, g, at, cap, cnt, items, nullptr, err);
     }
-    count_launches(3);
+    count_launches(1);
+    if (stride) {
+        k_rsqf_scan_bases<<<1, 1024, 0, s>>>(cnt, g.nb, base);
+        count_launches(1);
+    }
     GQF_CK(cudaGetLastError());
     return GQF_OK;
 }
@@ -602,7 +630,7 @@ int GQF_RSQF_API(lookup_sorted)(const gqf_rsqf *cqf, int n, const uint32_t *d_ke
     int st = call_begin(ar, s, ms != nullptr);
     if (st) return st;
     if (n > 0) {
-        st = rsqf_bucket(d_keys, (uint32_t)n, g, items, idx, cnt, base, ar.err, s);
+        st = rsqf_bucket(d_keys, (uint32_t)n, g, 0, items, idx, cnt, base, ar.err, s);
         if (st) return st;
         RsqfView v{static_cast<const uint8_t *>(cqf->blocks), cqf->numBlocks};
         k_rsqf_lookup_bucketed<<<g.nb, RSQF_LOOKUP_THREADS, 0, s>>>(items, idx, base, cnt, v, cqf->qbits, d_out);
@@ -679,9 +707,15 @@ int GQF_RSQF_API(insert)(const gqf_rsqf *cqf, int n, const uint32_t *d_keys, int
     uint8_t *table = static_cast<uint8_t *>(cqf->blocks);
     Arena &ar = arena(current_device(), s);
     std::lock_guard<std::mutex> lk(ar.mu);
+    // one scatter into regions of the average bucket and a margin; a bucket
+    // past its region means a second try with exact bases
+    const double avg = (double)n / g.nb;
+    const uint32_t stride = (uint32_t)align_up((size_t)(avg + 10.0 * std::sqrt(avg) + 64.0), 32);
+    const size_t nraw = std::max<size_t>((size_t)g.nb * stride, std::max(n, 1));
     Sizer z;
     z.take<uint32_t>(g.nb);
     z.take<uint32_t>(g.nb + 1);
+    z.take<uint32_t>(nraw);
     z.take<uint32_t>(std::max(n, 1));
     z.take<int32_t>(g.nb);
     z.take<int32_t>(g.nb);
@@ -699,7 +733,7 @@ int GQF_RSQF_API(insert)(const gqf_rsqf *cqf, int n, const uint32_t *d_keys, int
     if (!basep) return GQF_ERR_NOMEM;
     Carver c(basep);
     uint32_t *cnt = c.take<uint32_t>(g.nb), *base = c.take<uint32_t>(g.nb + 1);
-    uint32_t *items = c.take<uint32_t>(std::max(n, 1));
+    uint32_t *raw = c.take<uint32_t>(nraw), *items = c.take<uint32_t>(std::max(n, 1));
     int32_t *bmax = c.take<int32_t>(g.nb), *bpre = c.take<int32_t>(g.nb);
     uint32_t *fpos = c.take<uint32_t>(nbl + 1), *fhome = c.take<uint32_t>(nbl + 1);
     uint8_t *t0 = c.take<uint8_t>(tbytes);
@@ -715,20 +749,29 @@ int GQF_RSQF_API(insert)(const gqf_rsqf *cqf, int n, const uint32_t *d_keys, int
         GQF_CK(cudaMemsetAsync(ctl, 0, RCTL_WORDS * 4, s));
         k_rsqf_nonzero<<<di.sms * 4, 512, 0, s>>>(table, (size_t)(nbl + 1) * RSQF_BB, ctl);
         count_launches(1);
-        st = rsqf_bucket(d_keys, (uint32_t)n, g, items, nullptr, cnt, base, ar.err, s);
+        // per-bucket sort: a small capacity (two CTAs per SM), then whatever the shared memory allows
+        const size_t maxsm = (size_t)(di.smem_optin > 0 ? di.smem_optin : 99 * 1024) - 2048;
+        const size_t fixed = sort_smem_bytes(g.tb, 0);
+        const uint32_t cap = maxsm > fixed ? (uint32_t)std::min<size_t>((maxsm - fixed) / 4, 65535) : 0;
+        uint32_t cap1 = (uint32_t)std::min<size_t>(cap, fixed < 108 * 1024 ? (108 * 1024 - fixed) / 4 : 0);
+        if (cap1 < avg * 1.05) cap1 = cap;
+        GQF_CK(set_smem(k_bucket_sort, sort_smem_bytes(g.tb, cap)));
+        bool exact = false;
+    again:
+        st = rsqf_bucket(d_keys, (uint32_t)n, g, exact ? 0 : stride, raw, nullptr, cnt, base, ar.err, s);
         if (st) return st;
-        // per-bucket sort: capacity from the largest bucket the smem allows
-        size_t maxsm = (size_t)(di.smem_optin > 0 ? di.smem_optin : 99 * 1024) - 2048;
-        size_t fixed = sort_smem_bytes(g.tb, 0);
-        uint32_t cap = maxsm > fixed ? (uint32_t)std::min<size_t>((maxsm - fixed) / 4, 65535) : 0;
-        size_t sm = sort_smem_bytes(g.tb, cap);
-        GQF_CK(set_smem(k_bucket_sort, sm));
-        k_bucket_sort<<<g.nb, SORT_THREADS, sm, s>>>(items, base, cnt, g.tb, cap, ar.err, bmax);
+        k_bucket_sort<<<g.nb, SORT_THREADS, sort_smem_bytes(g.tb, cap1), s>>>(
+            raw, exact ? base : nullptr, stride, base, cnt, g.tb, 0u, cap1, cap1 == cap, items, ar.err, bmax);
+        if (cap1 < cap) {
+            k_bucket_sort<<<g.nb, SORT_THREADS, sort_smem_bytes(g.tb, cap), s>>>(
+                raw, exact ? base : nullptr, stride, base, cnt, g.tb, cap1, cap, 1, items, ar.err, bmax);
+            count_launches(1);
+        }
         k_rsqf_scan_max<<<1, 1024, 0, s>>>(bmax, g.nb, bpre);
         k_rsqf_positions<<<g.nb, RPOS_THREADS, 0, s>>>(items, (uint32_t)n, base, cnt, bpre, nbl, nbl * RSQF_SPB,
                                                        d_ret, fpos, fhome, ctl, ar.err);
-        const uint32_t agrid = std::min<uint32_t>((nbl + 1 + 7) / 8, di.sms * 64);
-        k_rsqf_assemble<<<agrid, 256, 0, s>>>(table, items, d_ret, (uint32_t)n, nbl, fpos, fhome, start, sus, ctl, ar.err);
+        k_rsqf_assemble<<<nbl / ASM_BLOCKS + 1, ASM_THREADS, 0, s>>>(table, items, d_ret, (uint32_t)n, nbl, fpos, fhome,
+                                                                     start, sus, ctl, ar.err);
         count_launches(4);
         GQF_CK(cudaGetLastError());
         k_rsqf_report<<<1, 1, 0, s>>>(ar.err, ctl, ar.report_dev);
@@ -736,6 +779,11 @@ int GQF_RSQF_API(insert)(const gqf_rsqf *cqf, int n, const uint32_t *d_keys, int
         GQF_CK(cudaEventRecord(ar.ev1, s));
         GQF_CK(cudaEventSynchronize(ar.ev1));
         const uint32_t h_err = ar.report[0], h_ctl = ar.report[1];
+        if ((h_err & DEV_ERR_BUCKET_OVER) && !exact) {  // nothing was written yet
+            exact = true;
+            GQF_CK(cudaMemsetAsync(ar.err, 0, sizeof(uint32_t), s));
+            goto again;
+        }
         if (h_err) return dev_err_to_status(h_err);
         const uint32_t grid = std::min<uint32_t>((nbl + 1 + 255) / 256, di.sms * 16);
         if (!(h_ctl & 3u)) {
