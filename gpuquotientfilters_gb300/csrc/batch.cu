@@ -21,27 +21,29 @@
 
 namespace gqf {
 
-// Slots past the last bucket's quotients only receive spill: clear them in
-// every filter that is rebuilt (the single-filter path does this with a
-// memset before its layout).
+// Slots past the last bucket's quotients only receive spill and start empty:
+// a filter's scatter chunks clear an equal share each, 16 bytes a store (the
+// tail starts 16-byte aligned).  One CTA per filter storing bytes took 89 us
+// for 256 filters of up to 2^22 slots, beside everything else.
 template <int BPE>
-__global__ void k_mf_clear_tails(MfParams p)
+__device__ __forceinline__ void mf_clear_tail(const MfFilter &f, uint32_t chunk, uint32_t nchunks)
 {
-    for (uint32_t fi = blockIdx.x; fi < p.nf; fi += gridDim.x) {
-        const MfFilter &f = p.f[fi];
-        if (!f.n_keys) continue;
-        const size_t tail = (size_t)(1u << f.q) * BPE;
-        for (size_t i = tail + threadIdx.x; i < f.T; i += blockDim.x) f.table[i] = 0;
-    }
+    const uint32_t t0 = BPE << f.q, len = f.T - t0, words = len / 16;
+    const uint32_t per = (words + nchunks - 1) / nchunks, w0 = min(words, chunk * per), w1 = min(words, w0 + per);
+    for (uint32_t i = w0 + threadIdx.x; i < w1; i += blockDim.x)
+        *reinterpret_cast<uint4 *>(f.table + t0 + 16 * (size_t)i) = make_uint4(0, 0, 0, 0);
+    if (chunk == 0)
+        for (uint32_t i = 16 * words + threadIdx.x; i < len; i += blockDim.x) f.table[t0 + i] = 0;
 }
 
-template <int THREADS, int IPT>
+template <int THREADS, int IPT, int BPE>
 __global__ void __launch_bounds__(THREADS) k_mf_hist(MfParams p)
 {
     __shared__ uint32_t s_f;
     if (threadIdx.x == 0) s_f = mf_owner<&MfFilter::chunk0>(p.f, p.nf, blockIdx.x);
     __syncthreads();
     const MfFilter &f = p.f[s_f];
+    mf_clear_tail<BPE>(f, blockIdx.x - f.chunk0, (f.n_keys + THREADS * IPT - 1) / (THREADS * IPT));
     bucket_hist_chunk<THREADS, IPT>(blockIdx.x - f.chunk0, f.keys, f.n_keys, mf_geom(f, p.tb), p.bcnt + f.bucket0);
 }
 
@@ -57,16 +59,28 @@ __global__ void __launch_bounds__(THREADS) k_mf_scatter(MfParams p)
                                            p.err);
 }
 
-// Exclusive scan of the bucket counts of all filters (one CTA).
+// Exclusive scan of the bucket counts of all filters.  A CTA scans one tile,
+// after summing all counts before it (52,000 counts are 200 KB in L2; one CTA
+// scanning them all took 43 us).
+constexpr uint32_t MF_SCAN_TILE = 4096;
 __global__ void __launch_bounds__(1024) k_mf_scan(const uint32_t *__restrict__ cnt, uint32_t nb,
                                                   uint32_t *__restrict__ base)
 {
-    __shared__ uint32_t sw[33];
-    const uint32_t per = (nb + 1023) / 1024;
-    const uint32_t b0 = min(nb, threadIdx.x * per), b1 = min(nb, b0 + per);
-    uint32_t sum = 0;
-    for (uint32_t b = b0; b < b1; b++) sum += cnt[b];
+    __shared__ uint32_t sw[33], s_before;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint32_t t0 = blockIdx.x * MF_SCAN_TILE, b0 = t0 + 4 * threadIdx.x;
+    uint32_t before = 0;
+    for (uint32_t i = threadIdx.x; i < t0; i += 1024) before += cnt[i];
+    before = __reduce_add_sync(~0u, before);
+    if (threadIdx.x == 0) s_before = 0;
+    __syncthreads();
+    if (lane == 0) atomicAdd(&s_before, before);
+    uint32_t c[4], sum = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        c[k] = b0 + k < nb ? cnt[b0 + k] : 0u;
+        sum += c[k];
+    }
     uint32_t incl = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -86,10 +100,11 @@ __global__ void __launch_bounds__(1024) k_mf_scan(const uint32_t *__restrict__ c
         sw[lane] = iv - v;
     }
     __syncthreads();
-    uint32_t run = sw[wid] + incl - sum;
-    for (uint32_t b = b0; b < b1; b++) {
-        base[b] = run;
-        run += cnt[b];
+    uint32_t run = s_before + sw[wid] + incl - sum;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        if (b0 + k < nb) base[b0 + k] = run;
+        run += c[k];
     }
 }
 
@@ -198,13 +213,13 @@ static cudaError_t mf_smem(K kernel, size_t bytes)
 }
 
 // Calls fn(kernel-set) for the scatter shape of the tuning.
-template <typename Fn>
+template <int BPE, typename Fn>
 static cudaError_t mf_with_scatter(uint32_t chunk, Fn fn)
 {
     switch (chunk) {
-    case 2048: return fn(k_mf_hist<256, 8>, k_mf_scatter<256, 8>, 256u, 2048u);
-    case 32768: return fn(k_mf_hist<1024, 32>, k_mf_scatter<1024, 32>, 1024u, 32768u);
-    default: return fn(k_mf_hist<256, 32>, k_mf_scatter<256, 32>, 256u, 8192u);
+    case 2048: return fn(k_mf_hist<256, 8, BPE>, k_mf_scatter<256, 8>, 256u, 2048u);
+    case 32768: return fn(k_mf_hist<1024, 32, BPE>, k_mf_scatter<1024, 32>, 1024u, 32768u);
+    default: return fn(k_mf_hist<256, 32, BPE>, k_mf_scatter<256, 32>, 256u, 8192u);
     }
 }
 
@@ -233,10 +248,10 @@ static int mf_record(Batch &b, cudaStream_t s)
     GQF_CK(cudaMemsetAsync(b.ctrl, 0, b.ctrl_bytes, s));
     if (b.any_build) {
         const uint32_t fgrid = std::min<uint32_t>(b.nf, (uint32_t)di.sms * 4);
-        k_mf_clear_tails<BPE><<<fgrid, 256, 0, s>>>(b.p);
-        GQF_CK(mf_with_scatter(b.tune.scatter_chunk, [&](auto khist, auto kscat, uint32_t threads, uint32_t chunk) {
+        GQF_CK(mf_with_scatter<BPE>(b.tune.scatter_chunk, [&](auto khist, auto kscat, uint32_t threads, uint32_t chunk) {
             khist<<<b.total_chunks, threads, (size_t)b.nbmax * 4, s>>>(b.p);
-            k_mf_scan<<<1, 1024, 0, s>>>(b.p.bcnt, b.total_buckets, b.p.bbase);
+            k_mf_scan<<<(b.total_buckets + MF_SCAN_TILE - 1) / MF_SCAN_TILE, 1024, 0, s>>>(
+                b.p.bcnt, b.total_buckets, b.p.bbase);
             kscat<<<b.total_chunks, threads, (size_t)chunk * 4 + (size_t)b.nbmax * 8, s>>>(b.p);
             return cudaGetLastError();
         }));
@@ -245,7 +260,7 @@ static int mf_record(Batch &b, cudaStream_t s)
             return cudaGetLastError();
         }));
         k_mf_fixup<BPE><<<fgrid, 256, 0, s>>>(b.p);
-        count_launches(6);
+        count_launches(5);
     }
     if (b.any_lookup) {
         const uint32_t grid = std::min<uint32_t>(b.total_qchunks, (uint32_t)di.sms * 8);
@@ -395,10 +410,12 @@ static int mf_create(Batch *b, const gqf_sqf_job *jobs, int count, int no_duplic
     b->p.bitmap_ok = bitmap ? 1 : 0;
     b->p.total_buckets = buckets;
     // kernel attributes, then the graph
-    GQF_CK(mf_with_scatter(b->tune.scatter_chunk, [&](auto khist, auto kscat, uint32_t, uint32_t chunk) {
+    auto scatter_attrs = [&](auto khist, auto kscat, uint32_t, uint32_t chunk) {
         cudaError_t e = mf_smem(khist, (size_t)b->nbmax * 4);
         return e != cudaSuccess ? e : mf_smem(kscat, (size_t)chunk * 4 + (size_t)b->nbmax * 8);
-    }));
+    };
+    GQF_CK(b->bpe == 1 ? mf_with_scatter<1>(b->tune.scatter_chunk, scatter_attrs)
+                       : mf_with_scatter<2>(b->tune.scatter_chunk, scatter_attrs));
     if (b->bpe == 1)
         GQF_CK(mf_with_layout<1>(tb, bitmap, [&](auto klay, int) { return mf_smem(klay, b->layout_smem); }));
     else
