@@ -367,7 +367,7 @@ static int mf_create(Batch *b, const gqf_sqf_job *jobs, int count, int no_duplic
     uint32_t cap = (uint32_t)std::min<double>(max_avg * 1.25 + 10.0 * std::sqrt(max_avg) + 512.0, 65520.0);
     cap = (cap + 15) & ~15u;
     // bitmap mode: thread counts of the graph (32 quotients a thread) and the persistent form
-    size_t sm = bitmap ? set_plan(tb, std::max(S / 32, (uint32_t)b->tune.cta_threads)).total
+    size_t sm = bitmap ? set_layout_smem(tb, std::max(S / 32, (uint32_t)b->tune.cta_threads))
                        : layout_smem_bytes(tb, cap, (int)b->bpe);
     if (sm > maxsm) return GQF_ERR_ARG;
     b->layout_smem = sm;

@@ -50,6 +50,7 @@ static uint32_t ceil_log2(uint64_t x)
 struct LayoutPlan {
     BucketGeom g;
     uint32_t stride;     // speculative bucket stride (items)
+    uint64_t n_expect;   // items it was made for
     uint32_t cap_items;  // per-CTA item capacity of k_bucket_layout
     size_t smem;
 };
@@ -80,6 +81,7 @@ static LayoutPlan plan_layout(uint32_t q, uint32_t r, uint64_t n_expect, uint64_
     p.g.fp_mask = (q + r >= 32) ? 0xFFFFFFFFu : ((1u << (q + r)) - 1u);
     double avg_b = (double)n_b_expect / p.g.nb;
     p.stride = (uint32_t)align_up((size_t)(avg_b + 10.0 * std::sqrt(avg_b) + 64.0), 32);
+    p.n_expect = n_expect;
     p.cap_items = 0;
     p.smem = 0;
     if (!general) return p;
@@ -153,6 +155,7 @@ struct Scratch {
     uint32_t fix_cap;
     uint32_t *bitems;  // batch fingerprints
     uint32_t *bidx;    // batch indices (sorted lookups)
+    void *rems;        // k_group_layout: remainders of large buckets
     // extracted table contents
     Counts3 *tiles;
     uint32_t *Q, *E, *abase, *acnt;
@@ -170,6 +173,7 @@ struct ScratchReq {
     size_t snap_bytes = 0;  // in-place update: snapshot of the table
     uint32_t upd_nb = 0;    // and its layout buckets
     bool every_fix = false; // room for a fix-up of every quotient
+    uint32_t rem_bytes = 0; // k_group_layout: scratch bytes per item
 };
 
 static Scratch carve(void *base, const ScratchReq &r, bool sizing_only, size_t *bytes_out)
@@ -189,6 +193,7 @@ static Scratch carve(void *base, const ScratchReq &r, bool sizing_only, size_t *
         s.fix_list = c.template take<uint32_t>(s.fix_cap);
         s.bitems = c.template take<uint32_t>(std::max<size_t>(r.batch_items, 1));
         s.bidx = r.pairs ? c.template take<uint32_t>(std::max<size_t>(r.batch_items, 1)) : nullptr;
+        s.rems = r.rem_bytes ? c.template take<uint8_t>(std::max<size_t>(r.batch_items, 1) * r.rem_bytes) : nullptr;
         if (r.extract) {
             size_t ntiles = (r.nslots + EXTRACT_TILE - 1) / EXTRACT_TILE;
             s.tiles = c.template take<Counts3>(ntiles + 1);
@@ -331,7 +336,7 @@ static int launch_layout(const LayoutPlan &p, const SqfGeom &tg, uint8_t *table,
         if (e == cudaSuccess) kernel<<<p.g.nb, threads, smem, s>>>(a);
     };
     if (BPE == 1 && set_ok) {
-        const size_t smem = set_plan(p.g.tb, threads).total;
+        const size_t smem = set_layout_smem(p.g.tb, threads);
         switch (p.g.tb) {
         case 15: go(k_set_layout<1024, 32>, smem); break;
         case 14: go(k_set_layout<512, 32>, smem); break;
@@ -346,7 +351,31 @@ static int launch_layout(const LayoutPlan &p, const SqfGeom &tg, uint8_t *table,
         GQF_CK(e);
         count_launches(1);
     }
-    if (!set_ok || a_dups) {
+    if (op == OP_BUILD && !set_ok) {
+        // shared memory for a third more than the average bucket; a larger
+        // one keeps its remainders in the scratch
+        a.rem_scratch = sc.rems;
+        const double avg = (double)p.n_expect / p.g.nb;
+        a.cap_items = (uint32_t)align_up((size_t)std::min(avg * 1.3 + 8.0 * std::sqrt(avg) + 64.0, 40000.0), 16);
+        const size_t smem = group_layout_smem(p.g.tb, threads, BPE, a.cap_items);
+        auto gg = [&](auto dup, auto uniq) {
+            if (nodup) go(uniq, smem);
+            else go(dup, smem);
+        };
+        switch (p.g.tb) {
+        case 15: gg(k_group_layout<1024, 32, BPE, false>, k_group_layout<1024, 32, BPE, true>); break;
+        case 14: gg(k_group_layout<512, 32, BPE, false>, k_group_layout<512, 32, BPE, true>); break;
+        case 13: gg(k_group_layout<256, 32, BPE, false>, k_group_layout<256, 32, BPE, true>); break;
+        case 12: gg(k_group_layout<256, 16, BPE, false>, k_group_layout<256, 16, BPE, true>); break;
+        case 11: gg(k_group_layout<128, 16, BPE, false>, k_group_layout<128, 16, BPE, true>); break;
+        case 10: gg(k_group_layout<128, 8, BPE, false>, k_group_layout<128, 8, BPE, true>); break;
+        case 9: gg(k_group_layout<64, 8, BPE, false>, k_group_layout<64, 8, BPE, true>); break;
+        case 8: gg(k_group_layout<32, 8, BPE, false>, k_group_layout<32, 8, BPE, true>); break;
+        default: gg(k_group_layout<32, 4, BPE, false>, k_group_layout<32, 4, BPE, true>); break;
+        }
+        GQF_CK(e);
+        count_launches(1);
+    } else if (!set_ok || a_dups) {
         switch (p.g.tb) {
         case 15: go(k_bucket_layout<1024, 32, BPE>, p.smem); break;
         case 14: go(k_bucket_layout<512, 32, BPE>, p.smem); break;
@@ -489,11 +518,12 @@ static int rebuild(const gqf_sqf *qf, const gqf_sqf *qf2, const uint32_t *keys, 
     const bool fused = BPE == 1 && set_ok && needA;
     // an update's batch keeps the large buckets (a layout bucket reads its
     // part of one); a build's are the layout's
-    LayoutPlan p = plan_layout(tg.q, tg.r, expect, bFromTable ? 0 : n, !set_ok || update, !fused);
+    LayoutPlan p = plan_layout(tg.q, tg.r, expect, bFromTable ? 0 : n, (!set_ok && op != OP_BUILD) || update, !fused);
     ScratchReq req{p.g.nb, bFromTable ? 0 : (size_t)p.g.nb * p.stride, false, needA, bFromTable, tg.nslots};
     // small filters are laid out in small buckets, which a nearly full table's
     // spill can pass whole
     req.every_fix = tg.q <= 22;
+    if (op == OP_BUILD && !set_ok) req.rem_bytes = BPE;
     int dev = current_device();
     Arena &ar = arena(dev, s);
     std::lock_guard<std::mutex> lk(ar.mu);
@@ -877,8 +907,9 @@ static int bulk_build_noalloc_t(const gqf_sqf *qf, uint32_t n, const uint32_t *k
     char *base = static_cast<char *>(nd->base);
     const SqfGeom tg = geom_of(qf);
     const bool set_ok = tg.r == 5 && nodup;
-    LayoutPlan p = plan_layout(tg.q, tg.r, n, n, !set_ok, false);  // few buckets: the fix-up list is small
+    LayoutPlan p = plan_layout(tg.q, tg.r, n, n, false, false);  // few buckets: the fix-up list is small
     ScratchReq req{p.g.nb, std::max<size_t>(n, 1), false, false, false, tg.nslots};
+    if (!set_ok) req.rem_bytes = BPE;
     size_t need = 0;
     carve(nullptr, req, true, &need);
     const size_t err_off = GQF_NOALLOC_SCRATCH_BYTES - 256;  // device error word

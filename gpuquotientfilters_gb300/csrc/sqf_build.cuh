@@ -457,6 +457,7 @@ struct LayoutArgs {
     // bucket that cannot be decoded (duplicate or out-of-order remainders in
     // an insert or delete, runs past its slice) sets *fused_fail and the op
     // is done the general way.
+    void *rem_scratch = nullptr;  // k_group_layout: a remainder per item of B, for buckets past cap_items
     const uint8_t *src_table = nullptr, *src2 = nullptr;
     uint32_t sub = 0;
     uint32_t *fused_fail = nullptr;

@@ -1,7 +1,8 @@
-// Set layouts of one-byte slots (r = 5, no fingerprint stored twice): the
-// bucket layout of builds and merges from fingerprint lists (k_set_layout),
+// Item-parallel bucket layouts.  One-byte slots with no fingerprint stored
+// twice (r = 5): builds and merges from fingerprint lists (k_set_layout),
 // and the in-place merge and large insert, which decode a bucket's old
-// contents straight from the table (k_set_update).
+// contents straight from the table (k_set_update).  Builds that keep every
+// copy, or of two-byte slots: k_group_layout.
 #pragma once
 
 #include "sqf_build.cuh"
@@ -28,19 +29,23 @@ constexpr uint32_t SET_R = 5;
 constexpr uint32_t SET_SPILL = 2048;   // tile slots past the bucket; the rest goes straight to the table
 constexpr uint32_t SET_ESCAPE = 255;   // displacement that does not fit a byte: recomputed from the thread's start
 
-struct SetPlan {
-    size_t disp, tile, occ, gc, total;
+// Shared memory of a layout CTA: run displacements, tile, occupied bits, the
+// threads' first free slots, then the bucket's contents.
+struct ItemsPlan {
+    size_t tile, occ, gc, contents;
 };
-__host__ __device__ inline SetPlan set_plan(uint32_t tb, uint32_t threads)
+__host__ __device__ constexpr ItemsPlan items_plan(size_t S, size_t threads, size_t bpe)
 {
-    const size_t S = (size_t)1 << tb;
-    SetPlan m;
-    m.disp = 4 * S;
-    m.tile = m.disp + S;
-    m.occ = m.tile + S + SET_SPILL + 16;
+    ItemsPlan m{};
+    m.tile = (S + 15) & ~(size_t)15;
+    m.occ = m.tile + (S + SET_SPILL) * bpe + 16;
     m.gc = m.occ + ((S / 8 + 15) & ~(size_t)15);
-    m.total = m.gc + 4 * ((size_t)threads + 4);
+    m.contents = m.gc + 4 * (threads + 4);
     return m;
+}
+__host__ __device__ inline size_t set_layout_smem(uint32_t tb, uint32_t threads)  // remainder sets
+{
+    return items_plan((size_t)1 << tb, threads, 1).contents + ((size_t)4 << tb);
 }
 
 // Shared-memory byte offset of the remainder set of local quotient x: the
@@ -99,7 +104,7 @@ struct ListSource {
         abase = na ? a.A.start(b) : 0;
         bbase = nb ? a.B.start(b) : 0;
     }
-    __device__ __forceinline__ void index(uint32_t) {}
+    __device__ __forceinline__ void index() {}
     // every fingerprint of the table, then those of the batch (local
     // quotient, remainder), shared by NT threads of which this is number t
     template <int NT, typename F>
@@ -114,15 +119,223 @@ struct ListSource {
     }
 };
 
+// Contents of a bucket as remainder sets, fed by a source (lists, or tables).
 template <int THREADS, int QPT, template <int, int> class Source>
-__device__ __forceinline__ void bucket_layout_set(const LayoutArgs &a, const uint32_t b)
+struct SetContents {
+    static constexpr int BPE = 1;
+    static constexpr bool SMALL = true;  // at most 32 items a quotient
+    static constexpr uint32_t S = THREADS * QPT;
+    uint8_t *mask;  // u32 at set_addr(x)
+    Source<THREADS, QPT> src;
+    __device__ __forceinline__ SetContents(const LayoutArgs &a, uint32_t b, uint8_t *mem) : mask(mem), src(a, b, mem + 4 * S) {}
+    __device__ __forceinline__ uint32_t &at(uint32_t x) const { return *reinterpret_cast<uint32_t *>(mask + set_addr(x)); }
+    __device__ __forceinline__ bool fits() const { return true; }
+    __device__ __forceinline__ void load()
+    {
+        for (uint32_t i = threadIdx.x; i < S / 4; i += THREADS) reinterpret_cast<uint4 *>(mask)[i] = make_uint4(0, 0, 0, 0);
+        src.index();
+        __syncthreads();
+        each<THREADS>(threadIdx.x, [&](uint32_t x, uint32_t rem) { atomicOr(&at(x), 1u << rem); });
+        __syncthreads();
+    }
+    __device__ __forceinline__ void sizes(uint32_t x, uint32_t (&k)[4]) const  // of quotients x .. x + 3
+    {
+        const uint4 m = *reinterpret_cast<const uint4 *>(mask + set_addr(x));
+        k[0] = __popc(m.x);
+        k[1] = __popc(m.y);
+        k[2] = __popc(m.z);
+        k[3] = __popc(m.w);
+    }
+    __device__ __forceinline__ uint32_t size(uint32_t x) const { return __popc(at(x)); }
+    template <int NT, typename F>
+    __device__ __forceinline__ void each(uint32_t t, F &&f) const
+    {
+        src.template table_items<NT>(t, f);
+        src.template batch_items<NT>(t, f);
+    }
+    // put(slot, element) for an item of a run that starts at slot st; the
+    // element's occupied bit is not set
+    template <typename Put>
+    __device__ __forceinline__ void put_item(uint32_t x, uint32_t rem, uint32_t st, Put &&put) const
+    {
+        const uint32_t below = __popc(at(x) & ((1u << rem) - 1u)), p = st + below;
+        put(p, (rem << 3) + 2 * min(below, 1u) + min(p - x, 1u));
+    }
+    template <typename Put>
+    __device__ __forceinline__ void put_run(uint32_t x, uint32_t st, Put &&put) const
+    {
+        uint32_t f = 0;
+        for (uint32_t m = at(x); m; m &= m - 1u, st++, f = 2u) put(st, ((__ffs(m) - 1) << 3) + f + min(st - x, 1u));
+    }
+    template <int NT, typename Start, typename Put>
+    __device__ __forceinline__ void put_big(uint32_t, Start &&, Put &&) const
+    {
+    }
+};
+
+// Contents of a bucket as groups: the remainders of each quotient next to
+// each other (counting sort), in any order.  Every copy is kept, or (UNIQUE)
+// repeats are struck out.  An item's slot is its run's start plus the smaller
+// ones of its group; equal copies each write all of their slots.  Groups of
+// more than BIG items are sorted and laid out by one thread each instead.  A
+// bucket with more items than the shared memory was sized for keeps its
+// remainders in global scratch.
+//
+// A thread sorting and walking its 32 quotients' groups one after the other
+// took 396 us for 12.3M fingerprints over 2^24 quotients; this takes 172 us.
+template <int THREADS, int QPT, int BPE_, bool UNIQUE>
+struct GroupContents {
+    static constexpr int BPE = BPE_;
+    static constexpr bool SMALL = false;
+    static constexpr uint32_t S = THREADS * QPT, R = BPE == 1 ? 5 : 13, BIG = 48;
+    using Rem = typename std::conditional<BPE == 1, uint8_t, uint16_t>::type;
+    static constexpr uint32_t STRUCK = BPE == 1 ? 0xFFu : 0xFFFFu;  // above every remainder
+    const LayoutArgs &a;
+    uint32_t *cnt;  // u16 per quotient: end of its group
+    Rem *rem;
+    uint32_t n, stray;
+    size_t base;
+    __device__ __forceinline__ GroupContents(const LayoutArgs &args, uint32_t b, uint8_t *mem) : a(args)
+    {
+        n = a.B.count(b);
+        base = n ? a.B.start(b) : 0;
+        cnt = reinterpret_cast<uint32_t *>(mem);
+        rem = n <= a.cap_items ? reinterpret_cast<Rem *>(mem + group_cnt_bytes(S))
+                               : static_cast<Rem *>(a.rem_scratch) + base;
+    }
+    static __host__ __device__ constexpr size_t group_cnt_bytes(size_t s) { return (4 * (s / 2 + s / 32 + 8) + 15) & ~(size_t)15; }
+    __device__ __forceinline__ bool fits() const { return n <= 65520; }  // u16 positions
+    __device__ __forceinline__ uint32_t end(uint32_t x) const { return cnt16_get(cnt, x); }
+    __device__ __forceinline__ uint32_t begin(uint32_t x) const { return x ? cnt16_get(cnt, x - 1) : 0u; }
+    __device__ __forceinline__ void load()
+    {
+        __shared__ uint32_t s_w[THREADS / 32];
+        const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+        for (uint32_t i = tid; i < S / 2 + S / 32 + 8; i += THREADS) cnt[i] = 0;
+        __syncthreads();
+        each<THREADS>(tid, [&](uint32_t x, uint32_t) { cnt16_fetch_inc(cnt, x); });
+        __syncthreads();
+        uint32_t sum = 0;
+        for (uint32_t j = 0; j < QPT; j += 2) {
+            const uint32_t c = cnt[skew16((tid * QPT + j) >> 1)];
+            sum += (c & 0xFFFFu) + (c >> 16);
+        }
+        uint32_t incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+            if ((int)lane >= o) incl += v;
+        }
+        if (lane == 31) s_w[wid] = incl;
+        __syncthreads();
+        uint32_t run = incl - sum;
+        for (uint32_t w = 0; w < wid; w++) run += s_w[w];
+        for (uint32_t j = 0; j < QPT; j += 2) {  // both counters of a word
+            const uint32_t w = skew16((tid * QPT + j) >> 1), c = cnt[w], c0 = c & 0xFFFFu;
+            cnt[w] = run | ((run + c0) << 16);
+            run += c0 + (c >> 16);
+        }
+        __syncthreads();
+        each<THREADS>(tid, [&](uint32_t x, uint32_t r) { rem[cnt16_fetch_inc(cnt, x)] = (Rem)r; });
+        __syncthreads();
+        for (uint32_t x = tid; x < S; x += THREADS) {
+            const uint32_t g0 = begin(x), g1 = end(x);
+            if (g1 - g0 < 2) continue;
+            if (g1 - g0 > BIG) {
+                small_sort(rem + g0, g1 - g0);
+                if (UNIQUE) {
+                    uint32_t k = g0 + 1;
+                    for (uint32_t i = g0 + 1; i < g1; i++)
+                        if (rem[i] != rem[k - 1]) rem[k++] = rem[i];
+                    for (; k < g1; k++) rem[k] = (Rem)STRUCK;
+                }
+            } else if (UNIQUE) {
+                for (uint32_t i = g0 + 1; i < g1; i++) {
+                    const Rem v = rem[i];
+                    for (uint32_t j = g0; j < i; j++)
+                        if (rem[j] == v) {
+                            rem[i] = (Rem)STRUCK;
+                            break;
+                        }
+                }
+            }
+        }
+        __syncthreads();
+    }
+    __device__ __forceinline__ uint32_t kept(uint32_t g0, uint32_t g1) const
+    {
+        if (!UNIQUE || g1 - g0 < 2) return g1 - g0;
+        uint32_t k = 0;
+        for (uint32_t i = g0; i < g1; i++) k += rem[i] != (Rem)STRUCK ? 1u : 0u;
+        return k;
+    }
+    __device__ __forceinline__ void sizes(uint32_t x, uint32_t (&k)[4]) const
+    {
+        uint32_t g = begin(x);
+        const uint32_t w0 = cnt[skew16(x >> 1)], w1 = cnt[skew16((x >> 1) + 1)];
+        const uint32_t e[4] = {w0 & 0xFFFFu, w0 >> 16, w1 & 0xFFFFu, w1 >> 16};
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            k[i] = kept(g, e[i]);
+            g = e[i];
+        }
+    }
+    __device__ __forceinline__ uint32_t size(uint32_t x) const { return kept(begin(x), end(x)); }
+    template <int NT, typename F>
+    __device__ __forceinline__ void each(uint32_t t, F &&f) const
+    {
+        for_each_item<NT>(a.B.items, base, n, t, [&](uint32_t v) { f((v >> R) & (S - 1), v & ((1u << R) - 1u)); });
+    }
+    template <typename Put>
+    __device__ __forceinline__ void put_item(uint32_t x, uint32_t r, uint32_t st, Put &&put) const
+    {
+        const uint32_t g0 = begin(x), g1 = end(x);
+        uint32_t less = 0, same = 1;
+        if (g1 - g0 > 1) {
+            if (g1 - g0 > BIG) return;  // put_big
+            same = 0;
+            for (uint32_t i = g0; i < g1; i++) {
+                less += rem[i] < (Rem)r ? 1u : 0u;
+                same += rem[i] == (Rem)r ? 1u : 0u;
+            }
+        }
+        for (uint32_t k = less; k < less + same; k++)
+            put(st + k, (r << 3) + 2 * min(k, 1u) + min(st + k - x, 1u));
+    }
+    template <typename Put>
+    __device__ __forceinline__ void put_run(uint32_t x, uint32_t st, Put &&put) const
+    {
+        const uint32_t g0 = begin(x), g1 = end(x);
+        const bool sorted = g1 - g0 > BIG;
+        for (uint32_t i = g0; i < g1; i++) {
+            const uint32_t r = rem[i];
+            if (UNIQUE && r == STRUCK) continue;
+            uint32_t k = i - g0;
+            if (!sorted) {
+                k = 0;
+                for (uint32_t j = g0; j < g1; j++) k += (rem[j] < (Rem)r || (rem[j] == (Rem)r && j < i)) ? 1u : 0u;
+            }
+            put(st + k, (r << 3) + 2 * min(k, 1u) + min(st + k - x, 1u));
+        }
+    }
+    // the groups put_item leaves out
+    template <int NT, typename Start, typename Put>
+    __device__ __forceinline__ void put_big(uint32_t t, Start &&start, Put &&put) const
+    {
+        for (uint32_t x = t; x < S; x += NT)
+            if (end(x) - begin(x) > BIG) put_run(x, start(x), put);
+    }
+};
+
+template <int THREADS, int QPT, class Contents>
+__device__ __forceinline__ void bucket_layout_items(const LayoutArgs &a, const uint32_t b)
 {
     extern __shared__ __align__(16) uint8_t smem_layout[];
+    constexpr int BPE = Contents::BPE;
     constexpr uint32_t S = THREADS * QPT, BUF = S + SET_SPILL, NW = THREADS / 32;
-    const SetPlan pl = set_plan(a.tb, THREADS);
-    uint8_t *s_mask = smem_layout;            // u32 at set_addr(x)
-    uint8_t *s_disp = smem_layout + pl.disp;  // displacement of quotient x's run
-    uint8_t *s_tile = smem_layout + pl.tile;  // byte i = slot x0 + i
+    constexpr ItemsPlan pl = items_plan(S, THREADS, BPE);
+    uint8_t *s_disp = smem_layout;            // displacement of quotient x's run
+    uint8_t *s_tile = smem_layout + pl.tile;  // slot x0 + i at byte BPE * i
     uint32_t *s_occ = reinterpret_cast<uint32_t *>(smem_layout + pl.occ);
     uint32_t *s_gc = reinterpret_cast<uint32_t *>(smem_layout + pl.gc);  // first free slot (from x0) at each thread's quotients
     __shared__ uint32_t s_cin, s_cout, s_nfix, s_fbase, s_naff;
@@ -130,47 +343,58 @@ __device__ __forceinline__ void bucket_layout_set(const LayoutArgs &a, const uin
     __shared__ uint32_t s_fix[256];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const uint32_t x0 = b * S, qb = tid * QPT;
-    Source<THREADS, QPT> src(a, b, smem_layout + pl.total);
+    Contents con(a, b, smem_layout + pl.contents);
+    if (!con.fits()) {  // flag it and keep the chain alive
+        if (tid == 0) {
+            atomicOr(a.err, DEV_ERR_BUCKET_CAP);
+            st_relaxed_u64(a.status + b, lb_pack_inc(x0));
+        }
+        return;
+    }
     auto fix_lost = [&]() {
         if (a.fused_fail) atomicOr(a.fused_fail, 1u);
         else if (!a.fix_soft) atomicOr(a.err, DEV_ERR_BUCKET_CAP);
     };
-    auto mask_at = [&](uint32_t x) -> uint32_t & { return *reinterpret_cast<uint32_t *>(s_mask + set_addr(x)); };
+    auto put_tile = [&](uint32_t p, uint32_t e) {
+        if (p >= BUF) return;
+        if (BPE == 1) s_tile[p] = (uint8_t)e;
+        else reinterpret_cast<uint16_t *>(s_tile)[p] = (uint16_t)__byte_perm(e, 0, 0x4401);
+    };
 
     if (tid == 0) {
         s_nfix = 0;
         s_naff = 0;
     }
-    for (uint32_t i = tid; i < S / 4; i += THREADS) reinterpret_cast<uint4 *>(s_mask)[i] = make_uint4(0, 0, 0, 0);
-    for (uint32_t i = tid; i < BUF / 16; i += THREADS) reinterpret_cast<uint4 *>(s_tile)[i] = make_uint4(0, 0, 0, 0);
+    for (uint32_t i = tid; i < BUF * BPE / 16; i += THREADS)
+        reinterpret_cast<uint4 *>(s_tile)[i] = make_uint4(0, 0, 0, 0);
     if (QPT < 32)
         for (uint32_t i = tid; i < (S + 31) / 32; i += THREADS) s_occ[i] = 0;
-    src.index(x0);
-    __syncthreads();
-    // remainder sets: the table's contents, then the batch
-    auto set_bit = [&](uint32_t x, uint32_t rem) { atomicOr(&mask_at(x), 1u << rem); };
-    src.template table_items<THREADS>(tid, set_bit);
-    src.template batch_items<THREADS>(tid, set_bit);
-    __syncthreads();
+    con.load();
 
-    // this thread's quotients: set sizes (one per byte), occupied bits, map
+    // this thread's quotients: sizes (one per byte), occupied bits, map
     uint32_t kk[QPT / 4], nz = 0;
     LayoutFn fn{0u, 0u};
     {
         int u = -1;  // entering below the first quotient
 #pragma unroll
         for (uint32_t j4 = 0; j4 < QPT / 4; j4++) {
-            const uint4 m4 = *reinterpret_cast<const uint4 *>(s_mask + set_addr(qb + 4 * j4));
-            const uint32_t k0 = __popc(m4.x), k1 = __popc(m4.y), k2 = __popc(m4.z), k3 = __popc(m4.w);
-            u = set_step(u, (int)k0);
-            u = set_step(u, (int)k1);
-            u = set_step(u, (int)k2);
-            u = set_step(u, (int)k3);
-            const uint32_t pk = k0 + (k1 << 8) + (k2 << 16) + (k3 << 24);
-            kk[j4] = pk;
-            fn.n = __dp4a(pk, 0x01010101u, fn.n);
-            const uint32_t f = ((pk + 0x7F7F7F7Fu) >> 7) & 0x01010101u;  // byte e: quotient e has items
-            nz |= ((f * 0x01020408u) >> 24 & 15u) << (4 * j4);
+            uint32_t k[4];
+            con.sizes(qb + 4 * j4, k);
+#pragma unroll
+            for (int e = 0; e < 4; e++) u = set_step(u, (int)k[e]);
+            if constexpr (Contents::SMALL) {
+                const uint32_t pk = k[0] + (k[1] << 8) + (k[2] << 16) + (k[3] << 24);
+                kk[j4] = pk;
+                fn.n = __dp4a(pk, 0x01010101u, fn.n);
+                const uint32_t f = ((pk + 0x7F7F7F7Fu) >> 7) & 0x01010101u;  // byte e: quotient e has items
+                nz |= ((f * 0x01020408u) >> 24 & 15u) << (4 * j4);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    fn.n += k[e];
+                    nz |= (k[e] ? 1u : 0u) << (4 * j4 + e);
+                }
+            }
         }
         fn.F = (uint32_t)((int)(x0 + qb + QPT) + u);
     }
@@ -218,11 +442,17 @@ __device__ __forceinline__ void bucket_layout_set(const LayoutArgs &a, const uin
         int u = (int)c - (int)(x0 + qb);
 #pragma unroll
         for (uint32_t j4 = 0; j4 < QPT / 4; j4++) {
-            uint32_t pk = 0;
+            uint32_t pk = 0, k[4];
+            if constexpr (Contents::SMALL) {
+#pragma unroll
+                for (int e = 0; e < 4; e++) k[e] = (kk[j4] >> (8 * e)) & 0xFFu;
+            } else {
+                con.sizes(qb + 4 * j4, k);
+            }
 #pragma unroll
             for (uint32_t e = 0; e < 4; e++) {
                 const int d = max(u, 0);
-                u = d + (int)((kk[j4] >> (8 * e)) & 0xFFu) - 1;
+                u = d + (int)k[e] - 1;
                 pk |= (uint32_t)min(d, (int)SET_ESCAPE) << (8 * e);
             }
             reinterpret_cast<uint32_t *>(s_disp)[(qb >> 2) + j4] = pk;
@@ -232,20 +462,14 @@ __device__ __forceinline__ void bucket_layout_set(const LayoutArgs &a, const uin
     displace(cspec);
     __syncthreads();
 
-    // slot (from x0) and byte of an item
-    auto place = [&](uint32_t x, uint32_t rem, uint32_t &e) -> uint32_t {
-        const uint32_t d = s_disp[x], set = mask_at(x);
-        const uint32_t below = __popc(set & ((1u << rem) - 1u));
-        uint32_t st = x + d;
-        if (d == SET_ESCAPE) {  // walk the thread's quotients up to x
-            const uint32_t y0 = x & ~(uint32_t)(QPT - 1);
-            int u = (int)s_gc[x / QPT] - (int)y0;
-            for (uint32_t y = y0; y < x; y++) u = set_step(u, __popc(mask_at(y)));
-            st = x + (uint32_t)max(u, 0);
-        }
-        const uint32_t p = st + below;
-        e = (rem << 3) + 2 * min(below, 1u) + min(p - x, 1u);
-        return p;
+    // first slot (from x0) of quotient x's run
+    auto start_of = [&](uint32_t x) -> uint32_t {
+        const uint32_t d = s_disp[x];
+        if (d != SET_ESCAPE) return x + d;
+        const uint32_t y0 = x & ~(uint32_t)(QPT - 1);  // walk the thread's quotients up to x
+        int u = (int)s_gc[x / QPT] - (int)y0;
+        for (uint32_t y = y0; y < x; y++) u = set_step(u, (int)con.size(y));
+        return x + (uint32_t)max(u, 0);
     };
     if (wid == 0) {
         uint32_t cin = 0;
@@ -261,13 +485,8 @@ __device__ __forceinline__ void bucket_layout_set(const LayoutArgs &a, const uin
         // every item writes its slot of the tile
         constexpr int NT = NW == 1 ? THREADS : THREADS - 32;
         const uint32_t t = NW == 1 ? tid : tid - 32;
-        auto emit = [&](uint32_t x, uint32_t rem) {
-            uint32_t e;
-            const uint32_t p = place(x, rem, e);
-            if (p < BUF) s_tile[p] = (uint8_t)e;
-        };
-        src.template table_items<NT>(t, emit);
-        src.template batch_items<NT>(t, emit);
+        con.template each<NT>(t, [&](uint32_t x, uint32_t rem) { con.put_item(x, rem, start_of(x), put_tile); });
+        con.template put_big<NT>(t, start_of, put_tile);
     }
     __syncthreads();
     const uint32_t cin = s_cin, cout = s_cout;
@@ -291,22 +510,11 @@ __device__ __forceinline__ void bucket_layout_set(const LayoutArgs &a, const uin
         const uint32_t naff = s_naff;
         // their slots end where the first unmoved thread's begin
         const uint32_t zend = naff < THREADS ? min(s_gc[naff], BUF) : BUF;
-        for (uint32_t i = tid; i < zend; i += THREADS) s_tile[i] = 0;
+        for (uint32_t i = tid; i < zend * BPE; i += THREADS) s_tile[i] = 0;
         __syncthreads();
         for (uint32_t y0 = 32 * wid; y0 < naff * QPT; y0 += THREADS) {
             const uint32_t x = y0 + lane;
-            if (x < naff * QPT) {
-                uint32_t st = x + s_disp[x], m = mask_at(x);
-                if (st - x == SET_ESCAPE) {
-                    const uint32_t z0 = x & ~(uint32_t)(QPT - 1);
-                    int u = (int)s_gc[x / QPT] - (int)z0;
-                    for (uint32_t y = z0; y < x; y++) u = set_step(u, __popc(mask_at(y)));
-                    st = x + (uint32_t)max(u, 0);
-                }
-                uint32_t f = 0;
-                for (; m; m &= m - 1u, st++, f = 2u)
-                    if (st < BUF) s_tile[st] = (uint8_t)(((__ffs(m) - 1) << 3) + f + min(st - x, 1u));
-            }
+            if (x < naff * QPT) con.put_run(x, start_of(x), put_tile);
         }
     }
     // occupied bits; those below lo (their slot was written by an earlier
@@ -331,13 +539,18 @@ __device__ __forceinline__ void bucket_layout_set(const LayoutArgs &a, const uin
     }
     if (cout > x0 + BUF) {  // spill past the tile: those items straight to the table
         __syncthreads();
-        auto spill = [&](uint32_t x, uint32_t rem) {
-            uint32_t e;
-            const uint32_t p = place(x, rem, e);
-            if (p >= BUF && p < hi_l) a.table[(size_t)x0 + p] = (uint8_t)e;  // past the table: reported as FULL
+        auto put_far = [&](uint32_t p, uint32_t e) {  // past the table: reported as FULL
+            if (p < BUF || p >= hi_l) return;
+            uint8_t *d = a.table + ((size_t)x0 + p) * BPE;
+            if (BPE == 1) {
+                d[0] = (uint8_t)e;
+            } else {
+                d[0] = (uint8_t)(e >> 8);
+                d[1] = (uint8_t)e;
+            }
         };
-        src.template table_items<THREADS>(tid, spill);
-        src.template batch_items<THREADS>(tid, spill);
+        con.template each<THREADS>(tid, [&](uint32_t x, uint32_t rem) { con.put_item(x, rem, start_of(x), put_far); });
+        con.template put_big<THREADS>(tid, start_of, put_far);
     }
     __syncthreads();
     {
@@ -352,25 +565,39 @@ __device__ __forceinline__ void bucket_layout_set(const LayoutArgs &a, const uin
             }
         }
     }
-    // store slots [lo, x0 + lim) with the occupied bits merged in: 16-byte
-    // words, bytes at a ragged start or end
-    for (uint32_t g = (lo_l & ~15u) + 16 * tid; g < lim; g += 16 * THREADS) {
-        uint4 v = *reinterpret_cast<const uint4 *>(s_tile + g);
-        const uint32_t bits = g < S ? (s_occ[g >> 5] >> (g & 16u)) & 0xFFFFu : 0u;
-        auto spread4 = [](uint32_t x4) -> uint32_t { return ((x4 * 0x00204081u) & 0x01010101u) << 2; };
-        v.x |= spread4(bits & 15u);
-        v.y |= spread4((bits >> 4) & 15u);
-        v.z |= spread4((bits >> 8) & 15u);
-        v.w |= spread4((bits >> 12) & 15u);
-        uint8_t *dst = a.table + (size_t)x0 + g;
-        if (g >= lo_l && g + 16 <= lim) {
+    // store slots [lo, x0 + lim) with the occupied bits merged in (bit 2 of a
+    // slot's last byte): 16-byte words, bytes at a ragged start or end
+    constexpr uint32_t SPW = 16 / BPE;  // slots per word
+    for (uint32_t g = (lo_l & ~(SPW - 1)) + SPW * tid; g < lim; g += SPW * THREADS) {
+        uint4 v = *reinterpret_cast<const uint4 *>(s_tile + g * BPE);
+        const uint32_t bits = g < S ? s_occ[g >> 5] >> (g & 31u) : 0u;
+        if (BPE == 1) {
+            auto spread4 = [](uint32_t x4) -> uint32_t { return ((x4 * 0x00204081u) & 0x01010101u) << 2; };
+            v.x |= spread4(bits & 15u);
+            v.y |= spread4((bits >> 4) & 15u);
+            v.z |= spread4((bits >> 8) & 15u);
+            v.w |= spread4((bits >> 12) & 15u);
+        } else {
+            auto spread2 = [](uint32_t x2) -> uint32_t { return ((x2 & 1u) << 10) | ((x2 & 2u) << 25); };
+            v.x |= spread2(bits);
+            v.y |= spread2(bits >> 2);
+            v.z |= spread2(bits >> 4);
+            v.w |= spread2(bits >> 6);
+        }
+        uint8_t *dst = a.table + ((size_t)x0 + g) * BPE;
+        if (g >= lo_l && g + SPW <= lim) {
             *reinterpret_cast<uint4 *>(dst) = v;
         } else {
             const uint32_t w[4] = {v.x, v.y, v.z, v.w};
             for (uint32_t k = 0; k < 16; k++)
-                if (g + k >= lo_l && g + k < lim) dst[k] = (uint8_t)(w[k >> 2] >> (8 * (k & 3)));
+                if (g + k / BPE >= lo_l && g + k / BPE < lim) dst[k] = (uint8_t)(w[k >> 2] >> (8 * (k & 3)));
         }
     }
+}
+template <int THREADS, int QPT, template <int, int> class Source>
+__device__ __forceinline__ void bucket_layout_set(const LayoutArgs &a, const uint32_t b)
+{
+    bucket_layout_items<THREADS, QPT, SetContents<THREADS, QPT, Source>>(a, b);
 }
 
 // ---------------------------------------------------------------------
@@ -569,7 +796,7 @@ struct TableSource {
         nb = a.B.count(b >> a.sub);
         bbase = nb ? a.B.start(b >> a.sub) : 0;
     }
-    __device__ __forceinline__ void index(uint32_t)
+    __device__ __forceinline__ void index()
     {
         __shared__ uint32_t s_w[2 * (THREADS / 32)];
         // a merge's result holds every fingerprint once whatever the tables repeat
@@ -602,7 +829,7 @@ using TwoTables = TableSource<THREADS, QPT, true>;
 
 __host__ __device__ inline size_t set_update_smem(uint32_t tb, uint32_t threads, bool two)
 {
-    return set_plan(tb, threads).total + (two ? 2 : 1) * slice_index_plan(tb).total;
+    return set_layout_smem(tb, threads) + (two ? 2 : 1) * slice_index_plan(tb).total;
 }
 
 // One CTA per bucket, taken in ticket order so every bucket's predecessors
@@ -616,6 +843,21 @@ __global__ void __launch_bounds__(THREADS, (THREADS >= 1024 ? 1 : 1024 / THREADS
     if (threadIdx.x == 0) s_ticket = atomicAdd(a.ticket, 1u);
     __syncthreads();
     bucket_layout_set<THREADS, QPT, ListSource>(a, s_ticket);
+}
+
+// A build that keeps every copy, or of two-byte slots.
+template <int THREADS, int QPT, int BPE, bool UNIQUE>
+__global__ void __launch_bounds__(THREADS, (THREADS >= 1024 ? 1 : 1024 / THREADS)) k_group_layout(LayoutArgs a)
+{
+    __shared__ uint32_t s_ticket;
+    if (threadIdx.x == 0) s_ticket = atomicAdd(a.ticket, 1u);
+    __syncthreads();
+    bucket_layout_items<THREADS, QPT, GroupContents<THREADS, QPT, BPE, UNIQUE>>(a, s_ticket);
+}
+__host__ __device__ inline size_t group_layout_smem(uint32_t tb, uint32_t threads, uint32_t bpe, size_t cap_items)
+{
+    const size_t S = (size_t)1 << tb;
+    return items_plan(S, threads, bpe).contents + GroupContents<32, 4, 1, false>::group_cnt_bytes(S) + cap_items * bpe;
 }
 
 // In-place merge and large insert: writes the live table, reads only the
