@@ -54,9 +54,8 @@ __global__ void __launch_bounds__(THREADS) k_mf_scatter(MfParams p)
     if (threadIdx.x == 0) s_f = mf_owner<&MfFilter::chunk0>(p.f, p.nf, blockIdx.x);
     __syncthreads();
     const MfFilter &f = p.f[s_f];
-    hash_bucket_chunk<THREADS, IPT, false>(blockIdx.x - f.chunk0, f.keys, f.n_keys, mf_geom(f, p.tb),
-                                           p.bbase + f.bucket0, 0xFFFFFFFFu, p.bfill + f.bucket0, p.items, nullptr,
-                                           p.err);
+    hash_bucket_chunk<THREADS, IPT>(blockIdx.x - f.chunk0, f.keys, f.n_keys, mf_geom(f, p.tb),
+                                           p.bbase + f.bucket0, 0xFFFFFFFFu, p.bfill + f.bucket0, p.items, p.err);
 }
 
 // Exclusive scan of the bucket counts of all filters.  A CTA scans one tile,

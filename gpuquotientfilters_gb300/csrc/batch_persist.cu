@@ -64,9 +64,8 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_mf_persistent(MfPara
             if (tid == 0) s_f = mf_owner<&MfFilter::pchunk0>(p.f, p.nf, u);
             __syncthreads();
             const MfFilter &f = p.f[s_f];
-            hash_bucket_chunk<THREADS, IPT, false>(u - f.pchunk0, f.keys, f.n_keys, mf_geom(f, p.tb),
-                                                   p.bbase + f.bucket0, 0xFFFFFFFFu, p.bfill + f.bucket0, p.items,
-                                                   nullptr, p.err);
+            hash_bucket_chunk<THREADS, IPT>(u - f.pchunk0, f.keys, f.n_keys, mf_geom(f, p.tb),
+                                                   p.bbase + f.bucket0, 0xFFFFFFFFu, p.bfill + f.bucket0, p.items, p.err);
         }
         if (!grid_sync(x.bar, p.err)) return;
         for (;;) {

@@ -184,6 +184,23 @@ int call_end(Arena &a, cudaStream_t s, float *ms)
     return dev_err_to_status(rep[0]);
 }
 
+int plain_begin(Arena &a, cudaStream_t s, bool timed)
+{
+    if (!arena_reserve(a, 0)) return GQF_ERR_NOMEM;
+    if (timed) GQF_CK(cudaEventRecord(a.ev0, s));
+    return GQF_OK;
+}
+
+int plain_end(Arena &a, cudaStream_t s, float *ms)
+{
+    GQF_CK(cudaGetLastError());
+    if (!ms) return GQF_OK;
+    GQF_CK(cudaEventRecord(a.ev1, s));
+    GQF_CK(cudaEventSynchronize(a.ev1));
+    GQF_CK(cudaEventElapsedTime(ms, a.ev0, a.ev1));
+    return GQF_OK;
+}
+
 }  // namespace gqf
 
 using namespace gqf;

@@ -97,6 +97,10 @@ int call_begin(Arena &a, cudaStream_t s, bool timed);
 // device error word to a status; otherwise ORs the error word into the
 // device latch for gqf_stream_status.
 int call_end(Arena &a, cudaStream_t s, float *ms);
+// The same for calls whose kernels set no error word: nothing to clear, latch
+// or read back, so a queued call is its kernels alone.
+int plain_begin(Arena &a, cudaStream_t s, bool timed);
+int plain_end(Arena &a, cudaStream_t s, float *ms);
 // Synchronous end of a step of a call: the device copies the error word
 // (and *extra, if given) into the arena's mapped host words, the host waits
 // for the stream and returns them in out[0], out[1].

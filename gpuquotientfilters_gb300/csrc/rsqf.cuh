@@ -147,18 +147,6 @@ __global__ void __launch_bounds__(RSQF_LOOKUP_THREADS) k_rsqf_lookup_unsorted(co
         out[i] = rsqf_lookup(v, q, aphash32(__ldg(keys + i)) & mask);
 }
 
-// launchLookups: queries grouped by quotient range (bucketed (fp, index)
-// pairs), results written to their input positions.
-__global__ void __launch_bounds__(RSQF_LOOKUP_THREADS) k_rsqf_lookup_bucketed(
-    const uint32_t *__restrict__ items, const uint32_t *__restrict__ idx, const uint32_t *__restrict__ base,
-    const uint32_t *__restrict__ cnt, RsqfView v, uint32_t q, int32_t *__restrict__ out)
-{
-    const uint32_t b = blockIdx.x;
-    const uint32_t n = cnt[b];
-    const size_t s0 = base[b];
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) out[idx[s0 + i]] = rsqf_lookup(v, q, items[s0 + i]);
-}
-
 // ----------------------------------------------------------------------------
 // Insert emulation.  A group is a run of blocks [glo, ghi); its thread inserts
 // the group's batch items (ascending fingerprints) with the reference's

@@ -523,16 +523,19 @@ int GQF_RSQF_API(lookup_unsorted)(const gqf_rsqf *cqf, int n, const uint32_t *d_
     Arena &ar = arena(current_device(), s);
     std::lock_guard<std::mutex> lk(ar.mu);
     const uint32_t nbl = cqf->numBlocks;
-    // one query per 16 slots pays for the mirror (the staging loads want a
-    // 16-byte aligned table, which initCQFGPU's is)
-    const bool mirror = (uint64_t)n * 16 >= (uint64_t)nbl * RSQF_SPB &&
+    // one query per 32 slots, and a million of them, pay for the mirror (2^19
+    // queries at q = 18: 20 us directly, 22 us through it; 2^21: 48 against
+    // 40; with 8-bit remainders 2^20 at q = 23: 32 against 37, 2^21: 54 against
+    // 52); the staging loads want a 16-byte aligned table, which
+    // initCQFGPU's is
+    const bool mirror = (uint64_t)n * 32 >= (uint64_t)nbl * RSQF_SPB && n >= (RSQF_R == 5 ? 1 << 20 : 3 << 19) &&
                         (reinterpret_cast<uintptr_t>(cqf->blocks) & 15u) == 0;
     uint64_t *rec = nullptr;
     if (mirror) {
         rec = static_cast<uint64_t *>(arena_reserve(ar, rmir_bytes(nbl)));
         if (!rec) return GQF_ERR_NOMEM;
     }
-    int st = call_begin(ar, s, ms != nullptr);
+    int st = plain_begin(ar, s, ms != nullptr);
     if (st) return st;
     const DeviceInfo &di = device_info(current_device());
     if (n > 0 && mirror) {
@@ -547,15 +550,15 @@ int GQF_RSQF_API(lookup_unsorted)(const gqf_rsqf *cqf, int n, const uint32_t *d_
         k_rsqf_lookup_unsorted<<<grid, RSQF_LOOKUP_THREADS, 0, s>>>(d_keys, (uint32_t)n, v, cqf->qbits, d_out);
         count_launches(1);
     }
-    return call_end(ar, s, ms);
+    return plain_end(ar, s, ms);
 }
 
-// Hash + bucketing of a batch: (items, optional idx) by bucket, counts, and
+// Hash + bucketing of a batch: items by bucket, counts, and
 // the counts' exclusive scan.  stride 0: histogram first, bucket b at base[b];
 // else one pass, bucket b at b * stride (a bucket past it sets
 // DEV_ERR_BUCKET_OVER).
 static int rsqf_bucket(const uint32_t *keys, uint32_t n, const BucketGeom &g, uint32_t stride, uint32_t *items,
-                       uint32_t *idx, uint32_t *cnt, uint32_t *base, uint32_t *err, cudaStream_t s)
+                       uint32_t *cnt, uint32_t *base, uint32_t *err, cudaStream_t s)
 {
     GQF_CK(cudaMemsetAsync(cnt, 0, g.nb * 4, s));
     // batches of up to 4M keys in 4096-key chunks, so that more than a few
@@ -577,22 +580,16 @@ static int rsqf_bucket(const uint32_t *keys, uint32_t n, const BucketGeom &g, ui
     }
     const uint32_t *at = stride ? nullptr : base;
     const uint32_t cap = stride ? stride : 0xFFFFFFFFu;
-    if (idx) {
-        auto kfn = k_hash_bucket<PAIR_THREADS, PAIR_IPT, true>;
-        size_t sm = (size_t)2 * PAIR_THREADS * PAIR_IPT * 4 + (size_t)g.nb * 8;
-        GQF_CK(set_smem(kfn, sm));
-        const uint32_t chunk = PAIR_THREADS * PAIR_IPT;
-        kfn<<<(n + chunk - 1) / chunk, PAIR_THREADS, sm, s>>>(keys, n, g, at, cap, cnt, items, idx, err);
-    } else if (small) {
-        auto kfn = k_hash_bucket<256, 16, false>;
+    if (small) {
+        auto kfn = k_hash_bucket<256, 16>;
         const size_t sm = (size_t)hchunk * 4 + (size_t)g.nb * 8;
         GQF_CK(set_smem(kfn, sm));
-        kfn<<<hgrid, 256, sm, s>>>(keys, n, g, at, cap, cnt, items, nullptr, err);
+        kfn<<<hgrid, 256, sm, s>>>(keys, n, g, at, cap, cnt, items, err);
     } else {
-        auto kfn = k_hash_bucket<SCATTER_THREADS, SCATTER_IPT, false>;
+        auto kfn = k_hash_bucket<SCATTER_THREADS, SCATTER_IPT>;
         const size_t sm = (size_t)hchunk * 4 + (size_t)g.nb * 8;
         GQF_CK(set_smem(kfn, sm));
-        kfn<<<hgrid, SCATTER_THREADS, sm, s>>>(keys, n, g, at, cap, cnt, items, nullptr, err);
+        kfn<<<hgrid, SCATTER_THREADS, sm, s>>>(keys, n, g, at, cap, cnt, items, err);
     }
     count_launches(1);
     if (stride) {
@@ -603,40 +600,13 @@ static int rsqf_bucket(const uint32_t *keys, uint32_t n, const BucketGeom &g, ui
     return GQF_OK;
 }
 
+// launchLookups: results go to the queries' input positions, so the queries are
+// probed in input order like unsorted ones (grouping them by block first took
+// 31 to 105 us where that takes 10 to 62).
 int GQF_RSQF_API(lookup_sorted)(const gqf_rsqf *cqf, int n, const uint32_t *d_keys, int32_t *d_out, void *stream,
                            float *ms)
 {
-    if (!rsqf_ok(cqf) || n < 0 || (n > 0 && (!d_keys || !d_out))) return GQF_ERR_ARG;
-    // Results go to the queries' input positions either way.  A batch of at
-    // least one query per 16 slots is answered faster by direct probes (a
-    // lookup is a rank and a select inside one or two blocks) than by grouping
-    // the queries by block first.
-    if ((uint64_t)n * 16 >= (uint64_t)cqf->numBlocks * 64)
-        return GQF_RSQF_API(lookup_unsorted)(cqf, n, d_keys, d_out, stream, ms);
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const BucketGeom g = rsqf_geom(cqf->qbits, (uint64_t)n);
-    Arena &ar = arena(current_device(), s);
-    std::lock_guard<std::mutex> lk(ar.mu);
-    Sizer z;
-    z.take<uint32_t>(g.nb);
-    z.take<uint32_t>(g.nb + 1);
-    z.take<uint32_t>(std::max(n, 1));
-    z.take<uint32_t>(std::max(n, 1));
-    void *basep = arena_reserve(ar, z.off);
-    if (!basep) return GQF_ERR_NOMEM;
-    Carver c(basep);
-    uint32_t *cnt = c.take<uint32_t>(g.nb), *base = c.take<uint32_t>(g.nb + 1);
-    uint32_t *items = c.take<uint32_t>(std::max(n, 1)), *idx = c.take<uint32_t>(std::max(n, 1));
-    int st = call_begin(ar, s, ms != nullptr);
-    if (st) return st;
-    if (n > 0) {
-        st = rsqf_bucket(d_keys, (uint32_t)n, g, 0, items, idx, cnt, base, ar.err, s);
-        if (st) return st;
-        RsqfView v{static_cast<const uint8_t *>(cqf->blocks), cqf->numBlocks};
-        k_rsqf_lookup_bucketed<<<g.nb, RSQF_LOOKUP_THREADS, 0, s>>>(items, idx, base, cnt, v, cqf->qbits, d_out);
-        count_launches(1);
-    }
-    return call_end(ar, s, ms);
+    return GQF_RSQF_API(lookup_unsorted)(cqf, n, d_keys, d_out, stream, ms);
 }
 
 // insertGPU (RSQF.cu:882-988): the batch is hashed and sorted, then applied
@@ -758,7 +728,7 @@ int GQF_RSQF_API(insert)(const gqf_rsqf *cqf, int n, const uint32_t *d_keys, int
         GQF_CK(set_smem(k_bucket_sort, sort_smem_bytes(g.tb, cap)));
         bool exact = false;
     again:
-        st = rsqf_bucket(d_keys, (uint32_t)n, g, exact ? 0 : stride, raw, nullptr, cnt, base, ar.err, s);
+        st = rsqf_bucket(d_keys, (uint32_t)n, g, exact ? 0 : stride, raw, cnt, base, ar.err, s);
         if (st) return st;
         k_bucket_sort<<<g.nb, SORT_THREADS, sort_smem_bytes(g.tb, cap1), s>>>(
             raw, exact ? base : nullptr, stride, base, cnt, g.tb, 0u, cap1, cap1 == cap, items, ar.err, bmax);

@@ -59,8 +59,7 @@ struct LayoutPlan {
 // per bucket (one CTA sorts a bucket in shared memory), at most 4096 buckets
 // (the scatter keeps two u32 per bucket in shared memory).  `spread`: also at
 // least 512 buckets (of 256 quotients or more), so a small filter's layout
-// uses every SM; its buckets cost little beyond their items.  (A bucketed
-// lookup stages spill slots with each bucket, so it keeps the large ones.)
+// uses every SM; its buckets cost little beyond their items.
 // `general`: k_bucket_layout may run.
 static LayoutPlan plan_layout(uint32_t q, uint32_t r, uint64_t n_expect, uint64_t n_b_expect, bool general,
                               bool spread)
@@ -107,12 +106,6 @@ static LayoutPlan plan_layout(uint32_t q, uint32_t r, uint64_t n_expect, uint64_
 // give less than 512 buckets, down to 1024.
 static uint32_t update_tb(uint32_t q) { return std::min<uint32_t>(q, std::min<uint32_t>(13, std::max<uint32_t>(10, q > 9 ? q - 9 : 0))); }
 
-static size_t scatter_smem(uint32_t nb, bool pairs)
-{
-    size_t chunk = pairs ? (size_t)PAIR_THREADS * PAIR_IPT : (size_t)SCATTER_THREADS * SCATTER_IPT;
-    return (pairs ? 2 : 1) * chunk * 4 + (size_t)nb * 8;
-}
-
 template <typename K>
 static cudaError_t set_smem(K kernel, size_t bytes)
 {
@@ -154,7 +147,6 @@ struct Scratch {
     uint32_t *fix_list;
     uint32_t fix_cap;
     uint32_t *bitems;  // batch fingerprints
-    uint32_t *bidx;    // batch indices (sorted lookups)
     void *rems;        // k_group_layout: remainders of large buckets
     // extracted table contents
     Counts3 *tiles;
@@ -166,7 +158,6 @@ struct Scratch {
 struct ScratchReq {
     uint32_t nb;
     size_t batch_items;  // capacity of the bucketed batch
-    bool pairs;
     bool extract;   // table contents needed
     bool extract2;  // second table (merge)
     uint32_t nslots;
@@ -192,7 +183,6 @@ static Scratch carve(void *base, const ScratchReq &r, bool sizing_only, size_t *
         s.fix_cap = std::max<uint32_t>(65536u, r.every_fix ? r.nslots : r.nslots / 8);
         s.fix_list = c.template take<uint32_t>(s.fix_cap);
         s.bitems = c.template take<uint32_t>(std::max<size_t>(r.batch_items, 1));
-        s.bidx = r.pairs ? c.template take<uint32_t>(std::max<size_t>(r.batch_items, 1)) : nullptr;
         s.rems = r.rem_bytes ? c.template take<uint8_t>(std::max<size_t>(r.batch_items, 1) * r.rem_bytes) : nullptr;
         if (r.extract) {
             size_t ntiles = (r.nslots + EXTRACT_TILE - 1) / EXTRACT_TILE;
@@ -262,41 +252,21 @@ static int bucket_batch_keys(const uint32_t *keys, uint32_t n, const LayoutPlan 
         GQF_CK(cudaMemsetAsync(sc.bcnt, 0, p.g.nb * 4, s));
     }
     count_launches(1);
-    auto kfn = k_hash_bucket<T, IPT, false>;
+    auto kfn = k_hash_bucket<T, IPT>;
     const size_t sm = (size_t)T * IPT * 4 + (size_t)p.g.nb * 8;
     GQF_CK(set_smem(kfn, sm));
     kfn<<<grid, T, sm, s>>>(keys, n, p.g, exact ? sc.bbase : nullptr, exact ? 0xFFFFFFFFu : p.stride, sc.bcnt,
-                            sc.bitems, nullptr, err);
+                            sc.bitems, err);
     GQF_CK(cudaGetLastError());
     return GQF_OK;
 }
 
-static int bucket_batch(const uint32_t *keys, uint32_t n, const LayoutPlan &p, Scratch &sc, bool exact, bool pairs,
-                        uint32_t *err, cudaStream_t s)
+static int bucket_batch(const uint32_t *keys, uint32_t n, const LayoutPlan &p, Scratch &sc, bool exact, uint32_t *err,
+                        cudaStream_t s)
 {
     if (n == 0) return GQF_OK;
-    if (!pairs) {
-        return n <= SMALL_BATCH ? bucket_batch_keys<SMALL_THREADS, SMALL_IPT>(keys, n, p, sc, exact, err, s)
-                                : bucket_batch_keys<SCATTER_THREADS, SCATTER_IPT>(keys, n, p, sc, exact, err, s);
-    }
-    const uint32_t chunk = PAIR_THREADS * PAIR_IPT;
-    const uint32_t grid = (n + chunk - 1) / chunk;
-    const size_t sm = scatter_smem(p.g.nb, pairs);
-    if (exact) {
-        count_launches(2);
-        GQF_CK(set_smem(k_bucket_hist<SCATTER_THREADS, SCATTER_IPT>, p.g.nb * 4));
-        const uint32_t hgrid = (n + SCATTER_THREADS * SCATTER_IPT - 1) / (SCATTER_THREADS * SCATTER_IPT);
-        k_bucket_hist<SCATTER_THREADS, SCATTER_IPT><<<hgrid, SCATTER_THREADS, p.g.nb * 4, s>>>(keys, n, p.g, sc.bcnt);
-        k_scan_bases<<<1, 1024, 0, s>>>(sc.bcnt, p.g.nb, sc.bbase);
-        GQF_CK(cudaMemsetAsync(sc.bcnt, 0, p.g.nb * 4, s));
-    }
-    count_launches(1);
-    auto kfn = k_hash_bucket<PAIR_THREADS, PAIR_IPT, true>;
-    GQF_CK(set_smem(kfn, sm));
-    kfn<<<grid, PAIR_THREADS, sm, s>>>(keys, n, p.g, exact ? sc.bbase : nullptr, exact ? 0xFFFFFFFFu : p.stride,
-                                       sc.bcnt, sc.bitems, sc.bidx, err);
-    GQF_CK(cudaGetLastError());
-    return GQF_OK;
+    return n <= SMALL_BATCH ? bucket_batch_keys<SMALL_THREADS, SMALL_IPT>(keys, n, p, sc, exact, err, s)
+                            : bucket_batch_keys<SCATTER_THREADS, SCATTER_IPT>(keys, n, p, sc, exact, err, s);
 }
 
 template <int BPE>
@@ -483,7 +453,7 @@ static size_t update_scratch_bytes(uint32_t q, uint32_t r, uint32_t n)
     const uint32_t nslots = gqf_sqf_num_slots(q);
     const uint64_t expect = std::min<uint64_t>((uint64_t)(nslots * 0.9) + n, (uint64_t)nslots * 2);
     LayoutPlan p = plan_layout(q, r, expect, n, true, false);
-    ScratchReq req{p.g.nb, (size_t)p.g.nb * p.stride, false, true, false, nslots};
+    ScratchReq req{p.g.nb, (size_t)p.g.nb * p.stride, true, false, nslots};
     size_t bytes = 0, bytes_exact = 0;
     carve(nullptr, req, true, &bytes);
     req.batch_items = std::max<size_t>(n, 1);
@@ -519,7 +489,7 @@ static int rebuild(const gqf_sqf *qf, const gqf_sqf *qf2, const uint32_t *keys, 
     // an update's batch keeps the large buckets (a layout bucket reads its
     // part of one); a build's are the layout's
     LayoutPlan p = plan_layout(tg.q, tg.r, expect, bFromTable ? 0 : n, (!set_ok && op != OP_BUILD) || update, !fused);
-    ScratchReq req{p.g.nb, bFromTable ? 0 : (size_t)p.g.nb * p.stride, false, needA, bFromTable, tg.nslots};
+    ScratchReq req{p.g.nb, bFromTable ? 0 : (size_t)p.g.nb * p.stride, needA, bFromTable, tg.nslots};
     // small filters are laid out in small buckets, which a nearly full table's
     // spill can pass whole
     req.every_fix = tg.q <= 22;
@@ -562,7 +532,7 @@ static int rebuild(const gqf_sqf *qf, const gqf_sqf *qf2, const uint32_t *keys, 
         GQF_CK(cudaMemsetAsync(sc.bcnt, 0, sc.ctrl_bytes, s));
         BucketSrc A{nullptr, nullptr, 0, nullptr}, B{nullptr, nullptr, 0, nullptr};
         if (n) {
-            st = bucket_batch(keys, n, p, sc, true, false, ar.err, s);
+            st = bucket_batch(keys, n, p, sc, true, ar.err, s);
             if (st) return st;
             B = BucketSrc{sc.bitems, sc.bbase, 0, sc.bcnt};
         }
@@ -630,7 +600,7 @@ static int rebuild(const gqf_sqf *qf, const gqf_sqf *qf2, const uint32_t *keys, 
             if (st) return st;
             B = BucketSrc{sc.E2, sc.a2base, 0, sc.a2cnt};
         } else if (n) {
-            st = bucket_batch(keys, n, p, sc, exact, false, ar.err, s);
+            st = bucket_batch(keys, n, p, sc, exact, ar.err, s);
             if (st) return st;
             B = exact ? BucketSrc{sc.bitems, sc.bbase, 0, sc.bcnt} : BucketSrc{sc.bitems, nullptr, p.stride, sc.bcnt};
         }
@@ -792,88 +762,52 @@ static int local_update(const gqf_sqf *qf, const uint32_t *keys, uint32_t n, int
     return call_end(ar, s, ms);
 }
 
+// Sorted and unsorted lookups alike: results go to the queries' input positions
+// either way (the reference sorts them back by index, quotientFilter.cu:
+// 304-305), and probing the table in input order was faster than bucketing
+// the queries first at every size (2^18 queries: 20 against 52 us at q = 22,
+// 19 against 127 us at q = 26).
 template <int BPE>
-static int lookup_unsorted_t(const gqf_sqf *qf, int n, const uint32_t *keys, uint32_t *out, cudaStream_t s, float *ms)
+static int lookup_t(const gqf_sqf *qf, int n, const uint32_t *keys, uint32_t *out, cudaStream_t s, float *ms)
 {
     const SqfGeom tg = geom_of(qf);
     Arena &ar = arena(current_device(), s);
     std::lock_guard<std::mutex> lk(ar.mu);
-    // one-byte slots and a batch of at least one query per 16 slots: transpose
-    // the table into the bit-plane mirror first
-    const bool mirror = BPE == 1 && (uint64_t)n * 16 >= tg.nslots;
-    uint4 *rec = nullptr;
-    if (mirror) {
-        rec = static_cast<uint4 *>(arena_reserve(ar, mir_bytes(tg.nslots)));
-        if (!rec) return GQF_ERR_NOMEM;
-        GQF_CK(set_smem(k_sqf_mirror, 2 * (size_t)MIR_TILE));
-    }
-    int st = call_begin(ar, s, ms != nullptr);
-    if (st) return st;
-    TableView v{qf->table, tg.q, tg.r, tg.nslots, (uint32_t)tg.T, (uint32_t)(tg.T / 8)};
-    if (n > 0 && mirror) {
-        const DeviceInfo &di = device_info(current_device());
-        const uint32_t ngroups = mir_groups(tg.nslots);
-        const uint32_t ntiles = (uint32_t)(((uint64_t)(ngroups + 1) * MIR_SLOTS + MIR_TILE - 1) / MIR_TILE);
-        k_sqf_mirror<<<std::min<uint32_t>(ntiles, (uint32_t)di.sms * 3), MIR_BUILD_THREADS, 2 * MIR_TILE, s>>>(
-            v, rec, ngroups, ntiles, ar.err);
-        const uint32_t grid = std::min<uint32_t>((n + MIR_LOOKUP_THREADS - 1) / MIR_LOOKUP_THREADS,
-                                                 (uint32_t)di.sms * 32);
-        k_lookup_mirror<<<grid, MIR_LOOKUP_THREADS, 0, s>>>(keys, (uint32_t)n, v, rec, out);
-        count_launches(2);
-    } else if (n > 0) {
-        const DeviceInfo &di = device_info(current_device());
-        // one or two queries per thread: more threads in flight beat more
-        // loads per thread for the dependent walks
-        constexpr int QPT = BPE == 1 ? 2 : 1;
-        const uint32_t per_block = LOOKUP_THREADS * QPT;
-        const uint32_t grid = std::min<uint32_t>((n + per_block - 1) / per_block, (uint32_t)di.sms * 32);
-        k_lookup_unsorted<BPE, QPT><<<grid, LOOKUP_THREADS, 0, s>>>(keys, (uint32_t)n, v, out);
-        count_launches(1);
-    }
-    return call_end(ar, s, ms);
-}
-
-template <int BPE>
-static int lookup_sorted_t(const gqf_sqf *qf, int n, const uint32_t *keys, uint32_t *out, cudaStream_t s, float *ms)
-{
-    const SqfGeom tg = geom_of(qf);
-    // Results go to the queries' input positions either way (the reference
-    // sorts them back by index, quotientFilter.cu:304-305).  On one-byte slots
-    // a batch of at least one query per 16 slots is answered faster through
-    // the bit-plane mirror than by bucketing the queries first.
-    if (BPE == 1 && (uint64_t)n * 16 >= tg.nslots) return lookup_unsorted_t<BPE>(qf, n, keys, out, s, ms);
-    LayoutPlan p = plan_layout(tg.q, tg.r, (uint64_t)tg.nslots * 8 / 10, (uint64_t)n, false, false);
-    // query buckets: aim for ~4k queries per bucket, table-aligned
-    ScratchReq req{p.g.nb, (size_t)std::max(n, 1), true, false, false, tg.nslots};
-    Arena &ar = arena(current_device(), s);
-    std::lock_guard<std::mutex> lk(ar.mu);
-    size_t bytes = 0;
-    carve(nullptr, req, true, &bytes);
-    void *base = arena_reserve(ar, bytes);
-    if (!base) return GQF_ERR_NOMEM;
-    Scratch sc = carve(base, req, false, &bytes);
-    int st = call_begin(ar, s, ms != nullptr);
-    if (st) return st;
-    if (n > 0) {
-        GQF_CK(cudaMemsetAsync(sc.bcnt, 0, sc.ctrl_bytes, s));
-        st = bucket_batch(keys, (uint32_t)n, p, sc, true, true, ar.err, s);
+    // One-byte slots: transposing the table into the bit-plane mirror first
+    // pays from one query per 32 slots and 768K queries on (2^19 queries: 26
+    // us directly, 26 to 29 us through the mirror for q = 15 to 22; 2^20: 37
+    // against 32 us).
+    const bool mirror = BPE == 1 && (uint64_t)n * 32 >= tg.nslots && n >= (3 << 18);
+    const TableView v{qf->table, tg.q, tg.r, tg.nslots, (uint32_t)tg.T, (uint32_t)(tg.T / 8)};
+    const DeviceInfo &di = device_info(current_device());
+    if (!mirror) {
+        const int st = plain_begin(ar, s, ms != nullptr);
         if (st) return st;
-        TableView v{qf->table, tg.q, tg.r, tg.nslots, (uint32_t)tg.T, (uint32_t)(tg.T / 8)};
-        BucketSrc src{sc.bitems, sc.bbase, 0, sc.bcnt};
-        const size_t lsm = lks_smem_bytes(p.g.tb);
-        const DeviceInfo &di = device_info(current_device());
-        if (BPE == 1 && (reinterpret_cast<uintptr_t>(qf->table) & 15) == 0 && p.g.tb >= 8 &&
-            lsm <= (size_t)(di.smem_optin > 0 ? di.smem_optin : 48 * 1024)) {
-            GQF_CK(set_smem(k_lookup_bucketed_s, lsm));
-            k_lookup_bucketed_s<<<p.g.nb, LKS_THREADS, lsm, s>>>(src, sc.bidx, v, p.g.tb, out);
-        } else {
-            k_lookup_bucketed<BPE><<<p.g.nb, LOOKUP_THREADS, 0, s>>>(src, sc.bidx, v, out);
+        if (n > 0) {
+            // one or two queries per thread: more threads in flight beat more
+            // loads per thread for the dependent walks
+            constexpr int QPT = BPE == 1 ? 2 : 1;
+            const uint32_t per_block = LOOKUP_THREADS * QPT;
+            const uint32_t grid = std::min<uint32_t>((n + per_block - 1) / per_block, (uint32_t)di.sms * 32);
+            k_lookup_unsorted<BPE, QPT><<<grid, LOOKUP_THREADS, 0, s>>>(keys, (uint32_t)n, v, out);
+            count_launches(1);
         }
-        count_launches(1);
+        return plain_end(ar, s, ms);
     }
+    uint4 *rec = static_cast<uint4 *>(arena_reserve(ar, mir_bytes(tg.nslots)));
+    if (!rec) return GQF_ERR_NOMEM;
+    GQF_CK(set_smem(k_sqf_mirror, 2 * (size_t)MIR_TILE));
+    const int st = call_begin(ar, s, ms != nullptr);
+    if (st) return st;
+    const uint32_t ngroups = mir_groups(tg.nslots);
+    const uint32_t ntiles = (uint32_t)(((uint64_t)(ngroups + 1) * MIR_SLOTS + MIR_TILE - 1) / MIR_TILE);
+    k_sqf_mirror<<<std::min<uint32_t>(ntiles, (uint32_t)di.sms * 3), MIR_BUILD_THREADS, 2 * MIR_TILE, s>>>(
+        v, rec, ngroups, ntiles, ar.err);
+    const uint32_t grid = std::min<uint32_t>((n + MIR_LOOKUP_THREADS - 1) / MIR_LOOKUP_THREADS, (uint32_t)di.sms * 32);
+    k_lookup_mirror<<<grid, MIR_LOOKUP_THREADS, 0, s>>>(keys, (uint32_t)n, v, rec, out);
+    count_launches(2);
     return call_end(ar, s, ms);
 }
-
 
 // ------------------------------------------------ no-allocation bulk build
 // Scratch for gqf_sqf_bulk_build_noalloc: a fixed array in the library's
@@ -908,7 +842,7 @@ static int bulk_build_noalloc_t(const gqf_sqf *qf, uint32_t n, const uint32_t *k
     const SqfGeom tg = geom_of(qf);
     const bool set_ok = tg.r == 5 && nodup;
     LayoutPlan p = plan_layout(tg.q, tg.r, n, n, false, false);  // few buckets: the fix-up list is small
-    ScratchReq req{p.g.nb, std::max<size_t>(n, 1), false, false, false, tg.nslots};
+    ScratchReq req{p.g.nb, std::max<size_t>(n, 1), false, false, tg.nslots};
     if (!set_ok) req.rem_bytes = BPE;
     size_t need = 0;
     carve(nullptr, req, true, &need);
@@ -922,7 +856,7 @@ static int bulk_build_noalloc_t(const gqf_sqf *qf, uint32_t n, const uint32_t *k
     GQF_CK(cudaMemsetAsync(sc.bcnt, 0, sc.ctrl_bytes, s));
     BucketSrc A{nullptr, nullptr, 0, nullptr}, B{nullptr, nullptr, 0, nullptr};
     if (n) {
-        int st = bucket_batch(keys, n, p, sc, true, false, err, s);
+        int st = bucket_batch(keys, n, p, sc, true, err, s);
         if (st) return st;
         B = BucketSrc{sc.bitems, sc.bbase, 0, sc.bcnt};
     }
@@ -1049,13 +983,13 @@ int gqf_sqf_merge(const gqf_sqf *qf1, const gqf_sqf *qf2, int no_duplicates, voi
 int gqf_sqf_lookup_unsorted(const gqf_sqf *qf, int n, const uint32_t *d_keys, uint32_t *d_out, void *stream, float *ms)
 {
     if (!sqf_ok(qf) || n < 0 || (n > 0 && (!d_keys || !d_out))) return GQF_ERR_ARG;
-    return BPE_DISPATCH(qf, lookup_unsorted_t, qf, n, d_keys, d_out, static_cast<cudaStream_t>(stream), ms);
+    return BPE_DISPATCH(qf, lookup_t, qf, n, d_keys, d_out, static_cast<cudaStream_t>(stream), ms);
 }
 
 int gqf_sqf_lookup_sorted(const gqf_sqf *qf, int n, const uint32_t *d_keys, uint32_t *d_out, void *stream, float *ms)
 {
     if (!sqf_ok(qf) || n < 0 || (n > 0 && (!d_keys || !d_out))) return GQF_ERR_ARG;
-    return BPE_DISPATCH(qf, lookup_sorted_t, qf, n, d_keys, d_out, static_cast<cudaStream_t>(stream), ms);
+    return BPE_DISPATCH(qf, lookup_t, qf, n, d_keys, d_out, static_cast<cudaStream_t>(stream), ms);
 }
 
 int gqf_debug_lookback_probe(const unsigned long long *status, unsigned int nb, unsigned int spin_limit,

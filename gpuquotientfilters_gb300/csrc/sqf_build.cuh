@@ -34,14 +34,10 @@ struct BucketGeom {
     uint32_t fp_mask;       // (1 << (q + r)) - 1
 };
 
-// Scatter CTA shapes: fingerprints only (build, insert, delete) take 32K
-// keys per CTA, halving the per-(CTA, bucket) global reservations; pairs
-// (sorted lookups) carry an index per key and take 16K.
+// Scatter CTA shape: 32K keys, halving the per-(CTA, bucket) global
+// reservations of 16K.
 constexpr int SCATTER_THREADS = 1024;
 constexpr int SCATTER_IPT = 32;
-constexpr int PAIR_THREADS = 512;
-constexpr int PAIR_IPT = 32;
-constexpr int LAYOUT_THREADS = 512;
 constexpr uint32_t SPILL_SLOTS = 4096;  // tile buffer headroom past the bucket
 constexpr uint32_t SPIN_LIMIT = 1u << 22;
 
@@ -93,21 +89,17 @@ __device__ uint32_t block_exclusive_scan_u32(uint32_t *cnt, uint32_t nvals, uint
 // speculative mode (bucket_base == nullptr); a bucket that would exceed cap
 // sets DEV_ERR_BUCKET_OVER and the host reruns with exact bases.
 // Dynamic smem: items[THREADS*IPT] + cursor[nb] + gbase[nb] (u32).
-// With `vals` non-null the kernel scatters (fingerprint, index) pairs: the
-// pair payload is the key's position in the input (sorted lookups).
 // ---------------------------------------------------------------------
-template <int THREADS, int IPT, bool PAIRS>
+template <int THREADS, int IPT>
 __device__ __forceinline__ void hash_bucket_chunk(
     uint32_t chunk, const uint32_t *__restrict__ keys, uint32_t n, const BucketGeom &g,
     const uint32_t *__restrict__ bucket_base, uint32_t cap,
-    uint32_t *__restrict__ bucket_cnt, uint32_t *__restrict__ out,
-    uint32_t *__restrict__ out_idx, uint32_t *__restrict__ err)
+    uint32_t *__restrict__ bucket_cnt, uint32_t *__restrict__ out, uint32_t *__restrict__ err)
 {
     extern __shared__ __align__(16) uint32_t smem_scatter[];
     constexpr uint32_t CHUNK = THREADS * IPT;
     uint32_t *s_items = smem_scatter;
-    uint32_t *s_idx = s_items + CHUNK;  // only when PAIRS
-    uint32_t *s_cur = s_items + (PAIRS ? 2 * CHUNK : CHUNK);
+    uint32_t *s_cur = s_items + CHUNK;
     uint32_t *s_gb = s_cur + g.nb;
     __shared__ uint32_t s_warp[33];
     const int tid = threadIdx.x;
@@ -181,7 +173,6 @@ __device__ __forceinline__ void hash_bucket_chunk(
         if (j < cnt) {
             uint32_t p = atomicAdd(&s_cur[fp[k] >> g.shift], 1u);
             s_items[p] = fp[k];
-            if (PAIRS) s_idx[p] = (uint32_t)(c0 + j);
         }
     }
     __syncthreads();
@@ -216,23 +207,20 @@ __device__ __forceinline__ void hash_bucket_chunk(
         const uint32_t b = v >> g.shift;
         const uint2 dlim = reinterpret_cast<const uint2 *>(s_cur)[b];
         if (i < dlim.y) {
-            const uint32_t dst = i + dlim.x;
-            out[dst] = v;
-            if (PAIRS) out_idx[dst] = s_idx[i];
+            out[i + dlim.x] = v;
         } else {
             atomicOr(err, DEV_ERR_BUCKET_OVER);
         }
     }
 }
 
-template <int THREADS, int IPT, bool PAIRS>
+template <int THREADS, int IPT>
 __global__ void __launch_bounds__(THREADS) k_hash_bucket(
     const uint32_t *__restrict__ keys, uint32_t n, BucketGeom g,
     const uint32_t *__restrict__ bucket_base, uint32_t cap,
-    uint32_t *__restrict__ bucket_cnt, uint32_t *__restrict__ out,
-    uint32_t *__restrict__ out_idx, uint32_t *__restrict__ err)
+    uint32_t *__restrict__ bucket_cnt, uint32_t *__restrict__ out, uint32_t *__restrict__ err)
 {
-    hash_bucket_chunk<THREADS, IPT, PAIRS>(blockIdx.x, keys, n, g, bucket_base, cap, bucket_cnt, out, out_idx, err);
+    hash_bucket_chunk<THREADS, IPT>(blockIdx.x, keys, n, g, bucket_base, cap, bucket_cnt, out, err);
 }
 
 // Histogram-only pass for exact bucket bases (used when a speculative

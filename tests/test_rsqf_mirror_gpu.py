@@ -1,5 +1,5 @@
-"""RSQF lookups through the aligned mirror (batches of at least one query per
-16 slots): the oracle's answers on regular and irregular tables (incremental
+"""RSQF lookups through the aligned mirror (batches of a million queries and
+more, here the same ones over and over): the oracle's answers on regular and irregular tables (incremental
 batches, spills over several blocks, a nearly full filter, the last blocks),
 and the same as the direct lookups of small batches."""
 import numpy as np
@@ -32,6 +32,8 @@ def test_mirror_lookups(gqf, cuda, q, alpha, batches, hot, rbits):
         assert np.array_equal(gqf.rsqf_blocks_bytes(f), o)
         look = np.concatenate([keys, O.mt_keys(602 + q, max(keys.size, 64))])
         want = O.rsqf_lookup(o, q, look, rbits)
+        reps = -(-(3 << 19) // look.size)
+        look, want = np.tile(look, reps), np.tile(want, reps)
         for op in (gqf.launchLookups, gqf.launchUnsortedLookupsRSQF):
             out = cuda.empty(look.size, dtype=cuda.int32, device="cuda")
             op(f, look.size, to_dev(cuda, look), out)
