@@ -10,6 +10,8 @@
 
 namespace gqf {
 
+constexpr uint32_t SPIN_LIMIT = 1u << 22;  // passes of a bounded wait
+
 // Device error word bits (latched per stream by the host layer).
 enum : uint32_t {
     DEV_ERR_FULL = 1u,          // a layout ran past (1<<q)*1.1 slots

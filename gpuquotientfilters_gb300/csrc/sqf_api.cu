@@ -57,9 +57,11 @@ struct LayoutPlan {
 
 // Bucket geometry for `n_expect` items over 2^q quotients: about 12k items
 // per bucket (one CTA sorts a bucket in shared memory), at most 4096 buckets
-// (the scatter keeps two u32 per bucket in shared memory).  `spread`: also at
-// least 512 buckets (of 256 quotients or more), so a small filter's layout
-// uses every SM; its buckets cost little beyond their items.
+// (the scatter keeps two u32 per bucket in shared memory).  `spread`: also
+// enough buckets (of 256 quotients or more) that a small filter's layout uses
+// every SM: 512 from q = 21 on, 256 below, where a launch and the look-back
+// count for more (NoDup build, 512 against 256 buckets: q = 17 0.061 and
+// 0.057 ms, q = 19 0.061 and 0.058, q = 21 0.058 and 0.060).
 // `general`: k_bucket_layout may run.
 static LayoutPlan plan_layout(uint32_t q, uint32_t r, uint64_t n_expect, uint64_t n_b_expect, bool general,
                               bool spread)
@@ -68,7 +70,8 @@ static LayoutPlan plan_layout(uint32_t q, uint32_t r, uint64_t n_expect, uint64_
     LayoutPlan p;
     uint32_t tb_lo = std::max<uint32_t>(7, q > 12 ? q - 12 : 0);
     uint32_t tb_hi = std::min<uint32_t>(q, 15);
-    if (spread) tb_hi = std::min(tb_hi, std::max<uint32_t>(q > 9 ? q - 9 : 0, std::min<uint32_t>(q, 8)));
+    const uint32_t lg_spread = q >= 21 ? 9 : 8;
+    if (spread) tb_hi = std::min(tb_hi, std::max<uint32_t>(q > lg_spread ? q - lg_spread : 0, std::min<uint32_t>(q, 8)));
     uint64_t denom = n_expect ? n_expect : 1;
     uint32_t tb = ceil_log2((12000ull << q) / denom);
     tb = std::min(std::max(tb, tb_lo), tb_hi);
@@ -183,7 +186,10 @@ static Scratch carve(void *base, const ScratchReq &r, bool sizing_only, size_t *
         s.fix_cap = std::max<uint32_t>(65536u, r.every_fix ? r.nslots : r.nslots / 8);
         s.fix_list = c.template take<uint32_t>(s.fix_cap);
         s.bitems = c.template take<uint32_t>(std::max<size_t>(r.batch_items, 1));
-        s.rems = r.rem_bytes ? c.template take<uint8_t>(std::max<size_t>(r.batch_items, 1) * r.rem_bytes) : nullptr;
+        s.rems = r.rem_bytes ? c.template take<uint8_t>((std::max<size_t>(r.batch_items, 1) +
+                                                         (r.extract ? r.nslots : 0) + (r.extract2 ? r.nslots : 0)) *
+                                                        r.rem_bytes)
+                             : nullptr;
         if (r.extract) {
             size_t ntiles = (r.nslots + EXTRACT_TILE - 1) / EXTRACT_TILE;
             s.tiles = c.template take<Counts3>(ntiles + 1);
@@ -321,7 +327,7 @@ static int launch_layout(const LayoutPlan &p, const SqfGeom &tg, uint8_t *table,
         GQF_CK(e);
         count_launches(1);
     }
-    if (op == OP_BUILD && !set_ok) {
+    if ((op == OP_BUILD || op == OP_MERGE) && !set_ok) {
         // shared memory for a third more than the average bucket; a larger
         // one keeps its remainders in the scratch
         a.rem_scratch = sc.rems;
@@ -488,12 +494,12 @@ static int rebuild(const gqf_sqf *qf, const gqf_sqf *qf2, const uint32_t *keys, 
     const bool fused = BPE == 1 && set_ok && needA;
     // an update's batch keeps the large buckets (a layout bucket reads its
     // part of one); a build's are the layout's
-    LayoutPlan p = plan_layout(tg.q, tg.r, expect, bFromTable ? 0 : n, (!set_ok && op != OP_BUILD) || update, !fused);
+    LayoutPlan p = plan_layout(tg.q, tg.r, expect, bFromTable ? 0 : n, op == OP_INSERT, !fused);
     ScratchReq req{p.g.nb, bFromTable ? 0 : (size_t)p.g.nb * p.stride, needA, bFromTable, tg.nslots};
     // small filters are laid out in small buckets, which a nearly full table's
     // spill can pass whole
     req.every_fix = tg.q <= 22;
-    if (op == OP_BUILD && !set_ok) req.rem_bytes = BPE;
+    if ((op == OP_BUILD || op == OP_MERGE) && !set_ok) req.rem_bytes = BPE;
     int dev = current_device();
     Arena &ar = arena(dev, s);
     std::lock_guard<std::mutex> lk(ar.mu);

@@ -12,13 +12,16 @@
 //                   CTA-local counting sort by bucket (bucket = the top
 //                   q - tb quotient bits) and coalesced runs into per-bucket
 //                   regions (one global atomic per CTA and bucket).
-//   k_bucket_layout one CTA per bucket (2^tb quotients): counting sort by
-//                   quotient in shared memory, tiny per-quotient remainder
-//                   sorts, then the slot recurrence as a block scan of
-//                   c -> max(c + n, F) maps, chained across buckets with a
-//                   decoupled look-back; every slot of the bucket's write
-//                   range is produced in shared memory and stored once with
-//                   16-byte stores (no read-modify-write of the table).
+//   k_set_layout, k_group_layout (sqf_set.cuh)
+//                   one CTA per bucket (2^tb quotients): the slot recurrence
+//                   as a block scan of c -> max(c + n, F) maps, chained
+//                   across buckets with a decoupled look-back; every item
+//                   then writes its own slot of the bucket's range in shared
+//                   memory, stored once with 16-byte stores (no
+//                   read-modify-write of the table).
+//   k_bucket_layout the general form with two sources (updates that fall
+//                   back): counting sort by quotient, a thread per stretch
+//                   of quotients.
 //   k_fixup_occ     occupied bits of quotients whose slot was written by an
 //                   earlier bucket (the spill of a cluster that crosses a
 //                   bucket boundary).
@@ -34,12 +37,13 @@ struct BucketGeom {
     uint32_t fp_mask;       // (1 << (q + r)) - 1
 };
 
-// Scatter CTA shape: 32K keys, halving the per-(CTA, bucket) global
-// reservations of 16K.
-constexpr int SCATTER_THREADS = 1024;
+// Scatter CTA shape: 16K keys, two CTAs per SM, so that one's barriers and
+// loads overlap the other's work (32K keys in one CTA halve the global
+// reservations but took 1 to 6% longer: dup build at q = 24 0.283 against
+// 0.266 ms).
+constexpr int SCATTER_THREADS = 512;
 constexpr int SCATTER_IPT = 32;
 constexpr uint32_t SPILL_SLOTS = 4096;  // tile buffer headroom past the bucket
-constexpr uint32_t SPIN_LIMIT = 1u << 22;
 
 // Exclusive scan of `cnt` (nvals entries of u32 in shared memory) in place,
 // by a block of THREADS threads; returns the total.  Each thread owns a
@@ -445,7 +449,7 @@ struct LayoutArgs {
     // bucket that cannot be decoded (duplicate or out-of-order remainders in
     // an insert or delete, runs past its slice) sets *fused_fail and the op
     // is done the general way.
-    void *rem_scratch = nullptr;  // k_group_layout: a remainder per item of B, for buckets past cap_items
+    void *rem_scratch = nullptr;  // k_group_layout: a remainder per item of A and B, for buckets past cap_items
     const uint8_t *src_table = nullptr, *src2 = nullptr;
     uint32_t sub = 0;
     uint32_t *fused_fail = nullptr;

@@ -1,8 +1,8 @@
 // Item-parallel bucket layouts.  One-byte slots with no fingerprint stored
 // twice (r = 5): builds and merges from fingerprint lists (k_set_layout),
 // and the in-place merge and large insert, which decode a bucket's old
-// contents straight from the table (k_set_update).  Builds that keep every
-// copy, or of two-byte slots: k_group_layout.
+// contents straight from the table (k_set_update).  Builds and merges that
+// keep every copy, or of two-byte slots: k_group_layout.
 #pragma once
 
 #include "sqf_build.cuh"
@@ -193,15 +193,19 @@ struct GroupContents {
     const LayoutArgs &a;
     uint32_t *cnt;  // u16 per quotient: end of its group
     Rem *rem;
-    uint32_t n, stray;
-    size_t base;
+    uint32_t n, na;
+    size_t abase, bbase;
     __device__ __forceinline__ GroupContents(const LayoutArgs &args, uint32_t b, uint8_t *mem) : a(args)
     {
-        n = a.B.count(b);
-        base = n ? a.B.start(b) : 0;
+        na = a.A.count(b);
+        n = na + a.B.count(b);
+        abase = na ? a.A.start(b) : 0;
+        bbase = n > na ? a.B.start(b) : 0;
         cnt = reinterpret_cast<uint32_t *>(mem);
+        // (the lists before this bucket's hold A.start + B.start items)
         rem = n <= a.cap_items ? reinterpret_cast<Rem *>(mem + group_cnt_bytes(S))
-                               : static_cast<Rem *>(a.rem_scratch) + base;
+                               : static_cast<Rem *>(a.rem_scratch) +
+                                     ((a.A.cnt ? a.A.start(b) : 0) + (a.B.cnt ? a.B.start(b) : 0));
     }
     static __host__ __device__ constexpr size_t group_cnt_bytes(size_t s) { return (4 * (s / 2 + s / 32 + 8) + 15) & ~(size_t)15; }
     __device__ __forceinline__ bool fits() const { return n <= 65520; }  // u16 positions
@@ -284,7 +288,9 @@ struct GroupContents {
     template <int NT, typename F>
     __device__ __forceinline__ void each(uint32_t t, F &&f) const
     {
-        for_each_item<NT>(a.B.items, base, n, t, [&](uint32_t v) { f((v >> R) & (S - 1), v & ((1u << R) - 1u)); });
+        auto item = [&](uint32_t v) { f((v >> R) & (S - 1), v & ((1u << R) - 1u)); };
+        if (na) for_each_item<NT>(a.A.items, abase, na, t, item);
+        if (n > na) for_each_item<NT>(a.B.items, bbase, n - na, t, item);
     }
     template <typename Put>
     __device__ __forceinline__ void put_item(uint32_t x, uint32_t r, uint32_t st, Put &&put) const
@@ -845,7 +851,7 @@ __global__ void __launch_bounds__(THREADS, (THREADS >= 1024 ? 1 : 1024 / THREADS
     bucket_layout_set<THREADS, QPT, ListSource>(a, s_ticket);
 }
 
-// A build that keeps every copy, or of two-byte slots.
+// A build or merge that keeps every copy, or of two-byte slots.
 template <int THREADS, int QPT, int BPE, bool UNIQUE>
 __global__ void __launch_bounds__(THREADS, (THREADS >= 1024 ? 1 : 1024 / THREADS)) k_group_layout(LayoutArgs a)
 {

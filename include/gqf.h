@@ -103,16 +103,14 @@ int gqf_sqf_bulk_build(const gqf_sqf *qf, int n, const uint32_t *d_keys,
 
 /* launchUnsortedLookups, quotientFilter.cu:359-381: d_out[i] = slot of
  * key i's remainder, or GQF_NOT_FOUND.  On one-byte slots a batch of at least
- * one query per 16 slots first transposes the table into a bit-plane mirror
- * (stream workspace, 32 bytes per 31 slots) and answers each query from two
- * of its 32-byte records. */
+ * one query per 32 slots and 786432 queries first transposes the table into
+ * a bit-plane mirror (stream workspace, 32 bytes per 31 slots) and answers
+ * each query from two of its 32-byte records. */
 int gqf_sqf_lookup_unsorted(const gqf_sqf *qf, int n, const uint32_t *d_keys,
                             uint32_t *d_out, void *stream, float *ms);
 
 /* launchSortedLookups, quotientFilter.cu:272-318: same results as the
- * unsorted lookup (input order).  Batches of at least one query per 16 slots
- * take the unsorted path above; smaller ones group the queries by table
- * region. */
+ * unsorted lookup (input order), by the same kernels. */
 int gqf_sqf_lookup_sorted(const gqf_sqf *qf, int n, const uint32_t *d_keys,
                           uint32_t *d_out, void *stream, float *ms);
 
@@ -179,9 +177,8 @@ int gqf_rsqf_free(gqf_rsqf *cqf);
  * fingerprint of the batch, or -1 */
 int gqf_rsqf_insert(const gqf_rsqf *cqf, int n, const uint32_t *d_keys,
                     int32_t *d_ret, void *stream, float *ms);
-/* launchLookups, RSQF.cu:411-456 (slot or -1, in input order).  Batches of
- * at least one query per 16 slots are probed directly, smaller ones grouped
- * by block first. */
+/* launchLookups, RSQF.cu:411-456 (slot or -1, in input order), by the
+ * kernels of the unsorted lookup. */
 int gqf_rsqf_lookup_sorted(const gqf_rsqf *cqf, int n, const uint32_t *d_keys,
                            int32_t *d_out, void *stream, float *ms);
 /* launchUnsortedLookups, RSQF.cu:540-563 */

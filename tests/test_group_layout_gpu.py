@@ -50,3 +50,35 @@ def test_group_build_many_copies(gqf, cuda, q, r, nodup):
     keys = np.concatenate([np.full(5000, 99, np.uint32), np.repeat(few, 60), narrow, O.mt_keys(722 + q, n)])
     keys = keys[np.random.default_rng(1).permutation(keys.size)]
     build_and_check(gqf, cuda, q, r, keys, nodup)
+
+
+@pytest.mark.parametrize("q,r,nodup", [(8, 5, False), (12, 13, True), (13, 13, False), (16, 5, False), (18, 13, True),
+                                       (20, 5, False)])
+@pytest.mark.parametrize("na,nb", [(0.45, 0.45), (0.7, 0.02), (0.0, 0.3)])
+def test_group_merge(gqf, cuda, q, r, nodup, na, nb):
+    """Merges that keep every copy, or of two-byte slots: both contents, one
+    of them small, the first filter empty; one key a thousand times on both
+    sides where the filter has room for it."""
+    G, torch = gqf, cuda
+    many = np.full(1000 if q >= 14 else 3, 99, np.uint32)
+    a, b = O.mt_keys(740 + q, int(na * (1 << q))), np.concatenate([many, O.mt_keys(760 + q, int(nb * (1 << q)))])
+    if na:
+        a = np.concatenate([a, many])
+    ta, tb = O.sqf_new(q, r), O.sqf_new(q, r)
+    if na:
+        assert O.sqf_bulk_build(ta, q, r, a, False) == 0
+    assert O.sqf_bulk_build(tb, q, r, b, False) == 0
+    assert O.sqf_merge_two(ta, tb.copy(), q, r, nodup) == 0
+    for sync in (True, False):
+        fa, fb = G.initFilterGPU(q, r), G.initFilterGPU(q, r)
+        try:
+            if na:
+                G.bulkBuildSegmentedLayouts(fa, a.size, to_dev(torch, a), False)
+            G.bulkBuildSegmentedLayouts(fb, b.size, to_dev(torch, b), False)
+            G.mergeTwoFilters(fa, fb, nodup, sync=sync)
+            G.stream_status()
+            assert np.array_equal(G.table_bytes(fa), ta)
+            assert np.array_equal(G.table_bytes(fb), tb)  # the second filter is only read
+        finally:
+            G.freeFilterGPU(fa)
+            G.freeFilterGPU(fb)
