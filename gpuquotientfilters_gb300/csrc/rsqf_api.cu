@@ -282,12 +282,18 @@ __global__ void __launch_bounds__(32 * WARPS) k_rsqf_round_warp(
 // A write past the group's end marks it crossed (merged with its successor
 // and done again); one past the window, or below it, hands the group to
 // k_rsqf_round_big through list 2.
+// Skipping and ending early leave blocks as k_rsqf_assemble wrote them and
+// take ret[] for canonical slots.  That holds in the first round only: the
+// second part of a merged group may have been replayed by itself in the round
+// before, for a batch without the first part's spill.  Later rounds (few, and
+// of few groups) replay every item from the first departure on and store all
+// blocks from there.
 template <uint32_t MAXB>
 __global__ void __launch_bounds__(32) k_rsqf_replay_build(
     uint8_t *__restrict__ t, const uint8_t *__restrict__ t0, uint32_t nblocks, uint32_t q,
     const uint32_t *__restrict__ fps, const uint32_t *__restrict__ fhome, const uint32_t *__restrict__ list,
     uint32_t *__restrict__ counts, uint8_t *__restrict__ crossed, uint32_t *n_crossed, int32_t *__restrict__ ret,
-    const uint8_t *__restrict__ sus, const uint32_t *__restrict__ fpos, uint32_t *__restrict__ list2)
+    const uint8_t *__restrict__ sus, const uint32_t *__restrict__ fpos, uint32_t *__restrict__ list2, int first)
 {
     constexpr uint32_t EXPB = 4;  // blocks that spilled items are compared in
     __shared__ __align__(16) uint8_t sm[MAXB * RSQF_SB];
@@ -349,7 +355,7 @@ __global__ void __launch_bounds__(32) k_rsqf_replay_build(
         uint32_t hcur = (fps[i] >> RSQF_R) / RSQF_SPB, wb = we;  // blocks [W, wb) are written back
         while (i < i1) {
             const uint32_t h = (fps[i] >> RSQF_R) / RSQF_SPB;
-            if (h > hcur && h < we && i == fhome[h]) {
+            if (first && h > hcur && h < we && i == fhome[h]) {
                 hcur = h;
                 // canonical again from block h on?
                 const uint32_t p0 = fpos[h], nsp = i > p0 ? i - p0 : 0u;
@@ -395,6 +401,7 @@ __global__ void __launch_bounds__(32) k_rsqf_replay_build(
             i++;
         }
         __syncwarp();
+        if (wb == we && we < e) f.crossed = true;  // the blocks past the window were not looked at
         if (f.crossed) {
             if (lane == 0) {
                 if (f.left || we < e) {
@@ -636,7 +643,7 @@ static int rsqf_replay_rounds(uint8_t *t, const uint8_t *t0, uint32_t nbl, uint3
         if (sus) {
             k_rsqf_replay_build<RSQF_WARP_GROUP_MAX><<<di.sms * 4, 32, 0, s>>>(
                 t, t0, nbl, q, items, fhome, wlist + 2 * (size_t)(nbl + 1), ctr, crossed, ctr + 3, d_ret, sus, fpos,
-                blist);
+                blist, round == 0 ? 1 : 0);
         } else {
             // the long groups' serial replays run beside the many short ones
             // (other blocks, other items), on the side stream
