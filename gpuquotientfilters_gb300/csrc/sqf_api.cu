@@ -328,11 +328,17 @@ static int launch_layout(const LayoutPlan &p, const SqfGeom &tg, uint8_t *table,
         count_launches(1);
     }
     if ((op == OP_BUILD || op == OP_MERGE) && !set_ok) {
-        // shared memory for a third more than the average bucket; a larger
-        // one keeps its remainders in the scratch
+        // shared memory for a third more than the average bucket, as far as
+        // the SM's goes (two-byte buckets of 32768 quotients); a larger one
+        // keeps its remainders in the scratch
         a.rem_scratch = sc.rems;
         const double avg = (double)p.n_expect / p.g.nb;
-        a.cap_items = (uint32_t)align_up((size_t)std::min(avg * 1.3 + 8.0 * std::sqrt(avg) + 64.0, 40000.0), 16);
+        const DeviceInfo &dv = device_info(current_device());
+        const size_t maxsm = (size_t)(dv.smem_optin > 0 ? dv.smem_optin : 99 * 1024) - 4096;  // less the static arrays
+        const size_t fixed = group_layout_smem(p.g.tb, threads, BPE, 0);
+        const size_t most = maxsm > fixed ? ((maxsm - fixed) / BPE) & ~(size_t)15 : 0;
+        a.cap_items = (uint32_t)std::min(
+            align_up((size_t)std::min(avg * 1.3 + 8.0 * std::sqrt(avg) + 64.0, 40000.0), 16), most);
         const size_t smem = group_layout_smem(p.g.tb, threads, BPE, a.cap_items);
         auto gg = [&](auto dup, auto uniq) {
             if (nodup) go(uniq, smem);
