@@ -1,59 +1,9 @@
 // C ABI of the standard quotient filter: host orchestration of the kernels.
-#include <algorithm>
-#include <cmath>
-#include <cstring>
-#include <map>
-#include <mutex>
-#include <type_traits>
-
-#include "host_common.cuh"
-#include "sqf_build.cuh"
-#include "sqf_extract.cuh"
-#include "sqf_fallback.cuh"
+#include "sqf_host.cuh"
 #include "sqf_lookup.cuh"
 #include "sqf_mirror.cuh"
-#include "sqf_update.cuh"
 
 namespace gqf {
-
-// ------------------------------------------------------------------ geometry
-static bool qr_ok(unsigned q, unsigned r)
-{
-    // quotientFilter.cu:46-47 asserts q + r <= 32 and (r + 3) % 8 == 0; a
-    // 32-bit fingerprint would need `1 << 32` in the hash modulus (:268), so
-    // q + r <= 31 here.  q >= 7 keeps a bucket at least 128 quotients.
-    return (r + 3) % 8 == 0 && (r + 3) / 8 <= 2 && q >= 7 && q + r <= 31 && r >= 1;
-}
-
-struct SqfGeom {
-    uint32_t q, r, bpe, nslots;
-    size_t T;
-};
-static SqfGeom geom_of(const gqf_sqf *qf)
-{
-    SqfGeom g;
-    g.q = qf->qbits;
-    g.r = qf->rbits;
-    g.bpe = (g.r + 3) / 8;
-    g.nslots = gqf_sqf_num_slots(g.q);
-    g.T = gqf_sqf_table_bytes(g.q, g.r);
-    return g;
-}
-
-static uint32_t ceil_log2(uint64_t x)
-{
-    uint32_t l = 0;
-    while ((1ull << l) < x) l++;
-    return l;
-}
-
-struct LayoutPlan {
-    BucketGeom g;
-    uint32_t stride;     // speculative bucket stride (items)
-    uint64_t n_expect;   // items it was made for
-    uint32_t cap_items;  // per-CTA item capacity of k_bucket_layout
-    size_t smem;
-};
 
 // Bucket geometry for `n_expect` items over 2^q quotients: about 12k items
 // per bucket (one CTA sorts a bucket in shared memory), at most 4096 buckets
@@ -104,26 +54,6 @@ static LayoutPlan plan_layout(uint32_t q, uint32_t r, uint64_t n_expect, uint64_
     return p;
 }
 
-// Layout buckets of an in-place update: 8192 quotients (three CTAs per SM
-// hold their sets, index and tile), fewer where the filter would otherwise
-// give less than 512 buckets, down to 1024.
-static uint32_t update_tb(uint32_t q) { return std::min<uint32_t>(q, std::min<uint32_t>(13, std::max<uint32_t>(10, q > 9 ? q - 9 : 0))); }
-
-template <typename K>
-static cudaError_t set_smem(K kernel, size_t bytes)
-{
-    // the attribute is per function and device; set it only when it grows
-    static std::mutex mu;
-    static std::map<std::pair<const void *, int>, size_t> done;
-    const std::pair<const void *, int> key(reinterpret_cast<const void *>(kernel), current_device());
-    std::lock_guard<std::mutex> lk(mu);
-    size_t &cur = done[key];
-    if (bytes <= cur) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess) cur = bytes;
-    return e;
-}
-
 // Device-side exclusive scan of bucket counts into bases (nb <= 4096).
 __global__ void __launch_bounds__(1024) k_scan_bases(const uint32_t *cnt, uint32_t nb, uint32_t *base)
 {
@@ -133,88 +63,6 @@ __global__ void __launch_bounds__(1024) k_scan_bases(const uint32_t *cnt, uint32
     __syncthreads();
     block_exclusive_scan_u32<1024>(s, nb, sw);
     for (uint32_t i = threadIdx.x; i < nb; i += blockDim.x) base[i] = s[i];
-}
-
-// ------------------------------------------------------------ the pipeline
-// Scratch for one rebuild: control words, look-back descriptors, fix-ups,
-// the bucketed batch (B) and optionally the table's extracted contents (A).
-struct Scratch {
-    uint32_t *bcnt;              // nb  : batch items per bucket
-    unsigned long long *status;  // nb  : look-back descriptors
-    uint32_t *ticket;
-    uint32_t *fix_cnt;
-    uint32_t *a_dups;  // table holds duplicate fingerprints (set by extraction)
-    uint32_t *fused_fail;  // the in-place update could not decode some bucket
-    uint8_t *snap;         // table snapshot of the in-place update
-    uint32_t *bbase;  // nb+1: exact batch bases
-    uint32_t *fix_list;
-    uint32_t fix_cap;
-    uint32_t *bitems;  // batch fingerprints
-    void *rems;        // k_group_layout: remainders of large buckets
-    // extracted table contents
-    Counts3 *tiles;
-    uint32_t *Q, *E, *abase, *acnt;
-    uint32_t *E2, *a2base, *a2cnt;
-    size_t ctrl_bytes;
-};
-
-struct ScratchReq {
-    uint32_t nb;
-    size_t batch_items;  // capacity of the bucketed batch
-    bool extract;   // table contents needed
-    bool extract2;  // second table (merge)
-    uint32_t nslots;
-    size_t snap_bytes = 0;  // in-place update: snapshot of the table
-    uint32_t upd_nb = 0;    // and its layout buckets
-    bool every_fix = false; // room for a fix-up of every quotient
-    uint32_t rem_bytes = 0; // k_group_layout: scratch bytes per item
-};
-
-static Scratch carve(void *base, const ScratchReq &r, bool sizing_only, size_t *bytes_out)
-{
-    Scratch s{};
-    auto lay = [&](auto &c) {
-        size_t nb = r.nb;
-        s.bcnt = c.template take<uint32_t>(nb, 8);
-        s.status = c.template take<unsigned long long>(std::max<size_t>(nb, r.upd_nb), 8);
-        s.ticket = c.template take<uint32_t>(1, 4);
-        s.fix_cnt = c.template take<uint32_t>(1, 4);
-        s.a_dups = c.template take<uint32_t>(1, 4);
-        s.fused_fail = c.template take<uint32_t>(1, 4);
-        s.ctrl_bytes = c.off;
-        s.bbase = c.template take<uint32_t>(nb + 1);
-        s.fix_cap = std::max<uint32_t>(65536u, r.every_fix ? r.nslots : r.nslots / 8);
-        s.fix_list = c.template take<uint32_t>(s.fix_cap);
-        s.bitems = c.template take<uint32_t>(std::max<size_t>(r.batch_items, 1));
-        s.rems = r.rem_bytes ? c.template take<uint8_t>((std::max<size_t>(r.batch_items, 1) +
-                                                         (r.extract ? r.nslots : 0) + (r.extract2 ? r.nslots : 0)) *
-                                                        r.rem_bytes)
-                             : nullptr;
-        if (r.extract) {
-            size_t ntiles = (r.nslots + EXTRACT_TILE - 1) / EXTRACT_TILE;
-            s.tiles = c.template take<Counts3>(ntiles + 1);
-            s.Q = c.template take<uint32_t>(r.nslots);
-            s.E = c.template take<uint32_t>(r.nslots);
-            s.abase = c.template take<uint32_t>(nb + 1);
-            s.acnt = c.template take<uint32_t>(nb);
-            if (r.extract2) {
-                s.E2 = c.template take<uint32_t>(r.nslots);
-                s.a2base = c.template take<uint32_t>(nb + 1);
-                s.a2cnt = c.template take<uint32_t>(nb);
-            }
-        }
-        s.snap = r.snap_bytes ? c.template take<uint8_t>(r.snap_bytes) : nullptr;
-    };
-    if (sizing_only) {
-        Sizer z;
-        lay(z);
-        *bytes_out = z.off;
-    } else {
-        Carver c(base);
-        lay(c);
-        *bytes_out = c.off;
-    }
-    return s;
 }
 
 // Extract a table's fingerprints (sorted for canonical tables) into E and
@@ -273,166 +121,6 @@ static int bucket_batch(const uint32_t *keys, uint32_t n, const LayoutPlan &p, S
     if (n == 0) return GQF_OK;
     return n <= SMALL_BATCH ? bucket_batch_keys<SMALL_THREADS, SMALL_IPT>(keys, n, p, sc, exact, err, s)
                             : bucket_batch_keys<SCATTER_THREADS, SCATTER_IPT>(keys, n, p, sc, exact, err, s);
-}
-
-template <int BPE>
-static int launch_layout(const LayoutPlan &p, const SqfGeom &tg, uint8_t *table, const BucketSrc &A,
-                         const BucketSrc &B, int op, int nodup, bool set_ok, const uint32_t *a_dups, Scratch &sc,
-                         uint32_t *err, cudaStream_t s, const uint32_t *gate = nullptr)
-{
-    // slots past the last bucket's quotients only receive spill: clear them
-    // (a gated launch leaves that to k_fallback_prepare)
-    size_t tail = (size_t)(1u << tg.q) * BPE;
-    if (!gate && tg.T > tail) GQF_CK(cudaMemsetAsync(table + tail, 0, tg.T - tail, s));
-    LayoutArgs a;
-    a.A = A;
-    a.B = B;
-    a.table = table;
-    a.q = tg.q;
-    a.r = tg.r;
-    a.tb = p.g.tb;
-    a.nb = p.g.nb;
-    a.nslots = tg.nslots;
-    a.cap_items = p.cap_items;
-    a.op = op;
-    a.nodup = nodup;
-    a.set_ok = set_ok ? 1 : 0;
-    a.a_dups = a_dups;
-    a.status = sc.status;
-    a.ticket = sc.ticket;
-    a.fix_list = sc.fix_list;
-    a.fix_cnt = sc.fix_cnt;
-    a.fix_cap = sc.fix_cap;
-    a.err = err;
-    a.gate = gate;
-    const int threads = (int)layout_threads(p.g.tb);
-    cudaError_t e = cudaSuccess;
-    auto go = [&](auto kernel, size_t smem) {
-        e = set_smem(kernel, smem);
-        if (e == cudaSuccess) kernel<<<p.g.nb, threads, smem, s>>>(a);
-    };
-    if (BPE == 1 && set_ok) {
-        const size_t smem = set_layout_smem(p.g.tb, threads);
-        switch (p.g.tb) {
-        case 15: go(k_set_layout<1024, 32>, smem); break;
-        case 14: go(k_set_layout<512, 32>, smem); break;
-        case 13: go(k_set_layout<256, 32>, smem); break;
-        case 12: go(k_set_layout<256, 16>, smem); break;
-        case 11: go(k_set_layout<128, 16>, smem); break;
-        case 10: go(k_set_layout<128, 8>, smem); break;
-        case 9: go(k_set_layout<64, 8>, smem); break;
-        case 8: go(k_set_layout<32, 8>, smem); break;
-        default: go(k_set_layout<32, 4>, smem); break;
-        }
-        GQF_CK(e);
-        count_launches(1);
-    }
-    if ((op == OP_BUILD || op == OP_MERGE) && !set_ok) {
-        // shared memory for a third more than the average bucket, as far as
-        // the SM's goes (two-byte buckets of 32768 quotients); a larger one
-        // keeps its remainders in the scratch
-        a.rem_scratch = sc.rems;
-        const double avg = (double)p.n_expect / p.g.nb;
-        const DeviceInfo &dv = device_info(current_device());
-        const size_t maxsm = (size_t)(dv.smem_optin > 0 ? dv.smem_optin : 99 * 1024) - 4096;  // less the static arrays
-        const size_t fixed = group_layout_smem(p.g.tb, threads, BPE, 0);
-        const size_t most = maxsm > fixed ? ((maxsm - fixed) / BPE) & ~(size_t)15 : 0;
-        a.cap_items = (uint32_t)std::min(
-            align_up((size_t)std::min(avg * 1.3 + 8.0 * std::sqrt(avg) + 64.0, 40000.0), 16), most);
-        const size_t smem = group_layout_smem(p.g.tb, threads, BPE, a.cap_items);
-        auto gg = [&](auto dup, auto uniq) {
-            if (nodup) go(uniq, smem);
-            else go(dup, smem);
-        };
-        switch (p.g.tb) {
-        case 15: gg(k_group_layout<1024, 32, BPE, false>, k_group_layout<1024, 32, BPE, true>); break;
-        case 14: gg(k_group_layout<512, 32, BPE, false>, k_group_layout<512, 32, BPE, true>); break;
-        case 13: gg(k_group_layout<256, 32, BPE, false>, k_group_layout<256, 32, BPE, true>); break;
-        case 12: gg(k_group_layout<256, 16, BPE, false>, k_group_layout<256, 16, BPE, true>); break;
-        case 11: gg(k_group_layout<128, 16, BPE, false>, k_group_layout<128, 16, BPE, true>); break;
-        case 10: gg(k_group_layout<128, 8, BPE, false>, k_group_layout<128, 8, BPE, true>); break;
-        case 9: gg(k_group_layout<64, 8, BPE, false>, k_group_layout<64, 8, BPE, true>); break;
-        case 8: gg(k_group_layout<32, 8, BPE, false>, k_group_layout<32, 8, BPE, true>); break;
-        default: gg(k_group_layout<32, 4, BPE, false>, k_group_layout<32, 4, BPE, true>); break;
-        }
-        GQF_CK(e);
-        count_launches(1);
-    } else if (!set_ok || a_dups) {
-        switch (p.g.tb) {
-        case 15: go(k_bucket_layout<1024, 32, BPE>, p.smem); break;
-        case 14: go(k_bucket_layout<512, 32, BPE>, p.smem); break;
-        case 13: go(k_bucket_layout<256, 32, BPE>, p.smem); break;
-        case 12: go(k_bucket_layout<256, 16, BPE>, p.smem); break;
-        case 11: go(k_bucket_layout<128, 16, BPE>, p.smem); break;
-        case 10: go(k_bucket_layout<128, 8, BPE>, p.smem); break;
-        case 9: go(k_bucket_layout<64, 8, BPE>, p.smem); break;
-        case 8: go(k_bucket_layout<32, 8, BPE>, p.smem); break;
-        default: go(k_bucket_layout<32, 4, BPE>, p.smem); break;
-        }
-        GQF_CK(e);
-        count_launches(1);
-    }
-    const DeviceInfo &di = device_info(current_device());
-    count_launches(1);
-    k_fixup_occ<BPE><<<di.sms * 2, 256, 0, s>>>(table, sc.fix_list, sc.fix_cnt, sc.fix_cap, gate);
-    GQF_CK(cudaGetLastError());
-    return GQF_OK;
-}
-
-// In-place update of one-byte slots: old contents from the snapshot (and
-// `src2`), batch buckets of geometry p.
-static int launch_update(const LayoutPlan &p, const SqfGeom &tg, uint8_t *table, const uint8_t *src2,
-                         const BucketSrc &B, int op, Scratch &sc, uint32_t *err, cudaStream_t s)
-{
-    const size_t tail = (size_t)1 << tg.q;
-    if (tg.T > tail) GQF_CK(cudaMemsetAsync(table + tail, 0, tg.T - tail, s));
-    LayoutArgs a;
-    a.A = BucketSrc{nullptr, nullptr, 0, nullptr};
-    a.B = B;
-    a.table = table;
-    a.q = tg.q;
-    a.r = tg.r;
-    a.tb = update_tb(tg.q);
-    a.nb = 1u << (tg.q - a.tb);
-    a.nslots = tg.nslots;
-    a.cap_items = 0;
-    a.op = op;
-    a.nodup = 1;
-    a.set_ok = 1;
-    a.a_dups = nullptr;
-    a.status = sc.status;
-    a.ticket = sc.ticket;
-    a.fix_list = sc.fix_list;
-    a.fix_cnt = sc.fix_cnt;
-    a.fix_cap = sc.fix_cap;
-    a.err = err;
-    a.src_table = sc.snap;
-    a.src2 = src2;
-    a.sub = p.g.tb - a.tb;
-    a.fused_fail = sc.fused_fail;
-    const int threads = (int)layout_threads(a.tb);
-    const size_t smem = set_update_smem(a.tb, threads, src2 != nullptr);
-    cudaError_t e = cudaSuccess;
-    auto go = [&](auto one, auto two) {
-        auto kernel = src2 ? two : one;
-        e = set_smem(kernel, smem);
-        if (e == cudaSuccess) kernel<<<a.nb, threads, smem, s>>>(a);
-    };
-    switch (a.tb) {
-    case 13: go(k_set_update<256, 32, false>, k_set_update<256, 32, true>); break;
-    case 12: go(k_set_update<256, 16, false>, k_set_update<256, 16, true>); break;
-    case 11: go(k_set_update<128, 16, false>, k_set_update<128, 16, true>); break;
-    case 10: go(k_set_update<128, 8, false>, k_set_update<128, 8, true>); break;
-    case 9: go(k_set_update<64, 8, false>, k_set_update<64, 8, true>); break;
-    case 8: go(k_set_update<32, 8, false>, k_set_update<32, 8, true>); break;
-    default: go(k_set_update<32, 4, false>, k_set_update<32, 4, true>); break;
-    }
-    GQF_CK(e);
-    const DeviceInfo &di = device_info(current_device());
-    k_fixup_occ<1><<<di.sms * 2, 256, 0, s>>>(table, sc.fix_list, sc.fix_cnt, sc.fix_cap, nullptr);
-    count_launches(2);
-    GQF_CK(cudaGetLastError());
-    return GQF_OK;
 }
 
 // Asynchronous in-place update that could not place some bucket (*gate
@@ -635,144 +323,10 @@ static int rebuild(const gqf_sqf *qf, const gqf_sqf *qf2, const uint32_t *keys, 
     return GQF_ERR_FULL;
 }
 
-// ------------------------------------------------------ cluster-local updates
 // An insert of at most one key per 16 quotients, and every delete
 // (sqf_update.cuh), with the general path behind it on the device.  Larger
 // inserts connect ever longer runs of clusters and are rebuilt instead.
 static bool insert_is_local(uint32_t q, uint32_t n) { return (uint64_t)n * 16 <= (1ull << q); }
-
-template <int BPE>
-static int local_update(const gqf_sqf *qf, const uint32_t *keys, uint32_t n, int op, cudaStream_t s, float *ms)
-{
-    const SqfGeom tg = geom_of(qf);
-    const DeviceInfo &di = device_info(current_device());
-    const bool ins = op == OP_INSERT;
-    // insert buckets of about 128 keys, one CTA each
-    InsBatch ib{};
-    uint32_t lg = 0;
-    while ((128ull << lg) < n && lg < std::min<uint32_t>(tg.q, 18)) lg++;
-    ib.nb = 1u << lg;
-    ib.shift = tg.q + tg.r - lg;
-    const double avg = (double)n / ib.nb;
-    ib.stride = (uint32_t)align_up((size_t)(avg + 10.0 * std::sqrt(avg) + 32.0), 32);
-    uint32_t hsize = 1024;
-    while (hsize < 2ull * n) hsize <<= 1;
-    ib.hmask = hsize - 1;
-    const size_t nkey = (size_t)ib.nb * ib.stride + n;
-    // a table shorter than any walk's limit needs no fallback
-    const bool fb = tg.nslots > FAR_SLOTS;
-    static_assert((uint64_t)((1u << (FB_TB - 1)) * 1.1) <= FAR_SLOTS, "a fallback table spans whole buckets");
-    const uint32_t fnb = fb ? 1u << (tg.q - FB_TB) : 1u;
-    const uint32_t ntiles = (tg.nslots + EXTRACT_TILE - 1) / EXTRACT_TILE;
-    FallbackArgs f{};
-    uint32_t *far = nullptr, *claim = nullptr, *n_units = nullptr;
-    uint2 *units = nullptr;
-    uint4 *lead = nullptr;
-    size_t zero_bytes = 0;
-    // control words | delete claims (both zeroed) | then either the update's
-    // arrays or, when the fallback runs, its own over them
-    auto lay = [&](auto &c) {
-        far = c.template take<uint32_t>(1);
-        f.bar = c.template take<uint32_t>(4, 16);
-        f.lay.ticket = c.template take<uint32_t>(1, 4);
-        f.lay.fix_cnt = c.template take<uint32_t>(1, 4);
-        ib.n_over = c.template take<uint32_t>(1, 4);
-        ib.pool = c.template take<uint32_t>(1, 4);
-        n_units = ib.n_group = c.template take<uint32_t>(1, 4);
-        f.bcnt = c.template take<uint32_t>(fnb, 4);
-        f.bfill = c.template take<uint32_t>(fnb, 4);
-        f.lay.status = c.template take<unsigned long long>(fnb, 8);
-        if (ins) ib.cnt = c.template take<uint32_t>(ib.nb, 4);
-        else claim = c.template take<uint32_t>(2 * ((tg.nslots + 31) / 32), 16);
-        zero_bytes = c.off;
-        const size_t at = c.off;
-        if (ins) {
-            ib.seen = c.template take<uint32_t>(hsize);
-            ib.base = c.template take<uint32_t>(ib.nb);
-            ib.key = c.template take<uint4>(nkey);
-            ib.over = c.template take<uint4>(n);
-        } else {
-            lead = c.template take<uint4>(n);
-            units = c.template take<uint2>(n);
-        }
-        const size_t end = c.off;
-        if (fb) {
-            c.off = at;
-            f.tiles = c.template take<Counts3>(ntiles + 1);
-            f.Q = c.template take<uint32_t>(tg.nslots);
-            f.E = c.template take<uint32_t>(tg.nslots);
-            f.abase = c.template take<uint32_t>(fnb + 1);
-            f.acnt = c.template take<uint32_t>(fnb);
-            f.bbase = c.template take<uint32_t>(fnb + 1);
-            f.bitems = c.template take<uint32_t>(n);
-            f.lay.fix_cap = std::max<uint32_t>(65536u, tg.nslots / 8);
-            f.lay.fix_list = c.template take<uint32_t>(f.lay.fix_cap);
-            c.off = std::max(c.off, end);
-        }
-    };
-    Sizer z;
-    lay(z);
-    Arena &ar = arena(current_device(), s);
-    std::lock_guard<std::mutex> lk(ar.mu);
-    void *base = arena_reserve(ar, z.off);
-    if (!base) return GQF_ERR_NOMEM;
-    Carver c(base);
-    lay(c);
-    int st = call_begin(ar, s, ms != nullptr);
-    if (st) return st;
-    if (n == 0) return call_end(ar, s, ms);
-    GQF_CK(cudaMemsetAsync(base, 0, zero_bytes, s));
-    const SlotTable<BPE> v{qf->table, tg.nslots};
-    const uint32_t grid = (n + UPD_THREADS - 1) / UPD_THREADS;
-    // a warp per listed unit or group, at most every key's
-    const uint32_t lgrid = std::min<uint32_t>((n + LIST_THREADS / 32 - 1) / (LIST_THREADS / 32), (uint32_t)di.sms * 32);
-    if (ins) {
-        GQF_CK(cudaMemsetAsync(ib.seen, 0xFF, (size_t)hsize * 4, s));
-        k_ins_stage<BPE><<<grid, UPD_THREADS, 0, s>>>(keys, n, v, tg.q, tg.r, ib, far);
-        k_ins_sort<<<ib.nb, INS_THREADS, 0, s>>>(ib, far);
-        k_ins_groups<BPE><<<ib.nb, INS_THREADS, 0, s>>>(v, ib, far);
-        k_ins_apply<BPE><<<ib.nb, INS_THREADS, 0, s>>>(v, tg.r, ib, ar.err, far);
-        k_ins_lists<BPE><<<lgrid, LIST_THREADS, 0, s>>>(v, tg.r, ib);
-        count_launches(5);
-    } else {
-        k_del_locate<BPE><<<grid, UPD_THREADS, 0, s>>>(keys, n, v, tg.q, tg.r, claim, lead, far);
-        k_del_apply<BPE><<<grid, UPD_THREADS, 0, s>>>(n, v, claim, lead, units, n_units, far);
-        k_del_units<BPE><<<lgrid, LIST_THREADS, 0, s>>>(v, claim, units, n_units);
-        count_launches(3);
-    }
-    GQF_CK(cudaGetLastError());
-    if (fb) {
-        f.far = far;
-        f.keys = keys;
-        f.n = n;
-        f.nbytes = (uint32_t)tg.T;
-        LayoutArgs &a = f.lay;
-        a.A = BucketSrc{f.E, f.abase, 0, f.acnt};
-        a.B = BucketSrc{f.bitems, f.bbase, 0, f.bcnt};
-        a.table = qf->table;
-        a.q = tg.q;
-        a.r = tg.r;
-        a.tb = FB_TB;
-        a.nb = fnb;
-        a.nslots = tg.nslots;
-        a.op = op;
-        a.nodup = ins ? 1 : 0;
-        a.set_ok = 0;
-        a.a_dups = nullptr;
-        a.err = ar.err;
-        // the most items a bucket's u16 counters allow (eight times its average)
-        a.cap_items = 65520;
-        const size_t smem = layout_smem_bytes(FB_TB, a.cap_items, BPE);
-        GQF_CK(set_smem(k_update_fallback<BPE>, smem));
-        // a quarter of the SMs: the launch must find room for all of its CTAs
-        // at once beside other streams' kernels, and it rarely runs
-        void *args[] = {&f};
-        GQF_CK(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_update_fallback<BPE>),
-                                           dim3(std::max(1, di.sms / 4)), dim3(FB_THREADS), args, smem, s));
-        count_launches(1);
-    }
-    return call_end(ar, s, ms);
-}
 
 // Sorted and unsorted lookups alike: results go to the queries' input positions
 // either way (the reference sorts them back by index, quotientFilter.cu:

@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(EXTRACT_THREADS) k_tile_counts(const uint8_t *
 
 // Exclusive scan of the tile counts by one CTA; total written at
 // tiles[ntiles].  Each thread loads its run of tiles with independent loads.
-__global__ void __launch_bounds__(1024) k_scan_counts3(Counts3 *tiles, uint32_t ntiles,
+static __global__ void __launch_bounds__(1024) k_scan_counts3(Counts3 *tiles, uint32_t ntiles,
                                                        const uint32_t *__restrict__ gate = nullptr)
 {
     if (gate && !*gate) return;
@@ -335,8 +335,8 @@ __global__ void __launch_bounds__(EXTRACT_THREADS) k_extract(const uint8_t *__re
 }
 
 // Bucket bounds of a sorted fingerprint list: base[b] = lower_bound(b << shift).
-__global__ void k_sorted_bounds(const uint32_t *__restrict__ E, const uint32_t *__restrict__ m_ptr, uint32_t nb,
-                                uint32_t shift, uint32_t *__restrict__ base, uint32_t *__restrict__ cnt,
+static __global__ void k_sorted_bounds(const uint32_t *__restrict__ E, const uint32_t *__restrict__ m_ptr, uint32_t nb,
+                                       uint32_t shift, uint32_t *__restrict__ base, uint32_t *__restrict__ cnt,
                                 const uint32_t *__restrict__ gate = nullptr)
 {
     if (gate && !*gate) return;
@@ -352,8 +352,8 @@ __global__ void k_sorted_bounds(const uint32_t *__restrict__ E, const uint32_t *
         base[b] = lo;
     }
 }
-__global__ void k_bounds_to_counts(const uint32_t *__restrict__ base, uint32_t nb, uint32_t *__restrict__ cnt,
-                                   const uint32_t *__restrict__ gate = nullptr)
+static __global__ void k_bounds_to_counts(const uint32_t *__restrict__ base, uint32_t nb, uint32_t *__restrict__ cnt,
+                                          const uint32_t *__restrict__ gate = nullptr)
 {
     if (gate && !*gate) return;
     for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x)

@@ -1,0 +1,62 @@
+// In-place merges and large inserts of one-byte slots.
+#include "sqf_host.cuh"
+
+namespace gqf {
+
+// In-place update of one-byte slots: old contents from the snapshot (and
+// `src2`), batch buckets of geometry p.
+int launch_update(const LayoutPlan &p, const SqfGeom &tg, uint8_t *table, const uint8_t *src2,
+                         const BucketSrc &B, int op, Scratch &sc, uint32_t *err, cudaStream_t s)
+{
+    const size_t tail = (size_t)1 << tg.q;
+    if (tg.T > tail) GQF_CK(cudaMemsetAsync(table + tail, 0, tg.T - tail, s));
+    LayoutArgs a;
+    a.A = BucketSrc{nullptr, nullptr, 0, nullptr};
+    a.B = B;
+    a.table = table;
+    a.q = tg.q;
+    a.r = tg.r;
+    a.tb = update_tb(tg.q);
+    a.nb = 1u << (tg.q - a.tb);
+    a.nslots = tg.nslots;
+    a.cap_items = 0;
+    a.op = op;
+    a.nodup = 1;
+    a.set_ok = 1;
+    a.a_dups = nullptr;
+    a.status = sc.status;
+    a.ticket = sc.ticket;
+    a.fix_list = sc.fix_list;
+    a.fix_cnt = sc.fix_cnt;
+    a.fix_cap = sc.fix_cap;
+    a.err = err;
+    a.src_table = sc.snap;
+    a.src2 = src2;
+    a.sub = p.g.tb - a.tb;
+    a.fused_fail = sc.fused_fail;
+    const int threads = (int)layout_threads(a.tb);
+    const size_t smem = set_update_smem(a.tb, threads, src2 != nullptr);
+    cudaError_t e = cudaSuccess;
+    auto go = [&](auto one, auto two) {
+        auto kernel = src2 ? two : one;
+        e = set_smem(kernel, smem);
+        if (e == cudaSuccess) kernel<<<a.nb, threads, smem, s>>>(a);
+    };
+    switch (a.tb) {
+    case 13: go(k_set_update<256, 32, false>, k_set_update<256, 32, true>); break;
+    case 12: go(k_set_update<256, 16, false>, k_set_update<256, 16, true>); break;
+    case 11: go(k_set_update<128, 16, false>, k_set_update<128, 16, true>); break;
+    case 10: go(k_set_update<128, 8, false>, k_set_update<128, 8, true>); break;
+    case 9: go(k_set_update<64, 8, false>, k_set_update<64, 8, true>); break;
+    case 8: go(k_set_update<32, 8, false>, k_set_update<32, 8, true>); break;
+    default: go(k_set_update<32, 4, false>, k_set_update<32, 4, true>); break;
+    }
+    GQF_CK(e);
+    const DeviceInfo &di = device_info(current_device());
+    k_fixup_occ<1><<<di.sms * 2, 256, 0, s>>>(table, sc.fix_list, sc.fix_cnt, sc.fix_cap, nullptr);
+    count_launches(2);
+    GQF_CK(cudaGetLastError());
+    return GQF_OK;
+}
+
+}  // namespace gqf

@@ -182,7 +182,9 @@ struct SetContents {
 // remainders in global scratch.
 //
 // A thread sorting and walking its 32 quotients' groups one after the other
-// took 396 us for 12.3M fingerprints over 2^24 quotients; this takes 172 us.
+// took 396 us for 12.3M fingerprints over 2^24 quotients; this took 172 us, and
+// takes about 145 us with its loops over groups of one to three items not
+// unrolled (which also compiles in a third of the time).
 template <int THREADS, int QPT, int BPE_, bool UNIQUE>
 struct GroupContents {
     static constexpr int BPE = BPE_;
@@ -215,6 +217,7 @@ struct GroupContents {
     {
         __shared__ uint32_t s_w[THREADS / 32];
         const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+#pragma unroll 1
         for (uint32_t i = tid; i < S / 2 + S / 32 + 8; i += THREADS) cnt[i] = 0;
         __syncthreads();
         each<THREADS>(tid, [&](uint32_t x, uint32_t) { cnt16_fetch_inc(cnt, x); });
@@ -242,6 +245,7 @@ struct GroupContents {
         __syncthreads();
         each<THREADS>(tid, [&](uint32_t x, uint32_t r) { rem[cnt16_fetch_inc(cnt, x)] = (Rem)r; });
         __syncthreads();
+#pragma unroll 1
         for (uint32_t x = tid; x < S; x += THREADS) {
             const uint32_t g0 = begin(x), g1 = end(x);
             if (g1 - g0 < 2) continue;
@@ -249,13 +253,16 @@ struct GroupContents {
                 small_sort(rem + g0, g1 - g0);
                 if (UNIQUE) {
                     uint32_t k = g0 + 1;
+#pragma unroll 1
                     for (uint32_t i = g0 + 1; i < g1; i++)
                         if (rem[i] != rem[k - 1]) rem[k++] = rem[i];
                     for (; k < g1; k++) rem[k] = (Rem)STRUCK;
                 }
             } else if (UNIQUE) {
+#pragma unroll 1
                 for (uint32_t i = g0 + 1; i < g1; i++) {
                     const Rem v = rem[i];
+#pragma unroll 1
                     for (uint32_t j = g0; j < i; j++)
                         if (rem[j] == v) {
                             rem[i] = (Rem)STRUCK;
@@ -270,6 +277,7 @@ struct GroupContents {
     {
         if (!UNIQUE || g1 - g0 < 2) return g1 - g0;
         uint32_t k = 0;
+#pragma unroll 1
         for (uint32_t i = g0; i < g1; i++) k += rem[i] != (Rem)STRUCK ? 1u : 0u;
         return k;
     }
@@ -300,11 +308,13 @@ struct GroupContents {
         if (g1 - g0 > 1) {
             if (g1 - g0 > BIG) return;  // put_big
             same = 0;
+#pragma unroll 1
             for (uint32_t i = g0; i < g1; i++) {
                 less += rem[i] < (Rem)r ? 1u : 0u;
                 same += rem[i] == (Rem)r ? 1u : 0u;
             }
         }
+#pragma unroll 1
         for (uint32_t k = less; k < less + same; k++)
             put(st + k, (r << 3) + 2 * min(k, 1u) + min(st + k - x, 1u));
     }
@@ -313,12 +323,14 @@ struct GroupContents {
     {
         const uint32_t g0 = begin(x), g1 = end(x);
         const bool sorted = g1 - g0 > BIG;
+#pragma unroll 1
         for (uint32_t i = g0; i < g1; i++) {
             const uint32_t r = rem[i];
             if (UNIQUE && r == STRUCK) continue;
             uint32_t k = i - g0;
             if (!sorted) {
                 k = 0;
+#pragma unroll 1
                 for (uint32_t j = g0; j < g1; j++) k += (rem[j] < (Rem)r || (rem[j] == (Rem)r && j < i)) ? 1u : 0u;
             }
             put(st + k, (r << 3) + 2 * min(k, 1u) + min(st + k - x, 1u));
@@ -328,6 +340,7 @@ struct GroupContents {
     template <int NT, typename Start, typename Put>
     __device__ __forceinline__ void put_big(uint32_t t, Start &&start, Put &&put) const
     {
+#pragma unroll 1
         for (uint32_t x = t; x < S; x += NT)
             if (end(x) - begin(x) > BIG) put_run(x, start(x), put);
     }
@@ -338,6 +351,9 @@ __device__ __forceinline__ void bucket_layout_items(const LayoutArgs &a, const u
 {
     extern __shared__ __align__(16) uint8_t smem_layout[];
     constexpr int BPE = Contents::BPE;
+    // (groups keep nothing in registers between the passes over a thread's
+    // quotients; unrolled, each of those kernels took 12 to 20 s to compile)
+    constexpr int JUNROLL = Contents::SMALL ? QPT / 4 : 1;
     constexpr uint32_t S = THREADS * QPT, BUF = S + SET_SPILL, NW = THREADS / 32;
     constexpr ItemsPlan pl = items_plan(S, THREADS, BPE);
     uint8_t *s_disp = smem_layout;            // displacement of quotient x's run
@@ -382,7 +398,7 @@ __device__ __forceinline__ void bucket_layout_items(const LayoutArgs &a, const u
     LayoutFn fn{0u, 0u};
     {
         int u = -1;  // entering below the first quotient
-#pragma unroll
+#pragma unroll(JUNROLL)
         for (uint32_t j4 = 0; j4 < QPT / 4; j4++) {
             uint32_t k[4];
             con.sizes(qb + 4 * j4, k);
@@ -446,7 +462,7 @@ __device__ __forceinline__ void bucket_layout_items(const LayoutArgs &a, const u
     auto displace = [&](uint32_t c) {
         s_gc[tid] = c - x0;
         int u = (int)c - (int)(x0 + qb);
-#pragma unroll
+#pragma unroll(JUNROLL)
         for (uint32_t j4 = 0; j4 < QPT / 4; j4++) {
             uint32_t pk = 0, k[4];
             if constexpr (Contents::SMALL) {
