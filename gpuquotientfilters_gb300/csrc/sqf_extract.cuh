@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(EXTRACT_THREADS) k_extract(const uint8_t *__re
 // Bucket bounds of a sorted fingerprint list: base[b] = lower_bound(b << shift).
 static __global__ void k_sorted_bounds(const uint32_t *__restrict__ E, const uint32_t *__restrict__ m_ptr, uint32_t nb,
                                        uint32_t shift, uint32_t *__restrict__ base, uint32_t *__restrict__ cnt,
-                                const uint32_t *__restrict__ gate = nullptr)
+                                       const uint32_t *__restrict__ gate = nullptr)
 {
     if (gate && !*gate) return;
     const uint32_t m = *m_ptr;

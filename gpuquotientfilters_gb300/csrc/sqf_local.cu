@@ -70,8 +70,10 @@ int local_update(const gqf_sqf *qf, const uint32_t *keys, uint32_t n, int op, cu
             f.acnt = c.template take<uint32_t>(fnb);
             f.bbase = c.template take<uint32_t>(fnb + 1);
             f.bitems = c.template take<uint32_t>(n);
-            f.lay.fix_cap = std::max<uint32_t>(65536u, tg.nslots / 8);
-            f.lay.fix_list = c.template take<uint32_t>(f.lay.fix_cap);
+            // a fix-up for every quotient: on an overfull table the spill
+            // passes whole buckets (the extraction is done with Q by then)
+            f.lay.fix_cap = tg.nslots;
+            f.lay.fix_list = f.Q;
             c.off = std::max(c.off, end);
         }
     };

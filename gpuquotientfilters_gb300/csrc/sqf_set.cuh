@@ -182,9 +182,9 @@ struct SetContents {
 // remainders in global scratch.
 //
 // A thread sorting and walking its 32 quotients' groups one after the other
-// took 396 us for 12.3M fingerprints over 2^24 quotients; this took 172 us, and
-// takes about 145 us with its loops over groups of one to three items not
-// unrolled (which also compiles in a third of the time).
+// took 396 us for 12.3M fingerprints over 2^24 quotients; this took 172 us.
+// Loops over a group (one to three items) are not unrolled: that build as a
+// whole took 276 us unrolled and takes 249, and compiles in a third of the time.
 template <int THREADS, int QPT, int BPE_, bool UNIQUE>
 struct GroupContents {
     static constexpr int BPE = BPE_;
