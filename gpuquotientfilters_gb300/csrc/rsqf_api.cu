@@ -70,11 +70,14 @@ __global__ void __launch_bounds__(1024) k_rsqf_scan_bases(const uint32_t *cnt, u
 // Buckets of lo < n <= cap items; a second launch with more shared memory
 // takes the few larger ones, so that two CTAs share an SM in the first.
 // 60.4M fingerprints, q = 26: one thread per quotient sorting its group, one
-// CTA per SM, took 852 us; this takes 335 us.
+// CTA per SM, took 852 us; this takes 335 us.  Ranking reads the square of a
+// group's size, so groups of more than SORT_BIG items are sorted by a thread
+// each.
 // With bmax non-null it also stores, per bucket, max(quotient_j - j) over
 // the bucket's items (j = index in the whole sorted array), the input of the
 // canonical-position scan.
 constexpr int SORT_THREADS = 512;
+constexpr uint32_t SORT_BIG = 48;
 __host__ __device__ inline size_t sort_smem_bytes(uint32_t tb, uint32_t cap)
 {
     size_t S = (size_t)1 << tb;
@@ -92,7 +95,7 @@ __global__ void __launch_bounds__(SORT_THREADS, 2) k_bucket_sort(const uint32_t 
     const uint32_t S = 1u << tb;
     uint32_t *s_cnt = smem_sort;
     uint32_t *s_it = smem_sort + (S / 2 + S / 32 + 8);
-    __shared__ uint32_t s_warp[33];
+    __shared__ uint32_t s_warp[33], s_big;
     const uint32_t b = blockIdx.x, n = src_base ? cnt[b] : min(cnt[b], stride);
     if (n > cap || (lo && n <= lo)) {  // the other launch's
         if (n > cap && last && threadIdx.x == 0) {
@@ -109,6 +112,7 @@ __global__ void __launch_bounds__(SORT_THREADS, 2) k_bucket_sort(const uint32_t 
         }
         return;
     }
+    if (threadIdx.x == 0) s_big = 0;
     for (uint32_t i = threadIdx.x; i < S / 2 + S / 32 + 8; i += SORT_THREADS) s_cnt[i] = 0;
     __syncthreads();
     for_each_item<SORT_THREADS>(src, s0, n, threadIdx.x,
@@ -158,6 +162,10 @@ __global__ void __launch_bounds__(SORT_THREADS, 2) k_bucket_sort(const uint32_t 
     for (uint32_t i = threadIdx.x; i < n; i += SORT_THREADS) {
         const uint32_t v = s_it[i], x = (v >> RSQF_R) & (S - 1);
         const uint32_t g0 = x ? cnt16_get(s_cnt, x - 1) : 0u, g1 = cnt16_get(s_cnt, x);
+        if (g1 - g0 > SORT_BIG) {
+            s_big = 1;
+            continue;
+        }
         uint32_t p = g0;
         for (uint32_t j = g0; j < g1; j++) {
             const uint32_t y = s_it[j];
@@ -166,6 +174,15 @@ __global__ void __launch_bounds__(SORT_THREADS, 2) k_bucket_sort(const uint32_t 
         dst[b0 + p] = v;
         m = max(m, (int32_t)(v >> RSQF_R) - (int32_t)(b0 + p));
     }
+    __syncthreads();
+    if (s_big)
+        for (uint32_t x = threadIdx.x; x < S; x += SORT_THREADS) {
+            const uint32_t g0 = x ? cnt16_get(s_cnt, x - 1) : 0u, g1 = cnt16_get(s_cnt, x);
+            if (g1 - g0 <= SORT_BIG) continue;
+            small_sort(s_it + g0, g1 - g0);
+            for (uint32_t i = g0; i < g1; i++) dst[b0 + i] = s_it[i];
+            m = max(m, (int32_t)(s_it[g0] >> RSQF_R) - (int32_t)(b0 + g0));
+        }
     int32_t tot;
     block_excl_max<SORT_THREADS>(m, reinterpret_cast<int32_t *>(s_warp), tot);
     if (threadIdx.x == 0) bmax[b] = tot;

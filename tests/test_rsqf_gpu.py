@@ -214,3 +214,23 @@ def test_rsqf8_width_limits(gqf, cuda):
         gqf.initCQFGPU(24, 8)  # q + 8 > 31
     with pytest.raises(gqf.GQFError):
         gqf.initCQFGPU(12, 6)
+
+
+@pytest.mark.parametrize("rbits", [5, 8])
+def test_rsqf_large_groups(gqf, cuda, rbits):
+    """Quotients of 47 to 1500 items, equal ones and different remainders
+    mixed: on both sides of the size from which a group is sorted by one
+    thread."""
+    q, rng = 14, np.random.default_rng(17)
+    cand = O.mt_keys(970, 1 << 21)
+    quot = O.aphash(cand, q, rbits) >> rbits
+    parts = [O.mt_keys(971, 6000)]
+    for x, size in ((40, 47), (700, 48), (1500, 49), (3000, 50), (5000, 200), (9000, 1500)):
+        mine = cand[quot == x]
+        parts += [np.repeat(mine[:3], size // 6), rng.choice(mine, size - 3 * (size // 6))]
+    keys = np.concatenate(parts)
+    keys = keys[rng.permutation(keys.size)]
+    f, o = RSQF(gqf, cuda, q, rbits), O.rsqf_new(q, rbits)
+    want = O.rsqf_insert_sorted(o, q, keys, rbits)
+    assert np.array_equal(f.insert(keys), want)
+    assert_same_blocks(f.blocks(), o, 17 + 8 * rbits)
