@@ -124,7 +124,8 @@ __device__ __forceinline__ void shift_right(const SlotTable<1> &v, uint32_t s, u
 }
 
 // Changes the bits `diff` of slot i's element (a word of 4 slot bytes inside
-// the table).
+// the table; k_del_units and k_ins_lists use this size only, the apply kernels
+// 8-byte words only).
 template <int BPE>
 __device__ __forceinline__ void xor_slot(const SlotTable<BPE> &v, uint32_t i, uint32_t diff)
 {
@@ -139,6 +140,25 @@ __device__ __forceinline__ void set_slot(const SlotTable<BPE> &v, uint32_t i, ui
 {
     xor_slot(v, i, (v.get(i) ^ e) & ~4u);
 }
+// Slots that one thread rewrites at the table's end, beside warps that change
+// neighbouring slots with xor_slot: the same word atomics wherever the word is
+// whole, single slots in the table's ragged last word, which xor_slot never
+// touches.
+template <int BPE>
+struct EndSlots {
+    const SlotTable<BPE> &v;
+    __device__ __forceinline__ uint32_t get(uint32_t i) const
+    {
+        if (BPE == 1) return __ldcg(v.t + i);
+        const uint32_t x = __ldcg(reinterpret_cast<const uint16_t *>(v.t) + i);
+        return ((x & 0xFFu) << 8) | (x >> 8);
+    }
+    __device__ __forceinline__ void put(uint32_t i, uint32_t e) const
+    {
+        if ((i | (4 / BPE - 1)) < v.nslots) xor_slot(v, i, get(i) ^ e);
+        else v.put(i, e);
+    }
+};
 constexpr int LIST_THREADS = 64;
 
 // ------------------------------------------------------------------ delete
@@ -377,7 +397,7 @@ __global__ void __launch_bounds__(LIST_THREADS) k_del_units(SlotTable<BPE> v, co
         if ((un.y | 3u) < v.nslots)
             del_unit_warp(v, claim, un.x, un.y);
         else if ((threadIdx.x & 31) == 0)
-            del_unit(v, [&](uint32_t t) { return (claim[t >> 4] >> (2 * (t & 15u))) & 1u; }, un.x, un.y);
+            del_unit(EndSlots<BPE>{v}, [&](uint32_t t) { return (claim[t >> 4] >> (2 * (t & 15u))) & 1u; }, un.x, un.y);
         __syncwarp();
     }
 }
@@ -670,7 +690,7 @@ __global__ void __launch_bounds__(INS_THREADS) k_ins_apply(SlotTable<BPE> v, uin
                 const bool head = (ent.y & INS_HEAD) != 0, newq = (ent.z & INS_NEWQ) != 0;
                 shift_right(v, ip, g, ((ent.x & ((1u << r) - 1u)) << 3) | (head ? 0u : 2u) | (ip != fq ? 1u : 0u),
                             head && !newq);
-                if (newq) xor_slot(v, fq, 4u);
+                if (newq) xorw(v, fq >> 3, 4ull << (8 * (fq & 7u)));  // (one word size per launch)
             }
         }
     }
@@ -771,7 +791,7 @@ __global__ void __launch_bounds__(LIST_THREADS) k_ins_lists(SlotTable<BPE> v, ui
         if ((e.z | 3u) < v.nslots)
             ins_group_warp(v, r, b, InsPos{e.x, e.y}, e.z, e.w, sc[threadIdx.x >> 5]);
         else if ((threadIdx.x & 31) == 0)
-            ins_group(v, r, b, InsPos{e.x, e.y}, e.z);
+            ins_group(EndSlots<BPE>{v}, r, b, InsPos{e.x, e.y}, e.z);
         __syncwarp();
     }
 }
