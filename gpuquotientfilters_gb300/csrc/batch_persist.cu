@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_mf_persistent(MfPara
             a.fix_cap = f.fix_cap;
             a.fix_soft = 1;
             a.err = p.err;
-            if (BPE == 1 && p.bitmap_ok) bucket_layout_set<THREADS, QPT, ListSource>(a, gb - f.bucket0);
+            if (BPE == 1 && p.bitmap_ok) bucket_layout_set<THREADS, QPT, OwnListSource>(a, gb - f.bucket0);
             else bucket_layout_body<THREADS, QPT, BPE>(a, gb - f.bucket0);
         }
         if (!grid_sync(x.bar, p.err)) return;

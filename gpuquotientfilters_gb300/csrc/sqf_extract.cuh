@@ -27,19 +27,19 @@ struct Counts3 {
 
 // Element values of 8 consecutive slots starting at slot s0 (zero past the
 // logical end).  One 8-byte load per 8 one-byte slots; two for 2-byte slots.
-template <int BPE>
+template <int BPE, bool NC>
 __device__ __forceinline__ void load8_elems(const uint8_t *t, uint32_t nslots, uint32_t nbytes, uint32_t s0,
                                             uint32_t e[8])
 {
     if (BPE == 1 && s0 + 8 <= nslots) {
-        uint64_t x = __ldg(reinterpret_cast<const unsigned long long *>(t + s0));
+        uint64_t x = ld_data<NC>(reinterpret_cast<const unsigned long long *>(t + s0));
 #pragma unroll
         for (int k = 0; k < 8; k++) e[k] = (uint32_t)(x >> (8 * k)) & 0xFFu;
         return;
     }
     if (BPE == 2 && s0 + 8 <= nslots && (size_t)(s0 + 8) * 2 <= nbytes) {
         const unsigned long long *p = reinterpret_cast<const unsigned long long *>(t + (size_t)s0 * 2);
-        uint64_t x0 = __ldg(p), x1 = __ldg(p + 1);
+        uint64_t x0 = ld_data<NC>(p), x1 = ld_data<NC>(p + 1);
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             e[k] = (((uint32_t)(x0 >> (16 * k)) & 0xFFu) << 8) | ((uint32_t)(x0 >> (16 * k + 8)) & 0xFFu);
@@ -78,11 +78,12 @@ struct ThreadSlots {
     uint32_t e[EXTRACT_WPT][8];
     uint32_t ne[EXTRACT_WPT], rs[EXTRACT_WPT], occ[EXTRACT_WPT];
     uint32_t s0;
+    template <bool NC>
     __device__ __forceinline__ void load(const uint8_t *t, uint32_t nslots, uint32_t nbytes, uint32_t tile)
     {
         s0 = tile * EXTRACT_TILE + threadIdx.x * (EXTRACT_WPT * 8);
 #pragma unroll
-        for (int w = 0; w < EXTRACT_WPT; w++) load8_elems<BPE>(t, nslots, nbytes, s0 + 8 * w, e[w]);
+        for (int w = 0; w < EXTRACT_WPT; w++) load8_elems<BPE, NC>(t, nslots, nbytes, s0 + 8 * w, e[w]);
 #pragma unroll
         for (int w = 0; w < EXTRACT_WPT; w++) masks_of(e[w], ne[w], rs[w], occ[w]);
     }
@@ -102,12 +103,12 @@ struct ThreadSlots {
 // Pass 1: per-tile counts.
 // When `dups` is non-null it is set to 1 if the table stores a fingerprint
 // twice: a continuation element whose remainder equals its predecessor's.
-template <int BPE>
+template <int BPE, bool NC = true>
 __device__ __forceinline__ void tile_counts(uint32_t tile, const uint8_t *t, uint32_t nslots, uint32_t nbytes,
                                             Counts3 *tiles, uint32_t *dups)
 {
     ThreadSlots<BPE> ts;
-    ts.load(t, nslots, nbytes, tile);
+    ts.template load<NC>(t, nslots, nbytes, tile);
     if (dups) {
         uint32_t prev = 0;
         if (ts.s0 > 0 && ts.s0 - 1 < nslots) {
@@ -265,12 +266,12 @@ __device__ __forceinline__ void flush_tile(const uint32_t *s_out, uint32_t cnt, 
 // Pass 2: positions of occupied slots, in slot order (Q[j] = quotient of
 // the j-th run).  A tile's entries are staged in shared memory and stored
 // coalesced.
-template <int BPE>
+template <int BPE, bool NC = true>
 __device__ __forceinline__ void occ_list(uint32_t tile, const uint8_t *t, uint32_t nslots, uint32_t nbytes,
                                          const Counts3 *tiles, uint32_t *Q, uint32_t *s_out)
 {
     ThreadSlots<BPE> ts;
-    ts.load(t, nslots, nbytes, tile);
+    ts.template load<NC>(t, nslots, nbytes, tile);
     const Counts3 ex = block_excl3(ts.totals());
     uint32_t o = ex.occ;
 #pragma unroll
@@ -298,12 +299,12 @@ __global__ void __launch_bounds__(EXTRACT_THREADS) k_occ_list(const uint8_t *__r
 
 // Pass 3: E[i] = fingerprint of the i-th stored element (staged per tile,
 // stored coalesced).
-template <int BPE>
+template <int BPE, bool NC = true>
 __device__ __forceinline__ void extract(uint32_t tile, const uint8_t *t, uint32_t nslots, uint32_t nbytes, uint32_t r,
                                         const Counts3 *tiles, const uint32_t *Q, uint32_t *E, uint32_t *s_out)
 {
     ThreadSlots<BPE> ts;
-    ts.load(t, nslots, nbytes, tile);
+    ts.template load<NC>(t, nslots, nbytes, tile);
     const Counts3 ex = block_excl3(ts.totals());
     uint32_t o = ex.ne;
     uint32_t runs_before = tiles[tile].rs + ex.rs;  // run starts strictly before this thread's slots

@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(FB_THREADS, 2) k_update_fallback(FallbackArgs 
     const uint32_t ntiles = (a.nslots + EXTRACT_TILE - 1) / EXTRACT_TILE;
     const uint32_t shift = a.r + a.tb, mask = (1u << (a.q + a.r)) - 1u;
     for (uint32_t u = blockIdx.x; u < ntiles; u += gridDim.x) {
-        tile_counts<BPE>(u, a.table, a.nslots, f.nbytes, f.tiles, nullptr);
+        tile_counts<BPE, false>(u, a.table, a.nslots, f.nbytes, f.tiles, nullptr);
         __syncthreads();
     }
     for (uint32_t i = gt; i < f.n; i += gn) atomicAdd(f.bcnt + ((aphash32(f.keys[i]) & mask) >> shift), 1u);
@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(FB_THREADS, 2) k_update_fallback(FallbackArgs 
     }
     if (!grid_sync(f.bar, a.err)) return;
     for (uint32_t u = blockIdx.x; u < ntiles; u += gridDim.x) {
-        occ_list<BPE>(u, a.table, a.nslots, f.nbytes, f.tiles, f.Q, s_out);
+        occ_list<BPE, false>(u, a.table, a.nslots, f.nbytes, f.tiles, f.Q, s_out);
         __syncthreads();
     }
     for (uint32_t i = gt; i < f.n; i += gn) {
@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(FB_THREADS, 2) k_update_fallback(FallbackArgs 
     }
     if (!grid_sync(f.bar, a.err)) return;
     for (uint32_t u = blockIdx.x; u < ntiles; u += gridDim.x) {
-        extract<BPE>(u, a.table, a.nslots, f.nbytes, a.r, f.tiles, f.Q, f.E, s_out);
+        extract<BPE, false>(u, a.table, a.nslots, f.nbytes, a.r, f.tiles, f.Q, f.E, s_out);
         __syncthreads();
     }
     if (!grid_sync(f.bar, a.err)) return;

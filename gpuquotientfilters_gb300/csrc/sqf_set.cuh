@@ -57,8 +57,8 @@ __device__ __forceinline__ uint32_t set_addr(uint32_t x) { return (x << 2) ^ ((x
 // f(item) for n items from items[start] (items 16-byte aligned), shared by
 // NT threads of which this is number t: single items up to the first and
 // from the last 16-byte boundary, 16-byte loads between.
-template <int NT, typename F>
-__device__ __forceinline__ void for_each_item(const uint32_t *__restrict__ items, size_t start, uint32_t n,
+template <int NT, bool NC = true, typename F>
+__device__ __forceinline__ void for_each_item(const uint32_t *items, size_t start, uint32_t n,
                                               uint32_t t, F &&f)
 {
     const uint32_t head = min(n, (uint32_t)(-(uint32_t)start & 3u)), nv = (n - head) >> 2, tail = head + 4 * nv;
@@ -66,7 +66,7 @@ __device__ __forceinline__ void for_each_item(const uint32_t *__restrict__ items
     const uint4 *v4 = reinterpret_cast<const uint4 *>(it + head);
     for (uint32_t j = t; j < nv; j += 2 * NT) {  // two loads in flight per thread
         const bool two = j + NT < nv;
-        const uint4 a = __ldg(v4 + j), b = two ? __ldg(v4 + j + NT) : make_uint4(0, 0, 0, 0);
+        const uint4 a = ld_data<NC>(v4 + j), b = two ? ld_data<NC>(v4 + j + NT) : make_uint4(0, 0, 0, 0);
         f(a.x);
         f(a.y);
         f(a.z);
@@ -78,8 +78,8 @@ __device__ __forceinline__ void for_each_item(const uint32_t *__restrict__ items
             f(b.w);
         }
     }
-    if (t < head) f(__ldg(it + t));
-    if (t < n - tail) f(__ldg(it + tail + t));
+    if (t < head) f(ld_data<NC>(it + t));
+    if (t < n - tail) f(ld_data<NC>(it + tail + t));
 }
 
 // One step of the layout map over consecutive quotients, relative to the
@@ -90,14 +90,14 @@ __device__ __forceinline__ void for_each_item(const uint32_t *__restrict__ items
 __device__ __forceinline__ int set_step(int u, int k) { return __viaddmax_s32(u, k - 1, k - 1); }
 
 // The bucket's fingerprints from lists: A (a table's extracted contents) and
-// B (the batch).
-template <int THREADS, int QPT>
-struct ListSource {
+// B (the batch).  NC: the lists are older than the launch.
+template <int THREADS, int QPT, bool NC>
+struct Lists {
     static constexpr uint32_t S = THREADS * QPT;
     const LayoutArgs &a;
     uint32_t na, nb;
     size_t abase, bbase;
-    __device__ __forceinline__ ListSource(const LayoutArgs &args, uint32_t b, uint8_t *) : a(args)
+    __device__ __forceinline__ Lists(const LayoutArgs &args, uint32_t b, uint8_t *) : a(args)
     {
         na = a.A.count(b);
         nb = a.B.count(b);
@@ -110,14 +110,18 @@ struct ListSource {
     template <int NT, typename F>
     __device__ __forceinline__ void table_items(uint32_t t, F &&f) const
     {
-        if (na) for_each_item<NT>(a.A.items, abase, na, t, [&](uint32_t v) { f((v >> SET_R) & (S - 1), v & 31u); });
+        if (na) for_each_item<NT, NC>(a.A.items, abase, na, t, [&](uint32_t v) { f((v >> SET_R) & (S - 1), v & 31u); });
     }
     template <int NT, typename F>
     __device__ __forceinline__ void batch_items(uint32_t t, F &&f) const
     {
-        for_each_item<NT>(a.B.items, bbase, nb, t, [&](uint32_t v) { f((v >> SET_R) & (S - 1), v & 31u); });
+        for_each_item<NT, NC>(a.B.items, bbase, nb, t, [&](uint32_t v) { f((v >> SET_R) & (S - 1), v & 31u); });
     }
 };
+template <int THREADS, int QPT>
+using ListSource = Lists<THREADS, QPT, true>;
+template <int THREADS, int QPT>
+using OwnListSource = Lists<THREADS, QPT, false>;
 
 // Contents of a bucket as remainder sets, fed by a source (lists, or tables).
 template <int THREADS, int QPT, template <int, int> class Source>
