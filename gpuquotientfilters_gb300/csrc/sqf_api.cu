@@ -70,17 +70,17 @@ __global__ void __launch_bounds__(1024) k_scan_bases(const uint32_t *cnt, uint32
 template <int BPE>
 static int extract_into(const uint8_t *table, uint32_t nslots, size_t nbytes, uint32_t r, const BucketGeom &g,
                         Counts3 *tiles, uint32_t *Q, uint32_t *E, uint32_t *base, uint32_t *cnt, uint32_t *dups,
-                        cudaStream_t s, const uint32_t *gate = nullptr)
+                        cudaStream_t s)
 {
     uint32_t ntiles = (nslots + EXTRACT_TILE - 1) / EXTRACT_TILE;
     count_launches(6);
-    k_tile_counts<BPE><<<ntiles, EXTRACT_THREADS, 0, s>>>(table, nslots, (uint32_t)nbytes, tiles, dups, gate);
-    k_scan_counts3<<<1, 1024, 0, s>>>(tiles, ntiles, gate);
-    k_occ_list<BPE><<<ntiles, EXTRACT_THREADS, 0, s>>>(table, nslots, (uint32_t)nbytes, tiles, Q, gate);
-    k_extract<BPE><<<ntiles, EXTRACT_THREADS, 0, s>>>(table, nslots, (uint32_t)nbytes, r, tiles, Q, E, gate);
+    k_tile_counts<BPE><<<ntiles, EXTRACT_THREADS, 0, s>>>(table, nslots, (uint32_t)nbytes, tiles, dups);
+    k_scan_counts3<<<1, 1024, 0, s>>>(tiles, ntiles);
+    k_occ_list<BPE><<<ntiles, EXTRACT_THREADS, 0, s>>>(table, nslots, (uint32_t)nbytes, tiles, Q);
+    k_extract<BPE><<<ntiles, EXTRACT_THREADS, 0, s>>>(table, nslots, (uint32_t)nbytes, r, tiles, Q, E);
     uint32_t grid = (g.nb + 1 + 255) / 256;
-    k_sorted_bounds<<<grid, 256, 0, s>>>(E, &tiles[ntiles].ne, g.nb, g.shift, base, cnt, gate);
-    k_bounds_to_counts<<<grid, 256, 0, s>>>(base, g.nb, cnt, gate);
+    k_sorted_bounds<<<grid, 256, 0, s>>>(E, &tiles[ntiles].ne, g.nb, g.shift, base, cnt);
+    k_bounds_to_counts<<<grid, 256, 0, s>>>(base, g.nb, cnt);
     GQF_CK(cudaGetLastError());
     return GQF_OK;
 }
@@ -123,97 +123,90 @@ static int bucket_batch(const uint32_t *keys, uint32_t n, const LayoutPlan &p, S
                             : bucket_batch_keys<SCATTER_THREADS, SCATTER_IPT>(keys, n, p, sc, exact, err, s);
 }
 
-// Asynchronous in-place update that could not place some bucket (*gate
-// set): reset what the general path's layout expects at zero -- look-back
-// descriptors, bucket ticket, fix-up count, duplicate flag, the call's error
-// word -- and clear the table's spill slots past the last bucket.  The
-// general path then rebuilds every slot from the snapshot's contents.
-__global__ void k_fallback_prepare(const uint32_t *__restrict__ gate, unsigned long long *status, uint32_t nb,
-                                   uint32_t *ticket, uint32_t *fix_cnt, uint32_t *dups, uint32_t *err,
-                                   uint8_t *tail, size_t tail_bytes)
-{
-    if (!*gate) return;
-    const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = i0; i < nb; i += step) status[i] = 0ull;
-    for (size_t i = i0; i < tail_bytes; i += step) tail[i] = 0;
-    if (i0 == 0) {
-        *ticket = 0;
-        *fix_cnt = 0;
-        *dups = 0;
-        *err = 0;
-    }
-}
-
+constexpr uint32_t ONE_LAUNCH_Q = 22;
 constexpr size_t SNAP_BESIDE = 16u << 20;  // table bytes from which a snapshot is copied on the side stream
 
-// Scratch bytes of rebuild() for an insert or delete of n keys (the same
-// sizing as below).
-static size_t update_scratch_bytes(uint32_t q, uint32_t r, uint32_t n)
+// What a rebuild runs and needs: A = current contents of the table (unless it
+// is a build), B = hashed batch keys or (two) the second table's contents.
+struct Rebuild {
+    bool needA, two;
+    bool set_ok;    // the layout from lists has set semantics (see LayoutArgs::set_ok)
+    bool in_place;  // one-byte slots, set semantics: decoded bucket by bucket from a snapshot
+    bool exact;     // exact bucket bases from the start
+    LayoutPlan p;
+    ScratchReq spec, req;  // scratch with speculative bucket strides, and as it runs otherwise
+    size_t bytes;
+};
+static Rebuild plan_rebuild(const SqfGeom &tg, uint32_t n, int op, int nodup, bool two, bool queued)
 {
-    const uint32_t nslots = gqf_sqf_num_slots(q);
-    const uint64_t expect = std::min<uint64_t>((uint64_t)(nslots * 0.9) + n, (uint64_t)nslots * 2);
-    LayoutPlan p = plan_layout(q, r, expect, n, true, false);
-    ScratchReq req{p.g.nb, (size_t)p.g.nb * p.stride, true, false, nslots};
-    size_t bytes = 0, bytes_exact = 0;
-    carve(nullptr, req, true, &bytes);
-    req.batch_items = std::max<size_t>(n, 1);
-    carve(nullptr, req, true, &bytes_exact);
-    return std::max(bytes, bytes_exact);
+    Rebuild b{};
+    b.needA = op != OP_BUILD;
+    b.two = two;
+    const bool update = op == OP_INSERT || op == OP_DELETE;
+    b.set_ok = tg.r == 5 && (((op == OP_BUILD || op == OP_MERGE) && nodup) || op == OP_INSERT);
+    b.in_place = tg.r == 5 && b.needA && (update || nodup);
+    // A timed build uses speculative bucket strides (one pass over the keys)
+    // and reruns with exact bucket bases if a bucket overflowed; the rerun
+    // rewrites the whole table from the keys.  Updates read the table, so
+    // they and all asynchronous calls bucket exactly.
+    b.exact = op != OP_BUILD || queued;
+    // expected items: the table holds at most nslots
+    const uint64_t expect = std::min<uint64_t>((b.needA ? (uint64_t)(tg.nslots * 0.9) : 0) +
+                                                   (two ? (uint64_t)(tg.nslots * 0.9) : n),
+                                               (uint64_t)tg.nslots * 2);
+    // an in-place update's batch keeps the large buckets (a layout bucket
+    // reads its part of one); a build's are the layout's
+    b.p = plan_layout(tg.q, tg.r, expect, two ? 0 : n, update || b.in_place, !b.in_place);
+    b.req = ScratchReq{b.p.g.nb, std::max<size_t>(n, 1), b.needA, two, tg.nslots};
+    // small filters are laid out in small buckets, which a nearly full table's
+    // spill can pass whole
+    b.req.every_fix = tg.q <= 22;
+    if ((op == OP_BUILD || op == OP_MERGE) && !b.set_ok) b.req.rem_bytes = tg.bpe;
+    b.spec = b.req;
+    if (!two) b.spec.batch_items = (size_t)b.p.g.nb * b.p.stride;
+    if (b.in_place) {
+        b.req.snap_bytes = tg.T;
+        b.req.upd_nb = 1u << (tg.q - update_tb(tg.q));
+        b.req.fallback = &tg;
+    }
+    carve(nullptr, b.req, true, &b.bytes);
+    if (!b.exact) {
+        size_t spec = 0;
+        carve(nullptr, b.spec, true, &spec);
+        b.bytes = std::max(b.bytes, spec);
+    }
+    return b;
 }
 
-// One rebuild: A = current contents of `table` (when the op needs them) or
-// of `table2`, B = hashed batch keys (or the second table's contents).
 template <int BPE>
 static int rebuild(const gqf_sqf *qf, const gqf_sqf *qf2, const uint32_t *keys, uint32_t n, int op, int nodup,
                    cudaStream_t s, float *ms)
 {
     const SqfGeom tg = geom_of(qf);
-    const bool needA = op != OP_BUILD;
-    const bool bFromTable = qf2 != nullptr;
-    // expected items: the table holds at most nslots
-    uint64_t expect = std::min<uint64_t>((needA ? (uint64_t)(tg.nslots * 0.9) : 0) + (bFromTable ? (uint64_t)(tg.nslots * 0.9) : n),
-                                         (uint64_t)tg.nslots * 2);
-    // r = 5 and set semantics: remainder sets (see LayoutArgs::set_ok)
-    const bool set_ok = tg.r == 5 && (((op == OP_BUILD || op == OP_MERGE) && nodup) || op == OP_INSERT);
+    Rebuild b = plan_rebuild(tg, n, op, nodup, qf2 != nullptr, ms == nullptr);
+    const LayoutPlan &p = b.p;
     // duplicates in the table veto the set mode of an insert
-    const bool update = op == OP_INSERT;
-    // In-place update: on one-byte slots with set semantics the old contents
-    // are decoded bucket by bucket from a snapshot of the table (no
-    // extraction pass, see LayoutArgs).  If a bucket cannot be decoded (a
-    // table holding duplicate fingerprints, a run past its slice), the op
-    // reruns the general way from the snapshot: a synchronous call decides on
-    // the host; an asynchronous one queues the general path behind the
-    // in-place kernels with every launch gated on the device-side failure
-    // flag, so it costs only empty launches when the in-place path held.
-    const bool fused = BPE == 1 && set_ok && needA;
-    // an update's batch keeps the large buckets (a layout bucket reads its
-    // part of one); a build's are the layout's
-    LayoutPlan p = plan_layout(tg.q, tg.r, expect, bFromTable ? 0 : n, op == OP_INSERT, !fused);
-    ScratchReq req{p.g.nb, bFromTable ? 0 : (size_t)p.g.nb * p.stride, needA, bFromTable, tg.nslots};
-    // small filters are laid out in small buckets, which a nearly full table's
-    // spill can pass whole
-    req.every_fix = tg.q <= 22;
-    if ((op == OP_BUILD || op == OP_MERGE) && !set_ok) req.rem_bytes = BPE;
-    int dev = current_device();
-    Arena &ar = arena(dev, s);
+    const bool insert = op == OP_INSERT;
+    Arena &ar = arena(current_device(), s);
     std::lock_guard<std::mutex> lk(ar.mu);
-    size_t bytes = 0;
-    carve(nullptr, req, true, &bytes);
-    // exact-mode batch needs n items at most
-    size_t bytes_exact = 0;
-    ScratchReq req_exact = req;
-    req_exact.batch_items = std::max<size_t>(n, 1);
-    carve(nullptr, req_exact, true, &bytes_exact);
-    ScratchReq req_fused = req_exact;
-    req_fused.snap_bytes = tg.T;
-    req_fused.upd_nb = 1u << (tg.q - update_tb(tg.q));
-    size_t bytes_fused = 0;
-    if (fused) carve(nullptr, req_fused, true, &bytes_fused);
-    void *base = arena_reserve(ar, std::max(std::max(bytes, bytes_exact), bytes_fused));
+    void *base = arena_reserve(ar, b.bytes);
     if (!base) return GQF_ERR_NOMEM;
-    float ms_fused = 0.0f;
-    if (fused) {
-        Scratch sc = carve(base, req_fused, false, &bytes);
+    size_t bytes = 0;
+    float ms_first = 0.0f;
+    FallbackArgs behind{};
+    // In-place update: the old contents are decoded bucket by bucket from a
+    // snapshot of the table (no extraction pass, see LayoutArgs).  If a bucket
+    // cannot be decoded (a table holding duplicate fingerprints, a run past
+    // its slice), the op is done the general way from the snapshot: a
+    // synchronous call decides on the host; behind an asynchronous one it is
+    // queued, and does nothing unless the device-side failure flag is set.  On
+    // tables up to ONE_LAUNCH_Q that is one cooperative launch; on larger ones
+    // the layout is a launch of its own, which uses the whole GPU (q = 24,
+    // overfull: 0.5 ms against 3.2).  A bucket that its shared memory cannot
+    // sort (a fingerprint with tens of thousands of copies) is left to another
+    // cooperative launch, which has more.
+    if (b.in_place) {
+        Scratch sc = carve(base, b.req, false, &bytes);
         int st = call_begin(ar, s, ms != nullptr);
         if (st) return st;
         // a large snapshot is copied on the side stream while the batch is
@@ -230,7 +223,7 @@ static int rebuild(const gqf_sqf *qf, const gqf_sqf *qf2, const uint32_t *keys, 
             GQF_CK(cudaMemcpyAsync(sc.snap, qf->table, tg.T, cudaMemcpyDeviceToDevice, s));
         }
         GQF_CK(cudaMemsetAsync(sc.bcnt, 0, sc.ctrl_bytes, s));
-        BucketSrc A{nullptr, nullptr, 0, nullptr}, B{nullptr, nullptr, 0, nullptr};
+        BucketSrc B{nullptr, nullptr, 0, nullptr};
         if (n) {
             st = bucket_batch(keys, n, p, sc, true, ar.err, s);
             if (st) return st;
@@ -241,60 +234,66 @@ static int rebuild(const gqf_sqf *qf, const gqf_sqf *qf2, const uint32_t *keys, 
         const uint8_t *src2 = !qf2 ? nullptr : qf2->table == qf->table ? sc.snap : qf2->table;
         st = launch_update(p, tg, qf->table, src2, B, op, sc, ar.err, s);
         if (st) return st;
+        FallbackArgs &f = sc.fb;
+        f.gate = sc.fused_fail;
+        f.gate_bits = ~0u;
+        f.src = sc.snap;
+        f.src2 = src2;
+        f.keys = keys;
+        f.n = n;
+        f.tiles = sc.tiles;
+        f.Q = sc.Q;
+        f.E = sc.E;
+        f.E2 = sc.E2;
+        f.bitems = sc.bitems;
         if (!ms) {
-            // the general path, gated on the failure flag: contents from the
-            // snapshot, the bucketed batch as it stands
-            const DeviceInfo &di = device_info(current_device());
-            const size_t tail = (size_t)(1u << tg.q) * BPE;
-            count_launches(1);
-            k_fallback_prepare<<<di.sms * 4, 256, 0, s>>>(sc.fused_fail, sc.status, p.g.nb, sc.ticket, sc.fix_cnt,
-                                                           sc.a_dups, ar.err, qf->table + tail,
-                                                           tg.T > tail ? tg.T - tail : 0);
-            GQF_CK(cudaGetLastError());
-            st = extract_into<BPE>(sc.snap, tg.nslots, tg.T, tg.r, p.g, sc.tiles, sc.Q, sc.E, sc.abase, sc.acnt,
-                                   update ? sc.a_dups : nullptr, s, sc.fused_fail);
-            if (st) return st;
-            A = BucketSrc{sc.E, sc.abase, 0, sc.acnt};
-            if (src2) {
-                st = extract_into<BPE>(src2, tg.nslots, tg.T, tg.r, p.g, sc.tiles, sc.Q, sc.E2, sc.a2base, sc.a2cnt,
-                                       nullptr, s, sc.fused_fail);
+            if (tg.q > ONE_LAUNCH_Q) {
+                FallbackArgs l = f;
+                l.n = 0;
+                l.lay.status = sc.status;
+                l.lay.ticket = sc.ticket;
+                l.lay.fix_cnt = sc.fix_cnt;
+                l.abase = sc.abase;
+                l.acnt = sc.acnt;
+                l.bbase = sc.a2base;
+                l.b2cnt = sc.a2cnt;
+                st = launch_fallback<BPE>(l, tg, qf->table, op, nodup, ar.err, s, &p.g);
                 if (st) return st;
-                B = BucketSrc{sc.E2, sc.a2base, 0, sc.a2cnt};
+                if (src2) B = BucketSrc{sc.E2, sc.a2base, 0, sc.a2cnt};
+                st = launch_layout<BPE>(p, tg, qf->table, BucketSrc{sc.E, sc.abase, 0, sc.acnt}, B, op, nodup, false,
+                                        nullptr, sc, ar.err, s, sc.fused_fail);
+                if (st) return st;
+                f.gate = ar.err;
+                f.gate_bits = DEV_ERR_BUCKET_CAP;
             }
-            st = launch_layout<BPE>(p, tg, qf->table, A, B, op, nodup, set_ok, update ? sc.a_dups : nullptr, sc,
-                                    ar.err, s, sc.fused_fail);
-            if (st) return st;
-            return call_end(ar, s, nullptr);
+            if (tg.q <= ONE_LAUNCH_Q || op != OP_MERGE)
+                st = launch_fallback<BPE>(f, tg, qf->table, op, nodup, ar.err, s);
+            return st ? st : call_end(ar, s, nullptr);
         }
         uint32_t rep[2];
         st = call_report(ar, s, sc.fused_fail, rep);
         if (st) return st;
-        const uint32_t e = rep[0], fail = rep[1];
-        GQF_CK(cudaEventElapsedTime(&ms_fused, ar.ev0, ar.ev1));
-        if (!fail) {
-            *ms = ms_fused;
-            return dev_err_to_status(e);
+        GQF_CK(cudaEventElapsedTime(&ms_first, ar.ev0, ar.ev1));
+        if (!rep[1]) {
+            *ms = ms_first;
+            return dev_err_to_status(rep[0]);
         }
-        GQF_CK(cudaMemcpy(qf->table, sc.snap, tg.T, cudaMemcpyDeviceToDevice));
+        behind = f;
+        GQF_CK(cudaMemcpyAsync(qf->table, sc.snap, tg.T, cudaMemcpyDeviceToDevice, s));
     }
-    // A timed build uses speculative bucket strides (one pass over the keys)
-    // and reruns with exact bucket bases if a bucket overflowed; the rerun
-    // rewrites the whole table from the keys.  Updates read the table, so
-    // they and all asynchronous calls bucket exactly.
-    bool exact = !(op == OP_BUILD && ms != nullptr);
-    for (int attempt = 0; attempt < 2; attempt++) {
-        Scratch sc = carve(base, exact ? req_exact : req, false, &bytes);
+    for (bool exact = b.exact;; exact = true) {
+        Scratch sc = carve(base, exact ? b.req : b.spec, false, &bytes);
         int st = call_begin(ar, s, ms != nullptr);
         if (st) return st;
         GQF_CK(cudaMemsetAsync(sc.bcnt, 0, sc.ctrl_bytes, s));  // counters, look-back, ticket, fix-ups
         BucketSrc A{nullptr, nullptr, 0, nullptr}, B{nullptr, nullptr, 0, nullptr};
-        if (needA) {
+        if (b.needA) {
             st = extract_into<BPE>(qf->table, tg.nslots, tg.T, tg.r, p.g, sc.tiles, sc.Q, sc.E, sc.abase, sc.acnt,
                                    sc.a_dups, s);
             if (st) return st;
             A = BucketSrc{sc.E, sc.abase, 0, sc.acnt};
         }
-        if (bFromTable) {
+        if (b.two) {
             st = extract_into<BPE>(qf2->table, tg.nslots, tg.T, tg.r, p.g, sc.tiles, sc.Q, sc.E2, sc.a2base, sc.a2cnt,
                                    nullptr, s);
             if (st) return st;
@@ -304,29 +303,64 @@ static int rebuild(const gqf_sqf *qf, const gqf_sqf *qf2, const uint32_t *keys, 
             if (st) return st;
             B = exact ? BucketSrc{sc.bitems, sc.bbase, 0, sc.bcnt} : BucketSrc{sc.bitems, nullptr, p.stride, sc.bcnt};
         }
-        st = launch_layout<BPE>(p, tg, qf->table, A, B, op, nodup, set_ok, update ? sc.a_dups : nullptr, sc, ar.err, s);
+        st = launch_layout<BPE>(p, tg, qf->table, A, B, op, nodup, b.set_ok, insert ? sc.a_dups : nullptr, sc, ar.err,
+                                s);
         if (st) return st;
         if (!ms) return call_end(ar, s, nullptr);
         // synchronous: look at the error word before deciding
         uint32_t rep[2];
         st = call_report(ar, s, nullptr, rep);
         if (st) return st;
-        const uint32_t e = rep[0];
-        if ((e & DEV_ERR_BUCKET_OVER) && !exact) {
-            exact = true;
-            continue;
-        }
+        if ((rep[0] & DEV_ERR_BUCKET_OVER) && !exact) continue;
         GQF_CK(cudaEventElapsedTime(ms, ar.ev0, ar.ev1));
-        *ms += ms_fused;
-        return dev_err_to_status(e);
+        *ms += ms_first;
+        if ((rep[0] & DEV_ERR_BUCKET_CAP) && b.in_place) {
+            ms_first = *ms;
+            behind.gate = ar.err;  // (holds the bit)
+            behind.gate_bits = DEV_ERR_BUCKET_CAP;
+            GQF_CK(cudaEventRecord(ar.ev0, s));
+            st = launch_fallback<BPE>(behind, tg, qf->table, op, nodup, ar.err, s);
+            if (st) return st;
+            st = call_end(ar, s, ms);
+            *ms += ms_first;
+            return st;
+        }
+        return dev_err_to_status(rep[0]);
     }
-    return GQF_ERR_FULL;
 }
 
-// An insert of at most one key per 16 quotients, and every delete
-// (sqf_update.cuh), with the general path behind it on the device.  Larger
-// inserts connect ever longer runs of clusters and are rebuilt instead.
-static bool insert_is_local(uint32_t q, uint32_t n) { return (uint64_t)n * 16 <= (1ull << q); }
+// ------------------------------------------------------------- update routes
+// All deletes, and inserts of at most a key per 16 quotients, touch only the
+// clusters they change (sqf_update.cuh); larger inserts update the whole table
+// in place.
+static uint32_t local_max_keys(uint32_t q, uint32_t, int op) { return op == OP_DELETE ? 0x7FFFFFFFu : 1u << (q - 4); }
+
+// Scratch bytes of an insert or delete of up to n keys, whichever way it goes.
+static size_t update_scratch_bytes(const SqfGeom &tg, uint32_t n)
+{
+    size_t most = 0;
+    for (int op : {OP_INSERT, OP_DELETE}) {
+        most = std::max(most, local_update_bytes(tg, std::min(n, local_max_keys(tg.q, tg.r, op)), op));
+        for (bool queued : {false, true})
+            most = std::max(most, plan_rebuild(tg, n, op, op == OP_INSERT, false, queued).bytes);
+    }
+    return most;
+}
+
+template <int BPE>
+static int update_t(const gqf_sqf *qf, const uint32_t *keys, uint32_t n, int op, cudaStream_t s, float *ms)
+{
+    float ms_local = 0.0f;
+    if (n <= local_max_keys(qf->qbits, qf->rbits, op)) {  // (and empty batches)
+        bool far = false;
+        const int st = local_update<BPE>(qf, keys, n, op, s, ms, &far);
+        if (st || !far) return st;
+        ms_local = *ms;
+    }
+    const int st = rebuild<BPE>(qf, nullptr, keys, n, op, op == OP_INSERT ? 1 : 0, s, ms);
+    if (ms) *ms += ms_local;
+    return st;
+}
 
 // Sorted and unsorted lookups alike: results go to the queries' input positions
 // either way (the reference sorts them back by index, quotientFilter.cu:
@@ -466,7 +500,10 @@ unsigned int gqf_sqf_num_slots(unsigned int q) { return (unsigned int)((double)(
 size_t gqf_sqf_update_workspace_bytes(unsigned int q, unsigned int r, int n)
 {
     if (!qr_ok(q, r) || n < 0) return 0;
-    return align_up(update_scratch_bytes(q, r, (uint32_t)n), 1u << 20);
+    gqf_sqf f{};
+    f.qbits = q;
+    f.rbits = r;
+    return align_up(update_scratch_bytes(geom_of(&f), (uint32_t)n), 1u << 20);
 }
 
 int gqf_sqf_init(gqf_sqf *qf, unsigned int q, unsigned int r)
@@ -516,16 +553,13 @@ int gqf_sqf_bulk_build_noalloc(const gqf_sqf *qf, int n, const uint32_t *d_keys,
 int gqf_sqf_insert(const gqf_sqf *qf, int n, const uint32_t *d_keys, void *stream, float *ms)
 {
     if (!sqf_ok(qf) || n < 0 || (n > 0 && !d_keys)) return GQF_ERR_ARG;
-    if (insert_is_local(qf->qbits, (uint32_t)n))
-        return BPE_DISPATCH(qf, local_update, qf, d_keys, (uint32_t)n, OP_INSERT, static_cast<cudaStream_t>(stream), ms);
-    return BPE_DISPATCH(qf, rebuild, qf, nullptr, d_keys, (uint32_t)n, OP_INSERT, 1, static_cast<cudaStream_t>(stream),
-                        ms);
+    return BPE_DISPATCH(qf, update_t, qf, d_keys, (uint32_t)n, OP_INSERT, static_cast<cudaStream_t>(stream), ms);
 }
 
 int gqf_sqf_delete(const gqf_sqf *qf, int n, const uint32_t *d_keys, void *stream, float *ms)
 {
     if (!sqf_ok(qf) || n < 0 || (n > 0 && !d_keys)) return GQF_ERR_ARG;
-    return BPE_DISPATCH(qf, local_update, qf, d_keys, (uint32_t)n, OP_DELETE, static_cast<cudaStream_t>(stream), ms);
+    return BPE_DISPATCH(qf, update_t, qf, d_keys, (uint32_t)n, OP_DELETE, static_cast<cudaStream_t>(stream), ms);
 }
 
 int gqf_sqf_insert_via_merge(const gqf_sqf *qf, const uint32_t *d_old, int n_old, const uint32_t *d_new, int n_new,

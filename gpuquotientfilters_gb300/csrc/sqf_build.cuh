@@ -453,9 +453,9 @@ struct LayoutArgs {
     const uint8_t *src_table = nullptr, *src2 = nullptr;
     uint32_t sub = 0;
     uint32_t *fused_fail = nullptr;
-    // When set, the launch does nothing unless *gate is nonzero (the general
-    // path queued behind an asynchronous in-place update, run only if that
-    // update could not place some bucket).
+    // When set, k_bucket_layout does nothing unless *gate is nonzero (the
+    // general path queued behind an asynchronous in-place update of a large
+    // table, run only if that update could not place some bucket).
     const uint32_t *gate = nullptr;
 };
 
@@ -800,9 +800,15 @@ __global__ void __launch_bounds__(THREADS, (THREADS >= 1024 ? 1 : 2)) k_bucket_l
     if (a.gate && !*a.gate) return;
     if (a.set_ok && !*a.a_dups) return;  // done by k_set_layout
     __shared__ uint32_t s_ticket;
-    if (threadIdx.x == 0) s_ticket = atomicAdd(a.ticket, 1u);
-    __syncthreads();
-    bucket_layout_body<THREADS, QPT_, BPE>(a, s_ticket);
+    for (;;) {  // (a gated launch has fewer CTAs than buckets)
+        if (threadIdx.x == 0) s_ticket = atomicAdd(a.ticket, 1u);
+        __syncthreads();
+        const uint32_t b = s_ticket;
+        if (b >= a.nb) break;
+        bucket_layout_body<THREADS, QPT_, BPE>(a, b);
+        if (!a.gate) break;
+        __syncthreads();
+    }
 }
 
 template <int BPE>

@@ -25,6 +25,17 @@ struct Counts3 {
     uint32_t ne, rs, occ;  // non-empty, run starts, occupied
 };
 
+// f(tile) for the CTA's tiles.
+template <typename F>
+__device__ __forceinline__ void for_each_tile(uint32_t nslots, F &&f)
+{
+    const uint32_t ntiles = (nslots + EXTRACT_TILE - 1) / EXTRACT_TILE;
+    for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        f(tile);
+        __syncthreads();
+    }
+}
+
 // Element values of 8 consecutive slots starting at slot s0 (zero past the
 // logical end).  One 8-byte load per 8 one-byte slots; two for 2-byte slots.
 template <int BPE, bool NC>
@@ -154,19 +165,15 @@ __device__ __forceinline__ void tile_counts(uint32_t tile, const uint8_t *t, uin
 template <int BPE>
 __global__ void __launch_bounds__(EXTRACT_THREADS) k_tile_counts(const uint8_t *__restrict__ t, uint32_t nslots,
                                                                 uint32_t nbytes, Counts3 *__restrict__ tiles,
-                                                                uint32_t *__restrict__ dups,
-                                                                const uint32_t *__restrict__ gate = nullptr)
+                                                                uint32_t *__restrict__ dups)
 {
-    if (gate && !*gate) return;
-    tile_counts<BPE>(blockIdx.x, t, nslots, nbytes, tiles, dups);
+    for_each_tile(nslots, [&](uint32_t tile) { tile_counts<BPE>(tile, t, nslots, nbytes, tiles, dups); });
 }
 
 // Exclusive scan of the tile counts by one CTA; total written at
 // tiles[ntiles].  Each thread loads its run of tiles with independent loads.
-static __global__ void __launch_bounds__(1024) k_scan_counts3(Counts3 *tiles, uint32_t ntiles,
-                                                       const uint32_t *__restrict__ gate = nullptr)
+static __global__ void __launch_bounds__(1024) k_scan_counts3(Counts3 *tiles, uint32_t ntiles)
 {
-    if (gate && !*gate) return;
     __shared__ uint32_t sw[3][32];
     const uint32_t per = (ntiles + 1023) / 1024;
     const uint32_t beg = min(ntiles, threadIdx.x * per), end = min(ntiles, beg + per);
@@ -289,12 +296,10 @@ __device__ __forceinline__ void occ_list(uint32_t tile, const uint8_t *t, uint32
 template <int BPE>
 __global__ void __launch_bounds__(EXTRACT_THREADS) k_occ_list(const uint8_t *__restrict__ t, uint32_t nslots,
                                                              uint32_t nbytes, const Counts3 *__restrict__ tiles,
-                                                             uint32_t *__restrict__ Q,
-                                                             const uint32_t *__restrict__ gate = nullptr)
+                                                             uint32_t *__restrict__ Q)
 {
-    if (gate && !*gate) return;
     __shared__ uint32_t s_out[EXTRACT_TILE];
-    occ_list<BPE>(blockIdx.x, t, nslots, nbytes, tiles, Q, s_out);
+    for_each_tile(nslots, [&](uint32_t tile) { occ_list<BPE>(tile, t, nslots, nbytes, tiles, Q, s_out); });
 }
 
 // Pass 3: E[i] = fingerprint of the i-th stored element (staged per tile,
@@ -327,20 +332,16 @@ template <int BPE>
 __global__ void __launch_bounds__(EXTRACT_THREADS) k_extract(const uint8_t *__restrict__ t, uint32_t nslots,
                                                             uint32_t nbytes, uint32_t r,
                                                             const Counts3 *__restrict__ tiles,
-                                                            const uint32_t *__restrict__ Q, uint32_t *__restrict__ E,
-                                                            const uint32_t *__restrict__ gate = nullptr)
+                                                            const uint32_t *__restrict__ Q, uint32_t *__restrict__ E)
 {
-    if (gate && !*gate) return;
     __shared__ uint32_t s_out[EXTRACT_TILE];
-    extract<BPE>(blockIdx.x, t, nslots, nbytes, r, tiles, Q, E, s_out);
+    for_each_tile(nslots, [&](uint32_t tile) { extract<BPE>(tile, t, nslots, nbytes, r, tiles, Q, E, s_out); });
 }
 
 // Bucket bounds of a sorted fingerprint list: base[b] = lower_bound(b << shift).
 static __global__ void k_sorted_bounds(const uint32_t *__restrict__ E, const uint32_t *__restrict__ m_ptr, uint32_t nb,
-                                       uint32_t shift, uint32_t *__restrict__ base, uint32_t *__restrict__ cnt,
-                                       const uint32_t *__restrict__ gate = nullptr)
+                                       uint32_t shift, uint32_t *__restrict__ base, uint32_t *__restrict__ cnt)
 {
-    if (gate && !*gate) return;
     const uint32_t m = *m_ptr;
     for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b <= nb; b += gridDim.x * blockDim.x) {
         uint64_t key = (uint64_t)b << shift;
@@ -353,10 +354,8 @@ static __global__ void k_sorted_bounds(const uint32_t *__restrict__ E, const uin
         base[b] = lo;
     }
 }
-static __global__ void k_bounds_to_counts(const uint32_t *__restrict__ base, uint32_t nb, uint32_t *__restrict__ cnt,
-                                          const uint32_t *__restrict__ gate = nullptr)
+static __global__ void k_bounds_to_counts(const uint32_t *__restrict__ base, uint32_t nb, uint32_t *__restrict__ cnt)
 {
-    if (gate && !*gate) return;
     for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x)
         cnt[b] = base[b + 1] - base[b];
 }

@@ -13,6 +13,8 @@
 #include "host_common.cuh"
 #include "sqf_build.cuh"
 #include "sqf_extract.cuh"
+#include "sqf_fallback.cuh"
+#include "sqf_walk.cuh"
 
 namespace gqf {
 
@@ -86,6 +88,7 @@ struct Scratch {
     uint32_t *a_dups;  // table holds duplicate fingerprints (set by extraction)
     uint32_t *fused_fail;  // the in-place update could not decode some bucket
     uint8_t *snap;         // table snapshot of the in-place update
+    FallbackArgs fb;       // the rebuild behind a queued one
     uint32_t *bbase;  // nb+1: exact batch bases
     uint32_t *fix_list;
     uint32_t fix_cap;
@@ -108,7 +111,26 @@ struct ScratchReq {
     uint32_t upd_nb = 0;    // and its layout buckets
     bool every_fix = false; // room for a fix-up of every quotient
     uint32_t rem_bytes = 0; // k_group_layout: scratch bytes per item
+    const SqfGeom *fallback = nullptr;  // in-place update: the rebuild behind it
 };
+
+inline uint32_t fallback_buckets(uint32_t q) { return q > FB_TB ? 1u << (q - FB_TB) : 1u; }
+// The rebuild's own buffers, apart from the lists (tiles, Q, E, E2, bitems)
+// and the words that start at zero.
+template <typename C>
+void carve_fallback(C &c, FallbackArgs &f, const SqfGeom &tg, bool two)
+{
+    const uint32_t nb = fallback_buckets(tg.q);
+    f.lay.status = c.template take<unsigned long long>(nb);
+    f.lay.ticket = c.template take<uint32_t>(1, 4);
+    f.lay.fix_cnt = c.template take<uint32_t>(1, 4);
+    f.bcnt = c.template take<uint32_t>(nb);
+    f.bfill = c.template take<uint32_t>(nb);
+    f.bbase = c.template take<uint32_t>(nb);
+    f.abase = c.template take<uint32_t>(nb);
+    f.acnt = c.template take<uint32_t>(nb);
+    if (two) f.b2cnt = c.template take<uint32_t>(nb);
+}
 
 inline Scratch carve(void *base, const ScratchReq &r, bool sizing_only, size_t *bytes_out)
 {
@@ -121,6 +143,7 @@ inline Scratch carve(void *base, const ScratchReq &r, bool sizing_only, size_t *
         s.fix_cnt = c.template take<uint32_t>(1, 4);
         s.a_dups = c.template take<uint32_t>(1, 4);
         s.fused_fail = c.template take<uint32_t>(1, 4);
+        s.fb.bar = c.template take<uint32_t>(4, 4);
         s.ctrl_bytes = c.off;
         s.bbase = c.template take<uint32_t>(nb + 1);
         s.fix_cap = std::max<uint32_t>(65536u, r.every_fix ? r.nslots : r.nslots / 8);
@@ -144,6 +167,7 @@ inline Scratch carve(void *base, const ScratchReq &r, bool sizing_only, size_t *
             }
         }
         s.snap = r.snap_bytes ? c.template take<uint8_t>(r.snap_bytes) : nullptr;
+        if (r.fallback) carve_fallback(c, s.fb, *r.fallback, r.extract2);
     };
     if (sizing_only) {
         Sizer z;
@@ -157,7 +181,8 @@ inline Scratch carve(void *base, const ScratchReq &r, bool sizing_only, size_t *
     return s;
 }
 
-// Bucket layout of A and B into the table, fix-ups included (sqf_layout.cuh).
+// Bucket layout of A and B into the table, fix-ups included (sqf_layout.cuh);
+// with a gate, by the general kernel, if *gate is set.
 template <int BPE>
 int launch_layout(const LayoutPlan &p, const SqfGeom &tg, uint8_t *table, const BucketSrc &A, const BucketSrc &B,
                   int op, int nodup, bool set_ok, const uint32_t *a_dups, Scratch &sc, uint32_t *err, cudaStream_t s,
@@ -165,8 +190,16 @@ int launch_layout(const LayoutPlan &p, const SqfGeom &tg, uint8_t *table, const 
 // In-place update of one-byte slots (sqf_inplace.cu).
 int launch_update(const LayoutPlan &p, const SqfGeom &tg, uint8_t *table, const uint8_t *src2, const BucketSrc &B,
                   int op, Scratch &sc, uint32_t *err, cudaStream_t s);
-// Cluster-local insert or delete (sqf_local.cu).
+// Cluster-local insert or delete (sqf_local.cu).  A synchronous call on
+// one-byte slots that met a stretch too long to walk leaves the table as it
+// was and sets *far; behind the others the rebuild runs on the device.
 template <int BPE>
-int local_update(const gqf_sqf *qf, const uint32_t *keys, uint32_t n, int op, cudaStream_t s, float *ms);
+int local_update(const gqf_sqf *qf, const uint32_t *keys, uint32_t n, int op, cudaStream_t s, float *ms, bool *far);
+size_t local_update_bytes(const SqfGeom &tg, uint32_t n, int op);
+// The gated rebuild: gate, src, src2, snap, keys, n and the buffers are set.
+// With `lists`, only the old contents' lists, in buckets of that geometry.
+template <int BPE>
+int launch_fallback(FallbackArgs &f, const SqfGeom &tg, uint8_t *table, int op, int nodup, uint32_t *err,
+                    cudaStream_t s, const BucketGeom *lists = nullptr);
 
 }  // namespace gqf

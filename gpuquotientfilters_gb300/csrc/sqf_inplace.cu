@@ -1,12 +1,23 @@
-// In-place merges and large inserts of one-byte slots.
+// In-place merges, inserts and deletes of one-byte slots.
 #include "sqf_host.cuh"
 
 namespace gqf {
 
+template <int THREADS, int QPT>
+static cudaError_t launch_shape(const LayoutArgs &a, size_t smem, cudaStream_t s)
+{
+    auto kernel = a.src2              ? k_set_update<THREADS, QPT, UPDATE_TWO>
+                  : a.op == OP_DELETE ? k_set_update<THREADS, QPT, UPDATE_DEL>
+                                      : k_set_update<THREADS, QPT, UPDATE_ADD>;
+    const cudaError_t e = set_smem(kernel, smem);
+    if (e == cudaSuccess) kernel<<<a.nb, THREADS, smem, s>>>(a);
+    return e;
+}
+
 // In-place update of one-byte slots: old contents from the snapshot (and
 // `src2`), batch buckets of geometry p.
 int launch_update(const LayoutPlan &p, const SqfGeom &tg, uint8_t *table, const uint8_t *src2,
-                         const BucketSrc &B, int op, Scratch &sc, uint32_t *err, cudaStream_t s)
+                  const BucketSrc &B, int op, Scratch &sc, uint32_t *err, cudaStream_t s)
 {
     const size_t tail = (size_t)1 << tg.q;
     if (tg.T > tail) GQF_CK(cudaMemsetAsync(table + tail, 0, tg.T - tail, s));
@@ -37,23 +48,18 @@ int launch_update(const LayoutPlan &p, const SqfGeom &tg, uint8_t *table, const 
     const int threads = (int)layout_threads(a.tb);
     const size_t smem = set_update_smem(a.tb, threads, src2 != nullptr);
     cudaError_t e = cudaSuccess;
-    auto go = [&](auto one, auto two) {
-        auto kernel = src2 ? two : one;
-        e = set_smem(kernel, smem);
-        if (e == cudaSuccess) kernel<<<a.nb, threads, smem, s>>>(a);
-    };
     switch (a.tb) {
-    case 13: go(k_set_update<256, 32, false>, k_set_update<256, 32, true>); break;
-    case 12: go(k_set_update<256, 16, false>, k_set_update<256, 16, true>); break;
-    case 11: go(k_set_update<128, 16, false>, k_set_update<128, 16, true>); break;
-    case 10: go(k_set_update<128, 8, false>, k_set_update<128, 8, true>); break;
-    case 9: go(k_set_update<64, 8, false>, k_set_update<64, 8, true>); break;
-    case 8: go(k_set_update<32, 8, false>, k_set_update<32, 8, true>); break;
-    default: go(k_set_update<32, 4, false>, k_set_update<32, 4, true>); break;
+    case 13: e = launch_shape<256, 32>(a, smem, s); break;
+    case 12: e = launch_shape<256, 16>(a, smem, s); break;
+    case 11: e = launch_shape<128, 16>(a, smem, s); break;
+    case 10: e = launch_shape<128, 8>(a, smem, s); break;
+    case 9: e = launch_shape<64, 8>(a, smem, s); break;
+    case 8: e = launch_shape<32, 8>(a, smem, s); break;
+    default: e = launch_shape<32, 4>(a, smem, s); break;
     }
     GQF_CK(e);
     const DeviceInfo &di = device_info(current_device());
-    k_fixup_occ<1><<<di.sms * 2, 256, 0, s>>>(table, sc.fix_list, sc.fix_cnt, sc.fix_cap, nullptr);
+    k_fixup_occ<1><<<di.sms * 2, 256, 0, s>>>(table, sc.fix_list, sc.fix_cnt, sc.fix_cap);
     count_launches(2);
     GQF_CK(cudaGetLastError());
     return GQF_OK;

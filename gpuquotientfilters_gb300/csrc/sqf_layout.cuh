@@ -8,9 +8,9 @@
 namespace gqf {
 
 template <int BPE>
-int launch_layout(const LayoutPlan &p, const SqfGeom &tg, uint8_t *table, const BucketSrc &A,
-                         const BucketSrc &B, int op, int nodup, bool set_ok, const uint32_t *a_dups, Scratch &sc,
-                         uint32_t *err, cudaStream_t s, const uint32_t *gate)
+int launch_layout(const LayoutPlan &p, const SqfGeom &tg, uint8_t *table, const BucketSrc &A, const BucketSrc &B,
+                  int op, int nodup, bool set_ok, const uint32_t *a_dups, Scratch &sc, uint32_t *err, cudaStream_t s,
+                  const uint32_t *gate)
 {
     // slots past the last bucket's quotients only receive spill: clear them
     // (a gated launch leaves that to k_fallback_prepare)
@@ -38,10 +38,13 @@ int launch_layout(const LayoutPlan &p, const SqfGeom &tg, uint8_t *table, const 
     a.err = err;
     a.gate = gate;
     const int threads = (int)layout_threads(p.g.tb);
+    const DeviceInfo &di = device_info(current_device());
+    // (an empty launch costs its CTAs: a gated one takes what is resident)
+    const uint32_t grid = gate ? std::min<uint32_t>(p.g.nb, (uint32_t)di.sms * 2) : p.g.nb;
     cudaError_t e = cudaSuccess;
     auto go = [&](auto kernel, size_t smem) {
         e = set_smem(kernel, smem);
-        if (e == cudaSuccess) kernel<<<p.g.nb, threads, smem, s>>>(a);
+        if (e == cudaSuccess) kernel<<<grid, threads, smem, s>>>(a);
     };
     if (BPE == 1 && set_ok) {
         const size_t smem = set_layout_smem(p.g.tb, threads);
@@ -59,14 +62,13 @@ int launch_layout(const LayoutPlan &p, const SqfGeom &tg, uint8_t *table, const 
         GQF_CK(e);
         count_launches(1);
     }
-    if ((op == OP_BUILD || op == OP_MERGE) && !set_ok) {
+    if ((op == OP_BUILD || op == OP_MERGE) && !set_ok && !gate) {
         // shared memory for a third more than the average bucket, as far as
         // the SM's goes (two-byte buckets of 32768 quotients); a larger one
         // keeps its remainders in the scratch
         a.rem_scratch = sc.rems;
         const double avg = (double)p.n_expect / p.g.nb;
-        const DeviceInfo &dv = device_info(current_device());
-        const size_t maxsm = (size_t)(dv.smem_optin > 0 ? dv.smem_optin : 99 * 1024) - 4096;  // less the static arrays
+        const size_t maxsm = (size_t)(di.smem_optin > 0 ? di.smem_optin : 99 * 1024) - 4096;  // less the static arrays
         const size_t fixed = group_layout_smem(p.g.tb, threads, BPE, 0);
         const size_t most = maxsm > fixed ? ((maxsm - fixed) / BPE) & ~(size_t)15 : 0;
         a.cap_items = (uint32_t)std::min(
@@ -104,7 +106,6 @@ int launch_layout(const LayoutPlan &p, const SqfGeom &tg, uint8_t *table, const 
         GQF_CK(e);
         count_launches(1);
     }
-    const DeviceInfo &di = device_info(current_device());
     count_launches(1);
     k_fixup_occ<BPE><<<di.sms * 2, 256, 0, s>>>(table, sc.fix_list, sc.fix_cnt, sc.fix_cap, gate);
     GQF_CK(cudaGetLastError());

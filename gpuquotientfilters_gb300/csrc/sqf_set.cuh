@@ -93,6 +93,7 @@ __device__ __forceinline__ int set_step(int u, int k) { return __viaddmax_s32(u,
 // B (the batch).  NC: the lists are older than the launch.
 template <int THREADS, int QPT, bool NC>
 struct Lists {
+    static constexpr bool DEL = false;
     static constexpr uint32_t S = THREADS * QPT;
     const LayoutArgs &a;
     uint32_t na, nb;
@@ -128,6 +129,7 @@ template <int THREADS, int QPT, template <int, int> class Source>
 struct SetContents {
     static constexpr int BPE = 1;
     static constexpr bool SMALL = true;  // at most 32 items a quotient
+    static constexpr bool DEL = Source<THREADS, QPT>::DEL;
     static constexpr uint32_t S = THREADS * QPT;
     uint8_t *mask;  // u32 at set_addr(x)
     Source<THREADS, QPT> src;
@@ -139,7 +141,13 @@ struct SetContents {
         for (uint32_t i = threadIdx.x; i < S / 4; i += THREADS) reinterpret_cast<uint4 *>(mask)[i] = make_uint4(0, 0, 0, 0);
         src.index();
         __syncthreads();
-        each<THREADS>(threadIdx.x, [&](uint32_t x, uint32_t rem) { atomicOr(&at(x), 1u << rem); });
+        if constexpr (DEL) {  // a table without copies loses the batch's fingerprints
+            src.template table_items<THREADS>(threadIdx.x, [&](uint32_t x, uint32_t rem) { atomicOr(&at(x), 1u << rem); });
+            __syncthreads();
+            src.template batch_items<THREADS>(threadIdx.x, [&](uint32_t x, uint32_t rem) { atomicAnd(&at(x), ~(1u << rem)); });
+        } else {
+            each<THREADS>(threadIdx.x, [&](uint32_t x, uint32_t rem) { atomicOr(&at(x), 1u << rem); });
+        }
         __syncthreads();
     }
     __device__ __forceinline__ void sizes(uint32_t x, uint32_t (&k)[4]) const  // of quotients x .. x + 3
@@ -155,14 +163,15 @@ struct SetContents {
     __device__ __forceinline__ void each(uint32_t t, F &&f) const
     {
         src.template table_items<NT>(t, f);
-        src.template batch_items<NT>(t, f);
+        if (!DEL) src.template batch_items<NT>(t, f);
     }
     // put(slot, element) for an item of a run that starts at slot st; the
     // element's occupied bit is not set
     template <typename Put>
     __device__ __forceinline__ void put_item(uint32_t x, uint32_t rem, uint32_t st, Put &&put) const
     {
-        const uint32_t below = __popc(at(x) & ((1u << rem) - 1u)), p = st + below;
+        const uint32_t m = at(x), below = __popc(m & ((1u << rem) - 1u)), p = st + below;
+        if (DEL && !((m >> rem) & 1u)) return;
         put(p, (rem << 3) + 2 * min(below, 1u) + min(p - x, 1u));
     }
     template <typename Put>
@@ -627,8 +636,8 @@ __device__ __forceinline__ void bucket_layout_set(const LayoutArgs &a, const uin
 }
 
 // ---------------------------------------------------------------------
-// The bucket's fingerprints from the table itself (in-place merge and large
-// insert), plus the batch.  Runs are stored in quotient order, one per
+// The bucket's fingerprints from the table itself (in-place merge, insert and
+// delete), and the batch.  Runs are stored in quotient order, one per
 // occupied quotient: of the runs starting at or past x0, the first D0 belong
 // to quotients below x0 (the lookup's walk back, done once per bucket), the
 // next ones to the bucket's occupied quotients in order.  index() keeps, per
@@ -654,7 +663,7 @@ __host__ __device__ inline SliceIndexPlan slice_index_plan(uint32_t tb)
     return m;
 }
 
-template <int THREADS, int QPT>
+template <int THREADS, int QPT, bool NC>
 struct Slice {
     static constexpr uint32_t S = THREADS * QPT;
     const uint8_t *t;
@@ -675,7 +684,7 @@ struct Slice {
     }
     __device__ __forceinline__ uint32_t byte_at(uint32_t i) const  // slot x0 + i
     {
-        return x0 + i < nslots ? (uint32_t)__ldg(t + x0 + i) : 0u;
+        return x0 + i < nslots ? (uint32_t)ld_data<NC>(t + x0 + i) : 0u;
     }
     // Builds the index.  Returns (on thread 0) whether the slice cannot be
     // decoded; dups: also when a run holds a remainder twice or out of order.
@@ -688,7 +697,7 @@ struct Slice {
         if (tid == 0) ctl[4] = 0;
         __syncthreads();
         if (wid == 0) {
-            const int D = pending_runs_warp(t, x0);
+            const int D = pending_runs_warp<NC>(t, x0);
             if (lane == 0) ctl[0] = (uint32_t)D;
         }
         const uint32_t per = (LW + THREADS - 1) / THREADS;
@@ -699,8 +708,8 @@ struct Slice {
             uint64_t v[4];
             const uint32_t s0 = x0 + 32 * w;
             if (s0 + 32 <= nslots) {
-                const ulonglong2 p0 = __ldg(reinterpret_cast<const ulonglong2 *>(t + s0));
-                const ulonglong2 p1 = __ldg(reinterpret_cast<const ulonglong2 *>(t + s0) + 1);
+                const ulonglong2 p0 = ld_data<NC>(reinterpret_cast<const ulonglong2 *>(t + s0));
+                const ulonglong2 p1 = ld_data<NC>(reinterpret_cast<const ulonglong2 *>(t + s0) + 1);
                 v[0] = p0.x;
                 v[1] = p0.y;
                 v[2] = p1.x;
@@ -713,7 +722,7 @@ struct Slice {
                 }
             }
             uint32_t rsm = 0, ocm = 0, nem = 0;
-            uint64_t before = (dups && s0 > 0 && s0 - 1 < nslots) ? (uint64_t)__ldg(t + s0 - 1) : 0ull;
+            uint64_t before = (dups && s0 > 0 && s0 - 1 < nslots) ? (uint64_t)ld_data<NC>(t + s0 - 1) : 0ull;
 #pragma unroll
             for (int h = 0; h < 4; h++) {
                 const Flags8 f = flags8(v[h]);
@@ -798,11 +807,14 @@ struct Slice {
     }
 };
 
-template <int THREADS, int QPT, bool TWO>
+// TWO: also the second table of a merge.  DELETES: the batch is taken out.
+// NC: the tables and the batch's list are older than the launch.
+template <int THREADS, int QPT, bool TWO, bool DELETES, bool NC>
 struct TableSource {
+    static constexpr bool DEL = DELETES;
     static constexpr uint32_t S = THREADS * QPT;
     const LayoutArgs &a;
-    Slice<THREADS, QPT> s1, s2;
+    Slice<THREADS, QPT, NC> s1, s2;
     uint32_t x0, nb;
     size_t bbase;
     __device__ __forceinline__ TableSource(const LayoutArgs &args, uint32_t b, uint8_t *mem) : a(args)
@@ -842,16 +854,23 @@ struct TableSource {
     template <int NT, typename F>
     __device__ __forceinline__ void batch_items(uint32_t t, F &&f) const
     {
-        for_each_item<NT>(a.B.items, bbase, nb, t, [&](uint32_t v) {
+        for_each_item<NT, NC>(a.B.items, bbase, nb, t, [&](uint32_t v) {
             const uint32_t x = (v >> SET_R) - x0;  // the batch bucket spans 2^sub layout buckets
             if (x < S) f(x, v & 31u);
         });
     }
 };
 template <int THREADS, int QPT>
-using OneTable = TableSource<THREADS, QPT, false>;
+using OneTable = TableSource<THREADS, QPT, false, false, true>;
 template <int THREADS, int QPT>
-using TwoTables = TableSource<THREADS, QPT, true>;
+using TwoTables = TableSource<THREADS, QPT, true, false, true>;
+template <int THREADS, int QPT>
+using LessTable = TableSource<THREADS, QPT, false, true, true>;
+// the same in a launch that made the snapshot and the list itself
+template <int THREADS, int QPT>
+using OwnTable = TableSource<THREADS, QPT, false, false, false>;
+template <int THREADS, int QPT>
+using OwnLessTable = TableSource<THREADS, QPT, false, true, false>;
 
 __host__ __device__ inline size_t set_update_smem(uint32_t tb, uint32_t threads, bool two)
 {
@@ -863,7 +882,6 @@ __host__ __device__ inline size_t set_update_smem(uint32_t tb, uint32_t threads,
 template <int THREADS, int QPT>
 __global__ void __launch_bounds__(THREADS, (THREADS >= 1024 ? 1 : 1024 / THREADS)) k_set_layout(LayoutArgs a)
 {
-    if (a.gate && !*a.gate) return;
     if (a.a_dups && *a.a_dups) return;  // the table holds duplicates: left to k_bucket_layout
     __shared__ uint32_t s_ticket;
     if (threadIdx.x == 0) s_ticket = atomicAdd(a.ticket, 1u);
@@ -886,15 +904,17 @@ __host__ __device__ inline size_t group_layout_smem(uint32_t tb, uint32_t thread
     return items_plan(S, threads, bpe).contents + GroupContents<32, 4, 1, false>::group_cnt_bytes(S) + cap_items * bpe;
 }
 
-// In-place merge and large insert: writes the live table, reads only the
+// In-place merge, insert and delete: writes the live table, reads only the
 // snapshot (and the second table).
-template <int THREADS, int QPT, bool TWO>
+enum UpdateKind : int { UPDATE_ADD = 0, UPDATE_TWO = 1, UPDATE_DEL = 2 };
+template <int THREADS, int QPT, int KIND>
 __global__ void __launch_bounds__(THREADS, (THREADS >= 1024 ? 1 : 768 / THREADS)) k_set_update(LayoutArgs a)
 {
     __shared__ uint32_t s_ticket;
     if (threadIdx.x == 0) s_ticket = atomicAdd(a.ticket, 1u);
     __syncthreads();
-    if (TWO) bucket_layout_set<THREADS, QPT, TwoTables>(a, s_ticket);
+    if constexpr (KIND == UPDATE_TWO) bucket_layout_set<THREADS, QPT, TwoTables>(a, s_ticket);
+    else if constexpr (KIND == UPDATE_DEL) bucket_layout_set<THREADS, QPT, LessTable>(a, s_ticket);
     else bucket_layout_set<THREADS, QPT, OneTable>(a, s_ticket);
 }
 

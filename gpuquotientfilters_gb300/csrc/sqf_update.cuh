@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(UPD_THREADS) k_del_locate(const uint32_t *__re
                         D += (uint32_t)__popc(occ);
                     }
                     const uint32_t end = k.first_clear(s + 1, [](const Sector<BPE> &x) { return x.sh; });
-                    if (end == UPD_NONE || end - p.unit > FAR_SLOTS) *far = 1;
+                    if (end == UPD_NONE || end - p.unit > v.far) *far = 1;
                     mine = make_uint4(s, ((s - p.unit) << 16) | (end - s), fq, D);
                 }
                 break;
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(UPD_THREADS) k_del_locate(const uint32_t *__re
             const uint32_t open = ~was & 0x55555555u & (~0u << (2 * (s & 15u)));
             const uint32_t to = open ? (s & ~15u) + (((uint32_t)__ffs(open) - 1u) >> 1) : (s | 15u) + 1;
             if (k.s.rs & low32(min(to - (s & ~31u) + 1, 32u)) & ~low32((s & 31u) + 1)) break;
-            if (to - p.pos > FAR_SLOTS || *reinterpret_cast<volatile uint32_t *>(far)) {
+            if (to - p.pos > v.far || *reinterpret_cast<volatile uint32_t *>(far)) {
                 *far = 1;
                 break;
             }
@@ -449,7 +449,7 @@ __global__ void __launch_bounds__(UPD_THREADS) k_ins_stage(const uint32_t *__res
     const RunPlace p = find_run(w, fq);
     uint32_t ip = p.pos, head = INS_HEAD;
     if (p.occ && !p.far) {
-        for (; ip < v.nslots && ip - p.pos <= FAR_SLOTS; ip++) {
+        for (; ip < v.nslots && ip - p.pos <= v.far; ip++) {
             const uint32_t e = w.elem(ip);
             if (ip > p.pos && !(e & 2u)) break;  // end of the run
             const uint32_t rem = e >> 3;
@@ -458,7 +458,7 @@ __global__ void __launch_bounds__(UPD_THREADS) k_ins_stage(const uint32_t *__res
         }
         if (ip != p.pos) head = 0;
     }
-    const uint32_t gap = p.far || ip - p.pos > FAR_SLOTS ? UPD_NONE : ip >= v.nslots ? v.nslots : w.next_empty(ip);
+    const uint32_t gap = p.far || ip - p.pos > v.far ? UPD_NONE : ip >= v.nslots ? v.nslots : w.next_empty(ip);
     if (gap == UPD_NONE) *far = 1;
     const uint4 entry = make_uint4(fp, ip | head, (gap & INS_GAP) | (p.occ ? 0u : INS_NEWQ), 0u);
     const uint32_t bk = fp >> b.shift, k = atomicAdd(b.cnt + bk, 1u);
@@ -599,7 +599,7 @@ __device__ __forceinline__ uint32_t ins_walk(const InsBatch &b, const SlotTable<
         Walk<BPE> w(v, g + 1);
         w.s.planes();
         g = w.next_empty(g + 1);
-        if (g - g0 > FAR_SLOTS) return g == v.nslots ? g : UPD_NONE;
+        if (g - g0 > v.far) return g == v.nslots ? g : UPD_NONE;
     }
 }
 

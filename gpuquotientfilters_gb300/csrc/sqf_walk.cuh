@@ -8,17 +8,18 @@
 namespace gqf {
 
 constexpr uint32_t WALK_NONE = 0xFFFFFFFFu;
-// A longer stretch (a nearly full table) is not walked.  An update that meets
-// one sets *far: nothing has been changed yet, the apply kernels do nothing,
-// and k_update_fallback rebuilds the table.  A lookup goes on slot by slot.
-constexpr uint32_t FAR_SLOTS = 5120;  // more than the slots of q = 12
+// A longer stretch (a nearly full table) is not walked: SlotTable::far slots
+// for an update, FAR_SLOTS at most.  An update that meets one sets *far:
+// nothing has been changed yet, the apply kernels do nothing, and the table is
+// updated as a whole.  A lookup goes on slot by slot.
+constexpr uint32_t FAR_SLOTS = 5120;
 
 // Slots of a table: element i = rem << 3 | occupied << 2 |
 // continuation << 1 | shifted.
 template <int BPE>
 struct SlotTable {
     uint8_t *t;
-    uint32_t nslots;
+    uint32_t nslots, far = FAR_SLOTS;
     __device__ __forceinline__ uint32_t get(uint32_t i) const
     {
         if (BPE == 1) return t[i];
@@ -141,7 +142,7 @@ struct Walk {
         return s.elem(v, slot);
     }
     // first slot at or after `slot` for which the plane pick(sector) is clear
-    // (the table's end reads as clear; WALK_NONE: further than FAR_SLOTS)
+    // (the table's end reads as clear; WALK_NONE: further than v.far)
     template <typename Pick>
     __device__ __forceinline__ uint32_t first_clear(uint32_t slot, Pick &&pick)
     {
@@ -152,7 +153,7 @@ struct Walk {
             if (m) return min(32 * si + (uint32_t)__ffs(m) - 1u, v.nslots);
             slot = 32 * si + 32;
             if (slot >= v.nslots) return v.nslots;
-            if (slot - from > FAR_SLOTS) return WALK_NONE;
+            if (slot - from > v.far) return WALK_NONE;
         }
     }
     // first empty slot at or after `slot` (nslots: none)
@@ -169,7 +170,7 @@ struct Walk {
 //   occ:  fq has a run;
 //   pos:  occ: the run's first slot; otherwise the slot a first element of fq
 //         goes in front of (the next run's start or the first empty slot);
-//   far:  the walk went past FAR_SLOTS, pos is not known.
+//   far:  the walk went past k.v.far, pos is not known.
 struct RunPlace {
     uint32_t unit, pos;
     bool occ, far;
@@ -191,7 +192,7 @@ __device__ __forceinline__ RunPlace find_run(Walk<BPE> &k, uint32_t fq)
         while (!st) {
             D += __popc(b.occ & in) - __popc(b.rs & in);
             if (bi == 0) break;
-            if (k.si - bi > FAR_SLOTS / 32) {
+            if (k.si - bi > k.v.far / 32) {
                 r.far = true;
                 return r;
             }
@@ -223,7 +224,7 @@ __device__ __forceinline__ RunPlace find_run(Walk<BPE> &k, uint32_t fq)
         D -= c;
         const uint32_t next = 32 * k.si + 32;
         if (next >= k.v.nslots) return r;
-        if (next - fq > FAR_SLOTS) {
+        if (next - fq > k.v.far) {
             r.far = true;
             return r;
         }

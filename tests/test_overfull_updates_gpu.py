@@ -5,6 +5,7 @@ import pytest
 
 import oracle as O
 from conftest import to_dev
+from sqf_model import Contents, check
 
 pytestmark = pytest.mark.gpu
 
@@ -17,24 +18,21 @@ def distinct_keys(seed, q, r, n):
 
 
 @pytest.mark.parametrize("sync", [True, False])
-@pytest.mark.parametrize("load", [1.03, 1.05])
-@pytest.mark.parametrize("q,r", [(18, 5), (20, 5), (22, 5), (18, 13)])
+@pytest.mark.parametrize("q,r,load", [(18, 5, 1.03), (18, 5, 1.05), (20, 5, 1.03), (20, 5, 1.05), (22, 5, 1.05),
+                                      (18, 13, 1.03), (18, 13, 1.05)])
 def test_overfull_updates(gqf, cuda, q, r, load, sync):
     n, m = int(load * (1 << q)), 24
     keys = distinct_keys(850 + q, q, r, n + m)
-    t = O.sqf_new(q, r)
-    assert O.sqf_bulk_build(t, q, r, keys[:n], True) == 0
+    c = Contents(q, r, keys[:n], True)
     f = gqf.initFilterGPU(q, r)
     try:
         gqf.bulkBuildSegmentedLayouts(f, n, to_dev(cuda, keys[:n]), True)
-        assert np.array_equal(gqf.table_bytes(f), t)
-        for op, ref, k in ((gqf.superclusterDeletes, O.sqf_delete, keys[:1]),
-                           (gqf.insert, O.sqf_insert, keys[n:]),
-                           (gqf.superclusterDeletes, O.sqf_delete, keys[n // 2: n // 2 + m])):
+        check(gqf, f, c.table(), "build")
+        for op, ref, k in ((gqf.superclusterDeletes, c.delete, keys[:1]), (gqf.insert, c.insert, keys[n:]),
+                           (gqf.superclusterDeletes, c.delete, keys[n // 2: n // 2 + m])):
             op(f, k.size, to_dev(cuda, k), sync=sync)
             gqf.stream_status()
-            ref(t, q, r, k)
-            raw = gqf.table_bytes(f)
-            assert np.array_equal(raw, t), "%s: %d bytes differ" % (op.__name__, np.count_nonzero(raw != t))
+            ref(k)
+            check(gqf, f, c.table(), op.__name__)
     finally:
         gqf.freeFilterGPU(f)

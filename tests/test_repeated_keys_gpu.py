@@ -6,6 +6,7 @@ import pytest
 
 import oracle as O
 from conftest import to_dev
+from sqf_model import Contents, check
 
 pytestmark = pytest.mark.gpu
 
@@ -15,19 +16,18 @@ pytestmark = pytest.mark.gpu
 def test_deletes_of_many_copies(gqf, cuda, q, r, copies, sync):
     keys = np.concatenate([np.full(copies, 99, np.uint32), O.mt_keys(900 + q, int(0.4 * (1 << q)))])
     near = keys[copies: copies + 500]
-    t = O.sqf_new(q, r)
-    assert O.sqf_bulk_build(t, q, r, keys, False) == 0
+    c = Contents(q, r, keys, False)
     f = gqf.initFilterGPU(q, r)
     try:
         gqf.bulkBuildSegmentedLayouts(f, keys.size, to_dev(cuda, keys), False)
         part = np.concatenate([np.full(copies // 3, 99, np.uint32), near])
-        for op, ref, k in ((gqf.superclusterDeletes, O.sqf_delete, part),
-                           (gqf.insert, O.sqf_insert, part),  # all stored already but the deleted ones
-                           (gqf.superclusterDeletes, O.sqf_delete, np.full(copies, 99, np.uint32))):
+        for op, ref, k in ((gqf.superclusterDeletes, c.delete, part),
+                           (gqf.insert, c.insert, part),  # all stored already but the deleted ones
+                           (gqf.superclusterDeletes, c.delete, np.full(copies, 99, np.uint32))):
             op(f, k.size, to_dev(cuda, k), sync=sync)
             gqf.stream_status()
-            ref(t, q, r, k)
-            assert np.array_equal(gqf.table_bytes(f), t), op.__name__
+            ref(k)
+            check(gqf, f, c.table(), op.__name__)
     finally:
         gqf.freeFilterGPU(f)
 
