@@ -330,10 +330,27 @@ static int rebuild(const gqf_sqf *qf, const gqf_sqf *qf2, const uint32_t *keys, 
 }
 
 // ------------------------------------------------------------- update routes
-// All deletes, and inserts of at most a key per 16 quotients, touch only the
-// clusters they change (sqf_update.cuh); larger inserts update the whole table
-// in place.
-static uint32_t local_max_keys(uint32_t q, uint32_t, int op) { return op == OP_DELETE ? 0x7FFFFFFFu : 1u << (q - 4); }
+// Inserts and deletes of at most a key per 64 quotients on tables of 2^22
+// quotients and more touch only the clusters they change (sqf_update.cuh);
+// larger batches, and any on smaller tables, update the whole table in place,
+// which costs the same at every fill.  A synchronous insert / delete in us,
+// fill 0.8:
+//               2^q / 1024 keys     2^q / 64           2^q / 16
+//               local    in place   local     in place local      in place
+//     q = 20    87/58    80/82      97/65     80/80    171/72     84/83
+//     q = 22    88/65    110/110    115/76    111/110  252/107    116/114
+//     q = 24    95/71    186/183    165/107   188/189  527/256    201/196
+//     q = 26    104/79   551/552    372/276   569/568  1560/955   629/620
+// and at fill 0.9 local ones of 2^q / 64 take 178/98 (in place 87/81), 221/127
+// (113/110), 325/205 (192/188) and 592/476 (572/571).
+//
+// Two-byte slots (q <= 18) have no in-place form: all deletes, and inserts of
+// at most a key per 16 quotients, are local.
+static uint32_t local_max_keys(uint32_t q, uint32_t r, int op)
+{
+    if (r != 5) return op == OP_DELETE ? 0x7FFFFFFFu : 1u << (q - 4);
+    return q >= 22 ? 1u << (q - 6) : 0u;
+}
 
 // Scratch bytes of an insert or delete of up to n keys, whichever way it goes.
 static size_t update_scratch_bytes(const SqfGeom &tg, uint32_t n)

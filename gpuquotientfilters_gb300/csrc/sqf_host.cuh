@@ -190,6 +190,13 @@ int launch_layout(const LayoutPlan &p, const SqfGeom &tg, uint8_t *table, const 
 // In-place update of one-byte slots (sqf_inplace.cu).
 int launch_update(const LayoutPlan &p, const SqfGeom &tg, uint8_t *table, const uint8_t *src2, const BucketSrc &B,
                   int op, Scratch &sc, uint32_t *err, cudaStream_t s);
+// Slots an update walks before it gives the stretch up.  On a nearly full
+// table the walks are lost time: the larger the table, the more its update as
+// a whole costs, and the longer they may be.
+inline uint32_t walk_limit(uint32_t q)
+{
+    return std::min(FAR_SLOTS, 1280u << (q > 22 ? std::min(q - 22, 2u) : 0));
+}
 // Cluster-local insert or delete (sqf_local.cu).  A synchronous call on
 // one-byte slots that met a stretch too long to walk leaves the table as it
 // was and sets *far; behind the others the rebuild runs on the device.

@@ -137,7 +137,7 @@ int local_update(const gqf_sqf *qf, const uint32_t *keys, uint32_t n, int op, cu
     if (st) return st;
     if (n == 0) return call_end(ar, s, ms);
     GQF_CK(cudaMemsetAsync(base, 0, b.zero_bytes, s));
-    const SlotTable<BPE> v{qf->table, tg.nslots};
+    const SlotTable<BPE> v{qf->table, tg.nslots, walk_limit(tg.q)};
     const uint32_t grid = (n + UPD_THREADS - 1) / UPD_THREADS;
     // a warp per listed unit or group, at most every key's
     const uint32_t lgrid = std::min<uint32_t>((n + LIST_THREADS / 32 - 1) / (LIST_THREADS / 32), (uint32_t)di.sms * 32);
