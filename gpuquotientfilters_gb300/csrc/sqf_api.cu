@@ -124,6 +124,7 @@ static int bucket_batch(const uint32_t *keys, uint32_t n, const LayoutPlan &p, S
 }
 
 constexpr uint32_t ONE_LAUNCH_Q = 22;
+constexpr uint32_t ONE_PASS_ITEMS = 1u << 20;
 constexpr size_t SNAP_BESIDE = 16u << 20;  // table bytes from which a snapshot is copied on the side stream
 
 // What a rebuild runs and needs: A = current contents of the table (unless it
@@ -133,11 +134,13 @@ struct Rebuild {
     bool set_ok;    // the layout from lists has set semantics (see LayoutArgs::set_ok)
     bool in_place;  // one-byte slots, set semantics: decoded bucket by bucket from a snapshot
     bool exact;     // exact bucket bases from the start
+    bool one_pass;  // the in-place batch in strides that hold all of it
     LayoutPlan p;
     ScratchReq spec, req;  // scratch with speculative bucket strides, and as it runs otherwise
     size_t bytes;
 };
-static Rebuild plan_rebuild(const SqfGeom &tg, uint32_t n, int op, int nodup, bool two, bool queued)
+static Rebuild plan_rebuild(const SqfGeom &tg, uint32_t n, int op, int nodup, bool two, bool queued,
+                            bool strides = true)
 {
     Rebuild b{};
     b.needA = op != OP_BUILD;
@@ -165,6 +168,14 @@ static Rebuild plan_rebuild(const SqfGeom &tg, uint32_t n, int op, int nodup, bo
     b.spec = b.req;
     if (!two) b.spec.batch_items = (size_t)b.p.g.nb * b.p.stride;
     if (b.in_place) {
+        // A small batch on a small table is bucketed in one pass, with room
+        // for all of it in every bucket: three launches fewer than exact bases
+        // need (a synchronous delete of 4096 keys at q = 15: 70 us, now 56).
+        b.one_pass = strides && (uint64_t)b.p.g.nb * n <= ONE_PASS_ITEMS;
+        if (b.one_pass) {
+            b.p.stride = (uint32_t)align_up(n, 4);
+            b.req.batch_items = std::max<size_t>((size_t)b.p.g.nb * b.p.stride, 1);
+        }
         b.req.snap_bytes = tg.T;
         b.req.upd_nb = 1u << (tg.q - update_tb(tg.q));
         b.req.fallback = &tg;
@@ -225,9 +236,9 @@ static int rebuild(const gqf_sqf *qf, const gqf_sqf *qf2, const uint32_t *keys, 
         GQF_CK(cudaMemsetAsync(sc.bcnt, 0, sc.ctrl_bytes, s));
         BucketSrc B{nullptr, nullptr, 0, nullptr};
         if (n) {
-            st = bucket_batch(keys, n, p, sc, true, ar.err, s);
+            st = bucket_batch(keys, n, p, sc, !b.one_pass, ar.err, s);
             if (st) return st;
-            B = BucketSrc{sc.bitems, sc.bbase, 0, sc.bcnt};
+            B = b.one_pass ? BucketSrc{sc.bitems, nullptr, p.stride, sc.bcnt} : BucketSrc{sc.bitems, sc.bbase, 0, sc.bcnt};
         }
         if (beside) GQF_CK(cudaStreamWaitEvent(s, ar.join, 0));
         // a filter merged with itself is read from the snapshot twice
@@ -337,12 +348,12 @@ static int rebuild(const gqf_sqf *qf, const gqf_sqf *qf2, const uint32_t *keys, 
 // fill 0.8:
 //               2^q / 1024 keys     2^q / 64           2^q / 16
 //               local    in place   local     in place local      in place
-//     q = 20    87/58    80/82      97/65     80/80    171/72     84/83
+//     q = 20    87/58    71/71      97/65     75/71    171/72     84/83
 //     q = 22    88/65    110/110    115/76    111/110  252/107    116/114
 //     q = 24    95/71    186/183    165/107   188/189  527/256    201/196
 //     q = 26    104/79   551/552    372/276   569/568  1560/955   629/620
-// and at fill 0.9 local ones of 2^q / 64 take 178/98 (in place 87/81), 221/127
-// (113/110), 325/205 (192/188) and 592/476 (572/571).
+// and at fill 0.9 local ones of 2^q / 64 from q = 22 on take 221/127 (in place
+// 113/110), 325/205 (192/188) and 592/476 (572/571).
 //
 // Two-byte slots (q <= 18) have no in-place form: all deletes, and inserts of
 // at most a key per 16 quotients, are local.
@@ -356,10 +367,13 @@ static uint32_t local_max_keys(uint32_t q, uint32_t r, int op)
 static size_t update_scratch_bytes(const SqfGeom &tg, uint32_t n)
 {
     size_t most = 0;
+    // smaller batches may take the strides of one pass where this one does not
+    const uint64_t buckets = 1ull << (tg.q - update_tb(tg.q));
+    const size_t strides = tg.r == 5 ? 4 * std::min<uint64_t>(buckets * (n + 4ull), ONE_PASS_ITEMS + 4 * buckets) : 0;
     for (int op : {OP_INSERT, OP_DELETE}) {
         most = std::max(most, local_update_bytes(tg, std::min(n, local_max_keys(tg.q, tg.r, op)), op));
         for (bool queued : {false, true})
-            most = std::max(most, plan_rebuild(tg, n, op, op == OP_INSERT, false, queued).bytes);
+            most = std::max(most, plan_rebuild(tg, n, op, op == OP_INSERT, false, queued, false).bytes + strides);
     }
     return most;
 }
