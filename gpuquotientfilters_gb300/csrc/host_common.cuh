@@ -109,6 +109,17 @@ int dev_err_to_status(uint32_t e);
 
 int current_device();
 
+// Loads kernels that would otherwise be loaded, one by one, by the first call
+// that launches each.
+template <typename... K>
+inline void load_kernels(K... kernels)
+{
+    cudaFuncAttributes a;
+    (void)(int[]){(int)cudaFuncGetAttributes(&a, kernels)...};
+}
+// The kernels of a server's lookups, inserts and deletes (sqf_api.cu).
+void load_served_kernels();
+
 // Kernel launches issued by this library (instrumentation for benchmarks).
 void count_launches(unsigned n);
 

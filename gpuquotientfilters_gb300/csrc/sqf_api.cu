@@ -440,6 +440,15 @@ static int lookup_t(const gqf_sqf *qf, int n, const uint32_t *keys, uint32_t *ou
     return call_end(ar, s, ms);
 }
 
+void load_served_kernels()
+{
+    load_local_kernels();
+    load_inplace_kernels();
+    load_kernels(k_bucket_hist<SMALL_THREADS, SMALL_IPT>, k_hash_bucket<SMALL_THREADS, SMALL_IPT>,
+                 k_bucket_hist<SCATTER_THREADS, SCATTER_IPT>, k_hash_bucket<SCATTER_THREADS, SCATTER_IPT>, k_scan_bases,
+                 k_fixup_occ<1>, k_sqf_mirror, k_lookup_mirror, k_lookup_unsorted<1, 2>, k_lookup_unsorted<2, 1>);
+}
+
 // ------------------------------------------------ no-allocation bulk build
 // Scratch for gqf_sqf_bulk_build_noalloc: a fixed array in the library's
 // device image.  Host code must not use the symbol itself as an address;

@@ -202,6 +202,8 @@ inline uint32_t walk_limit(uint32_t q)
 // was and sets *far; behind the others the rebuild runs on the device.
 template <int BPE>
 int local_update(const gqf_sqf *qf, const uint32_t *keys, uint32_t n, int op, cudaStream_t s, float *ms, bool *far);
+void load_local_kernels();
+void load_inplace_kernels();
 size_t local_update_bytes(const SqfGeom &tg, uint32_t n, int op);
 // The gated rebuild: gate, src, src2, snap, keys, n and the buffers are set.
 // With `lists`, only the old contents' lists, in buckets of that geometry.

@@ -65,4 +65,20 @@ int launch_update(const LayoutPlan &p, const SqfGeom &tg, uint8_t *table, const 
     return GQF_OK;
 }
 
+template <int THREADS, int QPT>
+static void load_shape()
+{
+    load_kernels(k_set_update<THREADS, QPT, UPDATE_ADD>, k_set_update<THREADS, QPT, UPDATE_DEL>);
+}
+void load_inplace_kernels()
+{
+    load_shape<256, 32>();
+    load_shape<256, 16>();
+    load_shape<128, 16>();
+    load_shape<128, 8>();
+    load_shape<64, 8>();
+    load_shape<32, 8>();
+    load_shape<32, 4>();
+}
+
 }  // namespace gqf

@@ -177,4 +177,17 @@ int local_update(const gqf_sqf *qf, const uint32_t *keys, uint32_t n, int op, cu
 template int local_update<1>(const gqf_sqf *, const uint32_t *, uint32_t, int, cudaStream_t, float *, bool *);
 template int local_update<2>(const gqf_sqf *, const uint32_t *, uint32_t, int, cudaStream_t, float *, bool *);
 
+template <int BPE>
+static void load_local()
+{
+    load_kernels(k_ins_stage<BPE>, k_ins_groups<BPE>, k_ins_apply<BPE>, k_ins_lists<BPE>, k_del_locate<BPE>,
+                 k_del_apply<BPE>, k_del_units<BPE>, k_update_fallback<BPE>);
+}
+void load_local_kernels()
+{
+    load_local<1>();
+    load_local<2>();
+    load_kernels(k_ins_sort);
+}
+
 }  // namespace gqf

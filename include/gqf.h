@@ -86,8 +86,8 @@ int gqf_stream_status(void *stream);
  * fits allocates nothing); release frees it after the stream drains. */
 int gqf_workspace_reserve(void *stream, size_t bytes, size_t *reserved);
 int gqf_workspace_release(void *stream);
-/* Workspace bytes one gqf_sqf_insert / gqf_sqf_delete of n keys on a
- * filter of (q, r) needs. */
+/* Workspace bytes that cover every gqf_sqf_insert / gqf_sqf_delete of up to
+ * n keys on a filter of (q, r). */
 size_t gqf_sqf_update_workspace_bytes(unsigned int q, unsigned int r, int n);
 
 /* ---------------- standard quotient filter ------------------------------ */
