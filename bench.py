@@ -36,9 +36,9 @@ N_LOOKUP = 1 << 24
 N_INSERT = 1 << 20
 N_DELETE = 1 << 20
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one q=26 r=5 NoDup build of
-# N_KEYS keys, from one `ncu --set full` capture: k_hash_bucket 384,808,192 + k_bucket_layout
-# 261,271,808 (k_fixup_occ touches a few KB).
-BUILD_DRAM_BYTES = 384808192 + 261271808
+# N_KEYS keys, from one `ncu --set full` capture: k_hash_bucket 398,502,912 + k_set_layout
+# 262,929,664 (k_fixup_occ touches a few KB).
+BUILD_DRAM_BYTES = 398502912 + 262929664
 # ops timed in every step but not counted in `value`
 EXTRA_OPS = ("build_dup",)
 
@@ -236,7 +236,7 @@ def run_gpu(args, world, rank, local):
         "roofline": {"bound": "hbm", "kernel": "bulk build pipeline (hash+bucket scatter, bucket layout, fixup)",
                      "achieved": b["alg_GBps"], "peak": peak, "unit": "GB/s", "frac": b["frac_hbm"],
                      "traffic": BUILD_DRAM_BYTES if q == Q else None,
-                     "traffic_source": "ncu capture of the same build (k_hash_bucket + k_bucket_layout)",
+                     "traffic_source": "ncu capture of the same build (k_hash_bucket + k_set_layout)",
                      "peak_source": peak_kind},
     }
 

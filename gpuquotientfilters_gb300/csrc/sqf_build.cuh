@@ -428,8 +428,8 @@ struct LayoutArgs {
     int op, nodup;
     // Set mode (k_set_layout): r = 5 and the op has set semantics (NoDup
     // build or merge, insert into a table without duplicate fingerprints);
-    // `a_dups` (device flag, may be null) vetoes it at run
-    // time when the table holds duplicates, and k_bucket_layout runs.
+    // `a_dups` (device flag, may be null) vetoes it at run time when the
+    // table holds duplicates, and k_bucket_layout runs.
     int set_ok;
     const uint32_t *a_dups;
     unsigned long long *status;
