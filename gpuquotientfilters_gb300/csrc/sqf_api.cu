@@ -277,8 +277,7 @@ static int rebuild(const gqf_sqf *qf, const gqf_sqf *qf2, const uint32_t *keys, 
                 f.gate = ar.err;
                 f.gate_bits = DEV_ERR_BUCKET_CAP;
             }
-            if (tg.q <= ONE_LAUNCH_Q || op != OP_MERGE)
-                st = launch_fallback<BPE>(f, tg, qf->table, op, nodup, ar.err, s);
+            st = launch_fallback<BPE>(f, tg, qf->table, op, nodup, ar.err, s);
             return st ? st : call_end(ar, s, nullptr);
         }
         uint32_t rep[2];

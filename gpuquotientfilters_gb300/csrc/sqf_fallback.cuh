@@ -6,7 +6,8 @@
 //   - an in-place update, or that one, met a bucket it cannot decode (a table
 //     holding duplicate fingerprints, a run past its slice): the old contents
 //     are extracted, from the snapshot, and every bucket is laid out again
-//     from both lists.
+//     from both lists (as remainder sets where no copies are kept: any number
+//     of items).
 // One launch, because the usual case is the empty one: a kernel per step was
 // 12 to 18 launches behind every queued in-place update or merge (q = 20, an
 // insert of a key per 8 quotients: 117 us, now 67).
@@ -21,7 +22,8 @@ namespace gqf {
 constexpr int FB_THREADS = EXTRACT_THREADS;
 constexpr uint32_t FB_TB = 13;  // quotients per bucket: 32 per thread (a smaller filter is one bucket)
 static_assert((1u << FB_TB) == FB_THREADS * 32, "one layout CTA shape");
-// Items a bucket may hold: what its u16 counters allow, eight times the average.
+// Items a bucket of a table with copies, or of two-byte slots, may hold: what
+// its u16 counters allow, eight times the average.
 constexpr uint32_t FB_CAP = 65520;
 
 struct FallbackArgs {
@@ -37,7 +39,8 @@ struct FallbackArgs {
     uint32_t n, nbytes;
     Counts3 *tiles;
     uint32_t *Q, *E, *E2, *abase, *acnt, *bbase, *b2cnt, *bcnt, *bfill, *bitems;
-    uint32_t *bar;  // four zero words
+    uint32_t *dups;  // set when the table holds copies
+    uint32_t *bar;   // four zero words
 };
 
 // Exclusive scans of NV interleaved words per entry by one CTA of FB_THREADS
@@ -100,7 +103,7 @@ __global__ void __launch_bounds__(FB_THREADS, 2) k_update_fallback(FallbackArgs 
     // what the layouts expect at zero
     auto reset = [&]() {
         for (uint32_t b = gt; b < a.nb; b += gn) a.status[b] = 0ull;
-        if (gt == 0) *a.ticket = *a.fix_cnt = 0u;
+        if (gt == 0) *a.ticket = *a.fix_cnt = *f.dups = 0u;
     };
     auto buckets = [&](auto &&body) {
         for (;;) {
@@ -160,7 +163,7 @@ __global__ void __launch_bounds__(FB_THREADS, 2) k_update_fallback(FallbackArgs 
         const uint8_t *src = k ? f.src2 : f.src;
         uint32_t *E = k ? f.E2 : f.E, *base = k ? f.bbase : f.abase, *cnt = k ? f.b2cnt : f.acnt;
         if (!grid_sync(f.bar, a.err)) return;
-        for_each_tile(a.nslots, [&](uint32_t u) { tile_counts<BPE, false>(u, src, a.nslots, f.nbytes, f.tiles, nullptr); });
+        for_each_tile(a.nslots, [&](uint32_t u) { tile_counts<BPE, false>(u, src, a.nslots, f.nbytes, f.tiles, k ? nullptr : f.dups); });
         if (!grid_sync(f.bar, a.err)) return;
         if (blockIdx.x == 0)
             fb_scan<3>(reinterpret_cast<const uint32_t *>(f.tiles), reinterpret_cast<uint32_t *>(f.tiles), ntiles, true);
@@ -190,7 +193,14 @@ __global__ void __launch_bounds__(FB_THREADS, 2) k_update_fallback(FallbackArgs 
     for (size_t i = ((size_t)BPE << a.q) + gt; i < f.nbytes; i += gn) a.table[i] = 0;
     if (f.lists_only) return;
     if (!grid_sync(f.bar, a.err)) return;
-    buckets([&](uint32_t b) { bucket_layout_body<FB_THREADS, 32, BPE>(a, b); });
+    // (the set layout's map of a bucket reaches its last quotient: whole
+    // buckets only)
+    if (BPE == 1 && a.q >= a.tb && (a.op == OP_MERGE || !__ldcg(f.dups))) {
+        if (a.op == OP_DELETE) buckets([&](uint32_t b) { bucket_layout_set<FB_THREADS, 32, OwnLessSource>(a, b); });
+        else buckets([&](uint32_t b) { bucket_layout_set<FB_THREADS, 32, OwnListSource>(a, b); });
+    } else {
+        buckets([&](uint32_t b) { bucket_layout_body<FB_THREADS, 32, BPE>(a, b); });
+    }
     if (!grid_sync(f.bar, a.err)) return;
     const uint32_t nf = min(__ldcg(a.fix_cnt), a.fix_cap);
     for (uint32_t i = gt; i < nf; i += gn) a.table[(size_t)__ldcg(a.fix_list + i) * BPE + (BPE - 1)] |= 4u;

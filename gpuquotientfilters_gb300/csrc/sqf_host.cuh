@@ -124,6 +124,7 @@ void carve_fallback(C &c, FallbackArgs &f, const SqfGeom &tg, bool two)
     f.lay.status = c.template take<unsigned long long>(nb);
     f.lay.ticket = c.template take<uint32_t>(1, 4);
     f.lay.fix_cnt = c.template take<uint32_t>(1, 4);
+    f.dups = c.template take<uint32_t>(1, 4);
     f.bcnt = c.template take<uint32_t>(nb);
     f.bfill = c.template take<uint32_t>(nb);
     f.bbase = c.template take<uint32_t>(nb);

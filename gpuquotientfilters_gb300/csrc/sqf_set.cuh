@@ -90,10 +90,11 @@ __device__ __forceinline__ void for_each_item(const uint32_t *items, size_t star
 __device__ __forceinline__ int set_step(int u, int k) { return __viaddmax_s32(u, k - 1, k - 1); }
 
 // The bucket's fingerprints from lists: A (a table's extracted contents) and
-// B (the batch).  NC: the lists are older than the launch.
-template <int THREADS, int QPT, bool NC>
+// B (the batch).  DELETES: the batch is taken out.  NC: the lists are older
+// than the launch.
+template <int THREADS, int QPT, bool DELETES, bool NC>
 struct Lists {
-    static constexpr bool DEL = false;
+    static constexpr bool DEL = DELETES;
     static constexpr uint32_t S = THREADS * QPT;
     const LayoutArgs &a;
     uint32_t na, nb;
@@ -120,9 +121,11 @@ struct Lists {
     }
 };
 template <int THREADS, int QPT>
-using ListSource = Lists<THREADS, QPT, true>;
+using ListSource = Lists<THREADS, QPT, false, true>;
 template <int THREADS, int QPT>
-using OwnListSource = Lists<THREADS, QPT, false>;
+using OwnListSource = Lists<THREADS, QPT, false, false>;
+template <int THREADS, int QPT>
+using OwnLessSource = Lists<THREADS, QPT, true, false>;
 
 // Contents of a bucket as remainder sets, fed by a source (lists, or tables).
 template <int THREADS, int QPT, template <int, int> class Source>

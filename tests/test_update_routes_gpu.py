@@ -63,6 +63,46 @@ def test_update_of_a_bucket_too_large_for_the_steps(gqf, cuda, q, sync):
         gqf.freeFilterGPU(f)
 
 
+@pytest.mark.parametrize("sync", [True, False])
+@pytest.mark.parametrize("op", ["insert", "delete", "merge", "via"])
+@pytest.mark.parametrize("q,lo,width", [(16, 100, 2130), (7, 20, 3), (11, 500, 50), (12, 40, 120), (13, 300, 260)])
+def test_dense_range(gqf, cuda, op, q, lo, width, sync):
+    """Nearly every remainder of neighbouring quotients, in one cluster that no
+    slice of the table holds: at q = 16 more items than a bucket of the rebuild
+    counts in 16 bits, and filters smaller than one bucket."""
+    G, r = gqf, 5
+    cand = O.mt_keys(1130, 1 << (23 if q == 16 else 20))
+    quot = O.aphash(cand, q, r) >> r
+    dense = cand[(quot >= lo) & (quot < lo + width)]
+    if q == 16:
+        assert 66000 < np.unique(O.aphash(dense, q, r)).size < 68160
+    more = O.mt_keys(1131, (1 << q) // 32)
+    c = Contents(q, r, dense, True)
+    f, f2 = G.initFilterGPU(q, r), G.initFilterGPU(q, r)
+    try:
+        G.bulkBuildSegmentedLayouts(f, dense.size, to_dev(cuda, dense), True)
+        d = to_dev(cuda, more)
+        if op == "insert":
+            c.insert(more)
+            G.insert(f, more.size, d, sync=sync)
+        elif op == "delete":
+            gone = np.concatenate([dense[: dense.size // 50], more])
+            c.delete(gone)
+            G.superclusterDeletes(f, gone.size, to_dev(cuda, gone), sync=sync)
+        elif op == "via":
+            c.merge(c.fps(more), True)
+            G.insertViaMerge(f, d, 0, d, more.size, True, sync=sync)
+        else:
+            c.merge(np.unique(c.fps(more)), True)
+            G.bulkBuildSegmentedLayouts(f2, more.size, d, True)
+            G.mergeTwoFilters(f, f2, True, sync=sync)
+        G.stream_status()
+        check(G, f, c.table(), op)
+    finally:
+        G.freeFilterGPU(f)
+        G.freeFilterGPU(f2)
+
+
 @pytest.mark.parametrize("q,na,nb", [(7, 0.4, 0.4), (12, 0.5, 0.3), (16, 0.5, 0.5), (22, 0.5, 0.55), (23, 0.2, 0.2)])
 @pytest.mark.parametrize("dup", [False, True])
 def test_queued_merges(gqf, cuda, q, na, nb, dup):
