@@ -89,6 +89,55 @@ __device__ __forceinline__ void fb_scan(const uint32_t *in, uint32_t *out, uint3
     }
 }
 
+// Leaves of bucket b's batch what changes the table: of deletes as many as
+// there are copies, of inserts the first of each new fingerprint.  For buckets
+// that a batch with a repeated key or of many times the table's size would take
+// past FB_CAP.  (One-byte slots: 18 bits of fingerprint in a bucket.)
+__device__ __forceinline__ void fb_reduce(const LayoutArgs &a, uint32_t b, uint32_t *items, uint32_t *cnt)
+{
+    extern __shared__ __align__(16) uint8_t smem_layout[];
+    uint32_t *s_words = reinterpret_cast<uint32_t *>(smem_layout);
+    __shared__ uint32_t s_kept;
+    constexpr uint32_t FP_BITS = FB_TB + 5, WORDS = 1u << (FP_BITS - 5);
+    const uint32_t tid = threadIdx.x, na = a.A.count(b), n = a.B.count(b);
+    const uint32_t *A = a.A.items + a.A.start(b);
+    uint32_t *B = items + a.B.start(b);
+    const bool del = a.op == OP_DELETE;
+    if (del && na > 2 * WORDS) return;  // (a counter of 16 bits per stored element)
+    for (uint32_t i = tid; i < WORDS; i += FB_THREADS) s_words[i] = 0;
+    if (tid == 0) s_kept = 0;
+    __syncthreads();
+    for (uint32_t i0 = 0; i0 < n; i0 += FB_THREADS) {
+        const uint32_t i = i0 + tid, fp = i < n ? __ldcg(B + i) : 0u;
+        bool keep = false;
+        if (i < n) {
+            uint32_t lo = 0, hi = na;
+            while (lo < hi) {
+                const uint32_t mid = (lo + hi) >> 1;
+                if (A[mid] < fp) lo = mid + 1;
+                else hi = mid;
+            }
+            const bool stored = lo < na && A[lo] == fp;
+            if (del && stored) {
+                const uint32_t sh = 16 * (lo & 1u);
+                uint32_t c = (*reinterpret_cast<volatile uint32_t *>(s_words + (lo >> 1)) >> sh) & 0xFFFFu;
+                if (lo + c < na && A[lo + c] == fp) {
+                    c = (atomicAdd(s_words + (lo >> 1), 1u << sh) >> sh) & 0xFFFFu;
+                    keep = lo + c < na && A[lo + c] == fp;
+                }
+            } else if (!del && !stored) {
+                const uint32_t x = fp & ((1u << FP_BITS) - 1u), bit = 1u << (x & 31u);
+                keep = !(atomicOr(s_words + (x >> 5), bit) & bit);
+            }
+        }
+        __syncthreads();  // the 256 items are read; places at or before them are written
+        if (keep) B[atomicAdd(&s_kept, 1u)] = fp;
+        __syncthreads();
+    }
+    if (tid == 0) cnt[b] = s_kept;
+    __syncthreads();
+}
+
 template <int BPE>
 __global__ void __launch_bounds__(FB_THREADS, 2) k_update_fallback(FallbackArgs f)
 {
@@ -199,7 +248,10 @@ __global__ void __launch_bounds__(FB_THREADS, 2) k_update_fallback(FallbackArgs 
         if (a.op == OP_DELETE) buckets([&](uint32_t b) { bucket_layout_set<FB_THREADS, 32, OwnLessSource>(a, b); });
         else buckets([&](uint32_t b) { bucket_layout_set<FB_THREADS, 32, OwnListSource>(a, b); });
     } else {
-        buckets([&](uint32_t b) { bucket_layout_body<FB_THREADS, 32, BPE>(a, b); });
+        buckets([&](uint32_t b) {
+            if (BPE == 1 && f.n && a.A.count(b) + a.B.count(b) > FB_CAP) fb_reduce(a, b, f.bitems, f.bcnt);
+            bucket_layout_body<FB_THREADS, 32, BPE>(a, b);
+        });
     }
     if (!grid_sync(f.bar, a.err)) return;
     const uint32_t nf = min(__ldcg(a.fix_cnt), a.fix_cap);

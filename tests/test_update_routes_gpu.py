@@ -103,6 +103,28 @@ def test_dense_range(gqf, cuda, op, q, lo, width, sync):
         G.freeFilterGPU(f2)
 
 
+@pytest.mark.parametrize("sync", [True, False])
+@pytest.mark.parametrize("q", [9, 14, 17, 23])
+def test_large_repeating_batches_on_a_table_with_copies(gqf, cuda, q, sync):
+    """Batches of many times the table's buckets, mostly repeats: the rebuild
+    keeps of them what changes the table."""
+    r = 5
+    n = min((1 << q) // 2, 1 << 20)
+    cand = O.mt_keys(1140 + q, 2 * n)
+    keys = np.concatenate([cand[:n], cand[: n // 4], np.repeat(cand[n: n + 3], 40 if q == 9 else 300)])
+    hot = np.concatenate([np.full(90000, cand[n], np.uint32), np.full(70000, cand[n + 5], np.uint32), cand[: n // 8],
+                          cand[-n // 8:], np.tile(cand[n // 3: n // 3 + 50], 200)])
+    f, c = gqf.initFilterGPU(q, r), Contents(q, r, keys, False)
+    assert c.table() is not None
+    try:
+        gqf.bulkBuildSegmentedLayouts(f, keys.size, to_dev(cuda, keys), False)
+        apply(gqf, cuda, f, c, "insert", hot, sync)
+        apply(gqf, cuda, f, c, "delete", hot, sync)
+        apply(gqf, cuda, f, c, "delete", np.concatenate([hot[:100000], cand[: n // 2]]), sync)
+    finally:
+        gqf.freeFilterGPU(f)
+
+
 @pytest.mark.parametrize("q,na,nb", [(7, 0.4, 0.4), (12, 0.5, 0.3), (16, 0.5, 0.5), (22, 0.5, 0.55), (23, 0.2, 0.2)])
 @pytest.mark.parametrize("dup", [False, True])
 def test_queued_merges(gqf, cuda, q, na, nb, dup):
